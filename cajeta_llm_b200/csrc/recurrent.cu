@@ -33,6 +33,8 @@
 #define CJ_LIB "recurrent"
 #include "common.cuh"
 
+#include <type_traits>
+
 using namespace cj;
 
 namespace {
@@ -447,6 +449,340 @@ __global__ void __launch_bounds__(128) scan_kernel(ScanArgs p, int DP, int TOK) 
     }
 }
 
+// The same scans for steps that bring many tokens a request.  scan_kernel's chain a token (shared-memory loads, a row's partial sum,
+// a butterfly, the store, one after the other) takes 600 to 700 ns whatever the state's size.  Here a thread keeps C columns, so that a
+// token's two vectors are loaded once for them; U tokens are walked before their C U read-outs are summed over the DP lanes all at once,
+// by halving (each lane hands half of its values to its partner: DP - 1 shuffles for DP values instead of log2 DP for one), after which
+// every lane holds one finished value; and what needs no state is worked out for WALK_TOK tokens side by side, a lane a token.
+// Every float32 operation on a (column, token) is scan_kernel's, in its order - the partial sums over a lane's rows, the butterfly's
+// tree, the update - so a state or a row has the same bits whichever of the two walked it.  2,048 tokens of one prompt, before and now:
+// state-space, 64 heads of 128 x 64, 1,266 and 356 us; delta rule, 16 of 128 x 128, 1,412 and 565 us; gated linear attention, 4 of
+// 128 x 256, 1,214 and 427 us; matrix memory, 8 of 128 x 256, 1,488 and 369 us.  Two columns a thread: with one 20 to 35 % slower (twice
+// the loads), with four up to 60 % (too few warps).  What bounds it: latencies with one warp a scheduler; in the delta rule the
+// chain from one token's state to the next (four dependent shuffles).
+constexpr int WALK_TOK = 32, WALK_COLS = 2;
+
+// Sums of V values over the DP lanes that share a column; lane `part` is left, in v[0], with the value its bits name, the first
+// exchanged the most significant.  The order of the exchanges is scan_kernel's: neighbouring parts first, but with a whole warp a
+// column the farthest.  (Written as a recursion, so that every index is a constant.)
+template <int DP, int N, int STEP, int V> __device__ __forceinline__ void halve_sum(float (&v)[V], int lane) {
+    constexpr int STEPS = DP == 8 ? 3 : DP == 16 ? 4 : 5;
+    if constexpr (STEP < STEPS) {
+        constexpr int O = DP == 32 ? 16 >> STEP : (32 / DP) << STEP;
+        if constexpr (N > 1) {
+            const bool up = (lane & O) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                const float give = up ? v[i] : v[N / 2 + i], keep = up ? v[N / 2 + i] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+            }
+            halve_sum<DP, N / 2, STEP + 1>(v, lane);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+            halve_sum<DP, 1, STEP + 1>(v, lane);
+        }
+    }
+}
+
+template <int DP, int NPER, int MODE, int C>
+__global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
+    constexpr bool DELTA = MODE == SCAN_DELTA;
+    constexpr int NVEC = MODE == SCAN_GLA ? 3 : 2, ROWS = DP * NPER, CPW = 32 / DP, CB = 4 * CPW * C, U = DP / C, V = U * C;
+    constexpr int OLD_CB = 4 * CPW;                                       // columns of a tile of the state's layout
+    constexpr int TILE_FLOATS = MODE == SCAN_MLSTM ? (2 * NPER + 1) * 128 : NPER * 128;
+    constexpr int TAIL = NVEC * ROWS + CB, STRIDE = TAIL + 4;             // a staged token: [a | b | (decays) | v: CB columns | 4 scalars]
+    constexpr int OWN = (STRIDE + 127) / 128;
+    cj::after_predecessor();
+    cj::release_successor();
+    extern __shared__ __align__(16) float staged[];
+    const int req = blockIdx.x, head = blockIdx.y;
+    const int slot = p.req_slot[req];
+    const int first = p.req_start[req], n = p.req_start[req + 1] - first;
+    if (slot < 0 || n <= 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int part = lane / CPW;
+    const int lcol = warp * CPW * C + lane % CPW;                         // the thread's columns: lcol + CPW k of the block's
+    const int col0 = blockIdx.z * CB;
+    const int group = head / (p.heads / p.groups);
+
+    // the sources of the entries of a staged token that this thread copies (entry tid + 128 k), for the request's first row; null: none
+    const float* src[OWN];
+    int ld[OWN];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+        const int e = tid + 128 * k;
+        src[k] = nullptr;
+        ld[k] = p.ld;
+        const float* x = p.x + (size_t)first * p.ld;
+        const float* raw = p.raw + (size_t)first * p.ld_raw;
+        if (e < NVEC * ROWS) {
+            const int which = e / ROWS, v = e - which * ROWS, d = v / NPER + DP * (v % NPER);      // index part * NPER + i -> row part + DP i
+            if (which == 2) { src[k] = raw + p.off_dt + head * ROWS + d; ld[k] = p.ld_raw; }
+            else src[k] = x + (which == 0 ? p.off_a : p.off_b) + group * ROWS + d;
+        } else if (e < TAIL) {
+            const int c = col0 + e - NVEC * ROWS;
+            if (c < p.cols) src[k] = x + p.off_v + head * p.cols + c;
+        } else if (e == TAIL && MODE != SCAN_GLA) { src[k] = raw + p.off_dt + head; ld[k] = p.ld_raw; }
+        else if (e == TAIL + 1 && (DELTA || MODE == SCAN_MLSTM)) { src[k] = raw + p.off_beta + head; ld[k] = p.ld_raw; }
+    }
+    auto stage = [&](int t0, float* buf) {
+        const int nt = min(WALK_TOK, n - t0);
+#pragma unroll
+        for (int k = 0; k < OWN; ++k) {
+            if (!src[k]) continue;
+            const float* s = src[k] + (size_t)t0 * ld[k];
+            float* d = buf + tid + 128 * k;
+#pragma unroll 4
+            for (int tt = 0; tt < nt; ++tt, s += ld[k], d += STRIDE) cp_async4(d, s);
+        }
+    };
+    // columns past the last read as zero in every staged token
+    for (int i = tid; i < 2 * WALK_TOK * CB; i += 128) {
+        const int t = i / CB, c = i - t * CB;
+        if (col0 + c >= p.cols) staged[t * STRIDE + NVEC * ROWS + c] = 0.0f;
+    }
+    stage(0, staged);
+    cp_async_commit();
+
+    // the state, in scan_kernel's layout: (tile of OLD_CB columns, i, thread of that kernel)
+    const int old_tiles = (p.cols + OLD_CB - 1) / OLD_CB;
+    float* S[C];
+    bool live[C];
+    float s[C][NPER];
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        const int col = col0 + lcol + CPW * k, in = col % OLD_CB;
+        live[k] = col / OLD_CB < old_tiles;                               // (columns that only pad the last tile belong to the layout)
+        S[k] = p.state + (size_t)slot * p.slot_stride + ((size_t)head * old_tiles + col / OLD_CB) * TILE_FLOATS
+               + (in / CPW) * 32 + part * CPW + in % CPW;
+#pragma unroll
+        for (int i = 0; i < NPER; ++i) s[k][i] = live[k] ? S[k][i * 128] : 0.0f;
+    }
+    const float A = MODE == SCAN_GLA ? 0.0f : (MODE == SCAN_MLSTM ? p.A_log[head] : expf(p.A_log[head]));
+    const float bias = MODE == SCAN_GLA ? 0.0f : p.dt_bias[head];
+    const float skip = MODE == SCAN_SSD ? p.skip[head] : 0.0f;
+    float nvec[MODE == SCAN_MLSTM ? NPER : 1];
+    float m_run = 0.0f;
+    if (MODE == SCAN_MLSTM) {
+#pragma unroll
+        for (int i = 0; i < NPER; ++i) nvec[i] = live[0] ? S[0][(NPER + i) * 128] : 0.0f;
+        // every tile and thread of the layout holds the maximum; this block's first tile is its own, whatever a thread's columns
+        m_run = p.state[(size_t)slot * p.slot_stride + ((size_t)head * old_tiles + col0 / OLD_CB) * TILE_FLOATS + 2 * NPER * 128];
+    }
+    // which finished value a lane is left with: token `my_u` of the batch, column `my_k` of the thread's
+    int my = 0;
+#pragma unroll
+    for (int b = 0, w = V >> 1; w > 0; ++b, w >>= 1) my += (lane & (DP == 32 ? 16 >> b : CPW << b)) ? w : 0;
+    const int my_u = my / C, my_k = my % C, my_col = lcol + CPW * my_k;
+    float* out = p.out + (size_t)first * p.heads * p.cols + head * p.cols + col0 + my_col;
+    const size_t out_ld = (size_t)p.heads * p.cols;
+    const bool writer = col0 + my_col < p.cols;
+
+    for (int t0 = 0, which = 0; t0 < n; t0 += WALK_TOK, which ^= 1) {
+        float* cur = staged + which * WALK_TOK * STRIDE;
+        if (t0 + WALK_TOK < n) stage(t0 + WALK_TOK, staged + (which ^ 1) * WALK_TOK * STRIDE);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const int nt = min(WALK_TOK, n - t0);
+        // what needs no state
+        if (DELTA) {
+            // unit vectors: a warp sums a token's squares (eight tokens a warp, their butterflies side by side)
+#pragma unroll 2
+            for (int tt = warp; tt < nt; tt += 4) {
+                float* tk = cur + tt * STRIDE;
+                float qq = 0.0f, kk = 0.0f;
+#pragma unroll
+                for (int d = 0; d < ROWS; d += 32)
+                    if (d + lane < ROWS) {
+                        qq = fmaf(tk[d + lane], tk[d + lane], qq);
+                        kk = fmaf(tk[ROWS + d + lane], tk[ROWS + d + lane], kk);
+                    }
+                qq = warp_sum(qq);
+                kk = warp_sum(kk);
+                const float qs = p.q_scale / sqrtf(qq + 1e-6f), ks = 1.0f / sqrtf(kk + 1e-6f);
+#pragma unroll
+                for (int d = 0; d < ROWS; d += 32)
+                    if (d + lane < ROWS) {
+                        tk[d + lane] *= qs;
+                        tk[ROWS + d + lane] *= ks;
+                    }
+            }
+            if (tid < nt) {
+                float* tk = cur + tid * STRIDE + TAIL;
+                tk[0] = expf(-A * softplus_f(tk[0] + bias));                                   // the decay
+                tk[1] = sigmoid_f(tk[1]);                                                      // beta
+            }
+        } else if (MODE == SCAN_GLA) {
+            for (int e = tid; e < nt * ROWS; e += 128) {
+                float* tk = cur + (e / ROWS) * STRIDE + e % ROWS;
+                tk[0] *= p.q_scale;
+                tk[2 * ROWS] = expf(log_sigmoid_f(tk[2 * ROWS]) * p.c0);
+            }
+        } else if (MODE == SCAN_MLSTM) {
+            float li = 0.0f, lf = 0.0f;
+            if (warp == 0) {
+                // the running maximum, token after token in every lane; a lane keeps its own token's
+                if (lane < nt) {
+                    const float* tk = cur + lane * STRIDE + TAIL;
+                    li = p.c0 * tanhf((tk[0] + bias) / p.c0);                                  // log of the input gate
+                    lf = log_sigmoid_f(p.c0 * tanhf((tk[1] + A) / p.c0));                      // log of the forget gate
+                }
+                float m = m_run, before = m_run, after = m_run;
+                for (int tt = 0; tt < nt; ++tt) {
+                    const float i = __shfl_sync(0xffffffffu, li, tt), f = __shfl_sync(0xffffffffu, lf, tt);
+                    const float mn = fmaxf(f + m, i);
+                    if (lane == tt) { before = m; after = mn; }
+                    m = mn;
+                }
+                if (lane < nt) {
+                    float* tk = cur + lane * STRIDE + TAIL;
+                    tk[0] = expf(lf + before - after);                                         // keep
+                    tk[1] = expf(li - after);                                                  // take
+                    tk[2] = expf(-after);
+                    tk[3] = after;
+                }
+            }
+            __syncthreads();
+            m_run = cur[(nt - 1) * STRIDE + TAIL + 3];
+            for (int e = tid; e < nt * ROWS; e += 128) {
+                float* tk = cur + (e / ROWS) * STRIDE;
+                tk[e % ROWS] *= p.q_scale;
+                tk[ROWS + e % ROWS] *= tk[TAIL + 1];
+            }
+        } else if (tid < nt) {
+            float* tk = cur + tid * STRIDE + TAIL;
+            const float dt = softplus_f(tk[0] + bias);
+            tk[0] = dt;
+            tk[1] = expf(-A * dt);
+        }
+        __syncthreads();
+        auto walk = [&](int b0, int nu, auto whole) {
+            constexpr bool WHOLE = decltype(whole)::value;
+            float y[V], nq[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!WHOLE && u >= nu) {
+#pragma unroll
+                    for (int k = 0; k < C; ++k) y[u * C + k] = 0.0f;
+                    nq[u] = 0.0f;
+                    continue;
+                }
+                const float* tk = cur + (b0 + u) * STRIDE;
+                float a[NPER], b[NPER], xv[C];
+#pragma unroll
+                for (int i = 0; i < NPER; i += 4) {
+                    const float4 va = *(const float4*)(tk + part * NPER + i);
+                    const float4 vb = *(const float4*)(tk + ROWS + part * NPER + i);
+                    a[i] = va.x; a[i + 1] = va.y; a[i + 2] = va.z; a[i + 3] = va.w;
+                    b[i] = vb.x; b[i + 1] = vb.y; b[i + 2] = vb.z; b[i + 3] = vb.w;
+                }
+#pragma unroll
+                for (int k = 0; k < C; ++k) xv[k] = tk[NVEC * ROWS + lcol + CPW * k];
+                if (DELTA) {
+                    const float decay = tk[TAIL], beta = tk[TAIL + 1];
+                    float dot[C];
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        dot[k] = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < NPER; ++i) {
+                            s[k][i] *= decay;
+                            dot[k] = fmaf(s[k][i], b[i], dot[k]);
+                        }
+                    }
+#pragma unroll
+                    for (int st = 0; st < (DP == 8 ? 3 : DP == 16 ? 4 : 5); ++st)
+#pragma unroll
+                        for (int k = 0; k < C; ++k) dot[k] += __shfl_xor_sync(0xffffffffu, dot[k], DP == 32 ? 16 >> st : CPW << st);
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        const float w = beta * (xv[k] - dot[k]);
+                        float sum = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < NPER; ++i) {
+                            s[k][i] = fmaf(b[i], w, s[k][i]);
+                            sum = fmaf(s[k][i], a[i], sum);
+                        }
+                        y[u * C + k] = sum;
+                    }
+                } else if (MODE == SCAN_GLA) {
+#pragma unroll
+                    for (int k = 0; k < C; ++k) y[u * C + k] = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < NPER; i += 4) {
+                        const float4 d4 = *(const float4*)(tk + 2 * ROWS + part * NPER + i);
+                        const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+#pragma unroll
+                            for (int k = 0; k < C; ++k) {
+                                s[k][i + j] = fmaf(d[j], s[k][i + j], __fmul_rn(b[i + j], xv[k]));
+                                y[u * C + k] = fmaf(s[k][i + j], a[i + j], y[u * C + k]);
+                            }
+                    }
+                } else if (MODE == SCAN_MLSTM) {
+                    const float keep = tk[TAIL];
+                    nq[u] = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < NPER; ++i) {
+                        nvec[i] = fmaf(keep, nvec[i], b[i]);
+                        nq[u] = fmaf(nvec[i], a[i], nq[u]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        float sum = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < NPER; ++i) {
+                            s[k][i] = fmaf(keep, s[k][i], __fmul_rn(b[i], xv[k]));
+                            sum = fmaf(s[k][i], a[i], sum);
+                        }
+                        y[u * C + k] = sum;
+                    }
+                } else {
+                    const float dt = tk[TAIL], decay = tk[TAIL + 1];
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        const float dx = dt * xv[k];
+                        float sum = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < NPER; ++i) {
+                            s[k][i] = fmaf(decay, s[k][i], __fmul_rn(a[i], dx));
+                            sum = fmaf(s[k][i], b[i], sum);
+                        }
+                        y[u * C + k] = sum;
+                    }
+                }
+            }
+            halve_sum<DP, V, 0>(y, lane);
+            if (MODE == SCAN_MLSTM) halve_sum<DP, U, 0>(nq, lane);
+            if (writer && (WHOLE || my_u < nu)) {
+                const float* tk = cur + (b0 + my_u) * STRIDE;
+                float v = y[0];
+                if (MODE == SCAN_SSD) v = fmaf(skip, tk[NVEC * ROWS + my_col], v);
+                if (MODE == SCAN_MLSTM) v = v / (fmaxf(fabsf(nq[0]), tk[TAIL + 2]) + p.c1);
+                out[(size_t)(t0 + b0 + my_u) * out_ld] = v;
+            }
+        };
+        int b0 = 0;
+#pragma unroll 1
+        for (; b0 + U <= nt; b0 += U) walk(b0, U, std::true_type{});
+        if (b0 < nt) walk(b0, nt - b0, std::false_type{});
+        __syncthreads();                                                  // everyone has walked this buffer before it is staged into again
+    }
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        if (!live[k]) continue;
+#pragma unroll
+        for (int i = 0; i < NPER; ++i) S[k][i * 128] = s[k][i];
+        if (MODE == SCAN_MLSTM) {
+#pragma unroll
+            for (int i = 0; i < NPER; ++i) S[k][(NPER + i) * 128] = nvec[i];
+            S[k][2 * NPER * 128] = m_run;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // y * silu(z) and an RMS over equal parts of the row, in either order:
 //   gate_first:  v = y * silu(z);  out = v / rms_part(v) * w
@@ -785,10 +1121,48 @@ CJ_EXPORT int cj_short_conv_commit(const float* in, int ld_in, int C, int taps, 
 //         forget gate's; c0 = the gates' cap, c1 = the floor added to the read-out's divisor).
 static long long scan_tile_floats(int mode, int nper) { return mode == 3 ? (long long)(2 * nper + 1) * 128 : (long long)nper * 128; }
 
+// Tokens a request, on average over the step, from which on walk_kernel takes over: at 4 tokens for each of 8 requests it takes 12.5 us
+// against scan_kernel's 18 (state-space, 64 heads of 128 x 64) and 13.5 against 18 (delta rule, 16 of 128 x 128); with one token a
+// request most of a batch would be empty.
+constexpr int WALK_MIN_ROWS = 4;
+
+template <int DP, int NPER, int MODE, int C>
+static int launch_walk_as(const ScanArgs& p, int requests, cudaStream_t stream) {
+    constexpr int CB = 4 * (32 / DP) * C;
+    constexpr int bytes = 2 * WALK_TOK * ((MODE == SCAN_GLA ? 3 : 2) * DP * NPER + CB + 4) * (int)sizeof(float);
+    static bool sized = false;
+    if (!sized) {
+        cudaError_t e = cudaFuncSetAttribute(walk_kernel<DP, NPER, MODE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+        sized = true;
+    }
+    const dim3 grid(requests, p.heads, (p.cols + CB - 1) / CB);
+    if (grid.z > 65535) return CJ_ERR_SIZE;
+    cj::launch(walk_kernel<DP, NPER, MODE, C>, grid, dim3(128), bytes, stream, p);
+    return launch_status();
+}
+
+// CJ_ERR_SIZE: not built for this share of the rows
+static int launch_walk(int mode, int DP, int nper, const ScanArgs& p, int requests, cudaStream_t stream) {
+#define WALK(D, N)                                                                                                      \
+    if (DP == D && nper == N) {                                                                                         \
+        switch (mode) {                                                                                                 \
+            case SCAN_SSD: return launch_walk_as<D, N, SCAN_SSD, WALK_COLS>(p, requests, stream);                       \
+            case SCAN_DELTA: return launch_walk_as<D, N, SCAN_DELTA, WALK_COLS>(p, requests, stream);                   \
+            case SCAN_GLA: return launch_walk_as<D, N, SCAN_GLA, WALK_COLS>(p, requests, stream);                       \
+            default: return launch_walk_as<D, N, SCAN_MLSTM, WALK_COLS>(p, requests, stream);                           \
+        }                                                                                                               \
+    }
+    // 64 or 128 rows a state
+    WALK(8, 8) WALK(8, 16) WALK(16, 4) WALK(16, 8) WALK(32, 4)
+#undef WALK
+    return CJ_ERR_SIZE;
+}
+
 CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off_b, int off_v, const float* raw, int ld_raw,
                             int off_dt, int off_beta, const float* A_log, const float* dt_bias, const float* skip, float* state,
                             long long slot_stride, long long state_floats, const int* req_start, const int* req_slot, float* out,
-                            int requests, int heads, int groups, int rows, int cols, float q_scale, float c0, float c1,
+                            int requests, int total_rows, int heads, int groups, int rows, int cols, float q_scale, float c0, float c1,
                             cudaStream_t stream) {
     if (requests <= 0) return 0;
     if (mode < 0 || mode > 3) return CJ_ERR_ARG;
@@ -806,6 +1180,12 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
                req_start, req_slot, out, heads, groups, rows, cols, q_scale, c0, c1};
     const int cols_per_block = 4 * (32 / DP);
     dim3 grid(requests, heads, (cols + cols_per_block - 1) / cols_per_block);
+    if (total_rows >= WALK_MIN_ROWS * requests && rows == DP * nper && grid.y <= 65535
+        && state_floats >= (long long)heads * grid.z * scan_tile_floats(mode, nper)) {
+        // many tokens a request: the same results from the kernel that walks several columns and tokens at a time, where it is built
+        const int st = launch_walk(mode, DP, nper, p, requests, stream);
+        if (st != CJ_ERR_SIZE) return st;
+    }
     if (grid.y > 65535 || grid.z > 65535) return CJ_ERR_SIZE;
     if (state_floats < (long long)heads * grid.z * scan_tile_floats(mode, nper)) return CJ_ERR_SIZE;
     // tokens staged at a time: up to 16, as many as 96 KB of shared memory hold twice
