@@ -1,0 +1,365 @@
+// Paged attention of the float32 path: float32 queries, cache and arithmetic, head sizes up to 128 that are multiples of four.
+// The formulas are attention_paged.cu's (window, capped scores, a gate per row and head, a constant sink score).
+//
+// Two kernels, one result.  A portion of a prompt goes 64 rows of a request and one head a block, so that a key read from the cache
+// serves 64 rows; a request with few rows (a decoded token) goes a row and head a block, its warps sharing the keys.  A row
+// must not depend on which of the two ran or on how its prompt was cut, so both do the same float32 operations for it, in this order:
+//   keys in chunks of 64 that begin at multiples of 64;  s_t = (q . k_t) scale, one chain of fused multiply-adds over the head;
+//   in a chunk m_c = max s_t, e_t = exp(s_t - m_c), l_c = sum e_t by a fixed tree, o_c = sum e_t v_t one chain over its keys;
+//   chunks joined in order:  m' = max(m, m_c), l = l exp(m - m') + l_c exp(m_c - m'), o likewise.
+// Keys outside a row's [from, p] enter none of its sums (they are skipped, not multiplied by zero).
+//
+// The prompt form keeps a thread on 4 rows x 4 keys of the scores and 4 rows x 8 entries of the output, operands as float4 from
+// shared memory (12 shared-memory wavefronts a 16 FMA clocks): bound by the FMA pipe and by waiting for a chunk's keys, which nothing
+// fetches ahead but the SM's other block.  1,777 rows of one prompt, 16 heads of 128: 961 us, where a row and head a block with a
+// key a lane took 12,700 us.  One row at 570 keys: 34 us, 120 us before.
+#define CJ_LIB "attention_f32"
+#include "common.cuh"
+
+using namespace cj;
+
+namespace {
+
+constexpr int KEYS = 64, ROWS = 64, MAX_DIM = 128;
+constexpr int TILE_THREADS = 256, ROW_WARPS = 8;
+
+struct Args {
+    const float* q; float* out; const float* kplane; const float* vplane;
+    const int* positions; const int* row_req; const int* req_start; int requests;
+    const int* table; int table_stride, page_tokens;
+    int n_heads, n_kv, hd, vd, window;
+    float scale, softcap;
+    const float* head_gate; int gate_ld;
+    float sink;
+    int few_rows;                  // requests with at most this many rows go row by row
+};
+
+__device__ __forceinline__ float score(float dot, const Args& p) {
+    // (products rounded by themselves: contracted into the subtraction that follows, the two kernels could differ)
+    float s = __fmul_rn(dot, p.scale);
+    if (p.softcap > 0.0f) s = __fmul_rn(p.softcap, tanhf(s / p.softcap));
+    return s;
+}
+__device__ __forceinline__ int first_key(int pos, int window) { return window > 0 && pos + 1 > window ? pos + 1 - window : 0; }
+__device__ __forceinline__ float chain4(float4 a, float4 b, float s) {
+    s = fmaf(a.x, b.x, s);
+    s = fmaf(a.y, b.y, s);
+    s = fmaf(a.z, b.z, s);
+    return fmaf(a.w, b.w, s);
+}
+__device__ __forceinline__ float gate_of(const Args& p, int row, int head) {
+    return p.head_gate ? 1.0f / (1.0f + expf(-p.head_gate[(size_t)row * p.gate_ld + head])) : 1.0f;
+}
+
+// VC: float4 of the output a thread holds per row (values of up to 64 VC entries)
+template <int VC>
+__global__ void __launch_bounds__(TILE_THREADS, 2) attention_f32_tile_kernel(const Args p) {
+    cj::after_predecessor();
+    cj::release_successor();
+    extern __shared__ __align__(16) float smem[];
+    const int ks = p.hd + 4;                        // row stride of queries and keys: 16 rows apart never share a bank
+    float* Qs = smem;                               // [ROWS][ks]
+    float* Ks = Qs + ROWS * ks;                     // [KEYS][ks]
+    float* Vs = Ks + KEYS * ks;                     // [KEYS][vd]
+    float* Ps = Vs + KEYS * p.vd;                   // [ROWS][KEYS + 4]
+    __shared__ int place[3];                        // request, first row of the tile, rows
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int head = blockIdx.y, kvh = head / (p.n_heads / p.n_kv);
+    if (tid < 32) {
+        // which rows: tile gridDim.x - 1 - blockIdx.x (a prompt's last rows, with the most keys, first) over all requests
+        const int tile = gridDim.x - 1 - blockIdx.x;
+        int before = 0, req = -1, row = 0, rows = 0;
+        for (int r0 = 0; r0 < p.requests; r0 += 32) {
+            const int r = r0 + lane;
+            const int a = r < p.requests ? p.req_start[r] : 0, c = r < p.requests ? p.req_start[r + 1] - a : 0;
+            const int n = c > p.few_rows ? (c + ROWS - 1) / ROWS : 0;
+            int inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            const int t = tile - (before + inc - n);
+            const unsigned who = __ballot_sync(0xffffffffu, t >= 0 && t < n);
+            if (who) {
+                const int l = __ffs(who) - 1;
+                req = r0 + l;
+                row = __shfl_sync(0xffffffffu, t, l) * ROWS;
+                rows = min(ROWS, __shfl_sync(0xffffffffu, c, l) - row);
+                row += __shfl_sync(0xffffffffu, a, l);
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) { place[0] = req; place[1] = row; place[2] = rows; }
+    }
+    __syncthreads();
+    const int row0 = place[1], rows = place[2];
+    if (place[0] < 0) return;
+    const int* tab = p.table + (size_t)place[0] * p.table_stride;
+    const int pos0 = p.positions[row0];             // the tile's rows are neighbours
+    const int hd4 = p.hd / 4, vd4 = p.vd / 4;
+    for (int i = tid; i < ROWS * hd4; i += TILE_THREADS) {
+        const int r = i / hd4, d = i - r * hd4;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < rows) v = *(const float4*)(p.q + ((size_t)(row0 + r) * p.n_heads + head) * p.hd + 4 * d);
+        *(float4*)(Qs + r * ks + 4 * d) = v;
+    }
+    const int tx = tid & 15, ty = tid >> 4;
+    const int first = first_key(pos0, p.window), last = pos0 + rows - 1;
+    float m[4], l[4], acc[4][VC][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = p.sink;
+        l[i] = p.sink == -INFINITY ? 0.0f : 1.0f;
+#pragma unroll
+        for (int c = 0; c < VC; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][c][e] = 0.0f;
+    }
+    for (int k0 = first & ~(KEYS - 1); k0 <= last; k0 += KEYS) {
+        __syncthreads();                            // the chunk before has been read
+        for (int i = tid; i < KEYS * 4; i += TILE_THREADS) {
+            const int j = i >> 2, key = k0 + j;     // four threads a key
+            const bool held = key >= first && key <= last;
+            size_t base = 0;
+            if (held) base = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
+            const float4* kr = (const float4*)(p.kplane + base * p.hd);
+            const float4* vr = (const float4*)(p.vplane + base * p.vd);
+            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+            for (int d = i & 3; d < hd4; d += 4) *(float4*)(Ks + j * ks + 4 * d) = held ? kr[d] : zero;
+#pragma unroll 4
+            for (int d = i & 3; d < vd4; d += 4) *(float4*)(Vs + j * p.vd + 4 * d) = held ? vr[d] : zero;
+        }
+        __syncthreads();
+        // scores: rows 4 ty + i, keys tx + 16 j
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 2
+        for (int d = 0; d < p.hd; d += 4) {
+            float4 a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *(const float4*)(Qs + (4 * ty + i) * ks + d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *(const float4*)(Ks + (tx + 16 * j) * ks + d);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = chain4(a[i], b[j], s[i][j]);
+        }
+        float keep[4], take[4];                     // factors of the sums so far and of this chunk's
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int pos = pos0 + 4 * ty + i, from = first_key(pos, p.window);
+            float mc = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = k0 + tx + 16 * j;
+                s[i][j] = key >= from && key <= pos ? score(s[i][j], p) : -INFINITY;
+                mc = fmaxf(mc, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mc = fmaxf(mc, __shfl_xor_sync(0xffffffffu, mc, o));
+            float e[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = k0 + tx + 16 * j;
+                e[j] = key >= from && key <= pos ? expf(s[i][j] - mc) : 0.0f;
+                Ps[(4 * ty + i) * (KEYS + 4) + tx + 16 * j] = e[j];
+            }
+            float lc = __fadd_rn(__fadd_rn(e[0], e[2]), __fadd_rn(e[1], e[3]));
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, o));
+            const bool any = from < k0 + KEYS && pos >= k0;          // the row sees a key of this chunk
+            const float mn = any ? fmaxf(m[i], mc) : m[i];
+            keep[i] = any ? expf(m[i] - mn) : 1.0f;
+            take[i] = any ? expf(mc - mn) : 0.0f;
+            if (any) {
+                l[i] = fmaf(lc, take[i], __fmul_rn(l[i], keep[i]));
+                m[i] = mn;
+            }
+        }
+        __syncwarp();                               // a row's weights were written by this warp's own lanes
+        float o[4][VC][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < VC; ++c)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[i][c][e] = 0.0f;
+        // whether every row of the tile sees every key of the chunk
+        const bool all = k0 + KEYS - 1 <= pos0 && k0 >= first_key(last, p.window);
+#pragma unroll 1
+        for (int k = 0; k < KEYS; k += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(Ps + (4 * ty + i) * (KEYS + 4) + k);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                float4 v[VC];
+#pragma unroll
+                for (int c = 0; c < VC; ++c) {
+                    const int d = 4 * tx + 64 * c;
+                    v[c] = d < p.vd ? *(const float4*)(Vs + (k + kk) * p.vd + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                    const int key = k0 + k + kk, pos = pos0 + 4 * ty + i;
+                    if (all || (key <= pos && key >= first_key(pos, p.window))) {
+#pragma unroll
+                        for (int c = 0; c < VC; ++c) {
+                            o[i][c][0] = fmaf(e, v[c].x, o[i][c][0]);
+                            o[i][c][1] = fmaf(e, v[c].y, o[i][c][1]);
+                            o[i][c][2] = fmaf(e, v[c].z, o[i][c][2]);
+                            o[i][c][3] = fmaf(e, v[c].w, o[i][c][3]);
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int pos = pos0 + 4 * ty + i;
+            if (!(first_key(pos, p.window) < k0 + KEYS && pos >= k0)) continue;
+#pragma unroll
+            for (int c = 0; c < VC; ++c)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][c][e] = fmaf(o[i][c][e], take[i], __fmul_rn(acc[i][c][e], keep[i]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 4 * ty + i;
+        if (r >= rows) continue;
+        const float inv = __fmul_rn(1.0f / l[i], gate_of(p, row0 + r, head));
+        float* o = p.out + ((size_t)(row0 + r) * p.n_heads + head) * p.vd;
+#pragma unroll
+        for (int c = 0; c < VC; ++c) {
+            const int d = 4 * tx + 64 * c;
+            if (d < p.vd)
+                *(float4*)(o + d) = make_float4(__fmul_rn(acc[i][c][0], inv), __fmul_rn(acc[i][c][1], inv), __fmul_rn(acc[i][c][2], inv),
+                                                __fmul_rn(acc[i][c][3], inv));
+        }
+    }
+}
+
+// A row and head a block: a warp a chunk of 64 keys, lane = keys lane and lane + 32 for the scores and four entries of the value for
+// the sums; after every round of chunks thread d joins them, in order, into entry d of the output.
+__global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const Args p) {
+    cj::after_predecessor();
+    cj::release_successor();
+    __shared__ __align__(16) float qs[MAX_DIM];
+    __shared__ __align__(16) float oc[ROW_WARPS][MAX_DIM];
+    __shared__ float mc_s[ROW_WARPS], lc_s[ROW_WARPS];
+    const int row = blockIdx.x, head = blockIdx.y, kvh = head / (p.n_heads / p.n_kv);
+    const int req = p.row_req[row];
+    if (p.req_start && p.req_start[req + 1] - p.req_start[req] > p.few_rows) return;      // the other kernel's
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int pos = p.positions[row], from = first_key(pos, p.window);
+    const int* tab = p.table + (size_t)req * p.table_stride;
+    if (tid < p.hd / 4) *(float4*)(qs + 4 * tid) = *(const float4*)(p.q + ((size_t)row * p.n_heads + head) * p.hd + 4 * tid);
+    __syncthreads();
+    float m = p.sink, l = p.sink == -INFINITY ? 0.0f : 1.0f, acc = 0.0f;
+    for (int k0 = from & ~(KEYS - 1); k0 <= pos; k0 += KEYS * ROW_WARPS) {
+        const int c0 = k0 + warp * KEYS;
+        if (c0 <= pos) {
+            float s[2], e[2];
+            size_t base[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int key = c0 + lane + 32 * j;
+                base[j] = 0;
+                s[j] = 0.0f;
+                if (key >= from && key <= pos)
+                    base[j] = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
+            }
+            const bool seen0 = c0 + lane >= from && c0 + lane <= pos, seen1 = c0 + lane + 32 >= from && c0 + lane + 32 <= pos;
+            const float4* k_a = (const float4*)(p.kplane + base[0] * p.hd);
+            const float4* k_b = (const float4*)(p.kplane + base[1] * p.hd);
+            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+            for (int d = 0; d < p.hd / 4; ++d) {
+                const float4 a = *(const float4*)(qs + 4 * d);
+                s[0] = chain4(a, seen0 ? k_a[d] : zero, s[0]);
+                s[1] = chain4(a, seen1 ? k_b[d] : zero, s[1]);
+            }
+            s[0] = seen0 ? score(s[0], p) : -INFINITY;
+            s[1] = seen1 ? score(s[1], p) : -INFINITY;
+            const float mc = warp_max(fmaxf(s[0], s[1]));
+            e[0] = seen0 ? expf(s[0] - mc) : 0.0f;
+            e[1] = seen1 ? expf(s[1] - mc) : 0.0f;
+            // the tree of the other kernel: keys 32 apart, then 16 apart, then 1, 2, 4, 8
+            float lc = __fadd_rn(e[0], e[1]);
+            lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, 16));
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, o));
+            if (lane == 0) { mc_s[warp] = mc; lc_s[warp] = lc; }
+            const int lo = max(from - c0, 0), hi = min(pos - c0, KEYS - 1);
+            float4 o = zero;
+            const bool mine = 4 * lane < p.vd;
+#pragma unroll 8
+            for (int j = lo; j <= hi; ++j) {
+                const float w = __shfl_sync(0xffffffffu, j < 32 ? e[0] : e[1], j & 31);
+                const size_t b = __shfl_sync(0xffffffffu, (unsigned long long)(j < 32 ? base[0] : base[1]), j & 31);
+                if (mine) {
+                    const float4 v = *(const float4*)(p.vplane + b * p.vd + 4 * lane);
+                    o.x = fmaf(w, v.x, o.x);
+                    o.y = fmaf(w, v.y, o.y);
+                    o.z = fmaf(w, v.z, o.z);
+                    o.w = fmaf(w, v.w, o.w);
+                }
+            }
+            if (mine) *(float4*)(oc[warp] + 4 * lane) = o;
+        }
+        __syncthreads();
+        const int n = min(ROW_WARPS, (pos - k0) / KEYS + 1);
+        for (int c = 0; c < n; ++c) {
+            const float mc = mc_s[c], mn = fmaxf(m, mc), keep = expf(m - mn), take = expf(mc - mn);
+            l = fmaf(lc_s[c], take, __fmul_rn(l, keep));
+            if (tid < p.vd) acc = fmaf(oc[c][tid], take, __fmul_rn(acc, keep));
+            m = mn;
+        }
+        __syncthreads();
+    }
+    if (tid < p.vd)
+        p.out[((size_t)row * p.n_heads + head) * p.vd + tid] = __fmul_rn(acc, __fmul_rn(1.0f / l, gate_of(p, row, head)));
+}
+
+}  // namespace
+
+// Arguments as cj_paged_attention's, float32 throughout; req_start [requests + 1]: the step's rows by request (neighbouring rows of a
+// request at neighbouring positions), or null: every row goes by itself.  tiles: an upper bound of the 64-row tiles of the
+// requests with more than few_rows rows, 0 for none; singles: whether a request has at most few_rows rows.
+CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, const float* vplane, const int* positions, const int* row_req,
+                               const int* req_start, int requests, const int* table, int table_stride, int page_tokens, int T, int n_heads,
+                               int n_kv, int hd, int vd, int window, float scale, float softcap, const float* head_gate, int gate_ld,
+                               float sink, int few_rows, int tiles, int singles, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (!q || !out || !kplane || !vplane || !positions || !row_req || !table || (tiles > 0 && !req_start)) return CJ_ERR_ARG;
+    if (hd <= 0 || hd > MAX_DIM || hd % 4 != 0 || vd <= 0 || vd > MAX_DIM || vd % 4 != 0) return CJ_ERR_SIZE;
+    if (n_heads <= 0 || n_heads > 65535 || n_kv <= 0 || n_heads % n_kv != 0 || page_tokens <= 0) return CJ_ERR_SIZE;
+    if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kplane | (uintptr_t)vplane) & 15) return CJ_ERR_ALIGN;
+    Args a{q, out, kplane, vplane, positions, row_req, req_start, requests, table, table_stride, page_tokens, n_heads, n_kv, hd, vd, window,
+           scale, softcap, head_gate, gate_ld, sink, few_rows};
+    if (tiles > 0) {
+        const int bytes = (int)sizeof(float) * ((ROWS + KEYS) * (hd + 4) + KEYS * vd + ROWS * (KEYS + 4));
+        auto kern = vd <= 64 ? attention_f32_tile_kernel<1> : attention_f32_tile_kernel<2>;
+        static bool sized[2] = {false, false};
+        if (!sized[vd <= 64]) {
+            const int most = (int)sizeof(float) * ((ROWS + KEYS) * (MAX_DIM + 4) + KEYS * MAX_DIM + ROWS * (KEYS + 4));
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+            if (e != cudaSuccess) return (int)e;
+            sized[vd <= 64] = true;
+        }
+        cj::launch(kern, dim3(tiles, n_heads), dim3(TILE_THREADS), bytes, stream, a);
+        if (int st = launch_status()) return st;
+    }
+    if (singles || tiles <= 0) cj::launch(attention_f32_row_kernel, dim3(T, n_heads), dim3(ROW_WARPS * 32), 0, stream, a);
+    return launch_status();
+}

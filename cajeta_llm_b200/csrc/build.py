@@ -34,6 +34,7 @@ LIBRARIES: Dict[str, str] = {
     "rowwise": "rowwise.cu",
     "gemm_simt": "gemm_simt.cu",
     "attention_paged": "attention_paged.cu",
+    "attention_f32": "attention_f32.cu",
     "attention_mixed": "attention_mixed.cu",
     "attention_diff": "attention_diff.cu",
     "moe_route": "moe_route.cu",

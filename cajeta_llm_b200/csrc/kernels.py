@@ -9,7 +9,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
-from typing import Dict, Optional
+from typing import Dict, Optional, Sequence
 
 import torch
 
@@ -379,12 +379,19 @@ def _gate(head_gate: Optional[torch.Tensor], gate_offset: int):
 NO_SINK = float("-inf")      # no key without a value joins the softmax
 
 
+# float32 attention: a request with at most this many rows in the step goes a row a block, one with more 64 rows a block.  Eight
+# rows at 520 keys in each of eight requests took 127 us a row a block; as a tile of 64 they would pay for 56 that are not there.
+F32_FEW_ROWS = 8
+
+
 def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor,
                     positions: torch.Tensor, row_req: torch.Tensor, table: torch.Tensor, page_tokens: int,
                     n_heads: int, n_kv: int, head_dim: int, window: int, scale: float, value_dim: int = 0,
                     softcap: float = 0.0, head_gate: Optional[torch.Tensor] = None, gate_offset: int = 0,
-                    sink: float = NO_SINK) -> None:
-    """Attention of every row over its request's cached keys [from, position].  ``value_dim``: the values'
+                    sink: float = NO_SINK, req_start: Optional[torch.Tensor] = None, h_req_start: Optional[Sequence[int]] = None) -> None:
+    """Attention of every row over its request's cached keys [from, position].  ``req_start`` ([requests + 1] int32, and
+    ``h_req_start``, the same on the host): the rows by request, a request's at neighbouring positions; with them the float32
+    form reads a key once for up to 64 rows (the result is the same without).  ``value_dim``: the values'
     size when it is not the keys'; ``softcap`` > 0: s <- cap tanh(s / cap); ``head_gate`` (float32 [T, ld]):
     head h of row t is multiplied by sigmoid(head_gate[t, gate_offset + h]).  ``sink``: a constant score of one more key that
     has no value (exp(sink) in the softmax's divisor alone, neither scaled nor capped; 0 adds one); NO_SINK: none."""
@@ -394,6 +401,22 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v
     if head_dim > 256:
         raise KernelError(f"paged_attention: head_dim {head_dim} is larger than 256")
     gate_ptr, gate_ld = _gate(head_gate, gate_offset)
+    vd = value_dim or head_dim
+    if (q.dtype == k_plane.dtype == torch.float32 and out.dtype == torch.float32 and head_dim % 4 == 0 and vd % 4 == 0
+            and max(head_dim, vd) <= 128 and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
+        tiles, singles, requests = 0, True, 0
+        if req_start is not None and h_req_start is not None:
+            _need(req_start, "req_start", torch.int32)
+            requests = len(h_req_start) - 1
+            rows = [b - a for a, b in zip(h_req_start, h_req_start[1:])]
+            tiles = sum(-(-n // 64) for n in rows if n > F32_FEW_ROWS)
+            singles = any(0 < n <= F32_FEW_ROWS for n in rows)
+        st = library("attention_f32").cj_attention_f32(
+            _ptr(q), _ptr(out), _ptr(k_plane), _ptr(v_plane), _ptr(positions), _ptr(row_req), _ptr(req_start if requests else None), _i(requests),
+            _ptr(table), _i(table.stride(0)), _i(page_tokens), _i(T), _i(n_heads), _i(n_kv), _i(head_dim), _i(vd), _i(window), _f(scale),
+            _f(softcap), gate_ptr, _i(gate_ld), _f(sink), _i(F32_FEW_ROWS), _i(tiles), _i(1 if singles else 0), _stream())
+        _check(st, "paged_attention")
+        return
     st = library("attention_paged").cj_paged_attention(
         _ptr(q), _ptr(out), _i(_code(q)), _ptr(k_plane), _ptr(v_plane), _i(_code(k_plane)), _ptr(positions),
         _ptr(row_req), _ptr(table), _i(table.stride(0)), _i(page_tokens), _i(T), _i(n_heads), _i(n_kv), _i(head_dim),

@@ -263,7 +263,8 @@ class PagedAttention(Part):
                                 entry.page_tokens, self.heads, self.kv_heads, self.head_dim, self.window, self.scale)
         else:
             K.paged_attention(q, out, entry.k_plane, entry.v_plane, ctx.positions, ctx.row_req, entry.block_table,
-                              entry.page_tokens, self.heads, self.kv_heads, self.head_dim, self.window, self.scale)
+                              entry.page_tokens, self.heads, self.kv_heads, self.head_dim, self.window, self.scale,
+                              req_start=getattr(ctx, "req_start", None), h_req_start=getattr(ctx, "h_req_start", None))
         K.tag = "o"
         parts = project_split(rt, out.view(T, self.q_dim), self.w_o, bias=self.b_o, out_scale=self.out_scale) if self.allow_pending else None
         if parts is None:
@@ -319,7 +320,8 @@ class PagedAttention(Part):
         else:
             K.paged_attention(q, out, entry.k_plane, entry.v_plane, ctx.positions, ctx.row_req, entry.block_table, entry.page_tokens,
                               self.heads, self.kv_heads, self.head_dim, self.window, self.scale, value_dim=self.value_dim,
-                              softcap=self.softcap, head_gate=gate, gate_offset=g_off, sink=self.sink_score)
+                              softcap=self.softcap, head_gate=gate, gate_offset=g_off, sink=self.sink_score,
+                              req_start=getattr(ctx, "req_start", None), h_req_start=getattr(ctx, "h_req_start", None))
         K.tag = "o"
         parts = project_split(rt, out.view(T, self.o_dim), self.w_o, out_scale=self.out_scale) if self.allow_pending else None
         if parts is None:

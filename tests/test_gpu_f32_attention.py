@@ -1,0 +1,70 @@
+"""float32 attention: rows in tiles of 64 and rows one by one give the same bits, and both hold to 64 bits."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("rows,prior,H,G,hd,vd,window,cap,gated,sink,page", [
+    ([9], [0], 4, 4, 128, 128, 0, 0.0, False, None, 16),                      # the fewest rows a tile takes
+    ([64, 63, 1], [0, 64, 63], 4, 4, 128, 128, 64, 0.0, True, 1.5, 16),       # a whole tile, one short, a row by itself; window = a chunk
+    ([130, 9, 8, 70], [0, 5, 200, 33], 6, 2, 64, 64, 0, 0.0, False, None, 16),
+    ([130, 9, 70, 3], [50, 5, 33, 100], 6, 2, 128, 64, 40, 30.0, True, None, 16),
+    ([65, 200], [7, 90], 4, 1, 24, 100, 33, 0.0, False, 0.0, 4),
+    ([12], [600], 2, 1, 4, 128, 0, 0.0, False, None, 16)])
+def test_tiles_and_rows_agree(rows, prior, H, G, hd, vd, window, cap, gated, sink, page):
+    from cajeta_llm_b200.csrc import kernels as K
+    g = torch.Generator().manual_seed(7)
+    total = [a + b for a, b in zip(rows, prior)]
+    width = max(-(-t // page) for t in total)
+    pages = sum(-(-t // page) for t in total) + 1
+    perm, at = torch.randperm(pages - 1, generator=g) + 1, 0
+    table = torch.full((len(rows), width), -1, dtype=torch.int32)
+    for r, t in enumerate(total):
+        n = -(-t // page)
+        table[r, :n] = perm[at:at + n].int()
+        at += n
+    kp, vp = (torch.randn(pages, G, page, d, generator=g).to(DEV) for d in (hd, vd))
+    T = sum(rows)
+    q = torch.randn(T, H, hd, generator=g).to(DEV)
+    gate = torch.randn(T, H + 3, generator=g).to(DEV) if gated else None
+    starts = [sum(rows[:i]) for i in range(len(rows) + 1)]
+    pos = torch.cat([torch.arange(p, p + n) for n, p in zip(rows, prior)]).int().to(DEV)
+    req = torch.cat([torch.full((n,), i) for i, n in enumerate(rows)]).int().to(DEV)
+    table, start = table.to(DEV), torch.tensor(starts, dtype=torch.int32, device=DEV)
+    scale = hd ** -0.5
+    kw = dict(value_dim=vd, softcap=cap, head_gate=gate, gate_offset=3 if gated else 0, sink=K.NO_SINK if sink is None else sink)
+    tiled, single = torch.empty(T, H, vd, device=DEV), torch.empty(T, H, vd, device=DEV)
+    K.paged_attention(q, tiled, kp, vp, pos, req, table, page, H, G, hd, window, scale, req_start=start, h_req_start=starts, **kw)
+    K.paged_attention(q, single, kp, vp, pos, req, table, page, H, G, hd, window, scale, **kw)
+    assert torch.equal(tiled, single)
+    for r, (n, p0) in enumerate(zip(rows, prior)):
+        held = table[r].long()[:-(-total[r] // page)]
+        k, v = (t[held].permute(1, 0, 2, 3).reshape(G, -1, t.shape[-1])[:, :total[r]].double() for t in (kp, vp))
+        i, j = torch.arange(p0, p0 + n, device=DEV)[:, None], torch.arange(total[r], device=DEV)[None]
+        seen = (j <= i) & ((j > i - window) if window else torch.ones_like(j, dtype=torch.bool))
+        for h in range(H):
+            s = q[starts[r]:starts[r + 1], h].double() @ k[h * G // H].t() * scale
+            s = (cap * torch.tanh(s / cap) if cap else s).masked_fill(~seen, -math.inf)
+            if sink is not None:
+                s = torch.cat([s, torch.full((n, 1), sink, dtype=torch.float64, device=DEV)], 1)
+            o = torch.softmax(s, 1)[:, :total[r]] @ v[h * G // H]
+            if gated:
+                o = o * torch.sigmoid(gate[starts[r]:starts[r + 1], 3 + h].double())[:, None]
+            assert torch.allclose(single[starts[r]:starts[r + 1], h].double(), o, atol=2e-5, rtol=1e-4)
+
+
+def test_a_later_rows_infinite_value_stays_with_the_rows_that_see_it():
+    from cajeta_llm_b200.csrc import kernels as K
+    T, H, hd = 40, 2, 64
+    g = torch.Generator().manual_seed(8)
+    kp, vp = (torch.randn(4, H, 16, hd, generator=g).to(DEV) for _ in range(2))
+    vp[1, :, 15] = float("inf")                                               # position 31
+    q, out = torch.randn(T, H, hd, generator=g).to(DEV), torch.empty(T, H, hd, device=DEV)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    K.paged_attention(q, out, kp, vp, pos, torch.zeros_like(pos), torch.arange(4, dtype=torch.int32, device=DEV)[None], 16, H, H, hd, 0, 0.125,
+                      req_start=torch.tensor([0, T], dtype=torch.int32, device=DEV), h_req_start=[0, T])
+    assert bool(torch.isfinite(out[:31]).all()) and not bool(torch.isfinite(out[31:]).any())
