@@ -33,6 +33,7 @@ NVCC_FLAGS = [
 LIBRARIES: Dict[str, str] = {
     "rowwise": "rowwise.cu",
     "gemm_simt": "gemm_simt.cu",
+    "gemm_f32_tc": "gemm_f32_tc.cu",
     "attention_paged": "attention_paged.cu",
     "attention_f32": "attention_f32.cu",
     "attention_mixed": "attention_mixed.cu",

@@ -1,0 +1,443 @@
+// Matrix products of float32 operands on the tensor cores, to float32's accuracy:
+//
+//     C[token, feature] (+)= scale (sum_k X[token, k] * W[feature, k] (+ bias))
+//
+// A float32 number is the sum of three bfloat16 numbers, 8 bits of its significand each (hi, mid, lo: the leading bits cut
+// off one after the other, so nothing is lost), and a product of two bfloat16 numbers is exact in float32.  Of the nine products
+// of the parts the six largest are summed; the three left out are together below 2^-24 of the product.  What decides the
+// accuracy is the sum, and tensor memory's adds truncate.  So a tensor-memory accumulator only ever holds
+// 32 products a term (one block of K) of three terms, the small terms first, and the blocks are added up in registers with
+// ordinary rounded float32 additions, in the order of K.  Measured against 64 bits, relative error of the result for normal operands:
+// K 2,048 1.8e-7, where the FMA pipe's chain of K fused multiply-adds gives 8.1e-7; K 5,632 2.6e-7 and 1.3e-6; 5,632 products of
+// one sign 2.2e-7 and 1.1e-6; K 132 1.2e-7 and 2.1e-7.
+//
+// A result's operations depend on its own row of X, its row of W and K alone: not on the other rows of the launch, the tile
+// sizes or the tile's place.  So a token's row has the same bits in a prompt's step and in a step of its own.
+//
+// A number that is infinite, or not a number, has no such parts.  The splitting threads notice one (its last remainder is no
+// number) and the tile's results are then summed on the FMA pipe instead, one chain over K as gemm_simt.cu has it.
+//
+// One block a tile of `feat_tile` (up to 128) features x N tokens; the weights are the rows of the product.  One thread sends for
+// the float32 tiles (TMA) into a ring as deep as shared memory allows; groups of eight warps split them into the six bfloat16
+// tiles of a stage, a group every G-th block of K; one warp issues the products; the last warps add the accumulators up
+// and store.  A block of K is a chain of short waits for a group (tile landed, stage free, stores visible to the products: some
+// 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
+// tokens that chain, with many the shared memory, which every operand crosses as float32 once and as bfloat16 parts once for each of
+// its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 35;
+// 250 x 6,144 x 2,048 328 and 117; 1,777 x 6,144 x 2,048 1,822 and 420; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
+// of 4 picks 802 / 1,915 / 6,045 and 181 / 575 / 1,607.  (With the float32 operands loaded into registers instead of by TMA
+// 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
+// Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
+#define CJ_LIB "gemm_f32_tc"
+#include "common.cuh"
+#include "tc_common.cuh"
+
+using namespace tc;
+
+namespace {
+
+constexpr int BK = 32;                    // K of a stage: 128 bytes of float32 (TMA's swizzle row), 64 bytes of bfloat16
+// groups of eight splitting warps, each with stages of bfloat16 parts of its own, and warps that add up: as many as registers
+// and shared memory hold
+constexpr int GROUP_WARPS = 8;
+constexpr int split_groups(int n) { return n <= 32 ? 3 : n <= 64 ? 2 : 1; }
+constexpr int split_stages(int n) { return n <= 32 ? 3 : 2; }
+constexpr int epi_warps(int n) { return n >= 64 ? 8 : 4; }
+// warps: the splitting groups, product issue, loads (and, so that the warps that add up begin at a multiple of four, idle ones), adding up
+constexpr int first_epi(int n) { return (GROUP_WARPS * split_groups(n) + 2 + 3) / 4 * 4; }
+constexpr int threads(int n) { return 32 * (first_epi(n) + epi_warps(n)); }
+
+struct Args {
+    const float* X; long long ldx;
+    const float* W; const float* W2;       // W2: the gated form's second weight
+    const float* bias; const float* bias2;
+    float* C; long long ldc;
+    int tokens, features, K;
+    int accumulate;
+    const int* group_offsets;
+    int groups;
+    float act_limit, act_alpha, act_cubic;
+    int act, act_feats;
+    float out_scale;
+    int feat_tile;                         // features of a tile: at most 128, of the gated form at most 64
+};
+
+template <int N> struct Smem {
+    static constexpr int W_PART = 128 * 64, X_PART = N * 64;           // one bfloat16 tile
+    static constexpr int STAGE = 3 * (W_PART + X_PART);
+    static constexpr int W_RAW = 128 * 128, X_RAW = N * 128;           // one float32 tile
+    static constexpr int RAW = W_RAW + X_RAW;
+    static constexpr int STAGES = split_stages(N);
+    // a multiple of the groups, so that a slot is always read by the same group: a wait by phase parity must not be two phases off
+    static constexpr int RING = (225 * 1024 - STAGES * STAGE) / RAW / STAGES * STAGES;
+    static constexpr int TOTAL = STAGES * STAGE + RING * RAW + 1024 /* alignment */;
+    static_assert(STAGES % split_groups(N) == 0, "a stage belongs to one group");
+};
+
+// eight float32 -> their three bfloat16 parts, packed; `odd` becomes no number when one of the eight is infinite or none
+__device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& hi, uint4& mid, uint4& lo, float& odd) {
+    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t a = __float_as_uint(f[2 * i]), b = __float_as_uint(f[2 * i + 1]);
+        h[i] = __byte_perm(a, b, 0x7632);
+        const float ra = f[2 * i] - __uint_as_float(a & 0xffff0000u), rb = f[2 * i + 1] - __uint_as_float(b & 0xffff0000u);
+        const uint32_t am = __float_as_uint(ra), bm = __float_as_uint(rb);
+        m[i] = __byte_perm(am, bm, 0x7632);
+        const float la = ra - __uint_as_float(am & 0xffff0000u), lb = rb - __uint_as_float(bm & 0xffff0000u);
+        l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+        odd = fmaf(la, 0.0f, odd);
+        odd = fmaf(lb, 0.0f, odd);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    mid = make_uint4(m[0], m[1], m[2], m[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// operand descriptor of a K-major bfloat16 tile of 64-byte rows, 64-byte swizzle (mode 4): 8-row groups 512 bytes apart; the other
+// fields as in umma_desc_sw128
+__device__ __forceinline__ uint64_t umma_desc_sw64(const void* smem_tile) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_u32(smem_tile) & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
+__device__ __noinline__ float chain(const float* x, const float* w, int K) {
+    float s = 0.0f;
+    for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
+    return s;
+}
+
+template <int N, bool DUAL>
+__global__ void __launch_bounds__(threads(N), 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                   const __grid_constant__ CUtensorMap map_w2, const Args p) {
+    using S = Smem<N>;
+    constexpr int G = split_groups(N), STAGES = S::STAGES, EPI_WARPS = epi_warps(N), RING = S::RING, ISSUE = GROUP_WARPS * G,
+                  LOAD = ISSUE + 1, FIRST_EPI = first_epi(N);
+    constexpr int XP = (N + 63) / 64;                         // rows of X a splitting thread takes (64 rows a pass)
+    constexpr int COLS = N * 4 / EPI_WARPS;                   // columns of an adding thread
+    constexpr uint32_t TMEM_COLS = 4 * N <= 64 ? 64 : 4 * N <= 128 ? 128 : 4 * N <= 256 ? 256 : 512;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* raw = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* stages = raw + RING * S::RAW;
+    __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int odd_flag;
+    __shared__ int place[3];                                  // group, first row, one past the last; group -1: no work
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < RING; ++s) {
+            mbar_init(&raw_full[s], 1);
+            mbar_init(&raw_empty[s], GROUP_WARPS);
+        }
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], GROUP_WARPS);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], EPI_WARPS);
+        }
+        odd_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == ISSUE) tmem_alloc(&tmem_slot, TMEM_COLS);
+    const bool grouped = p.group_offsets != nullptr;
+    if (grouped) cj::after_predecessor();
+    if (warp == 0) {
+        // which rows: token tile blockIdx.y of the whole launch, or of the group that holds it
+        if (grouped) {
+            int before = 0, found = -1, lo = 0, hi = 0;
+            for (int g0 = 0; g0 < p.groups; g0 += 32) {
+                const int g = g0 + lane;
+                const int a = g < p.groups ? p.group_offsets[g] : 0, b = g < p.groups ? p.group_offsets[g + 1] : 0;
+                const int n = g < p.groups ? (b - a + N - 1) / N : 0;
+                int inc = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                const int t = (int)blockIdx.y - (before + inc - n);
+                const unsigned who = __ballot_sync(0xffffffffu, t >= 0 && t < n);
+                if (who) {
+                    const int l = __ffs(who) - 1;
+                    found = g0 + l;
+                    lo = __shfl_sync(0xffffffffu, a, l) + __shfl_sync(0xffffffffu, t, l) * N;
+                    hi = min(__shfl_sync(0xffffffffu, b, l), lo + N);
+                    break;
+                }
+                before += __shfl_sync(0xffffffffu, inc, 31);
+            }
+            if (lane == 0) { place[0] = found; place[1] = lo; place[2] = hi; }
+        } else if (lane == 0) {
+            place[0] = 0;
+            place[1] = blockIdx.y * N;
+            place[2] = min(p.tokens, place[1] + N);
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    cj::release_successor();                                  // tensor memory is held
+    const int group = place[0], tok0 = place[1], n_tok = place[2] - place[1];
+    const uint32_t tmem = tmem_slot;
+    const int feat0 = blockIdx.x * p.feat_tile;
+    const int n_kb = (p.K + BK - 1) / BK;
+    const bool work = group >= 0 && n_tok > 0;
+    const int n16 = (n_tok + 15) & ~15;                       // the product's width; the parts of X lie n16 rows apart, side by side
+
+    if (work && warp == LOAD) {
+        // ---- float32 tiles: the weights' first ones leave before the kernel before this one has ended (no kernel writes weights) ----
+        if (elect_one()) {
+            const int w_row = group * p.features + feat0;
+            const uint32_t bytes = S::X_RAW + (DUAL ? 2u : 1u) * p.feat_tile * 128;
+            auto weights = [&](int kb, int s) {
+                uint8_t* at = raw + s * S::RAW;
+                tma_load_2d(at, &map_w, &raw_full[s], kb * BK, w_row);
+                if (DUAL) tma_load_2d(at + 64 * 128, &map_w2, &raw_full[s], kb * BK, w_row);
+            };
+            const int early = grouped ? 0 : min(RING, n_kb);
+            for (int kb = 0; kb < early; ++kb) {
+                mbar_expect_tx(&raw_full[kb], bytes);
+                weights(kb, kb);
+            }
+            if (!grouped) cj::after_predecessor();
+            bool ok = true;
+            for (int kb = 0; kb < n_kb && ok; ++kb) {
+                const int s = kb % RING;
+                if (kb >= early) {
+                    ok = mbar_wait(&raw_empty[s], ((kb / RING) & 1) ^ 1, 15);
+                    if (!ok) break;
+                    mbar_expect_tx(&raw_full[s], bytes);
+                    weights(kb, s);
+                }
+                tma_load_2d(raw + s * S::RAW + S::W_RAW, &map_x, &raw_full[s], kb * BK, tok0);
+            }
+        }
+    } else if (work && warp < ISSUE) {
+        // ---- splitting: thread = (row of 64, eight of the row's 32 float32) ------------------------
+        const int g = warp / GROUP_WARPS, piece = tid & 3, row0 = (tid & (32 * GROUP_WARPS - 1)) >> 2;
+        bool w_live[2], x_live[XP];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) w_live[i] = (DUAL ? row0 : row0 + 64 * i) < p.feat_tile;      // (rows past the last feature: read as they are, never stored)
+#pragma unroll
+        for (int i = 0; i < XP; ++i) x_live[i] = row0 + 64 * i < n_tok;
+        // 16-byte pieces 2 piece, 2 piece + 1 of a float32 row, piece `piece` of a bfloat16 row, each where its swizzle puts it
+        // (64 rows apart the swizzles are the same)
+        const int src0 = row0 * 128 + (((2 * piece) ^ (row0 & 7)) << 4), src1 = row0 * 128 + (((2 * piece + 1) ^ (row0 & 7)) << 4);
+        const int dst = row0 * 64 + ((piece ^ ((row0 >> 1) & 3)) << 4);
+        const int x_part = n16 * 64;
+        float odd = 0.0f;
+        bool ok = true;
+        for (int kb = g; kb < n_kb && ok; kb += G) {
+            const int rs = kb % RING, s = kb % STAGES;
+            ok = mbar_wait(&raw_full[rs], (kb / RING) & 1, 16) && mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 11);
+            if (!ok) break;
+            uint8_t* wt = stages + s * S::STAGE;
+            uint8_t* xt = wt + 3 * S::W_PART;
+            const uint8_t* wr = raw + rs * S::RAW;
+            const uint8_t* xr = wr + S::W_RAW;
+            uint4 hi, mid, lo;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (w_live[i]) {
+                    split8(*(const float4*)(wr + i * 64 * 128 + src0), *(const float4*)(wr + i * 64 * 128 + src1), hi, mid, lo, odd);
+                    uint8_t* at = wt + i * 64 * 64 + dst;
+                    *(uint4*)at = hi;
+                    *(uint4*)(at + S::W_PART) = mid;
+                    *(uint4*)(at + 2 * S::W_PART) = lo;
+                }
+#pragma unroll
+            for (int i = 0; i < XP; ++i)
+                if (x_live[i]) {
+                    split8(*(const float4*)(xr + i * 64 * 128 + src0), *(const float4*)(xr + i * 64 * 128 + src1), hi, mid, lo, odd);
+                    uint8_t* at = xt + i * 64 * 64 + dst;
+                    *(uint4*)at = hi;
+                    *(uint4*)(at + x_part) = mid;
+                    *(uint4*)(at + 2 * x_part) = lo;
+                }
+            if (kb + G >= n_kb && !(odd == 0.0f)) odd_flag = 1;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&raw_empty[rs]);
+                mbar_arrive(&full_bar[s]);
+            }
+        }
+    } else if (work && warp == ISSUE) {
+        // ---- product issue --------------------------------------------------------------------------
+        if (elect_one()) {
+            // two accumulators a block of K, D0 | D1, n16 columns each: D0 takes the products with the leading part of X, D1 the
+            // others; where both take the same part of W, one product twice as wide serves both
+            const uint32_t one = umma_idesc_bf16(128, n16), both = umma_idesc_bf16(128, 2 * n16);
+            const uint64_t first = umma_desc_sw64(stages);
+            const uint64_t w_step = S::W_PART >> 4, x_hi = 3 * w_step, x_lo = x_hi + (uint64_t)(2 * n16 * 64 >> 4);
+            bool ok = true;
+            for (int kb = 0; kb < n_kb && ok; ++kb) {
+                const int s = kb % STAGES, a = kb & 1;
+                ok = mbar_wait(&acc_empty[a], ((kb >> 1) & 1) ^ 1, 14) && mbar_wait(&full_bar[s], (kb / STAGES) & 1, 12);
+                if (!ok) break;
+                tcgen05_fence_after();
+                const uint64_t at = first + (uint64_t)((s * S::STAGE) >> 4);
+                const uint32_t d0 = tmem + a * 2 * N, d1 = d0 + n16;
+                // the smallest products first
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * w_step + 2 * k, at + x_hi + 2 * k, one, k > 0);          // lo hi
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma_bf16(d1, at + 2 * k, at + x_lo + 2 * k, one, k > 0);                       // hi lo
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + w_step + 2 * k, at + x_hi + 2 * k, both, 1);                 // mid hi | mid mid
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * k, at + x_hi + 2 * k, both, 1);                          // hi hi | hi mid
+                umma_commit(&empty_bar[s]);
+                umma_commit(&acc_full[a]);
+            }
+        }
+    } else if (work && warp >= FIRST_EPI) {
+        // ---- adding up: a thread has one row of the product (a feature) and COLS of its tokens --------------
+        const int quarter = warp & 3, r = quarter * 32 + lane, c_first = ((warp - FIRST_EPI) >> 2) * COLS;
+        float acc[COLS];
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
+        bool ok = true;
+        for (int kb = 0; kb < n_kb && ok; ++kb) {
+            const int a = kb & 1;
+            ok = mbar_wait(&acc_full[a], (kb >> 1) & 1, 13);
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t at = tmem + a * 2 * N + c_first + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+            for (int c = 0; c < COLS; c += 16) {
+                if (c_first + c >= n16) break;
+                uint32_t v[16];
+                tmem_ld16(at + n16 + c, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(v[j]);
+                tmem_ld16(at + c, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(v[j]);
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[a]);
+        }
+        if (!grouped) cj::after_predecessor();
+        const int fr = DUAL ? (r & 63) : r, feat = feat0 + fr;
+        const bool live = ok && fr < p.feat_tile && feat < p.features;
+        if (odd_flag && live) {
+            const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j)
+                if (c_first + j < n_tok) acc[j] = chain(p.X + (size_t)(tok0 + c_first + j) * p.ldx, w, p.K);
+        }
+        if (DUAL) {
+            // the second weight's sums cross to the threads that hold the first's: through the ring, which nothing reads any more
+            float* up = (float*)raw;
+            if (r >= 64) {
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) up[(c_first + j) * 64 + fr] = acc[j];
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+        }
+        if (live && !(DUAL && r >= 64)) {
+            const float b = p.bias ? p.bias[feat] : 0.0f;
+            const float b2 = DUAL && p.bias2 ? p.bias2[feat] : 0.0f;
+            float* out = p.C + (size_t)(tok0 + c_first) * p.ldc + feat;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) {
+                if (c_first + j >= n_tok) break;
+                float v = p.bias ? acc[j] + b : acc[j];
+                if (DUAL) {
+                    const float u = ((const float*)raw)[(c_first + j) * 64 + fr];
+                    v = cj::gated_act(v, p.bias2 ? u + b2 : u, p.act_limit, p.act_alpha, p.act_cubic);
+                } else if (p.act != cj::ACT_NONE && feat < p.act_feats) {
+                    v = cj::plain_act(v, p.act);
+                }
+                v *= p.out_scale;
+                float* o = out + (size_t)j * p.ldc;
+                *o = p.accumulate ? v + *o : v;
+            }
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == ISSUE) {
+        tcgen05_fence_after();
+        tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
+// a row-major float32 matrix in boxes of [box_rows, 32] with the 128-byte swizzle; out-of-range elements read as zero
+bool make_map_f32(CUtensorMap* map, const float* base, long long rows, long long cols, long long ld, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+    cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int N, bool DUAL>
+int launch(const Args& a, int tok_tiles, cudaStream_t stream) {
+    auto kern = gemm_f32_tc_kernel<N, DUAL>;
+    static bool sized = false;
+    if (!sized) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<N>::TOTAL);
+        if (e != cudaSuccess) return (int)e;
+        sized = true;
+    }
+    if (tok_tiles > 65535) return CJ_ERR_SIZE;
+    const long long w_rows = (long long)(a.group_offsets ? a.groups : 1) * a.features;
+    CUtensorMap mx, mw, mw2;
+    if (!make_map_f32(&mx, a.X, a.tokens, a.K, a.ldx, N) || !make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
+    mw2 = mw;
+    if (DUAL && !make_map_f32(&mw2, a.W2, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
+    cj::launch(kern, dim3((a.features + a.feat_tile - 1) / a.feat_tile, tok_tiles), dim3(threads(N)), Smem<N>::TOTAL, stream, mx, mw, mw2, a);
+    return cj::launch_status();
+}
+
+}  // namespace
+
+// X [tokens, K] float32 with row stride ldx (grouped: in the groups' order), W (and W2) [groups, features, K] contiguous float32; the
+// other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16, 32, 64 or 128); feat_tile: its features (32, 64 or 128; with W2 at most 64).
+CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
+                             long long ldc, int tokens, int features, int K, int accumulate, const int* group_offsets, int groups,
+                             float act_limit, float act_alpha, float act_cubic, int act, int act_feats, float out_scale, int n_tok,
+                             int feat_tile, cudaStream_t stream) {
+    if (tokens <= 0 || features <= 0) return 0;
+    if (!X || !W || !C || K <= 0) return CJ_ERR_ARG;
+    if (group_offsets && groups <= 0) return CJ_ERR_ARG;
+    if ((bias2 && !W2) || (act != cj::ACT_NONE && W2)) return CJ_ERR_ARG;
+    if (feat_tile != 32 && feat_tile != 64 && !(feat_tile == 128 && !W2)) return CJ_ERR_SIZE;
+    if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
+    if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2) & 15) return CJ_ERR_ALIGN;
+    Args a{X, ldx, W, W2, bias, bias2, C, ldc, tokens, features, K, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
+           act_feats > 0 ? act_feats : features, out_scale, feat_tile};
+    const int tok_tiles = (tokens + n_tok - 1) / max(n_tok, 1) + (group_offsets ? groups : 0);
+#define CASE(N) case N: return W2 ? launch<N, true>(a, tok_tiles, stream) : launch<N, false>(a, tok_tiles, stream);
+    switch (n_tok) {
+        CASE(16) CASE(32) CASE(64) CASE(128)
+    }
+#undef CASE
+    return CJ_ERR_SIZE;
+}
+
+// 0, or the code of the first bounded wait that ran out (15 loads, 11 and 16 splitting, 12 and 14 product issue, 13 adding up);
+// reading it synchronises the device.
+CJ_EXPORT int cj_gemm_f32_tc_error() {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, tc::g_error_flag, sizeof(int)) != cudaSuccess) return -1;
+    return v;
+}

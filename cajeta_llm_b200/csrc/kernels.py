@@ -265,12 +265,44 @@ def _gate_biases(w: torch.Tensor, w_up: Optional[torch.Tensor], bias: Optional[t
         raise KernelError(f"act must be one of {sorted(ACTS)} and goes with one weight, found '{act}'")
 
 
+F32_TC_TOKENS = (16, 32, 64, 128)      # token tiles of the float32 tensor-core product
+
+
+def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor], out: torch.Tensor) -> bool:
+    """Whether a product of these operands runs on the tensor cores in three bfloat16 parts an operand (csrc/gemm_f32_tc.cu): what TMA
+    can read, from K and features on that fill a tile (17 rows of 200 features and K 132: 12 us, 18 on the FMA pipe).  The
+    number of rows is no part of it: a row's bits must not depend on the others."""
+    N, K = w.shape[-2], w.shape[-1]
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K >= 128 and N >= 64 and K % 4 == 0
+            and a.stride(0) % 4 == 0 and a.stride(0) >= K and (a.data_ptr() | w.data_ptr() | (w_up.data_ptr() if w_up is not None else 0)) % 16 == 0)
+
+
+def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
+    """(tokens, features) of a tile of the float32 tensor-core product; a result's bits do not depend on them."""
+    most = 64 if gated else 128
+    if groups:
+        # tiles that most groups of an even split fill once (mean and two standard deviations), as their weights are read once a tile
+        mean = rows / groups
+        want = min(rows, mean + 2.0 * mean ** 0.5)
+        n_tok = next((n for n in F32_TC_TOKENS if want <= n), F32_TC_TOKENS[-1])
+        return n_tok, most if -(-features // most) * min(groups, rows) >= sms else most // 2
+
+    # rounds of the machine times what a block of K takes in a tile of these sizes (us, fitted to 2,048 x 2,048 for one row and
+    # 6,144 x 2,048 for 60, 250 and 1,777); 128 tokens only for many rows: with cold weights and one round 250 x 6,144 took 164 us
+    # with 128 and 117 with 64, 1,777 x 6,144 422 and 543
+    def cost(n, f):
+        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.18 + 0.0056 * min(n, rows) + 0.0023 * f * (2 if gated else 1))
+
+    return min(((n, f) for n in F32_TC_TOKENS if n <= 64 or rows >= 512 for f in (most, most // 2)), key=lambda t: cost(*t))
+
+
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
          accumulate: bool = False, w_up: Optional[torch.Tensor] = None, group_offsets: Optional[torch.Tensor] = None,
          a_row_index: Optional[torch.Tensor] = None, rows: Optional[int] = None, act_limit: float = 0.0,
          act_alpha: float = 1.0, out_scale: float = 1.0, act_cubic: float = 0.0, bias_up: Optional[torch.Tensor] = None,
          act: str = "", act_features: int = 0) -> None:
-    """out[M, N] (+)= out_scale (a[M, K] . w[N, K]^T (+ bias)) on the float32 FMA pipe.
+    """out[M, N] (+)= out_scale (a[M, K] . w[N, K]^T (+ bias)) to float32's accuracy: float32 operands of many features and
+    a long K on the tensor cores (see :func:`f32_tc_takes`), the others on the float32 FMA pipe.
 
     ``w_up`` selects the gated form: silu(a.w^T) * (a.w_up^T), or with ``act_limit`` > 0 the capped one,
     g = min(a.w^T, limit), u = clamp(a.w_up^T, +-limit), g * sigmoid(act_alpha g) * (u + 1); without a limit
@@ -302,6 +334,18 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
             raise KernelError("gemm: group_offsets must hold one more entry than w has groups")
     if a_row_index is not None:
         _need(a_row_index, "a_row_index", torch.int32)
+    if f32_tc_takes(a, w, w_up, out):
+        if a_row_index is not None:
+            gathered = torch.empty((M, K), dtype=a.dtype, device=a.device)
+            gather_rows(a, a_row_index, gathered)
+            a = gathered
+        n_tok, feat_tile = f32_tc_tile(M, N, G, w_up is not None, _sm_count())
+        st = library("gemm_f32_tc").cj_gemm_f32_tc(
+            _ptr(a), _ll(a.stride(0)), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
+            _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
+            _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
+        _check(st, "gemm")
+        return
     st = library("gemm_simt").cj_gemm_simt(
         _ptr(a), _ll(a.stride(0)), _i(_code(a)), _ptr(w), _ptr(w_up), _ll(K), _i(_code(w)), _ptr(bias), _ptr(bias_up),
         _ptr(out), _ll(out.stride(0)), _i(_code(out)), _i(M), _i(N), _i(K), _i(1 if accumulate else 0),
@@ -1462,7 +1506,7 @@ def wait_errors() -> Dict[str, int]:
     """Codes of bounded waits that ran out inside the tensor-core kernels, by library; empty
     when all is well.  Only libraries that are already loaded are asked."""
     found = {}
-    for name, symbol in (("gemm_tc", "cj_gemm_tc_error"), ("gemm_tc2", "cj_gemm_tc2_error"),
+    for name, symbol in (("gemm_tc", "cj_gemm_tc_error"), ("gemm_tc2", "cj_gemm_tc2_error"), ("gemm_f32_tc", "cj_gemm_f32_tc_error"),
                          ("attention_prefill_tc", "cj_prefill_attention_tc_error")):
         lib = _libs.get(name)
         if lib is not None:

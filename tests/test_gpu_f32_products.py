@@ -1,0 +1,87 @@
+"""The float32 product on the tensor cores (three bfloat16 parts an operand) against 64 bits, at the edges of its tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def K():
+    from cajeta_llm_b200.csrc import kernels
+    return kernels
+
+
+def rnd(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+def held(got, a, w, want):
+    """The sum's error is at most two roundings (2^-24 of the sum of magnitudes each) a block of 32 products, and a few for the terms
+    left out, the accumulator's truncation inside a block and the last addition."""
+    bound = (a.shape[-1] / 16 + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+    assert bool(((got.double() - want).abs() <= bound).all()), float(((got.double() - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 64, 128), (16, 128, 132), (17, 129, 160), (33, 200, 2048), (64, 130, 1000), (65, 1408, 256),
+                                     (129, 96, 1028), (300, 257, 136), (600, 260, 192)])
+def test_plain_bias_accumulate_scale(K, M, N, Kd):
+    a, w, b = rnd(M, Kd, seed=1), rnd(N, Kd, seed=2), rnd(N, seed=3)
+    out = torch.empty(M, N, device=DEV)
+    assert K.f32_tc_takes(a, w, None, out)
+    want = a.double() @ w.double().t()
+    K.gemm(a, w, out)
+    held(out, a, w, want)
+    base = rnd(M, N, seed=4)
+    acc = base.clone()
+    K.gemm(a, w, acc, bias=b, accumulate=True, out_scale=0.5)
+    assert torch.allclose(acc.double(), 0.5 * (want + b.double()) + base.double(), atol=1e-4, rtol=1e-5)
+    # rows do not depend on the batch: the same bits from a tile of any width
+    for lo, hi in ((0, 1), (M // 2, M)):
+        part = torch.empty(hi - lo, N, device=DEV)
+        K.gemm(a[lo:hi], w, part)
+        assert torch.equal(part, out[lo:hi])
+    assert K.wait_errors() == {}
+
+
+@pytest.mark.parametrize("n_tok", [16, 32, 64, 128])
+@pytest.mark.parametrize("feat_tile", [64, 128])
+def test_every_tile_gives_the_same_bits(K, monkeypatch, n_tok, feat_tile):
+    a, w = rnd(150, 292, seed=12), rnd(200, 292, seed=13)
+    out, other = torch.empty(150, 200, device=DEV), torch.empty(150, 200, device=DEV)
+    K.gemm(a, w, out)
+    monkeypatch.setattr(K, "f32_tc_tile", lambda *x: (n_tok, feat_tile))
+    K.gemm(a, w, other)
+    assert torch.equal(out, other)
+
+
+@pytest.mark.parametrize("T,inter", [(1, 64), (7, 100), (70, 192), (200, 65), (800, 64)])
+def test_gated_and_grouped(K, T, inter):
+    H, E, k = 260, 5, 2
+    x, wg, wu, wd = rnd(T, H, seed=5), rnd(E, inter, H, seed=6), rnd(E, inter, H, seed=7), rnd(E, H, inter, seed=8)
+    sel = torch.randint(0, E - 1, (T * k,), generator=torch.Generator().manual_seed(9))       # the last group is empty
+    order = torch.argsort(sel, stable=True)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(sel, minlength=E).cumsum(0)]).int().to(DEV)
+    index = (order // k).int().to(DEV)
+    out = torch.empty(T * k, inter, device=DEV)
+    K.gemm(x, wg, out, w_up=wu, group_offsets=offsets, a_row_index=index)
+    down = torch.empty(T * k, H, device=DEV)
+    K.gemm(out, wd, down, group_offsets=offsets)
+    for e in range(E):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        rows = x[index[lo:hi].long()].double()
+        g, u = rows @ wg[e].double().t(), rows @ wu[e].double().t()
+        assert torch.allclose(out[lo:hi].double(), g * torch.sigmoid(g) * u, atol=1e-3, rtol=1e-4)
+        assert torch.allclose(down[lo:hi].double(), out[lo:hi].double() @ wd[e].double().t(), atol=5e-3, rtol=1e-4)
+    assert K.wait_errors() == {}
+
+
+def test_infinite_and_missing_numbers_are_summed_as_the_fma_pipe_sums_them(K):
+    a, w = rnd(40, 192, seed=10), rnd(140, 192, seed=11)
+    a[3, 7], a[20, 100], a[21, 0], w[5, 9] = float("inf"), float("nan"), 3.4e38, float("-inf")
+    out = torch.empty(40, 140, device=DEV)
+    K.gemm(a, w, out)
+    want = a.double() @ w.double().t()
+    want = torch.where(want.abs() > 3.4028235e38, torch.sign(want) * float("inf"), want)
+    same = torch.isnan(out) == torch.isnan(want)
+    assert bool(same.all()) and torch.equal(torch.isinf(out), torch.isinf(want.float()))
