@@ -24,8 +24,8 @@
 // 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
 // tokens that chain, with many the shared memory, which every operand crosses as float32 once and as bfloat16 parts once for each of
 // its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 35;
-// 250 x 6,144 x 2,048 328 and 117; 1,777 x 6,144 x 2,048 1,822 and 420; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
-// of 4 picks 802 / 1,915 / 6,045 and 181 / 575 / 1,607.  (With the float32 operands loaded into registers instead of by TMA
+// 250 x 6,144 x 2,048 328 and 114; 1,777 x 6,144 x 2,048 1,822 and 375; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
+// of 4 picks 802 / 1,915 / 6,045 and 181 / 570 / 1,430.  (With the float32 operands loaded into registers instead of by TMA
 // 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
 #define CJ_LIB "gemm_f32_tc"
@@ -239,17 +239,37 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         bool ok = true;
         for (int kb = g; kb < n_kb && ok; kb += G) {
             const int rs = kb % RING, s = kb % STAGES;
-            ok = mbar_wait(&raw_full[rs], (kb / RING) & 1, 16) && mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 11);
+            ok = mbar_wait(&raw_full[rs], (kb / RING) & 1, 16);
             if (!ok) break;
-            uint8_t* wt = stages + s * S::STAGE;
-            uint8_t* xt = wt + 3 * S::W_PART;
             const uint8_t* wr = raw + rs * S::RAW;
             const uint8_t* xr = wr + S::W_RAW;
+            float4 w[2][2], x[XP][2];
+            auto read = [&]() {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    if (w_live[i]) {
+                        w[i][0] = *(const float4*)(wr + i * 64 * 128 + src0);
+                        w[i][1] = *(const float4*)(wr + i * 64 * 128 + src1);
+                    }
+#pragma unroll
+                for (int i = 0; i < XP; ++i)
+                    if (x_live[i]) {
+                        x[i][0] = *(const float4*)(xr + i * 64 * 128 + src0);
+                        x[i][1] = *(const float4*)(xr + i * 64 * 128 + src1);
+                    }
+            };
+            // a lone group reads while the stage is still in use (1,777 x 6,144: 396 -> 375 us); several cover each other's
+            if (G == 1) read();
+            ok = mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 11);
+            if (!ok) break;
+            if (G > 1) read();
+            uint8_t* wt = stages + s * S::STAGE;
+            uint8_t* xt = wt + 3 * S::W_PART;
             uint4 hi, mid, lo;
 #pragma unroll
             for (int i = 0; i < 2; ++i)
                 if (w_live[i]) {
-                    split8(*(const float4*)(wr + i * 64 * 128 + src0), *(const float4*)(wr + i * 64 * 128 + src1), hi, mid, lo, odd);
+                    split8(w[i][0], w[i][1], hi, mid, lo, odd);
                     uint8_t* at = wt + i * 64 * 64 + dst;
                     *(uint4*)at = hi;
                     *(uint4*)(at + S::W_PART) = mid;
@@ -258,7 +278,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
             for (int i = 0; i < XP; ++i)
                 if (x_live[i]) {
-                    split8(*(const float4*)(xr + i * 64 * 128 + src0), *(const float4*)(xr + i * 64 * 128 + src1), hi, mid, lo, odd);
+                    split8(x[i][0], x[i][1], hi, mid, lo, odd);
                     uint8_t* at = xt + i * 64 * 64 + dst;
                     *(uint4*)at = hi;
                     *(uint4*)(at + x_part) = mid;

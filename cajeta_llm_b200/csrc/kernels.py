@@ -289,7 +289,7 @@ def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
 
     # rounds of the machine times what a block of K takes in a tile of these sizes (us, fitted to 2,048 x 2,048 for one row and
     # 6,144 x 2,048 for 60, 250 and 1,777); 128 tokens only for many rows: with cold weights and one round 250 x 6,144 took 164 us
-    # with 128 and 117 with 64, 1,777 x 6,144 422 and 543
+    # with 128 and 114 with 64, 1,777 x 6,144 375 and 543
     def cost(n, f):
         return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.18 + 0.0056 * min(n, rows) + 0.0023 * f * (2 if gated else 1))
 

@@ -59,7 +59,7 @@ class Model:
 
     def libraries(self) -> set:
         """The kernel libraries this model's steps will call (embedding, norms and head included)."""
-        out = {"rowwise", "gemm_simt", "sampling"}
+        out = {"rowwise", "gemm_simt", "sampling"} | ({"gemm_f32_tc"} if self.runtime.act_dtype == torch.float32 else set())
         for p in self.parts():
             out |= p.libraries()
         return out

@@ -199,6 +199,8 @@ class PagedAttention(Part):
             libs |= {"attention_decode", "attention_prefill_tc" if self.head_dim == 128 else "attention_prefill"}
         else:
             libs.add("attention_paged")
+        if "attention_paged" in libs and self.runtime.act_dtype == torch.float32:
+            libs.add("attention_f32")
         if self.runtime.fast_kernels and self.hidden >= 128:
             libs |= {"gemm_tc", "gemm_tc2"}
         return libs

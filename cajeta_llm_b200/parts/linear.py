@@ -4,8 +4,9 @@
 a gated activation of two such products (SwiGLU and its like), for a dense weight or for the stacked weights of a
 mixture of experts.  On the bfloat16 path it runs on the tensor cores (tcgen05 / TMA)
 when the shapes allow TMA (K a multiple of 8, 16-byte aligned rows) and are large
-enough to fill a tile; otherwise, and always on the float32 path, it runs on the FMA
-pipe, whose results do not depend on the batch at all.  Few rows (decode) put the
+enough to fill a tile; otherwise, and always on the float32 path, it runs through
+``K.gemm`` (the FMA pipe, or three bfloat16 parts an operand on the tensor cores), whose
+results do not depend on the batch at all.  Few rows (decode) put the
 weights on the rows of the tensor-core product, many rows (prompt portions) the tokens.
 """
 from __future__ import annotations
