@@ -821,12 +821,15 @@ def cast_rows(x: torch.Tensor, out: torch.Tensor) -> None:
 
 
 def rmsnorm_add(hs: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float) -> None:
-    """hs[r] += y[r] / sqrt(mean(y[r]^2) + eps) * weight; everything float32."""
+    """hs[r] += y[r] / sqrt(mean(y[r]^2) + eps) * weight; everything float32.  ``y`` of three dimensions [S, rows, H]: partial
+    sums of the rows, added in order first."""
     _need(hs, "hs", torch.float32), _need(y, "y", torch.float32), _need(weight, "weight", torch.float32)
     rows, H = hs.shape
-    if y.shape != hs.shape or weight.numel() != H:
+    if y.shape[-2:] != hs.shape or y.dim() > 3 or weight.numel() != H:
         raise KernelError(f"rmsnorm_add: shapes hs {tuple(hs.shape)} y {tuple(y.shape)} weight {tuple(weight.shape)} do not agree")
-    _check(library("recurrent").cj_rmsnorm_add(_ptr(hs), _ptr(y), _ptr(weight), _f(eps), _i(rows), _i(H), _stream()), "rmsnorm_add")
+    parts, stride = (y.shape[0], y.stride(0)) if y.dim() == 3 else (1, 0)
+    _check(library("recurrent").cj_rmsnorm_add(_ptr(hs), _ptr(y), _i(parts), _ll(stride), _ptr(weight), _f(eps), _i(rows), _i(H), _stream()),
+           "rmsnorm_add")
 
 
 def scale_rows_gather(x: torch.Tensor, slot_of_pick: torch.Tensor, weights: torch.Tensor, top_k: int, out: torch.Tensor) -> None:
@@ -861,6 +864,28 @@ def short_conv(x: torch.Tensor, x_offset: int, channels: int, taps: int, weight:
                                             _ll(state.stride(0)), _ptr(row_req), _ptr(req_start), _ptr(req_slot), _ptr(out),
                                             _i(out.stride(0)), _i(_code(out)), _i(1 if activate else 0), _i(x.shape[0]), _stream())
     _check(st, "short_conv")
+
+
+def short_conv_moved(x: torch.Tensor, x_offset: int, channels: int, taps: int, weight: torch.Tensor, bias: Optional[torch.Tensor],
+                     state: torch.Tensor, ctx, out: torch.Tensor, activate: bool = True, state_offset: int = 0) -> None:
+    """``short_conv`` and ``short_conv_commit`` of a step (``ctx``: its :class:`StepContext`): one kernel when every request brings one
+    token, else the two after one another."""
+    if getattr(ctx, "all_single", False) and 2 <= taps <= 4:
+        _need(x, "x", torch.float32), _need(weight, "weight", torch.float32), _need(state, "state", torch.float32), _need(out, "out")
+        _need(ctx.row_req, "row_req", torch.int32), _need(ctx.req_slot, "req_slot", torch.int32)
+        if bias is not None:
+            _need(bias, "bias", torch.float32)
+        if weight.shape != (channels, taps) or x.shape[1] < x_offset + channels or out.shape[1] < channels or state[0].numel() < state_offset + (taps - 1) * channels:
+            raise KernelError("short_conv: sizes do not agree")
+        st = library("recurrent").cj_short_conv_single(
+            ctypes.c_void_p(x.data_ptr() + 4 * x_offset), _i(x.stride(0)), _i(channels), _i(taps), _ptr(weight), _ptr(bias),
+            ctypes.c_void_p(state.data_ptr() + 4 * state_offset), _ll(state.stride(0)), _ptr(ctx.row_req), _ptr(ctx.req_slot), _ptr(out),
+            _i(out.stride(0)), _i(_code(out)), _i(1 if activate else 0), _i(x.shape[0]), _stream())
+        _check(st, "short_conv")
+        return
+    short_conv(x, x_offset, channels, taps, weight, bias, state, ctx.row_req, ctx.req_start, ctx.req_slot, out, activate=activate,
+               state_offset=state_offset)
+    short_conv_commit(x, x_offset, channels, taps, state, ctx.req_start, ctx.req_slot, ctx.n_requests, state_offset=state_offset)
 
 
 def short_conv_commit(x: torch.Tensor, x_offset: int, channels: int, taps: int, state: torch.Tensor, req_start: torch.Tensor,

@@ -356,9 +356,7 @@ class PagedAttention(Part):
             at = getattr(entry, "state_offset", 0)
             conv = torch.empty((T, C), dtype=torch.float32, device=x.device)
             K.tag = "short conv"
-            K.short_conv(qkv, 0, C, self.taps, self.w_conv, None, entry.state, ctx.row_req, ctx.req_start, ctx.req_slot, conv,
-                         activate=False, state_offset=at)
-            K.short_conv_commit(qkv, 0, C, self.taps, entry.state, ctx.req_start, ctx.req_slot, ctx.n_requests, state_offset=at)
+            K.short_conv_moved(qkv, 0, C, self.taps, self.w_conv, None, entry.state, ctx, conv, activate=False, state_offset=at)
             qkv = conv
         q = torch.empty((T, self.heads, self.head_dim), dtype=rt.act_dtype, device=x.device)
         K.tag = "heads + cache write"

@@ -133,6 +133,8 @@ class OutputNormBlock(Part):
         super().__init__(spec, prefix, runtime)
         self.mixer_norm = make_part("norm", layer.mixer_norm, self.name(spec["mixer_norm_name"]), runtime)
         self.mixer = make_part("mixer", layer.mixer, self.name(spec["mixer_name"]), runtime)
+        if hasattr(self.mixer, "allow_pending"):
+            self.mixer.allow_pending = True        # partial sums are added by the kernel that norms them
         self.feed_forward = self.feed_forward_norm = None
         if layer.feed_forward is not None:
             self.feed_forward_norm = make_part("norm", layer.feed_forward_norm, self.name(spec["feed_forward_norm_name"]), runtime)
@@ -169,23 +171,27 @@ class OutputNormBlock(Part):
         K.cast_rows(hs, x)
         return x
 
-    def _add_normed(self, hs: torch.Tensor, y: torch.Tensor, pending, norm) -> None:
-        if pending is not None:
-            y += pending.sum(dim=0)
+    def _add_normed(self, hs: torch.Tensor, y: torch.Tensor, norm) -> None:
         K.tag = "norm + add"
         K.rmsnorm_add(hs, y, norm.weight, norm.eps)
         K.tag = None
 
     def forward(self, hs: torch.Tensor, ctx, entry) -> None:
-        y = torch.zeros_like(hs)
+        # a mixer that hands back partial sums leaves y alone: nothing to clear, and the norm adds them as it reads them
+        deferred = getattr(self.mixer, "defers", lambda n: False)(hs.shape[0])
+        y = torch.empty_like(hs) if deferred else torch.zeros_like(hs)
         pending = self.mixer.forward(self._input(hs), y, ctx, entry)
-        self._add_normed(hs, y, pending, self.mixer_norm)
+        if deferred and pending is None:
+            raise ValueError("a mixer that defers (defers(rows)) has to hand back partial sums")
+        if pending is not None and not deferred:
+            y += pending.sum(dim=0)
+        self._add_normed(hs, pending if deferred else y, self.mixer_norm)
         ff = self.feed_forward
         if ff is None:
             return
         y = torch.zeros_like(hs)
         ff.forward(self._input(hs), hs if getattr(ff, "needs_f32_input", False) else None, y, ctx)
-        self._add_normed(hs, y, None, self.feed_forward_norm)
+        self._add_normed(hs, y, self.feed_forward_norm)
 
 
 @register_part("block", "parallel")
@@ -390,10 +396,7 @@ class SandwichBlock(Part):
         h, _ = self.mixer_norm.forward(hs, out_dtype=torch.float32)
         x = torch.empty(h.shape, dtype=rt.act_dtype, device=hs.device)
         K.tag = "input conv"
-        K.short_conv(h, 0, self.hidden, self.taps, self.w_conv, None, entry.state, ctx.row_req, ctx.req_start, ctx.req_slot, x,
-                     activate=False, state_offset=entry.state_offset)
-        K.short_conv_commit(h, 0, self.hidden, self.taps, entry.state, ctx.req_start, ctx.req_slot, ctx.n_requests,
-                            state_offset=entry.state_offset)
+        K.short_conv_moved(h, 0, self.hidden, self.taps, self.w_conv, None, entry.state, ctx, x, activate=False, state_offset=entry.state_offset)
         K.tag = None
         return x
 

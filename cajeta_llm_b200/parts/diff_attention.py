@@ -145,10 +145,7 @@ class DifferentialAttention(Part):
             K.tag = "short conv"
             # one tap keeps no state: the kernel then reads none, and is given a word to point at
             state = entry.state if self.taps > 1 else torch.zeros((1, 1), dtype=torch.float32, device=dev)
-            K.short_conv(qkv, 0, C, self.taps, self.w_conv, None, state, ctx.row_req, ctx.req_start, ctx.req_slot, conv,
-                         activate=False, state_offset=at)
-            if self.taps > 1:
-                K.short_conv_commit(qkv, 0, C, self.taps, entry.state, ctx.req_start, ctx.req_slot, ctx.n_requests, state_offset=at)
+            K.short_conv_moved(qkv, 0, C, self.taps, self.w_conv, None, state, ctx, conv, activate=False, state_offset=at)
             qkv = conv
         kd = 2 * self.dim
         q = torch.empty((T, self.heads, kd), dtype=rt.act_dtype, device=dev)

@@ -1,0 +1,78 @@
+"""Row kernels around the recurrent mixers at the edges of their vector forms: against the plain formulas in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+@pytest.mark.parametrize("rows,H,parts", [(3, 4, 1), (5, 1020, 3), (2, 1024, 8), (9, 2048, 1), (4, 2052, 2), (3, 8192, 5), (2, 8196, 2), (3, 77, 2)])
+def test_rmsnorm_add_of_rows_and_of_partial_sums(rows, H, parts):
+    from cajeta_llm_b200.csrc import kernels as K
+    hs, y, w = rnd(rows, H, seed=1), rnd(parts, rows, H, seed=2), rnd(H, seed=3)
+    want_y = y.double().sum(0)
+    want = hs.double() + want_y / torch.sqrt((want_y ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    got = hs.clone()
+    K.rmsnorm_add(got, y if parts > 1 else y[0], w, 1e-6)
+    assert torch.allclose(got.double(), want, atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("channels,offset,lengths", [(512, 4, [1, 2, 200]), (516, 0, [127, 3, 17, 1]), (1028, 8, [130]), (510, 0, [140]), (512, 3, [128]),
+                                                      (64, 0, [5, 9])])
+@pytest.mark.parametrize("dtype,activate", [(torch.float32, True), (torch.bfloat16, False)])
+def test_short_conv_of_many_rows_equals_token_by_token(taps, channels, offset, lengths, dtype, activate):
+    from types import SimpleNamespace
+    from cajeta_llm_b200.csrc import kernels as K
+    R, T = len(lengths), sum(lengths)
+    x, w, b = rnd(T, channels + 12, seed=4), rnd(channels, taps, seed=5), rnd(channels, seed=6)
+    slots = torch.randperm(R + 1, generator=torch.Generator().manual_seed(7))[:R].int().to(DEV)
+    starts = [sum(lengths[:i]) for i in range(R + 1)]
+    req = torch.cat([torch.full((n,), i) for i, n in enumerate(lengths)]).int().to(DEV)
+    first = rnd(R + 1, (taps - 1) * channels + 5, seed=8)
+    results = []
+    for single in (False, True):
+        state, out = first.clone(), torch.empty(T, channels, device=DEV, dtype=dtype)
+
+        def conv(rows, row_req, req_start, slot, all_single):
+            part = torch.empty(len(rows), channels, device=DEV, dtype=dtype)
+            ctx = SimpleNamespace(row_req=row_req, req_start=torch.tensor(req_start, dtype=torch.int32, device=DEV), req_slot=slot,
+                                  n_requests=slot.numel(), all_single=all_single)
+            K.short_conv_moved(x[rows].contiguous(), offset, channels, taps, w, b, state, ctx, part, activate=activate, state_offset=5)
+            out[rows] = part
+
+        if single:
+            for t in range(max(lengths)):                                    # a step of every request that has a token t
+                live = [r for r in range(R) if t < lengths[r]]
+                conv([starts[r] + t for r in live], torch.arange(len(live), dtype=torch.int32, device=DEV), list(range(len(live) + 1)),
+                     slots[live].contiguous(), True)
+        else:
+            conv(list(range(T)), req, starts, slots, False)
+        results.append((out, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    if taps > 1:                                                             # and the formula, for the last request
+        r = R - 1
+        padded = torch.cat([first[slots[r], 5:5 + (taps - 1) * channels].view(taps - 1, channels), x[starts[r]:starts[r + 1], offset:offset + channels]]).double()
+        want = sum(w.double()[:, j] * padded[j:j + lengths[r]] for j in range(taps)) + b.double()
+        want = want * torch.sigmoid(want) if activate else want
+        tol = dict(atol=1e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=1e-2)
+        assert torch.allclose(results[0][0][starts[r]:].double(), want, **tol)
+
+
+@pytest.mark.parametrize("n,part,w_len,z_offset", [(512, 128, 128, 4), (1024, 256, 1024, 0), (1024, 512, 1024, 8), (2048, 1024, 1024, 0), (768, 384, 768, 0),
+                                                    (512, 128, 128, 3)])
+@pytest.mark.parametrize("gate_first,sigmoid", [(True, False), (False, False), (False, True)])
+def test_gated_group_norm(n, part, w_len, z_offset, gate_first, sigmoid):
+    from cajeta_llm_b200.csrc import kernels as K
+    y, z, w = rnd(5, n, seed=9), rnd(5, n + 12, seed=10), rnd(w_len, seed=11)
+    out = torch.empty(5, n, device=DEV)
+    K.gated_group_norm(y, part, z, z_offset, w, 1e-6, gate_first, out, sigmoid_gate=sigmoid)
+    zz = z[:, z_offset:z_offset + n].double()
+    gate = torch.sigmoid(zz) * (1.0 if sigmoid else zz)
+    v = (y.double() * gate if gate_first else y.double()).view(5, n // part, part)
+    v = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6)).reshape(5, n) * w.double().repeat(n // w_len)
+    assert torch.allclose(out.double(), v if gate_first else v * gate, atol=1e-5, rtol=1e-5)
