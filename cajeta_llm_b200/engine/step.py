@@ -448,12 +448,14 @@ class ModelRunner:
         if tokens.min() < 0 or tokens.max() >= vocab:
             bad = int(tokens[(tokens < 0) | (tokens >= vocab)][0])
             raise StepError(f"token id {bad} is outside the vocabulary [0, {vocab})")
-        for e in entries:
-            for w in e.want:
-                if not 0 <= w < len(e.tokens):
-                    raise StepError(f"want index {w} is outside the {len(e.tokens)} tokens of the entry")
+        # (whole arrays: a step that wants every row of a prompt of 2,048 tokens spent 250 us in a loop over them)
         n_want = np.fromiter((len(e.want) for e in entries), dtype=np.int32, count=len(entries))
-        wants = np.fromiter((w for e in entries for w in e.want), dtype=np.int32, count=int(n_want.sum()))
+        wants = np.concatenate([np.asarray(e.want) for e in entries if len(e.want) > 0] or [np.empty(0, dtype=np.int32)])
+        outside = ~((0 <= wants) & (wants < np.repeat(counts, n_want)))
+        if outside.any():
+            at = int(np.argmax(outside))
+            raise StepError(f"want index {wants[at]} is outside the {np.repeat(counts, n_want)[at]} tokens of the entry")
+        wants = wants.astype(np.int32)
         slot_arr = np.asarray(slots, dtype=np.int32)
         short = cache.books.reserve_step(slot_arr, counts)        # also refuses a slot that holds no request
         if short is not None:
