@@ -40,6 +40,8 @@ class SideBySide(Part):
                 m.allow_pending = False        # no norm follows that would add partial sums: each adds its own result
         self.graph_safe = all(getattr(m, "graph_safe", m.state_need() is None) for m in (self.left, self.right))
         self.capture_max_rows = min(int(getattr(m, "capture_max_rows", 1 << 30)) for m in (self.left, self.right))
+        self.capture_fresh = all(getattr(m, "capture_fresh", False) for m in (self.left, self.right)
+                                 if getattr(m, "capture_max_rows", 1 << 30) < 1 << 30)
         need = self.left.state_need()
         self.left_state = int(need.shape[0]) if need is not None else 0
         self.w_left = self.w_right = None

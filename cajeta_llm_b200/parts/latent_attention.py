@@ -22,7 +22,7 @@ the requests' tokens are built with two products over the gathered latents and a
 kernel on the tensor cores runs over them - a (query, key, head) pair then costs
 ``2 (dim + rot_dim + vdim)`` flops instead of ``2 (2 kv_rank + rot_dim)``.  Such a step reads
 the requests' lengths on the host, so it is not captured into a CUDA graph
-(``capture_max_rows``).  An entry that reads another entry's cache (``entry.writes_cache`` false) has no
+(``capture_max_rows``) - unless nothing is cached yet: then the tokens are the step's rows (``capture_fresh``).  An entry that reads another entry's cache (``entry.writes_cache`` false) has no
 ``W_dkv`` of its own: it attends over that entry's latents and key parts with its own
 queries, ``W_uk`` and ``W_uv``.
 
@@ -105,6 +105,8 @@ class LatentAttention(Part):
         """Steps with more rows than this are launched kernel by kernel: the plain form lays out the
         requests' tokens from their lengths on the host."""
         return self.EXPAND_MIN_ROWS - 1 if self.can_expand else 1 << 30
+
+    capture_fresh = True       # a step in which every request begins reads no lengths on the host
 
     def cache_need(self) -> Optional[KvNeed]:
         return KvNeed(1, self.rank + self.rot, self.window, values=False)
@@ -243,6 +245,10 @@ class LatentAttention(Part):
         T, H = proj.shape[0], self.heads
         layouts = ctx.__dict__.setdefault("_latent_tokens", {})
         layout = layouts.get(self.window)
+        if layout is None and not any(ctx.h_req_prior):
+            # nothing cached yet: the tokens are the step's rows, and the layout is the step's own metadata on the device (a step of
+            # this kind may be captured: what it reads is what a replay finds there)
+            layout = layouts[self.window] = (ctx.req_start, ctx.row_req, ctx.positions, T)
         if layout is None:
             # the tokens of the step's requests, cached and new, that its rows see, request after request (shared by the
             # step's layers of one window); base: where a request's position 0 lies, or would lie
