@@ -601,12 +601,15 @@ __global__ void __launch_bounds__(128) scan_kernel(ScanArgs p, int DP, int TOK) 
 // by halving (each lane hands half of its values to its partner: DP - 1 shuffles for DP values instead of log2 DP for one), after which
 // every lane holds one finished value; and what needs no state is worked out for WALK_TOK tokens side by side, a lane a token.
 // Every float32 operation on a (column, token) is scan_kernel's, in its order - the partial sums over a lane's rows, the butterfly's
-// tree, the update - so a state or a row has the same bits whichever of the two walked it.  2,048 tokens of one prompt, before and now:
-// state-space, 64 heads of 128 x 64, 1,266 and 356 us; delta rule, 16 of 128 x 128, 1,412 and 565 us; gated linear attention, 4 of
-// 128 x 256, 1,214 and 427 us; matrix memory, 8 of 128 x 256, 1,488 and 369 us.  Two columns a thread: with one 20 to 35 % slower (twice
-// the loads), with four up to 60 % (too few warps).  What bounds it: latencies with one warp a scheduler; in the delta rule the
-// chain from one token's state to the next (four dependent shuffles).
-constexpr int WALK_TOK = 32, WALK_COLS = 2;
+// tree, the update - so a state or a row has the same bits whichever of the two walked it.  Half of a block's warps walk; the other half
+// fetch the next tokens and work out what needs no state (unit norms, gates, decays' exponentials), a batch ahead.  2,048 tokens of
+// one prompt, scan_kernel, this kernel with every warp doing both, and as it is: state-space, 64 heads of 128 x 64, 1,266, 356 and
+// 274 us; delta rule, 16 of 128 x 128, 1,412, 565 and 333 us; gated linear attention, 4 of 128 x 256, 1,214, 427 and 385 us;
+// matrix memory, 8 of 128 x 256, 1,488, 369 and 296 us.  Two columns a thread: with one 20 to 35 % slower (twice the loads), with
+// four up to 60 % (too few warps).  What bounds it: latencies with one walking warp a scheduler - in the delta rule the chain from one
+// token's state to the next (four dependent shuffles), in gated linear attention the 128 exponentials and logarithms a token.
+constexpr int WALK_COLS = 2, WALK_BUFS = 3;
+constexpr int walk_tok(int mode) { return mode == SCAN_GLA ? 16 : 32; }      // (with the decays staged too, 32 would leave an SM room for one block)
 
 // Sums of V values over the DP lanes that share a column; lane `part` is left, in v[0], with the value its bits name, the first
 // exchanged the most significant.  The order of the exchanges is scan_kernel's: neighbouring parts first, but with a whole warp a
@@ -631,8 +634,9 @@ template <int DP, int N, int STEP, int V> __device__ __forceinline__ void halve_
 }
 
 template <int DP, int NPER, int MODE, int C>
-__global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
+__global__ void __launch_bounds__(256, 1) walk_kernel(ScanArgs p) {
     constexpr bool DELTA = MODE == SCAN_DELTA;
+    constexpr int TOK = walk_tok(MODE);
     constexpr int NVEC = MODE == SCAN_GLA ? 3 : 2, ROWS = DP * NPER, CPW = 32 / DP, CB = 4 * CPW * C, U = DP / C, V = U * C;
     constexpr int OLD_CB = 4 * CPW;                                       // columns of a tile of the state's layout
     constexpr int TILE_FLOATS = MODE == SCAN_MLSTM ? (2 * NPER + 1) * 128 : NPER * 128;
@@ -640,58 +644,166 @@ __global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
     constexpr int OWN = (STRIDE + 127) / 128;
     cj::after_predecessor();
     cj::release_successor();
-    extern __shared__ __align__(16) float staged[];
+    extern __shared__ __align__(16) float staged[];         // WALK_BUFS batches of TOK tokens: one walked, one made ready, one landing
+    __shared__ float m_last;
     const int req = blockIdx.x, head = blockIdx.y;
     const int slot = p.req_slot[req];
     const int first = p.req_start[req], n = p.req_start[req + 1] - first;
     if (slot < 0 || n <= 0) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // threads 0-127 walk, threads 128-255 fetch the tokens and work out what needs no state; both count from 0
+    const bool walker = threadIdx.x < 128;
+    const int tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5;
     const int part = lane / CPW;
     const int lcol = warp * CPW * C + lane % CPW;                         // the thread's columns: lcol + CPW k of the block's
     const int col0 = blockIdx.z * CB;
     const int group = head / (p.heads / p.groups);
+    const int batches = (n + TOK - 1) / TOK;
+    const float A = MODE == SCAN_GLA ? 0.0f : (MODE == SCAN_MLSTM ? p.A_log[head] : expf(p.A_log[head]));
+    const float bias = MODE == SCAN_GLA ? 0.0f : p.dt_bias[head];
+    const int old_tiles = (p.cols + OLD_CB - 1) / OLD_CB;
 
-    // the sources of the entries of a staged token that this thread copies (entry tid + 128 k), for the request's first row; null: none
-    const float* src[OWN];
-    int ld[OWN];
-#pragma unroll
-    for (int k = 0; k < OWN; ++k) {
-        const int e = tid + 128 * k;
-        src[k] = nullptr;
-        ld[k] = p.ld;
-        const float* x = p.x + (size_t)first * p.ld;
-        const float* raw = p.raw + (size_t)first * p.ld_raw;
-        if (e < NVEC * ROWS) {
-            const int which = e / ROWS, v = e - which * ROWS, d = v / NPER + DP * (v % NPER);      // index part * NPER + i -> row part + DP i
-            if (which == 2) { src[k] = raw + p.off_dt + head * ROWS + d; ld[k] = p.ld_raw; }
-            else src[k] = x + (which == 0 ? p.off_a : p.off_b) + group * ROWS + d;
-        } else if (e < TAIL) {
-            const int c = col0 + e - NVEC * ROWS;
-            if (c < p.cols) src[k] = x + p.off_v + head * p.cols + c;
-        } else if (e == TAIL && MODE != SCAN_GLA) { src[k] = raw + p.off_dt + head; ld[k] = p.ld_raw; }
-        else if (e == TAIL + 1 && (DELTA || MODE == SCAN_MLSTM)) { src[k] = raw + p.off_beta + head; ld[k] = p.ld_raw; }
-    }
-    auto stage = [&](int t0, float* buf) {
-        const int nt = min(WALK_TOK, n - t0);
+    if (!walker) {
+        // the sources of the entries of a staged token that this thread copies (entry tid + 128 k), for the request's first row; null: none
+        const float* src[OWN];
+        int ld[OWN];
 #pragma unroll
         for (int k = 0; k < OWN; ++k) {
-            if (!src[k]) continue;
-            const float* s = src[k] + (size_t)t0 * ld[k];
-            float* d = buf + tid + 128 * k;
-#pragma unroll 4
-            for (int tt = 0; tt < nt; ++tt, s += ld[k], d += STRIDE) cp_async4(d, s);
+            const int e = tid + 128 * k;
+            src[k] = nullptr;
+            ld[k] = p.ld;
+            const float* x = p.x + (size_t)first * p.ld;
+            const float* raw = p.raw + (size_t)first * p.ld_raw;
+            if (e < NVEC * ROWS) {
+                const int which = e / ROWS, v = e - which * ROWS, d = v / NPER + DP * (v % NPER);      // index part * NPER + i -> row part + DP i
+                if (which == 2) { src[k] = raw + p.off_dt + head * ROWS + d; ld[k] = p.ld_raw; }
+                else src[k] = x + (which == 0 ? p.off_a : p.off_b) + group * ROWS + d;
+            } else if (e < TAIL) {
+                const int c = col0 + e - NVEC * ROWS;
+                if (c < p.cols) src[k] = x + p.off_v + head * p.cols + c;
+            } else if (e == TAIL && MODE != SCAN_GLA) { src[k] = raw + p.off_dt + head; ld[k] = p.ld_raw; }
+            else if (e == TAIL + 1 && (DELTA || MODE == SCAN_MLSTM)) { src[k] = raw + p.off_beta + head; ld[k] = p.ld_raw; }
         }
-    };
-    // columns past the last read as zero in every staged token
-    for (int i = tid; i < 2 * WALK_TOK * CB; i += 128) {
-        const int t = i / CB, c = i - t * CB;
-        if (col0 + c >= p.cols) staged[t * STRIDE + NVEC * ROWS + c] = 0.0f;
+        auto stage = [&](int t0, float* buf) {
+            const int nt = min(TOK, n - t0);
+#pragma unroll
+            for (int k = 0; k < OWN; ++k) {
+                if (!src[k]) continue;
+                const float* s = src[k] + (size_t)t0 * ld[k];
+                float* d = buf + tid + 128 * k;
+#pragma unroll 4
+                for (int tt = 0; tt < nt; ++tt, s += ld[k], d += STRIDE) cp_async4(d, s);
+            }
+        };
+        auto prepare_sync = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };      // the fetching threads alone
+        float m_run = 0.0f;
+        if (MODE == SCAN_MLSTM) {
+            // every tile and thread of the layout holds the maximum; this block's first tile is its own, whatever a thread's columns
+            m_run = p.state[(size_t)slot * p.slot_stride + ((size_t)head * old_tiles + col0 / OLD_CB) * TILE_FLOATS + 2 * NPER * 128];
+        }
+        auto prepare = [&](int batch) {
+            float* cur = staged + batch % WALK_BUFS * TOK * STRIDE;
+            const int nt = min(TOK, n - batch * TOK);
+            // what needs no state
+            if (DELTA) {
+                // unit vectors: a warp sums a token's squares (eight tokens a warp, their butterflies side by side)
+#pragma unroll 2
+                for (int tt = warp; tt < nt; tt += 4) {
+                    float* tk = cur + tt * STRIDE;
+                    float qq = 0.0f, kk = 0.0f;
+#pragma unroll
+                    for (int d = 0; d < ROWS; d += 32)
+                        if (d + lane < ROWS) {
+                            qq = fmaf(tk[d + lane], tk[d + lane], qq);
+                            kk = fmaf(tk[ROWS + d + lane], tk[ROWS + d + lane], kk);
+                        }
+                    qq = warp_sum(qq);
+                    kk = warp_sum(kk);
+                    const float qs = p.q_scale / sqrtf(qq + 1e-6f), ks = 1.0f / sqrtf(kk + 1e-6f);
+#pragma unroll
+                    for (int d = 0; d < ROWS; d += 32)
+                        if (d + lane < ROWS) {
+                            tk[d + lane] *= qs;
+                            tk[ROWS + d + lane] *= ks;
+                        }
+                }
+                if (tid < nt) {
+                    float* tk = cur + tid * STRIDE + TAIL;
+                    tk[0] = expf(-A * softplus_f(tk[0] + bias));                                   // the decay
+                    tk[1] = sigmoid_f(tk[1]);                                                      // beta
+                }
+            } else if (MODE == SCAN_GLA) {
+#pragma unroll 4
+                for (int e = tid; e < nt * ROWS; e += 128) {
+                    float* tk = cur + (e / ROWS) * STRIDE + e % ROWS;
+                    tk[0] *= p.q_scale;
+                    tk[2 * ROWS] = expf(log_sigmoid_f(tk[2 * ROWS]) * p.c0);
+                }
+            } else if (MODE == SCAN_MLSTM) {
+                float li = 0.0f, lf = 0.0f;
+                if (warp == 0) {
+                    // the running maximum, token after token in every lane; a lane keeps its own token's
+                    if (lane < nt) {
+                        const float* tk = cur + lane * STRIDE + TAIL;
+                        li = p.c0 * tanhf((tk[0] + bias) / p.c0);                                  // log of the input gate
+                        lf = log_sigmoid_f(p.c0 * tanhf((tk[1] + A) / p.c0));                      // log of the forget gate
+                    }
+                    float m = m_run, before = m_run, after = m_run;
+                    for (int tt = 0; tt < nt; ++tt) {
+                        const float i = __shfl_sync(0xffffffffu, li, tt), f = __shfl_sync(0xffffffffu, lf, tt);
+                        const float mn = fmaxf(f + m, i);
+                        if (lane == tt) { before = m; after = mn; }
+                        m = mn;
+                    }
+                    if (lane < nt) {
+                        float* tk = cur + lane * STRIDE + TAIL;
+                        tk[0] = expf(lf + before - after);                                         // keep
+                        tk[1] = expf(li - after);                                                  // take
+                        tk[2] = expf(-after);
+                        tk[3] = after;
+                    }
+                }
+                prepare_sync();
+                m_run = cur[(nt - 1) * STRIDE + TAIL + 3];
+                if (tid == 0 && batch == batches - 1) m_last = m_run;
+#pragma unroll 4
+                for (int e = tid; e < nt * ROWS; e += 128) {
+                    float* tk = cur + (e / ROWS) * STRIDE;
+                    tk[e % ROWS] *= p.q_scale;
+                    tk[ROWS + e % ROWS] *= tk[TAIL + 1];
+                }
+            } else if (tid < nt) {
+                float* tk = cur + tid * STRIDE + TAIL;
+                const float dt = softplus_f(tk[0] + bias);
+                tk[0] = dt;
+                tk[1] = expf(-A * dt);
+            }
+        };
+        // columns past the last read as zero in every staged token
+        for (int i = tid; i < WALK_BUFS * TOK * CB; i += 128) {
+            const int t = i / CB, c = i - t * CB;
+            if (col0 + c >= p.cols) staged[t * STRIDE + NVEC * ROWS + c] = 0.0f;
+        }
+        stage(0, staged);
+        cp_async_commit();
+        if (batches > 1) stage(TOK, staged + TOK * STRIDE);
+        cp_async_commit();
+        cp_async_wait<1>();
+        prepare_sync();
+        prepare(0);
+        for (int batch = 0; batch < batches; ++batch) {
+            __syncthreads();                    // batch is ready, and the one before it walked: its buffer takes the one after next
+            if (batch + 2 < batches) stage((batch + 2) * TOK, staged + (batch + 2) % WALK_BUFS * TOK * STRIDE);
+            cp_async_commit();
+            if (batch + 1 < batches) {
+                cp_async_wait<1>();
+                prepare_sync();
+                prepare(batch + 1);
+            }
+        }
+        return;
     }
-    stage(0, staged);
-    cp_async_commit();
 
     // the state, in scan_kernel's layout: (tile of OLD_CB columns, i, thread of that kernel)
-    const int old_tiles = (p.cols + OLD_CB - 1) / OLD_CB;
     float* S[C];
     bool live[C];
     float s[C][NPER];
@@ -704,16 +816,11 @@ __global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
 #pragma unroll
         for (int i = 0; i < NPER; ++i) s[k][i] = live[k] ? S[k][i * 128] : 0.0f;
     }
-    const float A = MODE == SCAN_GLA ? 0.0f : (MODE == SCAN_MLSTM ? p.A_log[head] : expf(p.A_log[head]));
-    const float bias = MODE == SCAN_GLA ? 0.0f : p.dt_bias[head];
     const float skip = MODE == SCAN_SSD ? p.skip[head] : 0.0f;
     float nvec[MODE == SCAN_MLSTM ? NPER : 1];
-    float m_run = 0.0f;
     if (MODE == SCAN_MLSTM) {
 #pragma unroll
         for (int i = 0; i < NPER; ++i) nvec[i] = live[0] ? S[0][(NPER + i) * 128] : 0.0f;
-        // every tile and thread of the layout holds the maximum; this block's first tile is its own, whatever a thread's columns
-        m_run = p.state[(size_t)slot * p.slot_stride + ((size_t)head * old_tiles + col0 / OLD_CB) * TILE_FLOATS + 2 * NPER * 128];
     }
     // which finished value a lane is left with: token `my_u` of the batch, column `my_k` of the thread's
     int my = 0;
@@ -724,85 +831,10 @@ __global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
     const size_t out_ld = (size_t)p.heads * p.cols;
     const bool writer = col0 + my_col < p.cols;
 
-    for (int t0 = 0, which = 0; t0 < n; t0 += WALK_TOK, which ^= 1) {
-        float* cur = staged + which * WALK_TOK * STRIDE;
-        if (t0 + WALK_TOK < n) stage(t0 + WALK_TOK, staged + (which ^ 1) * WALK_TOK * STRIDE);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const int nt = min(WALK_TOK, n - t0);
-        // what needs no state
-        if (DELTA) {
-            // unit vectors: a warp sums a token's squares (eight tokens a warp, their butterflies side by side)
-#pragma unroll 2
-            for (int tt = warp; tt < nt; tt += 4) {
-                float* tk = cur + tt * STRIDE;
-                float qq = 0.0f, kk = 0.0f;
-#pragma unroll
-                for (int d = 0; d < ROWS; d += 32)
-                    if (d + lane < ROWS) {
-                        qq = fmaf(tk[d + lane], tk[d + lane], qq);
-                        kk = fmaf(tk[ROWS + d + lane], tk[ROWS + d + lane], kk);
-                    }
-                qq = warp_sum(qq);
-                kk = warp_sum(kk);
-                const float qs = p.q_scale / sqrtf(qq + 1e-6f), ks = 1.0f / sqrtf(kk + 1e-6f);
-#pragma unroll
-                for (int d = 0; d < ROWS; d += 32)
-                    if (d + lane < ROWS) {
-                        tk[d + lane] *= qs;
-                        tk[ROWS + d + lane] *= ks;
-                    }
-            }
-            if (tid < nt) {
-                float* tk = cur + tid * STRIDE + TAIL;
-                tk[0] = expf(-A * softplus_f(tk[0] + bias));                                   // the decay
-                tk[1] = sigmoid_f(tk[1]);                                                      // beta
-            }
-        } else if (MODE == SCAN_GLA) {
-            for (int e = tid; e < nt * ROWS; e += 128) {
-                float* tk = cur + (e / ROWS) * STRIDE + e % ROWS;
-                tk[0] *= p.q_scale;
-                tk[2 * ROWS] = expf(log_sigmoid_f(tk[2 * ROWS]) * p.c0);
-            }
-        } else if (MODE == SCAN_MLSTM) {
-            float li = 0.0f, lf = 0.0f;
-            if (warp == 0) {
-                // the running maximum, token after token in every lane; a lane keeps its own token's
-                if (lane < nt) {
-                    const float* tk = cur + lane * STRIDE + TAIL;
-                    li = p.c0 * tanhf((tk[0] + bias) / p.c0);                                  // log of the input gate
-                    lf = log_sigmoid_f(p.c0 * tanhf((tk[1] + A) / p.c0));                      // log of the forget gate
-                }
-                float m = m_run, before = m_run, after = m_run;
-                for (int tt = 0; tt < nt; ++tt) {
-                    const float i = __shfl_sync(0xffffffffu, li, tt), f = __shfl_sync(0xffffffffu, lf, tt);
-                    const float mn = fmaxf(f + m, i);
-                    if (lane == tt) { before = m; after = mn; }
-                    m = mn;
-                }
-                if (lane < nt) {
-                    float* tk = cur + lane * STRIDE + TAIL;
-                    tk[0] = expf(lf + before - after);                                         // keep
-                    tk[1] = expf(li - after);                                                  // take
-                    tk[2] = expf(-after);
-                    tk[3] = after;
-                }
-            }
-            __syncthreads();
-            m_run = cur[(nt - 1) * STRIDE + TAIL + 3];
-            for (int e = tid; e < nt * ROWS; e += 128) {
-                float* tk = cur + (e / ROWS) * STRIDE;
-                tk[e % ROWS] *= p.q_scale;
-                tk[ROWS + e % ROWS] *= tk[TAIL + 1];
-            }
-        } else if (tid < nt) {
-            float* tk = cur + tid * STRIDE + TAIL;
-            const float dt = softplus_f(tk[0] + bias);
-            tk[0] = dt;
-            tk[1] = expf(-A * dt);
-        }
-        __syncthreads();
+    for (int batch = 0; batch < batches; ++batch) {
+        const float* cur = staged + batch % WALK_BUFS * TOK * STRIDE;
+        const int t0 = batch * TOK, nt = min(TOK, n - t0);
+        __syncthreads();                        // the batch is ready
         auto walk = [&](int b0, int nu, auto whole) {
             constexpr bool WHOLE = decltype(whole)::value;
             float y[V], nq[U];
@@ -914,7 +946,6 @@ __global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
 #pragma unroll 1
         for (; b0 + U <= nt; b0 += U) walk(b0, U, std::true_type{});
         if (b0 < nt) walk(b0, nt - b0, std::false_type{});
-        __syncthreads();                                                  // everyone has walked this buffer before it is staged into again
     }
 #pragma unroll
     for (int k = 0; k < C; ++k) {
@@ -924,7 +955,7 @@ __global__ void __launch_bounds__(128) walk_kernel(ScanArgs p) {
         if (MODE == SCAN_MLSTM) {
 #pragma unroll
             for (int i = 0; i < NPER; ++i) S[k][(NPER + i) * 128] = nvec[i];
-            S[k][2 * NPER * 128] = m_run;
+            S[k][2 * NPER * 128] = m_last;        // (written before the last barrier)
         }
     }
 }
@@ -1360,24 +1391,32 @@ CJ_EXPORT int cj_short_conv_commit(const float* in, int ld_in, int C, int taps, 
 //         forget gate's; c0 = the gates' cap, c1 = the floor added to the read-out's divisor).
 static long long scan_tile_floats(int mode, int nper) { return mode == 3 ? (long long)(2 * nper + 1) * 128 : (long long)nper * 128; }
 
-// Tokens a request, on average over the step, from which on walk_kernel takes over: at 4 tokens for each of 8 requests it takes 12.5 us
-// against scan_kernel's 18 (state-space, 64 heads of 128 x 64) and 13.5 against 18 (delta rule, 16 of 128 x 128); with one token a
-// request most of a batch would be empty.
-constexpr int WALK_MIN_ROWS = 4;
+// Tokens a request, on average over the step, from which on walk_kernel takes over: at 8 tokens for each of 8 requests it takes 18, 27,
+// 17 and 19 us against scan_kernel's 27, 29, 30 and 30 (the four modes at the sizes above); at 4 the delta rule takes 24 against 18.
+constexpr int WALK_MIN_ROWS = 8;
 
 template <int DP, int NPER, int MODE, int C>
 static int launch_walk_as(const ScanArgs& p, int requests, cudaStream_t stream) {
     constexpr int CB = 4 * (32 / DP) * C;
-    constexpr int bytes = 2 * WALK_TOK * ((MODE == SCAN_GLA ? 3 : 2) * DP * NPER + CB + 4) * (int)sizeof(float);
+    constexpr int bytes = WALK_BUFS * walk_tok(MODE) * ((MODE == SCAN_GLA ? 3 : 2) * DP * NPER + CB + 4) * (int)sizeof(float);
+    // more than half of an SM's shared memory: one block an SM
+    constexpr int alone = bytes > 116 * 1024 ? bytes : 116 * 1024;
     static bool sized = false;
+    static int sms = 0;
     if (!sized) {
-        cudaError_t e = cudaFuncSetAttribute(walk_kernel<DP, NPER, MODE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaError_t e = cudaFuncSetAttribute(walk_kernel<DP, NPER, MODE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, alone);
+        int dev = 0;
+        if (e == cudaSuccess) e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return (int)e;
         sized = true;
     }
     const dim3 grid(requests, p.heads, (p.cols + CB - 1) / CB);
     if (grid.z > 65535) return CJ_ERR_SIZE;
-    cj::launch(walk_kernel<DP, NPER, MODE, C>, grid, dim3(128), bytes, stream, p);
+    // A grid that the machine holds a block an SM is made to spread: set up while the kernel before still runs, two of its blocks may
+    // otherwise land on one SM, and the scan takes as long as those two (64 heads of 128 x 64, 2,048 tokens: 650 us instead of 274).
+    const bool spread = (long long)grid.x * grid.y * grid.z <= sms;
+    cj::launch(walk_kernel<DP, NPER, MODE, C>, grid, dim3(256), spread ? alone : bytes, stream, p);
     return launch_status();
 }
 
