@@ -263,7 +263,191 @@ __global__ void __launch_bounds__(LA_HEADS * 32) latent_attention_kernel(
     }
 }
 
-// the stretches of a row's keys, merged in order: out = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z
+// The same for a bfloat16 cache whose entries are whole 16-byte pieces (rank a multiple of 64 up to 1,024, width of 8).  There a
+// warp scored 32 keys for its one head, three shared-memory reads for two multiply-adds, and a chunk came in nine round trips; here a
+// chunk's pieces are all sent for at once (cp.async, the next chunk's while this one is used), a warp takes an eighth of the entry for
+// all 8 heads (17 16-byte reads for 64 multiply-adds; lane j: key j), the warps' shares of a score meet in shared memory, warp h
+// keeps head h's maximum and sum, and for the weighted sum a warp takes 64 entries of every 512 of the latent, again for all
+// heads.  Rank 512, with the merge: 4 rows of 16 heads at 620 keys 30 -> 19 us, 8 of 32 at 520 40 -> 24, 64 of 16 at 520 122 -> 70,
+// 8 of 16 at 3,000 107 -> 59.  Bound by shared memory: 3 us a chunk of 32 keys and 8 heads.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+
+template <int NI>      // 512-entry pieces of the latent
+__global__ void __launch_bounds__(LA_HEADS * 32) latent_attention_tile_kernel(
+    const float* __restrict__ q_abs, const float* __restrict__ q_rot, const __nv_bfloat16* __restrict__ plane, int rank, int rot,
+    int heads, int T, const int* __restrict__ positions, const int* __restrict__ row_req, const int* __restrict__ table,
+    int table_stride, int page_tokens, int window, float scale, __nv_bfloat16* __restrict__ out, int split_keys,
+    float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ sink) {
+    cj::after_predecessor();
+    cj::release_successor();
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int width = rank + rot, pieces = width / 8, row_bytes = width * 2 + 16;      // (8 lanes reading 16 bytes of 8 keys: 32 banks)
+    float* qs = (float*)smem;                                   // [LA_HEADS][width]
+    float* sp = qs + LA_HEADS * width;                          // [warp][LA_HEADS][LA_KEYS]: the warps' shares of the scores
+    float* ps = sp + 8 * LA_HEADS * LA_KEYS;                    // [LA_KEYS][LA_HEADS]: weights
+    float* cs = ps + LA_KEYS * LA_HEADS;                        // [LA_HEADS]: the sums' factor; at the end 1 / l
+    unsigned char* ks = (unsigned char*)(cs + LA_HEADS);        // [2][LA_KEYS][row_bytes]
+    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int head0 = blockIdx.y * LA_HEADS;
+    const int pos = positions[r];
+    const int oldest = window > 0 ? max(0, pos + 1 - window) : 0;
+    const int key_begin = oldest + (split_keys > 0 ? (int)blockIdx.z * split_keys : 0);
+    const int key_end = split_keys > 0 ? min(pos + 1, key_begin + split_keys) : pos + 1;
+    if (key_begin >= key_end) return;                           // this stretch lies past the row's position
+    const int* pages = table + (size_t)row_req[r] * table_stride;
+    // a thread copies pieces tid & 7, + 8, ... of key tid / 8
+    auto fetch = [&](int k0, unsigned char* to) {
+        const int j = tid >> 3;
+        if (k0 + j < key_end) {
+            const int kp = k0 + j;
+            const unsigned char* src = (const unsigned char*)(plane + ((size_t)pages[kp / page_tokens] * page_tokens + kp % page_tokens) * width);
+            for (int u = tid & 7; u < pieces; u += 8) cp_async16(to + j * row_bytes + 16 * u, src + 16 * u);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the queries travel with the first chunk: warp h fetches head h's
+    if (head0 + warp < heads) {
+        const float* qa = q_abs + ((size_t)(head0 + warp) * T + r) * rank;
+        const float* qr = q_rot + ((size_t)r * heads + head0 + warp) * rot;
+        for (int e = 4 * lane; e < width; e += 128) cp_async16(qs + warp * width + e, e < rank ? qa + e : qr + e - rank);
+    } else {
+        for (int e = lane; e < width; e += 32) qs[warp * width + e] = 0.0f;
+    }
+    fetch(key_begin, ks);
+    float acc[NI][LA_HEADS][2];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int h = 0; h < LA_HEADS; ++h) acc[i][h][0] = acc[i][h][1] = 0.0f;
+    float m = -INFINITY, l = 0.0f;                              // warp h: head head0 + h
+    if (sink && head0 + warp < heads && key_begin == oldest) { m = sink[head0 + warp]; l = 1.0f; }
+    int at = 0;
+    for (int k0 = key_begin; k0 < key_end; k0 += LA_KEYS, at ^= 1) {
+        const int n_keys = min(LA_KEYS, key_end - k0);
+        const unsigned char* kc = ks + at * LA_KEYS * row_bytes;
+        if (k0 + LA_KEYS < key_end) {
+            fetch(k0 + LA_KEYS, ks + (at ^ 1) * LA_KEYS * row_bytes);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        float s[LA_HEADS];
+#pragma unroll
+        for (int h = 0; h < LA_HEADS; ++h) s[h] = 0.0f;
+        for (int u = warp; u < pieces; u += 8) {
+            const uint4 k4 = *(const uint4*)(kc + lane * row_bytes + 16 * u);       // (a key past the stretch: whatever the buffer held; not used)
+            const uint32_t kw[4] = {k4.x, k4.y, k4.z, k4.w};
+            float kf[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { kf[2 * i] = __uint_as_float(kw[i] << 16); kf[2 * i + 1] = __uint_as_float(kw[i] & 0xffff0000u); }
+#pragma unroll
+            for (int h = 0; h < LA_HEADS; ++h) {
+                const float4 a = *(const float4*)(qs + h * width + 8 * u), b = *(const float4*)(qs + h * width + 8 * u + 4);
+                s[h] = fmaf(a.x, kf[0], s[h]); s[h] = fmaf(a.y, kf[1], s[h]); s[h] = fmaf(a.z, kf[2], s[h]); s[h] = fmaf(a.w, kf[3], s[h]);
+                s[h] = fmaf(b.x, kf[4], s[h]); s[h] = fmaf(b.y, kf[5], s[h]); s[h] = fmaf(b.z, kf[6], s[h]); s[h] = fmaf(b.w, kf[7], s[h]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < LA_HEADS; ++h) sp[(warp * LA_HEADS + h) * LA_KEYS + lane] = s[h];
+        __syncthreads();
+        {
+            float dot = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) dot += sp[(w * LA_HEADS + warp) * LA_KEYS + lane];
+            const float sc = lane < n_keys ? dot * scale : -INFINITY;
+            const float m_new = fmaxf(m, warp_max(sc));
+            const float pj = lane < n_keys ? expf(sc - m_new) : 0.0f;
+            const float corr = expf(m - m_new);                 // 0 on the first chunk (m = -inf)
+            l = l * corr + warp_sum(pj);
+            m = m_new;
+            ps[lane * LA_HEADS + warp] = pj;
+            if (lane == 0) cs[warp] = corr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < LA_HEADS; ++h) {
+            const float corr = cs[h];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) { acc[i][h][0] *= corr; acc[i][h][1] *= corr; }
+        }
+#pragma unroll 4
+        for (int j = 0; j < n_keys; ++j) {
+            const float4 p0 = *(const float4*)(ps + j * LA_HEADS), p1 = *(const float4*)(ps + j * LA_HEADS + 4);
+            const float pw[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int e = 512 * i + 64 * warp + 2 * lane;
+                if (NI > 1 || rank < 512) if (e >= rank) continue;
+                const uint32_t w2 = *(const uint32_t*)(kc + j * row_bytes + 2 * e);
+                const float lo = __uint_as_float(w2 << 16), hi = __uint_as_float(w2 & 0xffff0000u);
+#pragma unroll
+                for (int h = 0; h < LA_HEADS; ++h) {
+                    acc[i][h][0] = fmaf(pw[h], lo, acc[i][h][0]);
+                    acc[i][h][1] = fmaf(pw[h], hi, acc[i][h][1]);
+                }
+            }
+        }
+        __syncthreads();                                        // the chunk, its weights and factors have been used
+    }
+    if (lane == 0) cs[warp] = 1.0f / l;
+    __syncthreads();
+    if (part_acc && lane == 0 && head0 + warp < heads) {
+        float* ml = part_ml + (((size_t)r * heads + head0 + warp) * gridDim.z + blockIdx.z) * 2;
+        ml[0] = m;
+        ml[1] = l;
+    }
+#pragma unroll
+    for (int h = 0; h < LA_HEADS; ++h) {
+        if (head0 + h >= heads) break;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int e = 512 * i + 64 * warp + 2 * lane;
+            if (e >= rank) continue;
+            if (part_acc)
+                *(float2*)(part_acc + (((size_t)r * heads + head0 + h) * gridDim.z + blockIdx.z) * rank + e) = make_float2(acc[i][h][0], acc[i][h][1]);
+            else
+                *(__nv_bfloat162*)(out + ((size_t)(head0 + h) * T + r) * rank + e) = __floats2bfloat162_rn(acc[i][h][0] * cs[h], acc[i][h][1] * cs[h]);
+        }
+    }
+}
+
+// the stretches of a row's keys, merged in order: out = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z.  The stretches' factors are worked
+// out side by side, a thread each, and the sums read four stretches at a time.
+constexpr int MERGE_MOST = 128;
+template <typename TC>
+__global__ void __launch_bounds__(MERGE_MOST) latent_merge_few_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits,
+                                                                       int split_keys, int window, int rank, int heads, int T,
+                                                                       const int* __restrict__ positions, TC* __restrict__ out) {
+    cj::after_predecessor();
+    cj::release_successor();
+    __shared__ float f[MERGE_MOST], top[4], sum[4];
+    const int r = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5;
+    const int n_keys = window > 0 ? min(positions[r] + 1, window) : positions[r] + 1;
+    const int nz = min(splits, (n_keys + split_keys - 1) / split_keys);
+    const size_t item = (size_t)r * heads + head;
+    const float2 ml = tid < nz ? *(const float2*)(part_ml + (item * splits + tid) * 2) : make_float2(-INFINITY, 0.0f);
+    const float wm = warp_max(ml.x);
+    if ((tid & 31) == 0) top[warp] = wm;
+    __syncthreads();
+    const float M = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+    const float e = tid < nz ? expf(ml.x - M) : 0.0f;
+    f[tid] = e;
+    const float ws = warp_sum(e * ml.y);
+    if ((tid & 31) == 0) sum[warp] = ws;
+    __syncthreads();
+    const float inv = 1.0f / ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+    const float* acc = part_acc + item * splits * rank;
+    for (int c = tid; c < rank; c += MERGE_MOST) {
+        float v = 0.0f;
+#pragma unroll 4
+        for (int z = 0; z < nz; ++z) v = fmaf(f[z], acc[(size_t)z * rank + c], v);
+        out[((size_t)head * T + r) * rank + c] = from_f32<TC>(v * inv);
+    }
+}
+
 template <typename TC>
 __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits, int split_keys,
                                     int window, int rank, int heads, int T, const int* __restrict__ positions, TC* __restrict__ out) {
@@ -390,10 +574,38 @@ CJ_EXPORT int cj_latent_attention(const float* q_abs, const float* q_rot, const 
         cj::launch(latent_attention_kernel<TC, N>, grid, dim3(LA_HEADS * 32), smem, stream, q_abs, q_rot, (const TC*)plane, \
                    rank, rot, heads, T, positions, row_req, table, table_stride, page_tokens, window, scale, (TC*)out, row_words, \
                    split_keys, pa, pm, sink);                                                                          \
-        if (split_keys > 0)                                                                                            \
-            cj::launch(latent_merge_kernel<TC>, dim3(T, heads), dim3(128), 0, stream, (const float*)pa, (const float*)pm, splits, \
-                       split_keys, window, rank, heads, T, positions, (TC*)out);                                               \
+        MERGE(TC);                                                                                                     \
     } while (0)
+#define MERGE(TC)                                                                                                      \
+    do {                                                                                                               \
+        if (split_keys > 0 && splits <= MERGE_MOST)                                                                    \
+            cj::launch(latent_merge_few_kernel<TC>, dim3(T, heads), dim3(MERGE_MOST), 0, stream, (const float*)pa, (const float*)pm, splits, \
+                       split_keys, window, rank, heads, T, positions, (TC*)out);                                       \
+        else if (split_keys > 0)                                                                                       \
+            cj::launch(latent_merge_kernel<TC>, dim3(T, heads), dim3(128), 0, stream, (const float*)pa, (const float*)pm, splits, \
+                       split_keys, window, rank, heads, T, positions, (TC*)out);                                       \
+    } while (0)
+    // a bfloat16 cache of 16-byte pieces
+    const size_t tile_smem = (size_t)LA_HEADS * width * 4 + (8 * LA_HEADS * LA_KEYS + LA_KEYS * LA_HEADS + LA_HEADS) * 4 + 2 * (size_t)LA_KEYS * (width * 2 + 16);
+    if (cache_dtype == CJ_BF16 && rank % 64 == 0 && width % 8 == 0 && tile_smem <= 200 * 1024 && (((uintptr_t)plane | (uintptr_t)out | (uintptr_t)q_abs | (uintptr_t)q_rot) & 15) == 0
+        && (((uintptr_t)pa | (uintptr_t)pm) & 15) == 0) {
+#define LAUNCH_TILE(NI)                                                                                                \
+        do {                                                                                                           \
+            static bool sized = false;                                                                                 \
+            if (!sized) {                                                                                              \
+                cudaFuncSetAttribute(latent_attention_tile_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
+                sized = true;                                                                                          \
+            }                                                                                                          \
+            cj::launch(latent_attention_tile_kernel<NI>, grid, dim3(LA_HEADS * 32), tile_smem, stream, q_abs, q_rot, (const __nv_bfloat16*)plane, \
+                       rank, rot, heads, T, positions, row_req, table, table_stride, page_tokens, window, scale, (__nv_bfloat16*)out, split_keys, \
+                       pa, pm, sink);                                                                                  \
+        } while (0)
+        if (rank <= 512) LAUNCH_TILE(1);
+        else LAUNCH_TILE(2);
+#undef LAUNCH_TILE
+        MERGE(__nv_bfloat16);
+        return launch_status();
+    }
 #define PICK(TC)                                  \
     do {                                          \
         if (nacc <= 4) LAUNCH(TC, 4);             \
@@ -406,6 +618,7 @@ CJ_EXPORT int cj_latent_attention(const float* q_abs, const float* q_rot, const 
     else return CJ_ERR_DTYPE;
 #undef PICK
 #undef LAUNCH
+#undef MERGE
     return launch_status();
 }
 
