@@ -11,17 +11,18 @@
 //
 // The prompt form keeps a thread on 4 rows x 4 keys of the scores and 4 rows x 8 entries of the output, operands as float4 from
 // shared memory (12 shared-memory wavefronts a 16 FMA clocks): bound by the FMA pipe and by waiting for a chunk's keys, which nothing
-// fetches ahead but the SM's other block.  1,777 rows of one prompt, 16 heads of 128: 961 us, where a row and head a block with a
+// fetches ahead but the SM's other block.  1,777 rows of one prompt, 16 heads of 128: 735 us, where a row and head a block with a
 // key a lane took 12,700 us.  One row at 570 keys: 34 us, 120 us before.
 #define CJ_LIB "attention_f32"
 #include "common.cuh"
+
+#include <type_traits>
 
 using namespace cj;
 
 namespace {
 
-constexpr int KEYS = 64, ROWS = 64, MAX_DIM = 128;
-constexpr int TILE_THREADS = 256, ROW_WARPS = 8;
+constexpr int KEYS = 64, MAX_DIM = 128, ROW_WARPS = 8;
 
 struct Args {
     const float* q; float* out; const float* kplane; const float* vplane;
@@ -51,9 +52,10 @@ __device__ __forceinline__ float gate_of(const Args& p, int row, int head) {
     return p.head_gate ? 1.0f / (1.0f + expf(-p.head_gate[(size_t)row * p.gate_ld + head])) : 1.0f;
 }
 
-// VC: float4 of the output a thread holds per row (values of up to 64 VC entries)
-template <int VC>
-__global__ void __launch_bounds__(TILE_THREADS, 2) attention_f32_tile_kernel(const Args p) {
+// VC: float4 of the output a thread holds per row (values of up to 64 VC entries); ROWS: rows of a tile, 64 or 32
+template <int VC, int ROWS>
+__global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const Args p) {
+    constexpr int TILE_THREADS = 4 * ROWS;
     cj::after_predecessor();
     cj::release_successor();
     extern __shared__ __align__(16) float smem[];
@@ -194,35 +196,40 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) attention_f32_tile_kernel(con
                 for (int e = 0; e < 4; ++e) o[i][c][e] = 0.0f;
         // whether every row of the tile sees every key of the chunk
         const bool all = k0 + KEYS - 1 <= pos0 && k0 >= first_key(last, p.window);
+        auto values = [&](auto whole) {
+            constexpr bool ALL = decltype(whole)::value;
 #pragma unroll 1
-        for (int k = 0; k < KEYS; k += 4) {
-            float4 w[4];
+            for (int k = 0; k < KEYS; k += 4) {
+                float4 w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(Ps + (4 * ty + i) * (KEYS + 4) + k);
+                for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(Ps + (4 * ty + i) * (KEYS + 4) + k);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                float4 v[VC];
+                for (int kk = 0; kk < 4; ++kk) {
+                    float4 v[VC];
 #pragma unroll
-                for (int c = 0; c < VC; ++c) {
-                    const int d = 4 * tx + 64 * c;
-                    v[c] = d < p.vd ? *(const float4*)(Vs + (k + kk) * p.vd + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
+                    for (int c = 0; c < VC; ++c) {
+                        const int d = 4 * tx + 64 * c;
+                        v[c] = d < p.vd ? *(const float4*)(Vs + (k + kk) * p.vd + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                    const int key = k0 + k + kk, pos = pos0 + 4 * ty + i;
-                    if (all || (key <= pos && key >= first_key(pos, p.window))) {
+                    for (int i = 0; i < 4; ++i) {
+                        const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                        const int key = k0 + k + kk, pos = pos0 + 4 * ty + i;
+                        if (ALL || (key <= pos && key >= first_key(pos, p.window))) {
 #pragma unroll
-                        for (int c = 0; c < VC; ++c) {
-                            o[i][c][0] = fmaf(e, v[c].x, o[i][c][0]);
-                            o[i][c][1] = fmaf(e, v[c].y, o[i][c][1]);
-                            o[i][c][2] = fmaf(e, v[c].z, o[i][c][2]);
-                            o[i][c][3] = fmaf(e, v[c].w, o[i][c][3]);
+                            for (int c = 0; c < VC; ++c) {
+                                o[i][c][0] = fmaf(e, v[c].x, o[i][c][0]);
+                                o[i][c][1] = fmaf(e, v[c].y, o[i][c][1]);
+                                o[i][c][2] = fmaf(e, v[c].z, o[i][c][2]);
+                                o[i][c][3] = fmaf(e, v[c].w, o[i][c][3]);
+                            }
                         }
                     }
                 }
             }
-        }
+        };
+        if (all) values(std::true_type{});         // (the test a row and key is what the other chunks pay for)
+        else values(std::false_type{});
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int pos = pos0 + 4 * ty + i;
@@ -335,11 +342,11 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
 
 // Arguments as cj_paged_attention's, float32 throughout; req_start [requests + 1]: the step's rows by request (neighbouring rows of a
 // request at neighbouring positions), or null: every row goes by itself.  tiles: an upper bound of the 64-row tiles of the
-// requests with more than few_rows rows, 0 for none; singles: whether a request has at most few_rows rows.
+// requests with more than few_rows rows, 0 for none, tiles32 the same of 32 rows; singles: whether a request has at most few_rows rows.
 CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, const float* vplane, const int* positions, const int* row_req,
                                const int* req_start, int requests, const int* table, int table_stride, int page_tokens, int T, int n_heads,
                                int n_kv, int hd, int vd, int window, float scale, float softcap, const float* head_gate, int gate_ld,
-                               float sink, int few_rows, int tiles, int singles, cudaStream_t stream) {
+                               float sink, int few_rows, int tiles, int tiles32, int singles, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (!q || !out || !kplane || !vplane || !positions || !row_req || !table || (tiles > 0 && !req_start)) return CJ_ERR_ARG;
     if (hd <= 0 || hd > MAX_DIM || hd % 4 != 0 || vd <= 0 || vd > MAX_DIM || vd % 4 != 0) return CJ_ERR_SIZE;
@@ -348,16 +355,18 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
     Args a{q, out, kplane, vplane, positions, row_req, req_start, requests, table, table_stride, page_tokens, n_heads, n_kv, hd, vd, window,
            scale, softcap, head_gate, gate_ld, sink, few_rows};
     if (tiles > 0) {
-        const int bytes = (int)sizeof(float) * ((ROWS + KEYS) * (hd + 4) + KEYS * vd + ROWS * (KEYS + 4));
-        auto kern = vd <= 64 ? attention_f32_tile_kernel<1> : attention_f32_tile_kernel<2>;
-        static bool sized[2] = {false, false};
-        if (!sized[vd <= 64]) {
-            const int most = (int)sizeof(float) * ((ROWS + KEYS) * (MAX_DIM + 4) + KEYS * MAX_DIM + ROWS * (KEYS + 4));
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        // Tiles of 32 rows when those of 64 would leave SMs without a second block: 256 rows at 950 keys, 16 heads 185 -> 138 us.
+        const int rows = (long long)tiles * n_heads >= 2 * 148 ? 64 : 32, wide = vd <= 64 ? 0 : 1;
+        auto smem = [rows](int h, int v) { return (int)sizeof(float) * ((rows + KEYS) * (h + 4) + KEYS * v + rows * (KEYS + 4)); };
+        auto kern = rows == 64 ? (wide ? attention_f32_tile_kernel<2, 64> : attention_f32_tile_kernel<1, 64>)
+                               : (wide ? attention_f32_tile_kernel<2, 32> : attention_f32_tile_kernel<1, 32>);
+        static bool sized[2][2] = {};
+        if (!sized[rows == 64][wide]) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(MAX_DIM, MAX_DIM));
             if (e != cudaSuccess) return (int)e;
-            sized[vd <= 64] = true;
+            sized[rows == 64][wide] = true;
         }
-        cj::launch(kern, dim3(tiles, n_heads), dim3(TILE_THREADS), bytes, stream, a);
+        cj::launch(kern, dim3(rows == 64 ? tiles : tiles32, n_heads), dim3(4 * rows), smem(hd, vd), stream, a);
         if (int st = launch_status()) return st;
     }
     if (singles || tiles <= 0) cj::launch(attention_f32_row_kernel, dim3(T, n_heads), dim3(ROW_WARPS * 32), 0, stream, a);

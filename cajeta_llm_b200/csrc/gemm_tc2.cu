@@ -241,14 +241,22 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         for (int tile = cluster; tile < total_tiles && ok; tile += clusters) {
             TileCoord c = decode_tile<N_TOK>(p, tile, feat_tiles, tok_tiles, tiles_before);
             const int as = acc_it % ACC_STAGES;
+            const int n_cols = c.tok_end - c.tok0;
+            const int feat = c.feat0 + (int)rank * 128 + r;
+            const bool live = feat < p.features;
+            // the rows that the sums are added to are read 32 columns ahead, the first ones while the products still run
+            float old[EPI == EPI_ACC_F32 ? 32 : 1];
+            auto read_old = [&](int c0) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    old[j] = live && c0 + j < n_cols ? ((const float*)p.out)[(long long)(c.tok0 + c0 + j) * p.ldo + feat] : 0.0f;
+            };
+            if constexpr (EPI == EPI_ACC_F32) read_old(0);
             ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[as], (acc_it / ACC_STAGES) & 1, 3));
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + as * STAGE_COLS + ((uint32_t)(quarter * 32) << 16);
-            const int n_cols = c.tok_end - c.tok0;
             {
-                const int feat = c.feat0 + (int)rank * 128 + r;
-                const bool live = feat < p.features;
                 const float b = (p.bias != nullptr && live) ? p.bias[feat] : 0.0f;
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_TOK; c0 += 32) {
@@ -260,13 +268,14 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                     if (!live) continue;
                     // column j is token tok0 + c0 + j: a warp writes 32 consecutive features of a token
                     const long long o0 = (long long)(c.tok0 + c0) * p.ldo + feat;
-                    if (EPI == EPI_ACC_F32) {
-                        float old[32];
+                    if constexpr (EPI == EPI_ACC_F32) {
+                        float sum[32];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) old[j] = c0 + j < n_cols ? ((const float*)p.out)[o0 + j * p.ldo] : 0.0f;
+                        for (int j = 0; j < 32; ++j) sum[j] = old[j] + (__uint_as_float(v[j]) + b) * p.out_scale;
+                        if (c0 + 32 < n_cols) read_old(c0 + 32);
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (c0 + j < n_cols) ((float*)p.out)[o0 + j * p.ldo] = old[j] + (__uint_as_float(v[j]) + b) * p.out_scale;
+                            if (c0 + j < n_cols) ((float*)p.out)[o0 + j * p.ldo] = sum[j];
                     } else {
                         float f[32];
 #pragma unroll

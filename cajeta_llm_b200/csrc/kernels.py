@@ -448,17 +448,17 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v
     vd = value_dim or head_dim
     if (q.dtype == k_plane.dtype == torch.float32 and out.dtype == torch.float32 and head_dim % 4 == 0 and vd % 4 == 0
             and max(head_dim, vd) <= 128 and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
-        tiles, singles, requests = 0, True, 0
+        tiles, tiles32, singles, requests = 0, 0, True, 0
         if req_start is not None and h_req_start is not None:
             _need(req_start, "req_start", torch.int32)
             requests = len(h_req_start) - 1
             rows = [b - a for a, b in zip(h_req_start, h_req_start[1:])]
-            tiles = sum(-(-n // 64) for n in rows if n > F32_FEW_ROWS)
+            tiles, tiles32 = (sum(-(-n // t) for n in rows if n > F32_FEW_ROWS) for t in (64, 32))
             singles = any(0 < n <= F32_FEW_ROWS for n in rows)
         st = library("attention_f32").cj_attention_f32(
             _ptr(q), _ptr(out), _ptr(k_plane), _ptr(v_plane), _ptr(positions), _ptr(row_req), _ptr(req_start if requests else None), _i(requests),
             _ptr(table), _i(table.stride(0)), _i(page_tokens), _i(T), _i(n_heads), _i(n_kv), _i(head_dim), _i(vd), _i(window), _f(scale),
-            _f(softcap), gate_ptr, _i(gate_ld), _f(sink), _i(F32_FEW_ROWS), _i(tiles), _i(1 if singles else 0), _stream())
+            _f(softcap), gate_ptr, _i(gate_ld), _f(sink), _i(F32_FEW_ROWS), _i(tiles), _i(tiles32), _i(1 if singles else 0), _stream())
         _check(st, "paged_attention")
         return
     st = library("attention_paged").cj_paged_attention(
