@@ -81,19 +81,21 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ hs, const float* __restri
     for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] += value(i) * scale * w[i];
 }
 
-// The same for widths that are multiples of four, up to 8,192, 16-byte aligned: a thread keeps its NV float4 of the row, which is read once
-// (2,048 rows of 2,048: 11.9 -> 6.6 us).  Bound by memory.
+// The same for widths that are multiples of four, up to 8,192, 16-byte aligned: a thread keeps its NV float4 of the row, which is read once.
+// The squares are added in the order of the kernel above with `order` threads (from shared memory, a thread for one or two of that kernel's),
+// so that both give the same bits.  Bound by memory: 2,048 rows of 2,048 out of HBM 21.6 us with the kernel above, 11.2 with this one (10.2
+// with sums in the order of the float4); 8 rows 2.5 and 2.2.
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_add4_kernel(float* __restrict__ hs, const float* __restrict__ y, int n_parts,
-                                                           long long part_stride, const float* __restrict__ w, float eps, int H) {
+                                                           long long part_stride, const float* __restrict__ w, float eps, int H, int order) {
     cj::after_predecessor();
     cj::release_successor();
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float row[1024 * NV];
+    __shared__ float sums[16];
     const float4* src = (const float4*)(y + (size_t)blockIdx.x * H);
     float4* dst = (float4*)(hs + (size_t)blockIdx.x * H);
     const int n4 = H / 4;
     float4 v[NV], old[NV];
-    float ss = 0.0f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int i = threadIdx.x + 256 * k;
@@ -105,11 +107,20 @@ __global__ void __launch_bounds__(256) rmsnorm_add4_kernel(float* __restrict__ h
                 const float4 a = src[s * (part_stride / 4) + i];
                 v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
             }
+            *(float4*)(row + 4 * i) = v[k];
         }
-        ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, ss))));
     }
-    ss = block_sum(ss, scratch);
-    const float scale = 1.0f / sqrtf(ss / (float)H + eps);
+    __syncthreads();
+    for (int t = threadIdx.x; t < order; t += 256) {
+        float ss = 0.0f;
+        for (int i = t; i < H; i += order) ss = fmaf(row[i], row[i], ss);
+        ss = warp_sum(ss);
+        if ((t & 31) == 0) sums[t >> 5] = ss;
+    }
+    __syncthreads();
+    float total = 0.0f;
+    for (int i = 0; i < order / 32; ++i) total += sums[i];
+    const float scale = 1.0f / sqrtf(total / (float)H + eps);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int i = threadIdx.x + 256 * k;
@@ -1001,41 +1012,41 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, int n, int 
     }
 }
 
-// The same for parts of 128 NV entries (16-byte aligned rows): a lane keeps its 4 NV entries, so y and z are read and the gate is worked
-// out once.  2,048 rows of 8 parts of 512: 41.5 -> 16.3 us, of 16 parts of 128: 16.7 -> 9.3 us.
+// The same for parts of 32 NV entries: a lane keeps its entries, so y and z are read and the gate is worked out once.  The operations and
+// their order are the kernel's above, so both give the same bits.  2,048 rows of 8 parts of 512 out of HBM: 49.9 us with the kernel above,
+// 16.1 with this one; of 16 parts of 128: 24.9 and 11.4.
 template <typename TO, int NV>
-__global__ void gated_group_norm4_kernel(const float* __restrict__ y, int n, const float* __restrict__ z, int ld_z, const float* __restrict__ w,
-                                         int w_len, float eps, int gate_first, TO* __restrict__ out) {
+__global__ void gated_group_norm_kept_kernel(const float* __restrict__ y, int n, const float* __restrict__ z, int ld_z, const float* __restrict__ w,
+                                             int w_len, float eps, int gate_first, TO* __restrict__ out) {
     cj::after_predecessor();
     cj::release_successor();
-    constexpr int PART = 128 * NV;
+    constexpr int PART = 32 * NV;
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, parts = n / PART;
     const bool plain_sigmoid = (gate_first & 2) != 0, first = (gate_first & 1) != 0;
     for (int g = blockIdx.y * nw + warp; g < parts; g += gridDim.y * nw) {
-        const int c0 = g * PART + 4 * lane;
-        float v[NV][4], gate[NV][4], ss = 0.0f;
+        const int c0 = g * PART + lane;
+        const float* yr = y + (size_t)r * n + c0;
+        const float* zr = z + (size_t)r * ld_z + c0;
+        float v[NV], gate[NV], ss = 0.0f;
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
-            const float4 a = *(const float4*)(y + (size_t)r * n + c0 + 128 * k), b = *(const float4*)(z + (size_t)r * ld_z + c0 + 128 * k);
-            const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+            v[k] = yr[32 * k];
+            gate[k] = zr[32 * k];
+        }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                gate[k][i] = (plain_sigmoid ? 1.0f : vb[i]) / (1.0f + expf(-vb[i]));
-                v[k][i] = first ? va[i] * gate[k][i] : va[i];
-                ss = fmaf(v[k][i], v[k][i], ss);
-            }
+        for (int k = 0; k < NV; ++k) {
+            gate[k] = (plain_sigmoid ? 1.0f : gate[k]) / (1.0f + expf(-gate[k]));
+            if (first) v[k] *= gate[k];
+            ss = fmaf(v[k], v[k], ss);
         }
         ss = warp_sum(ss);
         const float scale = 1.0f / sqrtf(ss / (float)PART + eps);
         const float* wp = w + c0 % w_len;                    // (w_len is a multiple of the part)
+        TO* o = out + (size_t)r * n + c0;
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
-            const float4 g4 = *(const float4*)(wp + 128 * k);
-            const float gw[4] = {g4.x, g4.y, g4.z, g4.w};
-            float o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = first ? v[k][i] * scale * gw[i] : v[k][i] * scale * gw[i] * gate[k][i];
-            store_four(out + (size_t)r * n + c0 + 128 * k, o);
+            const float u = v[k] * scale * wp[32 * k];
+            o[32 * k] = from_f32<TO>(first ? u : u * gate[k]);
         }
     }
 }
@@ -1288,8 +1299,9 @@ CJ_EXPORT int cj_rmsnorm_add(float* hs, const float* y, int n_parts, long long p
                              cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (!hs || !y || !w || H <= 0 || n_parts < 1) return CJ_ERR_ARG;
+    const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     if (H % 4 == 0 && H <= 8192 && part_stride % 4 == 0 && (((uintptr_t)hs | (uintptr_t)y | (uintptr_t)w) & 15) == 0) {
-#define LAUNCH_NV(NV) cj::launch(rmsnorm_add4_kernel<NV>, dim3(rows), dim3(256), 0, stream, hs, y, n_parts, part_stride, w, eps, H)
+#define LAUNCH_NV(NV) cj::launch(rmsnorm_add4_kernel<NV>, dim3(rows), dim3(256), 0, stream, hs, y, n_parts, part_stride, w, eps, H, threads)
         if (H <= 1024) LAUNCH_NV(1);
         else if (H <= 2048) LAUNCH_NV(2);
         else if (H <= 4096) LAUNCH_NV(4);
@@ -1297,7 +1309,6 @@ CJ_EXPORT int cj_rmsnorm_add(float* hs, const float* y, int n_parts, long long p
 #undef LAUNCH_NV
         return launch_status();
     }
-    int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     cj::launch(rmsnorm_add_kernel, dim3(rows), dim3(threads), 0, stream, hs, y, n_parts, part_stride, w, eps, H);
     return launch_status();
 }
@@ -1527,14 +1538,14 @@ CJ_EXPORT int cj_gated_group_norm(const float* y, int n, int part_len, const flo
     int by = (parts + warps - 1) / warps;
     if (by > 64) by = 64;
     dim3 grid(rows, by);
-    if (part_len % 128 == 0 && (part_len == 128 || part_len == 256 || part_len == 512 || part_len == 1024) && ld_z % 4 == 0 && w_len % part_len == 0
-        && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w) & 15) == 0 && ((uintptr_t)out & 15) == 0 && (out_dtype == CJ_F32 || out_dtype == CJ_BF16)) {
-#define LAUNCH_NV(TO, NV) cj::launch(gated_group_norm4_kernel<TO, NV>, grid, dim3(warps * 32), 0, stream, y, n, z, ld_z, w, w_len, eps, gate_first, (TO*)out)
+    if ((part_len == 128 || part_len == 256 || part_len == 512 || part_len == 1024) && w_len % part_len == 0
+        && (out_dtype == CJ_F32 || out_dtype == CJ_BF16)) {
+#define LAUNCH_NV(TO, NV) cj::launch(gated_group_norm_kept_kernel<TO, NV>, grid, dim3(warps * 32), 0, stream, y, n, z, ld_z, w, w_len, eps, gate_first, (TO*)out)
 #define LAUNCH_PART(TO)                                                                                                 \
-        if (part_len == 128) LAUNCH_NV(TO, 1);                                                                          \
-        else if (part_len == 256) LAUNCH_NV(TO, 2);                                                                     \
-        else if (part_len == 512) LAUNCH_NV(TO, 4);                                                                     \
-        else LAUNCH_NV(TO, 8)
+        if (part_len == 128) LAUNCH_NV(TO, 4);                                                                          \
+        else if (part_len == 256) LAUNCH_NV(TO, 8);                                                                     \
+        else if (part_len == 512) LAUNCH_NV(TO, 16);                                                                    \
+        else LAUNCH_NV(TO, 32)
         if (out_dtype == CJ_F32) { LAUNCH_PART(float); }
         else { LAUNCH_PART(__nv_bfloat16); }
 #undef LAUNCH_PART

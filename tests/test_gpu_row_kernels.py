@@ -1,4 +1,5 @@
-"""Row kernels around the recurrent mixers at the edges of their vector forms: against the plain formulas in 64 bits."""
+"""Row kernels around the recurrent mixers at the edges of their vector forms: against the plain formulas in 64 bits, and their order of sums."""
+import numpy as np
 import pytest
 import torch
 
@@ -76,3 +77,42 @@ def test_gated_group_norm(n, part, w_len, z_offset, gate_first, sigmoid):
     v = (y.double() * gate if gate_first else y.double()).view(5, n // part, part)
     v = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6)).reshape(5, n) * w.double().repeat(n // w_len)
     assert torch.allclose(out.double(), v if gate_first else v * gate, atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("rows,H", [(2, 100), (2, 512), (3, 2048), (2, 4100), (2, 8192), (2, 9000)])
+def test_rmsnorm_add_sums_a_row_in_one_order(rows, H):
+    """A thread's entries one after the other (every 128th, 256th or 512th of the row, by its width), a warp's threads in pairs 16, 8, 4, 2
+    and 1 apart, then the warps: the same bits whichever kernel ran."""
+    from cajeta_llm_b200.csrc import kernels as K
+    f, wide = np.float32, np.longdouble                      # (a product of two float32 is exact in the wide type)
+    hs, y, w = rnd(rows, H, seed=12), rnd(rows, H, seed=13), rnd(H, seed=14)
+    threads = 512 if H >= 2048 else 256 if H >= 512 else 128
+    want = []
+    for h, v in zip(hs.cpu().numpy(), y.cpu().numpy()):
+        part = np.zeros(threads, f)
+        for i in range(0, H, threads):
+            e = v[i:i + threads].astype(wide)
+            part[:len(e)] = (e * e + part[:len(e)]).astype(f)
+        part = part.reshape(-1, 32)
+        for o in (16, 8, 4, 2, 1):
+            part = part + part[:, np.arange(32) ^ o]
+        total = f(0.0)
+        for p in part[:, 0]:
+            total = f(total + p)
+        scale = f(1.0) / np.sqrt(f(f(total / f(H)) + f(1e-6)))
+        want.append(((v * scale).astype(wide) * w.cpu().numpy() + h).astype(f))
+    got = hs.clone()
+    K.rmsnorm_add(got, y, w, 1e-6)
+    assert np.array_equal(got.cpu().numpy(), np.stack(want))
+
+
+@pytest.mark.parametrize("part", [128, 256, 512, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gate_first,sigmoid", [(True, False), (False, True)])
+def test_gated_group_norm_gives_the_same_bits_for_any_weight_length(part, dtype, gate_first, sigmoid):
+    from cajeta_llm_b200.csrc import kernels as K
+    y, z, w = rnd(7, part, seed=15), rnd(7, part, seed=16), rnd(part + 32, seed=17)
+    outs = [torch.empty(7, part, device=DEV, dtype=dtype) for _ in range(2)]
+    K.gated_group_norm(y, part, z, 0, w, 1e-6, gate_first, outs[0], sigmoid_gate=sigmoid)          # a weight of another length: entry by entry
+    K.gated_group_norm(y, part, z, 0, w[:part].clone(), 1e-6, gate_first, outs[1], sigmoid_gate=sigmoid)
+    assert torch.equal(outs[0], outs[1])
