@@ -821,15 +821,12 @@ def cast_rows(x: torch.Tensor, out: torch.Tensor) -> None:
 
 
 def rmsnorm_add(hs: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float) -> None:
-    """hs[r] += y[r] / sqrt(mean(y[r]^2) + eps) * weight; everything float32.  ``y`` of three dimensions [S, rows, H]: partial
-    sums of the rows, added in order first."""
+    """hs[r] += y[r] / sqrt(mean(y[r]^2) + eps) * weight; everything float32."""
     _need(hs, "hs", torch.float32), _need(y, "y", torch.float32), _need(weight, "weight", torch.float32)
     rows, H = hs.shape
-    if y.shape[-2:] != hs.shape or y.dim() > 3 or weight.numel() != H:
+    if y.shape != hs.shape or weight.numel() != H:
         raise KernelError(f"rmsnorm_add: shapes hs {tuple(hs.shape)} y {tuple(y.shape)} weight {tuple(weight.shape)} do not agree")
-    parts, stride = (y.shape[0], y.stride(0)) if y.dim() == 3 else (1, 0)
-    _check(library("recurrent").cj_rmsnorm_add(_ptr(hs), _ptr(y), _i(parts), _ll(stride), _ptr(weight), _f(eps), _i(rows), _i(H), _stream()),
-           "rmsnorm_add")
+    _check(library("recurrent").cj_rmsnorm_add(_ptr(hs), _ptr(y), _ptr(weight), _f(eps), _i(rows), _i(H), _stream()), "rmsnorm_add")
 
 
 def scale_rows_gather(x: torch.Tensor, slot_of_pick: torch.Tensor, weights: torch.Tensor, top_k: int, out: torch.Tensor) -> None:

@@ -61,24 +61,17 @@ __global__ void cast_rows_kernel(const float* __restrict__ x, TO* __restrict__ o
         out[i] = from_f32<TO>(x[i]);
 }
 
-// The row is y, or the sum of `n_parts` partial sums (a product cut along K; added in order), part_stride apart.
-__global__ void rmsnorm_add_kernel(float* __restrict__ hs, const float* __restrict__ y, int n_parts, long long part_stride,
-                                   const float* __restrict__ w, float eps, int H) {
+__global__ void rmsnorm_add_kernel(float* __restrict__ hs, const float* __restrict__ y, const float* __restrict__ w, float eps, int H) {
     cj::after_predecessor();
     cj::release_successor();
     __shared__ float scratch[32];
     const float* src = y + (size_t)blockIdx.x * H;
     float* dst = hs + (size_t)blockIdx.x * H;
-    auto value = [&](int i) {
-        float v = src[i];
-        for (int s = 1; s < n_parts; ++s) v += src[s * part_stride + i];
-        return v;
-    };
     float ss = 0.0f;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) { const float v = value(i); ss = fmaf(v, v, ss); }
+    for (int i = threadIdx.x; i < H; i += blockDim.x) ss = fmaf(src[i], src[i], ss);
     ss = block_sum(ss, scratch);
     const float scale = 1.0f / sqrtf(ss / (float)H + eps);
-    for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] += value(i) * scale * w[i];
+    for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] += src[i] * scale * w[i];
 }
 
 // The same for widths that are multiples of four, up to 8,192, 16-byte aligned: a thread keeps its NV float4 of the row, which is read once.
@@ -86,8 +79,8 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ hs, const float* __restri
 // so that both give the same bits.  Bound by memory: 2,048 rows of 2,048 out of HBM 21.6 us with the kernel above, 11.2 with this one (10.2
 // with sums in the order of the float4); 8 rows 2.5 and 2.2.
 template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_add4_kernel(float* __restrict__ hs, const float* __restrict__ y, int n_parts,
-                                                           long long part_stride, const float* __restrict__ w, float eps, int H, int order) {
+__global__ void __launch_bounds__(256) rmsnorm_add4_kernel(float* __restrict__ hs, const float* __restrict__ y,
+                                                           const float* __restrict__ w, float eps, int H, int order) {
     cj::after_predecessor();
     cj::release_successor();
     __shared__ __align__(16) float row[1024 * NV];
@@ -103,10 +96,6 @@ __global__ void __launch_bounds__(256) rmsnorm_add4_kernel(float* __restrict__ h
         if (i < n4) {
             v[k] = src[i];
             old[k] = dst[i];
-            for (int s = 1; s < n_parts; ++s) {
-                const float4 a = src[s * (part_stride / 4) + i];
-                v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
-            }
             *(float4*)(row + 4 * i) = v[k];
         }
     }
@@ -1294,14 +1283,12 @@ CJ_EXPORT int cj_cast_rows(const float* x, void* out, int out_dtype, long long n
     return launch_status();
 }
 
-// y: [rows, H], or n_parts > 1 partial sums of it, part_stride floats apart
-CJ_EXPORT int cj_rmsnorm_add(float* hs, const float* y, int n_parts, long long part_stride, const float* w, float eps, int rows, int H,
-                             cudaStream_t stream) {
+CJ_EXPORT int cj_rmsnorm_add(float* hs, const float* y, const float* w, float eps, int rows, int H, cudaStream_t stream) {
     if (rows <= 0) return 0;
-    if (!hs || !y || !w || H <= 0 || n_parts < 1) return CJ_ERR_ARG;
+    if (!hs || !y || !w || H <= 0) return CJ_ERR_ARG;
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
-    if (H % 4 == 0 && H <= 8192 && part_stride % 4 == 0 && (((uintptr_t)hs | (uintptr_t)y | (uintptr_t)w) & 15) == 0) {
-#define LAUNCH_NV(NV) cj::launch(rmsnorm_add4_kernel<NV>, dim3(rows), dim3(256), 0, stream, hs, y, n_parts, part_stride, w, eps, H, threads)
+    if (H % 4 == 0 && H <= 8192 && (((uintptr_t)hs | (uintptr_t)y | (uintptr_t)w) & 15) == 0) {
+#define LAUNCH_NV(NV) cj::launch(rmsnorm_add4_kernel<NV>, dim3(rows), dim3(256), 0, stream, hs, y, w, eps, H, threads)
         if (H <= 1024) LAUNCH_NV(1);
         else if (H <= 2048) LAUNCH_NV(2);
         else if (H <= 4096) LAUNCH_NV(4);
@@ -1309,7 +1296,7 @@ CJ_EXPORT int cj_rmsnorm_add(float* hs, const float* y, int n_parts, long long p
 #undef LAUNCH_NV
         return launch_status();
     }
-    cj::launch(rmsnorm_add_kernel, dim3(rows), dim3(threads), 0, stream, hs, y, n_parts, part_stride, w, eps, H);
+    cj::launch(rmsnorm_add_kernel, dim3(rows), dim3(threads), 0, stream, hs, y, w, eps, H);
     return launch_status();
 }
 

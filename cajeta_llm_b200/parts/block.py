@@ -133,8 +133,6 @@ class OutputNormBlock(Part):
         super().__init__(spec, prefix, runtime)
         self.mixer_norm = make_part("norm", layer.mixer_norm, self.name(spec["mixer_norm_name"]), runtime)
         self.mixer = make_part("mixer", layer.mixer, self.name(spec["mixer_name"]), runtime)
-        if hasattr(self.mixer, "allow_pending"):
-            self.mixer.allow_pending = True        # partial sums are added by the kernel that norms them
         self.feed_forward = self.feed_forward_norm = None
         if layer.feed_forward is not None:
             self.feed_forward_norm = make_part("norm", layer.feed_forward_norm, self.name(spec["feed_forward_norm_name"]), runtime)
@@ -171,27 +169,23 @@ class OutputNormBlock(Part):
         K.cast_rows(hs, x)
         return x
 
-    def _add_normed(self, hs: torch.Tensor, y: torch.Tensor, norm) -> None:
+    def _add_normed(self, hs: torch.Tensor, y: torch.Tensor, pending, norm) -> None:
+        if pending is not None:
+            y += pending.sum(dim=0)
         K.tag = "norm + add"
         K.rmsnorm_add(hs, y, norm.weight, norm.eps)
         K.tag = None
 
     def forward(self, hs: torch.Tensor, ctx, entry) -> None:
-        # a mixer that hands back partial sums leaves y alone: nothing to clear, and the norm adds them as it reads them
-        deferred = getattr(self.mixer, "defers", lambda n: False)(hs.shape[0])
-        y = torch.empty_like(hs) if deferred else torch.zeros_like(hs)
+        y = torch.zeros_like(hs)
         pending = self.mixer.forward(self._input(hs), y, ctx, entry)
-        if deferred and pending is None:
-            raise ValueError("a mixer that defers (defers(rows)) has to hand back partial sums")
-        if pending is not None and not deferred:
-            y += pending.sum(dim=0)
-        self._add_normed(hs, pending if deferred else y, self.mixer_norm)
+        self._add_normed(hs, y, pending, self.mixer_norm)
         ff = self.feed_forward
         if ff is None:
             return
         y = torch.zeros_like(hs)
         ff.forward(self._input(hs), hs if getattr(ff, "needs_f32_input", False) else None, y, ctx)
-        self._add_normed(hs, y, self.feed_forward_norm)
+        self._add_normed(hs, y, None, self.feed_forward_norm)
 
 
 @register_part("block", "parallel")

@@ -52,7 +52,7 @@ import torch
 
 from ..csrc import kernels as K
 from .base import KvNeed, Part, make_part, register_part
-from .linear import project, project_split, splits_few_rows
+from .linear import project, project_split
 from .plan import ParamSpec
 
 
@@ -201,9 +201,6 @@ class LatentAttention(Part):
             project(rt, gated, self.w_o, residual, accumulate=True)
         K.tag = None
         return parts
-
-    def defers(self, rows: int) -> bool:
-        return self.allow_pending and splits_few_rows(self.runtime, rows, self.w_o)
 
     def _absorbed_form(self, proj: torch.Tensor, gate, ctx, entry) -> torch.Tensor:
         """``proj``: float32 rows whose first ``heads * (dim + rot_dim)`` columns are the queries; ``gate``: (matrix, column)

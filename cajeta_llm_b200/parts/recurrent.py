@@ -95,20 +95,9 @@ from .plan import ParamSpec
 
 class _StateMixer(Part):
     graph_safe = True          # rows, requests and slots come from the step's device metadata only
-    allow_pending = False      # a block that takes partial sums from its mixer sets this True
 
     def cache_need(self):
         return None
-
-    def defers(self, rows: int) -> bool:
-        return self.allow_pending and splits_few_rows(self.runtime, rows, self.w_o)
-
-    def _project_out(self, gated: torch.Tensor, residual: torch.Tensor) -> Optional[torch.Tensor]:
-        """The output projection, added into ``residual`` - or, for a block that takes them and a step of few rows, handed back as partial sums."""
-        parts = project_split(self.runtime, gated, self.w_o) if self.allow_pending else None
-        if parts is None:
-            project(self.runtime, gated, self.w_o, residual, accumulate=True)
-        return parts
 
     def libraries(self) -> set:
         libs = {"recurrent", "gemm_simt"}
@@ -186,9 +175,9 @@ class StateSpaceMixer(_StateMixer):
         K.tag = "gate + norm"
         K.gated_group_norm(y, self.inner // self.norm_groups, proj, 0, self.w_norm, self.eps, True, gated)
         K.tag = "o"
-        parts = self._project_out(gated, residual)
+        project(rt, gated, self.w_o, residual, accumulate=True)
         K.tag = None
-        return parts
+        return None
 
 
 @register_part("mixer", "gated_delta")
@@ -255,9 +244,9 @@ class GatedDeltaMixer(_StateMixer):
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, C + 2 * self.heads, self.w_norm, self.eps, False, gated)
         K.tag = "o"
-        parts = self._project_out(gated, residual)
+        project(rt, gated, self.w_o, residual, accumulate=True)
         K.tag = None
-        return parts
+        return None
 
 
 @register_part("mixer", "gla")
@@ -320,9 +309,9 @@ class GatedLinearAttention(_StateMixer):
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, off_g, self.w_norm, self.eps, False, gated)
         K.tag = "o"
-        parts = self._project_out(gated, residual)
+        project(rt, gated, self.w_o, residual, accumulate=True)
         K.tag = None
-        return parts
+        return None
 
 
 @register_part("mixer", "mlstm")
@@ -382,9 +371,9 @@ class MatrixMemoryMixer(_StateMixer):
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, off_g, self.w_norm, self.eps, False, gated, sigmoid_gate=True)
         K.tag = "o"
-        parts = self._project_out(gated, residual)
+        project(rt, gated, self.w_o, residual, accumulate=True)
         K.tag = None
-        return parts
+        return None
 
 
 @register_part("mixer", "mingru")
