@@ -53,6 +53,7 @@ struct Args {
     const float* bias; const float* bias2;
     float* C; long long ldc;
     int tokens, features, K;
+    int x_rows;                            // rows that X holds: nothing is read past them
     int accumulate;
     const int* group_offsets;
     int groups;
@@ -397,6 +398,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
 }
 
+// out[s, :] = x[index[s], :] for the rows of the groups (all rows without groups), zeros where the index names no row of x.  Rows outside
+// the groups are left alone: no product reads them, and their indices may be anything.  A warp a row.
+__global__ void __launch_bounds__(256) gather_group_rows_kernel(const float* __restrict__ x, long long ldx, int x_rows, const int* __restrict__ index,
+                                                                const int* __restrict__ group_offsets, int groups, int rows, int K, float* __restrict__ out) {
+    cj::after_predecessor();
+    cj::release_successor();
+    const int lane = threadIdx.x & 31, s = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lo = group_offsets ? group_offsets[0] : 0, hi = group_offsets ? min(rows, group_offsets[groups]) : rows;
+    if (s < lo || s >= hi) return;
+    const int from = index[s];
+    const bool there = from >= 0 && from < x_rows;
+    const float4* src = (const float4*)(x + (there ? from : 0) * ldx);
+    float4* dst = (float4*)(out + (size_t)s * K);
+#pragma unroll 4
+    for (int i = lane; i < K / 4; i += 32) dst[i] = there ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
 // a row-major float32 matrix in boxes of [box_rows, 32] with the 128-byte swizzle; out-of-range elements read as zero
 bool make_map_f32(CUtensorMap* map, const float* base, long long rows, long long cols, long long ld, int box_rows) {
     EncodeTiledFn fn = encode_fn();
@@ -421,7 +439,7 @@ int launch(const Args& a, int tok_tiles, cudaStream_t stream) {
     if (tok_tiles > 65535) return CJ_ERR_SIZE;
     const long long w_rows = (long long)(a.group_offsets ? a.groups : 1) * a.features;
     CUtensorMap mx, mw, mw2;
-    if (!make_map_f32(&mx, a.X, a.tokens, a.K, a.ldx, N) || !make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
+    if (!make_map_f32(&mx, a.X, a.x_rows, a.K, a.ldx, N) || !make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
     mw2 = mw;
     if (DUAL && !make_map_f32(&mw2, a.W2, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
     cj::launch(kern, dim3((a.features + a.feat_tile - 1) / a.feat_tile, tok_tiles), dim3(threads(N)), Smem<N>::TOTAL, stream, mx, mw, mw2, a);
@@ -430,20 +448,31 @@ int launch(const Args& a, int tok_tiles, cudaStream_t stream) {
 
 }  // namespace
 
-// X [tokens, K] float32 with row stride ldx (grouped: in the groups' order), W (and W2) [groups, features, K] contiguous float32; the
+// Rows of x (float32, row stride ldx, x_rows of them) in the groups' order, out [rows, K] contiguous: as cj_gemm_f32_tc takes them.
+CJ_EXPORT int cj_gather_group_rows(const float* x, long long ldx, int x_rows, const int* index, const int* group_offsets, int groups, int rows,
+                                   int K, float* out, cudaStream_t stream) {
+    if (rows <= 0) return 0;
+    if (!x || !index || !out || K <= 0 || x_rows <= 0 || (group_offsets && groups <= 0)) return CJ_ERR_ARG;
+    if (K % 4 != 0 || ldx % 4 != 0 || ldx < K || (((uintptr_t)x | (uintptr_t)out) & 15)) return CJ_ERR_ALIGN;
+    cj::launch(gather_group_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, x, ldx, x_rows, index, group_offsets, groups, rows, K, out);
+    return cj::launch_status();
+}
+
+// X [x_rows, K] float32 with row stride ldx (grouped: in the groups' order; no row from x_rows on is read), W (and W2) [groups, features, K]
+// contiguous float32; the
 // other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16, 32, 64 or 128); feat_tile: its features (32, 64 or 128; with W2 at most 64).
-CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
+CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
                              long long ldc, int tokens, int features, int K, int accumulate, const int* group_offsets, int groups,
                              float act_limit, float act_alpha, float act_cubic, int act, int act_feats, float out_scale, int n_tok,
                              int feat_tile, cudaStream_t stream) {
     if (tokens <= 0 || features <= 0) return 0;
-    if (!X || !W || !C || K <= 0) return CJ_ERR_ARG;
+    if (!X || !W || !C || K <= 0 || x_rows <= 0) return CJ_ERR_ARG;
     if (group_offsets && groups <= 0) return CJ_ERR_ARG;
     if ((bias2 && !W2) || (act != cj::ACT_NONE && W2)) return CJ_ERR_ARG;
     if (feat_tile != 32 && feat_tile != 64 && !(feat_tile == 128 && !W2)) return CJ_ERR_SIZE;
     if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2) & 15) return CJ_ERR_ALIGN;
-    Args a{X, ldx, W, W2, bias, bias2, C, ldc, tokens, features, K, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
+    Args a{X, ldx, W, W2, bias, bias2, C, ldc, tokens, features, K, x_rows, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
            act_feats > 0 ? act_feats : features, out_scale, feat_tile};
     const int tok_tiles = (tokens + n_tok - 1) / max(n_tok, 1) + (group_offsets ? groups : 0);
 #define CASE(N) case N: return W2 ? launch<N, true>(a, tok_tiles, stream) : launch<N, false>(a, tok_tiles, stream);

@@ -336,12 +336,15 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
         _need(a_row_index, "a_row_index", torch.int32)
     if f32_tc_takes(a, w, w_up, out):
         if a_row_index is not None:
+            # the groups' rows side by side (a row outside the groups has no index to follow, an index below 0 names a row of zeros)
             gathered = torch.empty((M, K), dtype=a.dtype, device=a.device)
-            gather_rows(a, a_row_index, gathered)
+            st = library("gemm_f32_tc").cj_gather_group_rows(_ptr(a), _ll(a.stride(0)), _i(a.shape[0]), _ptr(a_row_index), _ptr(group_offsets), _i(G),
+                                                             _i(M), _i(K), _ptr(gathered), _stream())
+            _check(st, "gather_rows")
             a = gathered
         n_tok, feat_tile = f32_tc_tile(M, N, G, w_up is not None, _sm_count())
         st = library("gemm_f32_tc").cj_gemm_f32_tc(
-            _ptr(a), _ll(a.stride(0)), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
+            _ptr(a), _ll(a.stride(0)), _i(min(M, a.shape[0])), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
             _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
             _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
         _check(st, "gemm")

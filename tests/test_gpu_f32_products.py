@@ -85,3 +85,24 @@ def test_infinite_and_missing_numbers_are_summed_as_the_fma_pipe_sums_them(K):
     want = torch.where(want.abs() > 3.4028235e38, torch.sign(want) * float("inf"), want)
     same = torch.isnan(out) == torch.isnan(want)
     assert bool(same.all()) and torch.equal(torch.isinf(out), torch.isinf(want.float()))
+
+
+def test_rows_by_index_of_a_column_slice_and_slots_outside_the_groups(K):
+    """Rows may be a column slice of a wider matrix; an index below 0 names a row of zeros; slots that no group holds are neither read nor
+    written, and x need not have rows for them."""
+    H, E, N, slots = 128, 3, 64, 40
+    x, w = rnd(20, H + 16, seed=14)[:, 8:8 + H], rnd(E, N, H, seed=15)
+    offsets = torch.tensor([2, 9, 9, 30], dtype=torch.int32, device=DEV)
+    index = torch.full((slots,), -1, dtype=torch.int32, device=DEV)
+    index[2:30] = torch.randint(0, 20, (28,), generator=torch.Generator().manual_seed(16)).int().to(DEV)
+    index[5] = -1
+    out = torch.full((slots, N), 7.0, device=DEV)
+    assert K.f32_tc_takes(x, w, None, out)
+    K.gemm(x, w, out, group_offsets=offsets, a_row_index=index)
+    assert bool((out[:2] == 7.0).all()) and bool((out[30:] == 7.0).all()) and bool((out[5] == 0.0).all())
+    rows = torch.where(index[:, None] >= 0, x[index.clamp(min=0).long()], 0.0)
+    for e, (lo, hi) in enumerate(((2, 9), (9, 9), (9, 30))):
+        held(out[lo:hi], rows[lo:hi], w[e], rows[lo:hi].double() @ w[e].double().t())
+    again = torch.full((slots, N), 7.0, device=DEV)
+    K.gemm(rows[:30].contiguous(), w, again, group_offsets=offsets, rows=slots)
+    assert torch.equal(out, again)
