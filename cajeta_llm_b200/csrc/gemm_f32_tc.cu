@@ -2,20 +2,26 @@
 //
 //     C[token, feature] (+)= scale (sum_k X[token, k] * W[feature, k] (+ bias))
 //
-// A float32 number is the sum of three bfloat16 numbers, 8 bits of its significand each (hi, mid, lo: the leading bits cut
-// off one after the other, so nothing is lost), and a product of two bfloat16 numbers is exact in float32.  Of the nine products
-// of the parts the six largest are summed; the three left out are together below 2^-24 of the product.  What decides the
-// accuracy is the sum, and tensor memory's adds truncate.  So a tensor-memory accumulator only ever holds
-// 32 products a term (one block of K) of three terms, the small terms first, and the blocks are added up in registers with
-// ordinary rounded float32 additions, in the order of K.  Measured against 64 bits, relative error of the result for normal operands:
-// K 2,048 1.8e-7, where the FMA pipe's chain of K fused multiply-adds gives 8.1e-7; K 5,632 2.6e-7 and 1.3e-6; 5,632 products of
-// one sign 2.2e-7 and 1.1e-6; K 132 1.2e-7 and 2.1e-7.
+// A float32 number is the sum of three bfloat16 numbers (hi: the number rounded to nearest; mid: what is left, rounded; lo: the rest, at most
+// seven bits), and a product of two bfloat16 numbers is exact in float32.  Of the nine products of the parts the six largest are summed; the
+// three left out (mid lo, lo mid, lo lo) are together at most 2^-24 (1 + 2^-10) of the product, of either sign.  What else decides the
+// accuracy is the sum, and tensor memory's adds truncate.  So a tensor-memory accumulator only ever holds 32 products a term (one block
+// of K): one the products of the leading parts, 16 bits each, another the five smaller terms; and the blocks are added up in registers with
+// ordinary rounded float32 additions, in the order of K.  Measured against 64 bits, relative error of the result, this and the FMA pipe's
+// chain of K fused multiply-adds: normal operands, K 132 7.3e-8 and 2.0e-7, K 2,048 2.1e-7 and 8.1e-7, K 5,632 3.4e-7 and 1.4e-6; 2,048
+// products of one sign 1.8e-7 and 7.0e-7, with the low 15 bits of every operand set 1.8e-7 and 4.5e-6; rows with a single entry
+// 2.6e-8 and 2.5e-8, at most 1.7 x 2^-24 and 2^-24.  (The parts cut off instead of rounded, as they were, lose up to 2^-21 of a product,
+// always towards zero: single entries 1.0e-7, at most 9.7 x 2^-24.  mid lo and lo mid summed as well: single entries as the chain, but 1 row x
+// 2,048 x 2,048 36.7 us instead of 31.5.)
 //
 // A result's operations depend on its own row of X, its row of W and K alone: not on the other rows of the launch, the tile
 // sizes or the tile's place.  So a token's row has the same bits in a prompt's step and in a step of its own.
 //
-// A number that is infinite, or not a number, has no such parts.  The splitting threads notice one (its last remainder is no
-// number) and the tile's results are then summed on the FMA pipe instead, one chain over K as gemm_simt.cu has it.
+// Not every number is the sum of three such parts: not one that is infinite, or not a number, or so large that its first part would be
+// infinite (from 2^128 - 2^119 on), or so small that its last one lies below the smallest bfloat16 (below 2^-110).  The splitting
+// threads notice one, and the tile's results are then summed on the FMA pipe instead, one chain over K as gemm_simt.cu has it.  So is a
+// result that is not finite (a part's product may overflow where the product itself does not) or below 2^-100 (whose smaller parts' products
+// are too small for float32).
 //
 // One block a tile of `feat_tile` (up to 128) features x N tokens; the weights are the rows of the product.  One thread sends for
 // the float32 tiles (TMA) into a ring as deep as shared memory allows; groups of eight warps split them into the six bfloat16
@@ -23,8 +29,8 @@
 // and store.  A block of K is a chain of short waits for a group (tile landed, stage free, stores visible to the products: some
 // 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
 // tokens that chain, with many the shared memory, which every operand crosses as float32 once and as bfloat16 parts once for each of
-// its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 35;
-// 250 x 6,144 x 2,048 328 and 114; 1,777 x 6,144 x 2,048 1,822 and 375; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
+// its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 32;
+// 250 x 6,144 x 2,048 328 and 101; 1,777 x 6,144 x 2,048 1,822 and 347; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
 // of 4 picks 802 / 1,915 / 6,045 and 181 / 570 / 1,430.  (With the float32 operands loaded into registers instead of by TMA
 // 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
@@ -75,21 +81,24 @@ template <int N> struct Smem {
     static_assert(STAGES % split_groups(N) == 0, "a stage belongs to one group");
 };
 
-// eight float32 -> their three bfloat16 parts, packed; `odd` becomes no number when one of the eight is infinite or none
-__device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& hi, uint4& mid, uint4& lo, float& odd) {
+// eight float32 -> their three bfloat16 parts, packed; some bit of `odd` is set when one of the eight is not the sum of its parts: infinite,
+// no number, so large that its first part rounds to infinity, or so small that its last part falls below the smallest bfloat16
+__device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& hi, uint4& mid, uint4& lo, uint32_t& odd) {
     const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
     uint32_t h[4], m[4], l[4];
+    auto pack = [](float a, float b) {
+        const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+        return *(const uint32_t*)&t;
+    };
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint32_t a = __float_as_uint(f[2 * i]), b = __float_as_uint(f[2 * i + 1]);
-        h[i] = __byte_perm(a, b, 0x7632);
-        const float ra = f[2 * i] - __uint_as_float(a & 0xffff0000u), rb = f[2 * i + 1] - __uint_as_float(b & 0xffff0000u);
-        const uint32_t am = __float_as_uint(ra), bm = __float_as_uint(rb);
-        m[i] = __byte_perm(am, bm, 0x7632);
-        const float la = ra - __uint_as_float(am & 0xffff0000u), lb = rb - __uint_as_float(bm & 0xffff0000u);
-        l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
-        odd = fmaf(la, 0.0f, odd);
-        odd = fmaf(lb, 0.0f, odd);
+        const float a = f[2 * i], b = f[2 * i + 1];
+        h[i] = pack(a, b);
+        const float ra = a - __uint_as_float(h[i] << 16), rb = b - __uint_as_float(h[i] & 0xffff0000u);
+        m[i] = pack(ra, rb);
+        const float la = ra - __uint_as_float(m[i] << 16), lb = rb - __uint_as_float(m[i] & 0xffff0000u);
+        l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);        // (a remainder has eight bits at most)
+        odd |= __float_as_uint(la) | __float_as_uint(lb);
     }
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     mid = make_uint4(m[0], m[1], m[2], m[3]);
@@ -113,6 +122,9 @@ __device__ __noinline__ float chain(const float* x, const float* w, int K) {
     for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
     return s;
 }
+
+// whether a sum of the parts' products stands as it is (see the head of the file)
+__device__ __forceinline__ bool chain_free(float v) { return (fabsf(v) >= 0x1p-100f && fabsf(v) <= 3.402823466e38f) || v == 0.0f; }
 
 template <int N, bool DUAL>
 __global__ void __launch_bounds__(threads(N), 1)
@@ -236,7 +248,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const int src0 = row0 * 128 + (((2 * piece) ^ (row0 & 7)) << 4), src1 = row0 * 128 + (((2 * piece + 1) ^ (row0 & 7)) << 4);
         const int dst = row0 * 64 + ((piece ^ ((row0 >> 1) & 3)) << 4);
         const int x_part = n16 * 64;
-        float odd = 0.0f;
+        uint32_t odd = 0;
         bool ok = true;
         for (int kb = g; kb < n_kb && ok; kb += G) {
             const int rs = kb % RING, s = kb % STAGES;
@@ -285,7 +297,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     *(uint4*)(at + x_part) = mid;
                     *(uint4*)(at + 2 * x_part) = lo;
                 }
-            if (kb + G >= n_kb && !(odd == 0.0f)) odd_flag = 1;
+            if (kb + G >= n_kb && (odd & 0xffffu)) odd_flag = 1;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
             __syncwarp();
             if (lane == 0) {
@@ -296,11 +308,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     } else if (work && warp == ISSUE) {
         // ---- product issue --------------------------------------------------------------------------
         if (elect_one()) {
-            // two accumulators a block of K, D0 | D1, n16 columns each: D0 takes the products with the leading part of X, D1 the
-            // others; where both take the same part of W, one product twice as wide serves both
+            // two accumulators a block of K, D0 | D1, n16 columns each: D0 takes the products of the leading parts alone, whose 16 bits an
+            // accumulator holds, D1 the others; the leading part of W meets the first two parts of X in one product twice as wide
             const uint32_t one = umma_idesc_bf16(128, n16), both = umma_idesc_bf16(128, 2 * n16);
             const uint64_t first = umma_desc_sw64(stages);
-            const uint64_t w_step = S::W_PART >> 4, x_hi = 3 * w_step, x_lo = x_hi + (uint64_t)(2 * n16 * 64 >> 4);
+            const uint64_t w_step = S::W_PART >> 4, x_hi = 3 * w_step, x_step = (uint64_t)(n16 * 64 >> 4);
             bool ok = true;
             for (int kb = 0; kb < n_kb && ok; ++kb) {
                 const int s = kb % STAGES, a = kb & 1;
@@ -309,15 +321,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 tcgen05_fence_after();
                 const uint64_t at = first + (uint64_t)((s * S::STAGE) >> 4);
                 const uint32_t d0 = tmem + a * 2 * N, d1 = d0 + n16;
-                // the smallest products first
+                auto add = [&](int pw, int px) {             // D1 += part pw of W . part px of X
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * w_step + 2 * k, at + x_hi + 2 * k, one, k > 0);          // lo hi
+                    for (int k = 0; k < BK / 16; ++k) umma_bf16(d1, at + pw * w_step + 2 * k, at + x_hi + px * x_step + 2 * k, one, 1);
+                };
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(d1, at + 2 * k, at + x_lo + 2 * k, one, k > 0);                       // hi lo
-#pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + w_step + 2 * k, at + x_hi + 2 * k, both, 1);                 // mid hi | mid mid
-#pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * k, at + x_hi + 2 * k, both, 1);                          // hi hi | hi mid
+                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * k, at + x_hi + 2 * k, both, k > 0);                      // hi hi | hi mid
+                add(1, 0); add(0, 2); add(1, 1); add(2, 0);
                 umma_commit(&empty_bar[s]);
                 umma_commit(&acc_full[a]);
             }
@@ -355,11 +365,20 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         if (!grouped) cj::after_predecessor();
         const int fr = DUAL ? (r & 63) : r, feat = feat0 + fr;
         const bool live = ok && fr < p.feat_tile && feat < p.features;
-        if (odd_flag && live) {
-            const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
+        bool again = odd_flag != 0;
 #pragma unroll
-            for (int j = 0; j < COLS; ++j)
-                if (c_first + j < n_tok) acc[j] = chain(p.X + (size_t)(tok0 + c_first + j) * p.ldx, w, p.K);
+        for (int j = 0; j < COLS; ++j) again = again || !chain_free(acc[j]);
+        if (again && live) {
+            // (rarely: through an array in memory, so that the sums keep their registers)
+            float sums[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
+            const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
+#pragma unroll 1
+            for (int j = 0; j < COLS && c_first + j < n_tok; ++j)
+                if (odd_flag || !chain_free(sums[j])) sums[j] = chain(p.X + (size_t)(tok0 + c_first + j) * p.ldx, w, p.K);
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
         }
         if (DUAL) {
             // the second weight's sums cross to the threads that hold the first's: through the ring, which nothing reads any more

@@ -42,8 +42,9 @@ class Runtime:
     ``dtype == "bfloat16"``: matrices, activations between kernels and the cache are
     bfloat16; statistics, sums, the residual stream, router inputs and logits are
     float32.  ``dtype == "float32"``: everything is float32 and every product is summed to
-    float32's accuracy (on the FMA pipe, or on the tensor cores with each operand in three
-    parts that lose nothing; no reduced-precision matrix mode).
+    float32's accuracy (on the FMA pipe, or on the tensor cores with each operand as the sum
+    of three bfloat16 parts and the parts' products down to 2^-24 of the operands'; no
+    reduced-precision matrix mode).
     """
 
     def __init__(self, dtype: str = "bfloat16", device: str = "cuda:0", fast_kernels: bool = True):

@@ -17,9 +17,9 @@ def rnd(*shape, seed):
 
 
 def held(got, a, w, want):
-    """The sum's error is at most two roundings (2^-24 of the sum of magnitudes each) a block of 32 products, and a few for the terms
-    left out, the accumulator's truncation inside a block and the last addition."""
-    bound = (a.shape[-1] / 16 + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+    """The sum's error is at most, in units of 2^-24 of the sum of magnitudes: two roundings a block of 32 products, one for the terms left
+    out, two for each of the leading products' two truncated adds inside a block, and one for the smaller terms'."""
+    bound = (a.shape[-1] / 16 + 6) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
     assert bool(((got.double() - want).abs() <= bound).all()), float(((got.double() - want).abs() / bound).max())
 
 
@@ -42,6 +42,65 @@ def test_plain_bias_accumulate_scale(K, M, N, Kd):
         K.gemm(a[lo:hi], w, part)
         assert torch.equal(part, out[lo:hi])
     assert K.wait_errors() == {}
+
+
+def low_bits(t):
+    """Operands that three bfloat16 parts hold worst: the low 15 bits all set."""
+    return (t.view(torch.int32) | 0x7FFF).view(torch.float32)
+
+
+def on_the_fma_pipe(K, monkeypatch, a, w):
+    out = torch.empty(a.shape[0], w.shape[0], device=DEV)
+    with monkeypatch.context() as m:
+        m.setattr(K, "f32_tc_takes", lambda *x: False)
+        K.gemm(a, w, out)
+    return out
+
+
+@pytest.mark.parametrize("kind", ["given", "normal", "low bits"])
+def test_rows_with_a_single_entry_are_right_to_their_last_place(K, kind):
+    """One product: half a place for its rounding and at most as much for the terms left out."""
+    n, Kd = 256, 128
+    x, y = rnd(n, seed=17), rnd(n, seed=18)
+    if kind == "given":
+        x, y = torch.full_like(x, 1 + 2.0 ** -7 - 2.0 ** -23), torch.full_like(y, 1 + 2.0 ** -7 - 2.0 ** -23)
+    if kind == "low bits":
+        x, y = low_bits(x), low_bits(y)
+    a = torch.zeros(n, Kd, device=DEV)
+    a[torch.arange(n), torch.arange(n) % Kd] = x
+    out = torch.empty(n, n, device=DEV)
+    K.gemm(a, y[:, None].expand(n, Kd).contiguous(), out)
+    want = x.double()[:, None] * y.double()[None, :]
+    assert bool(((out.double() - want).abs() <= 2.0 ** -23 * want.abs()).all())
+
+
+@pytest.mark.parametrize("Kd", [128, 2048])
+def test_sums_of_one_sign_are_no_further_off_than_the_fma_pipes(K, monkeypatch, Kd):
+    for low in (False, True):
+        a, w = rnd(64, Kd, seed=19).abs(), rnd(128, Kd, seed=20).abs()
+        if low:
+            a, w = low_bits(a), low_bits(w)
+        out, want = torch.empty(64, 128, device=DEV), a.double() @ w.double().t()
+        K.gemm(a, w, out)
+        held(out, a, w, want)
+        assert float((out.double() - want).norm()) <= float((on_the_fma_pipe(K, monkeypatch, a, w).double() - want).norm())
+
+
+@pytest.mark.parametrize("ea,ew", [(-124, 60), (-112, 60), (-104, 10), (-60, -58), (-149, 100), (126, -60), (64, 62)])
+def test_operands_and_products_near_the_ends_of_the_range(K, monkeypatch, ea, ew):
+    """Numbers that are not the sum of three parts, and products whose parts are not float32's, are as right as on the FMA pipe."""
+    n, Kd = 64, 128
+    g = torch.Generator().manual_seed(21)
+    x, y = ((1 + torch.rand(n, generator=g)).double().mul(2.0 ** e).float().to(DEV) for e in (ea, ew))
+    a = torch.zeros(n, Kd, device=DEV)
+    a[torch.arange(n), torch.arange(n)] = x
+    w = y[:, None].expand(n, Kd).contiguous()
+    out, want = torch.empty(n, n, device=DEV), x.double()[:, None] * y.double()[None, :]
+    K.gemm(a, w, out)
+    fma = on_the_fma_pipe(K, monkeypatch, a, w)
+    near = (out.double() - want).abs() <= 2.0 ** -23 * want.abs() + 2.0 ** -150
+    assert bool((near | (torch.isinf(out) & torch.isinf(fma))).all())
+    assert torch.equal(torch.isinf(out), torch.isinf(fma))
 
 
 @pytest.mark.parametrize("n_tok", [16, 32, 64, 128])
