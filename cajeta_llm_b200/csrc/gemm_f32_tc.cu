@@ -19,9 +19,9 @@
 //
 // Not every number is the sum of three such parts: not one that is infinite, or not a number, or so large that its first part would be
 // infinite (from 2^128 - 2^119 on), or so small that its last one lies below the smallest bfloat16 (below 2^-110).  The splitting
-// threads notice one, and the tile's results are then summed on the FMA pipe instead, one chain over K as gemm_simt.cu has it.  So is a
-// result that is not finite (a part's product may overflow where the product itself does not) or below 2^-100 (whose smaller parts' products
-// are too small for float32).
+// threads notice that a tile has one; the warps that add up then look for its rows of X and W, whose results, and no others, are summed on the
+// FMA pipe instead, one chain over K as gemm_simt.cu has it.  So is a result that is not finite (a part's product may overflow where the
+// product itself does not) or below 2^-100 (whose smaller parts' products are too small for float32).
 //
 // One block a tile of `feat_tile` (up to 128) features x N tokens; the weights are the rows of the product.  One thread sends for
 // the float32 tiles (TMA) into a ring as deep as shared memory allows; groups of eight warps split them into the six bfloat16
@@ -30,8 +30,8 @@
 // 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
 // tokens that chain, with many the shared memory, which every operand crosses as float32 once and as bfloat16 parts once for each of
 // its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 32;
-// 250 x 6,144 x 2,048 328 and 101; 1,777 x 6,144 x 2,048 1,822 and 347; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
-// of 4 picks 802 / 1,915 / 6,045 and 181 / 570 / 1,430.  (With the float32 operands loaded into registers instead of by TMA
+// 250 x 6,144 x 2,048 327 and 100; 1,777 x 6,144 x 2,048 1,817 and 352; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
+// of 4 picks among 60 of them 796 / 1,449 / 3,162 and 147 / 392 / 866.  (With the float32 operands loaded into registers instead of by TMA
 // 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
 #define CJ_LIB "gemm_f32_tc"
@@ -123,6 +123,20 @@ __device__ __noinline__ float chain(const float* x, const float* w, int K) {
     return s;
 }
 
+// Which of `rows` (at most 64) rows have an entry that is not the sum of three parts, a bit a row; the warp goes over a row together.
+__device__ __noinline__ unsigned long long odd_rows(const float* first, long long ld, int rows, int K) {
+    unsigned long long found = 0;
+    for (int r = 0; r < rows; ++r) {
+        uint32_t odd = 0;
+        for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+            uint4 hi, mid, lo;
+            split8(*(const float4*)(first + r * ld + k), make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi, mid, lo, odd);
+        }
+        if (__any_sync(0xffffffffu, (odd & 0xffffu) != 0)) found |= 1ull << r;
+    }
+    return found;
+}
+
 // whether a sum of the parts' products stands as it is (see the head of the file)
 __device__ __forceinline__ bool chain_free(float v) { return (fabsf(v) >= 0x1p-100f && fabsf(v) <= 3.402823466e38f) || v == 0.0f; }
 
@@ -141,7 +155,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     uint8_t* stages = raw + RING * S::RAW;
     __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int odd_flag;
+    __shared__ int odd_flag;                                  // some row of the tile has an entry that is not the sum of three parts
     __shared__ int place[3];                                  // group, first row, one past the last; group -1: no work
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -368,15 +382,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         bool again = odd_flag != 0;
 #pragma unroll
         for (int j = 0; j < COLS; ++j) again = again || !chain_free(acc[j]);
-        if (again && live) {
+        if (__any_sync(0xffffffffu, again)) {
             // (rarely: through an array in memory, so that the sums keep their registers)
             float sums[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
+            const int cols = min(COLS, n_tok - c_first);
+            const float* x = p.X + (size_t)(tok0 + c_first) * p.ldx;
             const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
+            unsigned long long odd_x = 0;
+            bool odd_w = false;
+            if (__any_sync(0xffffffffu, odd_flag != 0)) {
+                // some row of the tile: which of the warp's (its live features are its first lanes')
+                odd_x = odd_rows(x, p.ldx, cols, p.K);
+                odd_w = odd_rows(w - (long long)lane * p.K, p.K, __popc(__ballot_sync(0xffffffffu, live)), p.K) >> lane & 1;
+            }
 #pragma unroll 1
-            for (int j = 0; j < COLS && c_first + j < n_tok; ++j)
-                if (odd_flag || !chain_free(sums[j])) sums[j] = chain(p.X + (size_t)(tok0 + c_first + j) * p.ldx, w, p.K);
+            for (int j = 0; j < cols && live; ++j)
+                if (odd_w || (odd_x >> j & 1) || !chain_free(sums[j])) sums[j] = chain(x + (size_t)j * p.ldx, w, p.K);
 #pragma unroll
             for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
         }

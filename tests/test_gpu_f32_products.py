@@ -135,6 +135,38 @@ def test_gated_and_grouped(K, T, inter):
     assert K.wait_errors() == {}
 
 
+@pytest.mark.parametrize("n_tok", [16, 32, 64, 128])
+@pytest.mark.parametrize("feat_tile", [64, 128])
+def test_a_row_that_is_not_finite_changes_no_other_rows_bits(K, monkeypatch, n_tok, feat_tile):
+    monkeypatch.setattr(K, "f32_tc_tile", lambda *x: (n_tok, feat_tile))
+    a, w = rnd(140, 192, seed=22), rnd(200, 192, seed=23)
+    plain, out = torch.empty(140, 200, device=DEV), torch.empty(140, 200, device=DEV)
+    K.gemm(a, w, plain)
+    rows, feats = [3, 64, 139], [0, 70, 199]
+    a[3, 7], a[64, 100], a[139, 0], w[0, 9], w[70, 191], w[199, 31] = float("inf"), float("nan"), 2.0 ** -126, float("-inf"), 1e-40, float("nan")
+    K.gemm(a, w, out)
+    r, f = torch.ones(140, dtype=torch.bool), torch.ones(200, dtype=torch.bool)
+    r[rows], f[feats] = False, False
+    assert torch.equal(out[r][:, f], plain[r][:, f])
+    want = a.double() @ w.double().t()
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+
+
+@pytest.mark.parametrize("feat_tile", [32, 64])
+def test_another_groups_weights_change_no_bits(K, monkeypatch, feat_tile):
+    """Features that do not fill a group's last tile: the tile holds rows of the next group's weights too."""
+    monkeypatch.setattr(K, "f32_tc_tile", lambda *x: (16, feat_tile))
+    x, wg, wu = rnd(20, 128, seed=24), rnd(2, 72, 128, seed=25), rnd(2, 72, 128, seed=26)
+    offsets = torch.tensor([0, 11, 20], dtype=torch.int32, device=DEV)
+    plain, out = torch.empty(20, 72, device=DEV), torch.empty(20, 72, device=DEV)
+    for gated in (False, True):
+        K.gemm(x, wg, plain, w_up=wu if gated else None, group_offsets=offsets)
+        bad_g, bad_u = wg.clone(), wu.clone()
+        bad_g[1, 0, 3] = bad_u[1, 1, 5] = float("inf")
+        K.gemm(x, bad_g, out, w_up=bad_u if gated else None, group_offsets=offsets)
+        assert torch.equal(out[:11], plain[:11]) and torch.equal(out[11:, 2:], plain[11:, 2:])
+
+
 def test_infinite_and_missing_numbers_are_summed_as_the_fma_pipe_sums_them(K):
     a, w = rnd(40, 192, seed=10), rnd(140, 192, seed=11)
     a[3, 7], a[20, 100], a[21, 0], w[5, 9] = float("inf"), float("nan"), 3.4e38, float("-inf")
