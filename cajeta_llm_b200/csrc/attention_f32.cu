@@ -369,6 +369,7 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
         cj::launch(kern, dim3(rows == 64 ? tiles : tiles32, n_heads), dim3(4 * rows), smem(hd, vd), stream, a);
         if (int st = launch_status()) return st;
     }
+    if (tiles <= 0) a.req_start = nullptr;                     // no tile: every row by itself, whatever its request has
     if (singles || tiles <= 0) cj::launch(attention_f32_row_kernel, dim3(T, n_heads), dim3(ROW_WARPS * 32), 0, stream, a);
     return launch_status();
 }

@@ -452,10 +452,12 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v
     if (q.dtype == k_plane.dtype == torch.float32 and out.dtype == torch.float32 and head_dim % 4 == 0 and vd % 4 == 0
             and max(head_dim, vd) <= 128 and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
         tiles, tiles32, singles, requests = 0, 0, True, 0
-        if req_start is not None and h_req_start is not None:
+        if req_start is not None and h_req_start is not None and len(h_req_start) > 0:      # (an empty list: a step's lengths that nobody filled in)
             _need(req_start, "req_start", torch.int32)
             requests = len(h_req_start) - 1
             rows = [b - a for a, b in zip(h_req_start, h_req_start[1:])]
+            if h_req_start[0] != 0 or h_req_start[-1] != T or min(rows, default=0) < 0 or req_start.numel() <= requests:
+                raise KernelError(f"paged_attention: h_req_start {list(h_req_start)} does not share out {T} rows")
             tiles, tiles32 = (sum(-(-n // t) for n in rows if n > F32_FEW_ROWS) for t in (64, 32))
             singles = any(0 < n <= F32_FEW_ROWS for n in rows)
         st = library("attention_f32").cj_attention_f32(

@@ -70,3 +70,25 @@ def test_a_later_rows_infinite_value_stays_with_the_rows_that_see_it():
     K.paged_attention(q, out, kp, vp, pos, torch.zeros_like(pos), torch.arange(4, dtype=torch.int32, device=DEV)[None], 16, H, H, hd, 0, 0.125,
                       req_start=torch.tensor([0, T], dtype=torch.int32, device=DEV), h_req_start=[0, T])
     assert bool(torch.isfinite(out[:31]).all()) and not bool(torch.isfinite(out[31:]).any())
+
+
+def test_rows_by_request_have_to_cover_the_rows():
+    """A list that shares out other rows than the step's is refused; an empty one is none at all."""
+    from cajeta_llm_b200.csrc import kernels as K
+    T, H, hd = 20, 2, 64
+    g = torch.Generator().manual_seed(9)
+    kp, vp = (torch.randn(2, H, 16, hd, generator=g).to(DEV) for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g).to(DEV)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+
+    def run(**kw):
+        out = torch.full((T, H, hd), 7.0, device=DEV)
+        K.paged_attention(q, out, kp, vp, pos, torch.zeros_like(pos), torch.arange(2, dtype=torch.int32, device=DEV)[None], 16, H, H, hd, 0, 0.125, **kw)
+        return out
+
+    start = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    plain = run()
+    assert torch.equal(run(req_start=start, h_req_start=[]), plain) and torch.equal(run(req_start=start, h_req_start=[0, T]), plain)
+    for wrong in ([0], [0, T - 1], [0, T + 1], [1, T], [0, 12, 11, T], [0, 5, T]):
+        with pytest.raises(K.KernelError):
+            run(req_start=start, h_req_start=wrong)
