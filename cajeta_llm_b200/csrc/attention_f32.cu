@@ -7,6 +7,7 @@
 //   keys in chunks of 64 that begin at multiples of 64;  s_t = (q . k_t) scale, one chain of fused multiply-adds over the head;
 //   in a chunk m_c = max s_t, e_t = exp(s_t - m_c), l_c = sum e_t by a fixed tree, o_c = sum e_t v_t one chain over its keys;
 //   chunks joined in order:  m' = max(m, m_c), l = l exp(m - m') + l_c exp(m_c - m'), o likewise.
+// A score of -inf (a product that overflows) is a key without weight.
 // Keys outside a row's [from, p] enter none of its sums (they are skipped, not multiplied by zero).
 //
 // The prompt form keeps a thread on 4 rows x 4 keys of the scores and 4 rows x 8 entries of the output, operands as float4 from
@@ -41,6 +42,8 @@ __device__ __forceinline__ float score(float dot, const Args& p) {
     if (p.softcap > 0.0f) s = __fmul_rn(p.softcap, tanhf(s / p.softcap));
     return s;
 }
+// e^(s - top); with a top of -inf (every score so far is) zero: such a key has no weight, and the keys after it keep theirs
+__device__ __forceinline__ float weight(float s, float top) { return expf(s - (top == -INFINITY ? 0.0f : top)); }
 __device__ __forceinline__ int first_key(int pos, int window) { return window > 0 && pos + 1 > window ? pos + 1 - window : 0; }
 __device__ __forceinline__ float chain4(float4 a, float4 b, float s) {
     s = fmaf(a.x, b.x, s);
@@ -171,7 +174,7 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = k0 + tx + 16 * j;
-                e[j] = key >= from && key <= pos ? expf(s[i][j] - mc) : 0.0f;
+                e[j] = key >= from && key <= pos ? weight(s[i][j], mc) : 0.0f;
                 Ps[(4 * ty + i) * (KEYS + 4) + tx + 16 * j] = e[j];
             }
             float lc = __fadd_rn(__fadd_rn(e[0], e[2]), __fadd_rn(e[1], e[3]));
@@ -179,8 +182,8 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
             for (int o = 1; o < 16; o <<= 1) lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, o));
             const bool any = from < k0 + KEYS && pos >= k0;          // the row sees a key of this chunk
             const float mn = any ? fmaxf(m[i], mc) : m[i];
-            keep[i] = any ? expf(m[i] - mn) : 1.0f;
-            take[i] = any ? expf(mc - mn) : 0.0f;
+            keep[i] = any ? weight(m[i], mn) : 1.0f;
+            take[i] = any ? weight(mc, mn) : 0.0f;
             if (any) {
                 l[i] = fmaf(lc, take[i], __fmul_rn(l[i], keep[i]));
                 m[i] = mn;
@@ -299,8 +302,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
             s[0] = seen0 ? score(s[0], p) : -INFINITY;
             s[1] = seen1 ? score(s[1], p) : -INFINITY;
             const float mc = warp_max(fmaxf(s[0], s[1]));
-            e[0] = seen0 ? expf(s[0] - mc) : 0.0f;
-            e[1] = seen1 ? expf(s[1] - mc) : 0.0f;
+            e[0] = seen0 ? weight(s[0], mc) : 0.0f;
+            e[1] = seen1 ? weight(s[1], mc) : 0.0f;
             // the tree of the other kernel: keys 32 apart, then 16 apart, then 1, 2, 4, 8
             float lc = __fadd_rn(e[0], e[1]);
             lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, 16));
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
         __syncthreads();
         const int n = min(ROW_WARPS, (pos - k0) / KEYS + 1);
         for (int c = 0; c < n; ++c) {
-            const float mc = mc_s[c], mn = fmaxf(m, mc), keep = expf(m - mn), take = expf(mc - mn);
+            const float mc = mc_s[c], mn = fmaxf(m, mc), keep = weight(m, mn), take = weight(mc, mn);
             l = fmaf(lc_s[c], take, __fmul_rn(l, keep));
             if (tid < p.vd) acc = fmaf(oc[c][tid], take, __fmul_rn(acc, keep));
             m = mn;

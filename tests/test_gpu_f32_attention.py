@@ -92,3 +92,34 @@ def test_rows_by_request_have_to_cover_the_rows():
     for wrong in ([0], [0, T - 1], [0, T + 1], [1, T], [0, 12, 11, T], [0, 5, T]):
         with pytest.raises(K.KernelError):
             run(req_start=start, h_req_start=wrong)
+
+
+@pytest.mark.parametrize("tiled", [False, True])
+def test_keys_whose_scores_are_minus_infinity_have_no_weight(tiled):
+    """Whole chunks of such keys at a row's end, in its middle and at its beginning (the first score of all finite or not)."""
+    from cajeta_llm_b200.csrc import kernels as K
+    T, prior, H, hd = 9, 320, 2, 64
+    n = T + prior
+    g = torch.Generator().manual_seed(10)
+    kp, vp = (torch.randn(21, H, 16, hd, generator=g).to(DEV) for _ in range(2))
+    q = torch.randn(T, H, hd, generator=g).to(DEV)
+    q[..., 0] = 1.0
+    q[4:, :, 0] = 0.0                                                         # (0 x -inf is no number: the other rows' keys are finite)
+    kp[..., 0] = kp[..., 0].abs()
+    keys = kp.permute(1, 0, 2, 3).reshape(H, -1, hd)
+    dead = torch.zeros(keys.shape[1], dtype=torch.bool)
+    dead[:64], dead[128:192], dead[320:] = True, True, True
+    big = torch.zeros(hd, device=DEV)
+    big[0] = -3e38
+    keys[:, dead.to(DEV)] = big
+    kp = keys.reshape(H, 21, 16, hd).permute(1, 0, 2, 3).contiguous()
+    pos = torch.arange(prior, n, dtype=torch.int32, device=DEV)
+    out = torch.empty(T, H, hd, device=DEV)
+    more = dict(req_start=torch.tensor([0, T], dtype=torch.int32, device=DEV), h_req_start=[0, T]) if tiled else {}
+    K.paged_attention(q, out, kp, vp, pos, torch.zeros_like(pos), torch.arange(21, dtype=torch.int32, device=DEV)[None], 16, H, H, hd, 0, 2.0, **more)
+    values = vp.permute(1, 0, 2, 3).reshape(H, -1, hd).double()
+    for h in range(H):
+        s = (q[:4, h] @ kp.permute(1, 0, 2, 3).reshape(H, -1, hd)[h].t() * 2.0).double()
+        s = s.masked_fill(torch.arange(336, device=DEV)[None] > pos[:4, None], -math.inf)
+        assert bool(torch.isinf(s[:, :64]).all())
+        assert torch.allclose(out[:4, h].double(), torch.softmax(s, 1) @ values[h], atol=2e-5, rtol=1e-4)
