@@ -244,20 +244,23 @@ __global__ void __launch_bounds__(128) short_conv_single_kernel(const float* __r
                                                                 TO* __restrict__ out, int ld_out, int act) {
     cj::after_predecessor();
     cj::release_successor();
-    const int r = blockIdx.x, c = blockIdx.y * 128 + threadIdx.x;
+    const int r = blockIdx.x;
     const int slot = req_slot[row_req[r]];
-    if (c >= C || slot < 0) return;
-    float* st = state + (size_t)slot * slot_stride + c;
-    float v[TAPS], acc = bias ? bias[c] : 0.0f;
+    if (slot < 0) return;
+    // (one round, unless there are more channels than a grid has threads)
+    for (int c = blockIdx.y * 128 + threadIdx.x; c < C; c += gridDim.y * 128) {
+        float* st = state + (size_t)slot * slot_stride + c;
+        float v[TAPS], acc = bias ? bias[c] : 0.0f;
 #pragma unroll
-    for (int k = 0; k < TAPS - 1; ++k) v[k] = st[(size_t)k * C];
-    v[TAPS - 1] = in[(size_t)r * ld_in + c];
+        for (int k = 0; k < TAPS - 1; ++k) v[k] = st[(size_t)k * C];
+        v[TAPS - 1] = in[(size_t)r * ld_in + c];
 #pragma unroll
-    for (int k = 0; k < TAPS; ++k) acc = fmaf(w[(size_t)c * TAPS + k], v[k], acc);
-    if (act) acc = acc / (1.0f + expf(-acc));
-    out[(size_t)r * ld_out + c] = from_f32<TO>(acc);
+        for (int k = 0; k < TAPS; ++k) acc = fmaf(w[(size_t)c * TAPS + k], v[k], acc);
+        if (act) acc = acc / (1.0f + expf(-acc));
+        out[(size_t)r * ld_out + c] = from_f32<TO>(acc);
 #pragma unroll
-    for (int k = 0; k < TAPS - 1; ++k) st[(size_t)k * C] = v[k + 1];
+        for (int k = 0; k < TAPS - 1; ++k) st[(size_t)k * C] = v[k + 1];
+    }
 }
 
 __global__ void short_conv_commit_kernel(const float* __restrict__ in, int ld_in, int C, int taps, float* __restrict__ state,
@@ -1320,10 +1323,9 @@ CJ_EXPORT int cj_short_conv(const float* in, int ld_in, int C, int taps, const f
     if (!in || !w || !state || !row_req || !req_start || !req_slot || !out || C <= 0 || taps < 1) return CJ_ERR_ARG;
     // many rows: four channels and 16 rows a thread.  From 128 rows on: 8 x 12 blocks for 6,144 channels, a block an SM nearly
     const int out_bytes = out_dtype == CJ_F32 ? 16 : 8;
-    if (T >= CONV_MIN_ROWS && taps >= 2 && taps <= 4 && (C | ld_in | ld_out) % 4 == 0 && ((uintptr_t)in & 15) == 0 && (uintptr_t)out % out_bytes == 0
+    if (T >= CONV_MIN_ROWS && taps >= 2 && taps <= 4 && C <= 65535 * 512 && (C | ld_in | ld_out) % 4 == 0 && ((uintptr_t)in & 15) == 0 && (uintptr_t)out % out_bytes == 0
         && (out_dtype == CJ_F32 || out_dtype == CJ_BF16)) {
         const dim3 tiles((T + CONV_ROWS - 1) / CONV_ROWS, (C + 511) / 512);
-        if (tiles.y > 65535) return CJ_ERR_SIZE;
 #define LAUNCH_TILE(TO, N) cj::launch(short_conv_tile_kernel<TO, N>, tiles, dim3(128), 0, stream, in, ld_in, C, w, bias, state, slot_stride, row_req, \
                                       req_start, req_slot, (TO*)out, ld_out, act, T)
 #define LAUNCH_TAPS(TO)                                                                                                 \
@@ -1353,8 +1355,7 @@ CJ_EXPORT int cj_short_conv_single(const float* in, int ld_in, int C, int taps, 
     if (T <= 0) return 0;
     if (!in || !w || !state || !row_req || !req_slot || !out || C <= 0) return CJ_ERR_ARG;
     if (taps < 2 || taps > 4) return CJ_ERR_SIZE;
-    const dim3 grid(T, (C + 127) / 128);
-    if (grid.y > 65535) return CJ_ERR_SIZE;
+    const dim3 grid(T, min((C + 127) / 128, 65535));
 #define LAUNCH_ONE(TO, N) cj::launch(short_conv_single_kernel<TO, N>, grid, dim3(128), 0, stream, in, ld_in, C, w, bias, state, slot_stride, row_req, \
                                      req_slot, (TO*)out, ld_out, act)
 #define LAUNCH_TAPS(TO)                                                                                                 \

@@ -133,3 +133,14 @@ def test_a_normed_mixers_output_product_is_one_sum(monkeypatch, rows):
     monkeypatch.setattr(K, "gemm_tc", lambda *a, **k: (cuts.append(k.get("k_splits", 1)), plain(*a, **k)))
     r.step([StepEntry(r.admit(), [i], [0]) for i in range(rows)])
     assert cuts and set(cuts) == {1}
+
+
+def test_single_tokens_convolution_of_more_channels_than_a_grid_has_threads():
+    from types import SimpleNamespace
+    from cajeta_llm_b200.csrc import kernels as K
+    C, taps = 65535 * 128 + 5, 2
+    x, w, state = rnd(1, C, seed=18), rnd(C, taps, seed=19), rnd(1, C, seed=20)
+    at = torch.zeros(1, dtype=torch.int32, device=DEV)
+    want, out = w[:, 0] * state[0] + w[:, 1] * x[0], torch.empty(1, C, device=DEV)
+    K.short_conv_moved(x, 0, C, taps, w, None, state, SimpleNamespace(row_req=at, req_slot=at, all_single=True), out, activate=False)
+    assert torch.allclose(out[0], want, atol=1e-5, rtol=1e-5) and torch.equal(state, x)
