@@ -16,28 +16,30 @@ def test_walked_and_single_tokens_agree(mode, heads, groups, rows, cols, lengths
     if mode >= 2:
         groups = heads
     R, T = len(lengths), sum(lengths)
-    x = torch.randn(T, 2 * groups * rows + heads * cols + 7, generator=g).to(DEV)
-    raw = torch.randn(T, heads * (rows if mode == 2 else 1) + heads + 3, generator=g).to(DEV)
     off_dt, off_beta = 1, 2 + heads
     A, bias, skip = (torch.randn(heads, generator=g).to(DEV) * 0.3 for _ in range(3))
     n = K.state_scan_floats(heads, rows, cols, mode)
     slots = torch.randperm(R + 1, generator=g)[:R].int().to(DEV)
     starts = [sum(lengths[:i]) for i in range(R + 1)]
-    results = []
-    for single in (False, True):
-        state, out = torch.zeros(R + 1, n + 3, device=DEV), torch.zeros(T, heads * cols, device=DEV)
+    states = [torch.zeros(R + 1, n + 3, device=DEV) for _ in range(2)]
+    for step in range(2):                                                    # from empty states, then from those the first step left
+        x = torch.randn(T, 2 * groups * rows + heads * cols + 7, generator=g).to(DEV)
+        raw = torch.randn(T, heads * (rows if mode == 2 else 1) + heads + 3, generator=g).to(DEV)
+        outs = []
+        for single, state in zip((False, True), states):
+            out = torch.zeros(T, heads * cols, device=DEV)
 
-        def scan(lo, hi, slot, req_start):
-            K.state_scan(mode, x[lo:hi], 3, 3 + groups * rows, 3 + 2 * groups * rows, raw[lo:hi], off_dt, off_beta, A, bias, skip, state, 3,
-                         torch.tensor(req_start, dtype=torch.int32, device=DEV), slot, out[lo:hi], slot.numel(), heads, groups, rows, cols,
-                         q_scale=0.125, c0=5.0 if mode == 3 else 0.25, c1=1e-6)
+            def scan(lo, hi, slot, req_start):
+                K.state_scan(mode, x[lo:hi], 3, 3 + groups * rows, 3 + 2 * groups * rows, raw[lo:hi], off_dt, off_beta, A, bias, skip, state, 3,
+                             torch.tensor(req_start, dtype=torch.int32, device=DEV), slot, out[lo:hi], slot.numel(), heads, groups, rows, cols,
+                             q_scale=0.125, c0=5.0 if mode == 3 else 0.25, c1=1e-6)
 
-        if single:
-            for r in range(R):
-                for t in range(starts[r], starts[r + 1]):
-                    scan(t, t + 1, slots[r:r + 1].contiguous(), [0, 1])
-        else:
-            scan(0, T, slots, starts)
-        results.append((state, out))
-    assert bool(results[0][1].abs().sum() > 0)
-    assert torch.equal(results[0][1], results[1][1]) and torch.equal(results[0][0], results[1][0])
+            if single:
+                for r in range(R):
+                    for t in range(starts[r], starts[r + 1]):
+                        scan(t, t + 1, slots[r:r + 1].contiguous(), [0, 1])
+            else:
+                scan(0, T, slots, starts)
+            outs.append(out)
+        assert bool(outs[0].abs().sum() > 0) and bool(states[0][slots.long()].abs().sum(1).min() > 0)
+        assert torch.equal(outs[0], outs[1]) and torch.equal(states[0], states[1])
