@@ -414,59 +414,51 @@ __global__ void __launch_bounds__(LA_HEADS * 32) latent_attention_tile_kernel(
     }
 }
 
-// the stretches of a row's keys, merged in order: out = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z.  The stretches' factors are worked
-// out side by side, a thread each, and the sums read four stretches at a time.
-constexpr int MERGE_MOST = 128;
+// the stretches of a row's keys, merged in order: out = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z.  The factors of 128 stretches at a
+// time are worked out side by side, a thread each; a thread then has up to 8 entries of the sum.
+constexpr int MERGE = 128;
 template <typename TC>
-__global__ void __launch_bounds__(MERGE_MOST) latent_merge_few_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits,
-                                                                       int split_keys, int window, int rank, int heads, int T,
-                                                                       const int* __restrict__ positions, TC* __restrict__ out) {
+__global__ void __launch_bounds__(MERGE) latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits,
+                                                             int split_keys, int window, int rank, int heads, int T,
+                                                             const int* __restrict__ positions, TC* __restrict__ out) {
     cj::after_predecessor();
     cj::release_successor();
-    __shared__ float f[MERGE_MOST], top[4], sum[4];
+    __shared__ float f[MERGE], top[4], sum[4];
     const int r = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5;
     const int n_keys = window > 0 ? min(positions[r] + 1, window) : positions[r] + 1;
     const int nz = min(splits, (n_keys + split_keys - 1) / split_keys);
     const size_t item = (size_t)r * heads + head;
-    const float2 ml = tid < nz ? *(const float2*)(part_ml + (item * splits + tid) * 2) : make_float2(-INFINITY, 0.0f);
-    const float wm = warp_max(ml.x);
+    const float* ml = part_ml + item * splits * 2;              // (read a float at a time: it need not lie on 8 bytes)
+    float wm = -INFINITY;
+    for (int z = tid; z < nz; z += MERGE) wm = fmaxf(wm, ml[2 * z]);
+    wm = warp_max(wm);
     if ((tid & 31) == 0) top[warp] = wm;
     __syncthreads();
     const float M = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
-    const float e = tid < nz ? expf(ml.x - M) : 0.0f;
-    f[tid] = e;
-    const float ws = warp_sum(e * ml.y);
-    if ((tid & 31) == 0) sum[warp] = ws;
-    __syncthreads();
-    const float inv = 1.0f / ((sum[0] + sum[1]) + (sum[2] + sum[3]));
-    const float* acc = part_acc + item * splits * rank;
-    for (int c = tid; c < rank; c += MERGE_MOST) {
-        float v = 0.0f;
+    const float* acc = part_acc + item * splits * rank + tid;
+    float v[8] = {}, total = 0.0f;                              // (a latent has at most 1,024 entries)
+    for (int z0 = 0; z0 < nz; z0 += MERGE, acc += (size_t)MERGE * rank) {
+        const int z = z0 + tid;
+        const float e = z < nz ? expf(ml[2 * z] - M) : 0.0f;
+        const float ws = warp_sum(z < nz ? e * ml[2 * z + 1] : 0.0f);
+        if (z0 > 0) __syncthreads();                            // the factors before have been used
+        f[tid] = e;
+        if ((tid & 31) == 0) sum[warp] = ws;
+        __syncthreads();
+        total += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        const int n = min(MERGE, nz - z0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (tid + MERGE * i >= rank) break;
 #pragma unroll 4
-        for (int z = 0; z < nz; ++z) v = fmaf(f[z], acc[(size_t)z * rank + c], v);
-        out[((size_t)head * T + r) * rank + c] = from_f32<TC>(v * inv);
+            for (int k = 0; k < n; ++k) v[i] = fmaf(f[k], acc[(size_t)k * rank + MERGE * i], v[i]);
+        }
     }
-}
-
-template <typename TC>
-__global__ void latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits, int split_keys,
-                                    int window, int rank, int heads, int T, const int* __restrict__ positions, TC* __restrict__ out) {
-    cj::after_predecessor();
-    cj::release_successor();
-    const int r = blockIdx.x, head = blockIdx.y;
-    const int n_keys = window > 0 ? min(positions[r] + 1, window) : positions[r] + 1;
-    const int nz = min(splits, (n_keys + split_keys - 1) / split_keys);
-    const size_t item = (size_t)r * heads + head;
-    const float* ml = part_ml + item * splits * 2;
-    float M = -INFINITY;
-    for (int z = 0; z < nz; ++z) M = fmaxf(M, ml[2 * z]);
-    float L = 0.0f;
-    for (int z = 0; z < nz; ++z) L += expf(ml[2 * z] - M) * ml[2 * z + 1];
-    const float inv = 1.0f / L;
-    for (int e = threadIdx.x; e < rank; e += blockDim.x) {
-        float v = 0.0f;
-        for (int z = 0; z < nz; ++z) v = fmaf(expf(ml[2 * z] - M), part_acc[(item * splits + z) * rank + e], v);
-        out[((size_t)head * T + r) * rank + e] = from_f32<TC>(v * inv);
+    const float inv = 1.0f / total;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int c = tid + MERGE * i;
+        if (c < rank) out[((size_t)head * T + r) * rank + c] = from_f32<TC>(v[i] * inv);
     }
 }
 
@@ -574,15 +566,12 @@ CJ_EXPORT int cj_latent_attention(const float* q_abs, const float* q_rot, const 
         cj::launch(latent_attention_kernel<TC, N>, grid, dim3(LA_HEADS * 32), smem, stream, q_abs, q_rot, (const TC*)plane, \
                    rank, rot, heads, T, positions, row_req, table, table_stride, page_tokens, window, scale, (TC*)out, row_words, \
                    split_keys, pa, pm, sink);                                                                          \
-        MERGE(TC);                                                                                                     \
+        LAUNCH_MERGE(TC);                                                                                              \
     } while (0)
-#define MERGE(TC)                                                                                                      \
+#define LAUNCH_MERGE(TC)                                                                                               \
     do {                                                                                                               \
-        if (split_keys > 0 && splits <= MERGE_MOST)                                                                    \
-            cj::launch(latent_merge_few_kernel<TC>, dim3(T, heads), dim3(MERGE_MOST), 0, stream, (const float*)pa, (const float*)pm, splits, \
-                       split_keys, window, rank, heads, T, positions, (TC*)out);                                       \
-        else if (split_keys > 0)                                                                                       \
-            cj::launch(latent_merge_kernel<TC>, dim3(T, heads), dim3(128), 0, stream, (const float*)pa, (const float*)pm, splits, \
+        if (split_keys > 0)                                                                                            \
+            cj::launch(latent_merge_kernel<TC>, dim3(T, heads), dim3(MERGE), 0, stream, (const float*)pa, (const float*)pm, splits, \
                        split_keys, window, rank, heads, T, positions, (TC*)out);                                       \
     } while (0)
     // a bfloat16 cache of 16-byte pieces
@@ -603,7 +592,7 @@ CJ_EXPORT int cj_latent_attention(const float* q_abs, const float* q_rot, const 
         if (rank <= 512) LAUNCH_TILE(1);
         else LAUNCH_TILE(2);
 #undef LAUNCH_TILE
-        MERGE(__nv_bfloat16);
+        LAUNCH_MERGE(__nv_bfloat16);
         return launch_status();
     }
 #define PICK(TC)                                  \
@@ -618,7 +607,7 @@ CJ_EXPORT int cj_latent_attention(const float* q_abs, const float* q_rot, const 
     else return CJ_ERR_DTYPE;
 #undef PICK
 #undef LAUNCH
-#undef MERGE
+#undef LAUNCH_MERGE
     return launch_status();
 }
 
