@@ -28,11 +28,12 @@
 // tiles of a stage, a group every G-th block of K; one warp issues the products; the last warps add the accumulators up
 // and store.  A block of K is a chain of short waits for a group (tile landed, stage free, stores visible to the products: some
 // 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
-// tokens that chain, with many the shared memory, which every operand crosses as float32 once and as bfloat16 parts once for each of
-// its products.  Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 32;
-// 250 x 6,144 x 2,048 327 and 100; 1,777 x 6,144 x 2,048 1,817 and 352; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens
-// of 4 picks among 60 of them 796 / 1,449 / 3,162 and 147 / 392 / 866.  (With the float32 operands loaded into registers instead of by TMA
-// 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
+// tokens that chain, with many one group's going through read, split, write and wait (issue slots 61 % used, shared memory 44 %, integer and
+// conversion pipe 40 %, tensor pipe 33 %; shared memory has no room for a second group).
+// Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 32; 250 x 6,144 x 2,048 327 and 100;
+// 1,777 x 6,144 x 2,048 1,817 and 352; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens of 4 picks among 60 of them
+// 796 / 1,449 / 3,162 and 147 / 392 / 866.  (With the float32 operands loaded into registers instead of by TMA 1,777 x 6,144 took 815: one
+// load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
 #define CJ_LIB "gemm_f32_tc"
 #include "common.cuh"
