@@ -1,8 +1,8 @@
 // Paged attention of the float32 path: float32 queries, cache and arithmetic, head sizes up to 128 that are multiples of four.
 // The formulas are attention_paged.cu's (window, capped scores, a gate per row and head, a constant sink score).
 //
-// Two kernels, one result.  A portion of a prompt goes 64 rows of a request and one head a block, so that a key read from the cache
-// serves 64 rows; a request with few rows (a decoded token) goes a row and head a block, its warps sharing the keys.  A row
+// Two kernels, one result.  A portion of a prompt goes 64 or 32 rows of a request and one head a block, so that a key read from the cache
+// serves as many rows; a request with few rows (a decoded token) goes a row and head a block, its warps sharing the keys.  A row
 // must not depend on which of the two ran or on how its prompt was cut, so both do the same float32 operations for it, in this order:
 //   keys in chunks of 64 that begin at multiples of 64;  s_t = (q . k_t) scale, one chain of fused multiply-adds over the head;
 //   in a chunk m_c = max s_t, e_t = exp(s_t - m_c), l_c = sum e_t by a fixed tree, o_c = sum e_t v_t one chain over its keys;
@@ -12,8 +12,8 @@
 //
 // The prompt form keeps a thread on 4 rows x 4 keys of the scores and 4 rows x 8 entries of the output, operands as float4 from
 // shared memory (12 shared-memory wavefronts a 16 FMA clocks): bound by the FMA pipe and by waiting for a chunk's keys, which nothing
-// fetches ahead but the SM's other block.  1,777 rows of one prompt, 16 heads of 128: 735 us, where a row and head a block with a
-// key a lane took 12,700 us.  One row at 570 keys: 34 us, 120 us before.
+// fetches ahead but the SM's other block, where a second one fits.  1,777 rows of one prompt, 16 heads of 128: 713 us, where a row and head
+// a block with a key a lane took 12,700 us.  One row at 570 keys: 34 us, 120 us before.
 #define CJ_LIB "attention_f32"
 #include "common.cuh"
 
@@ -358,18 +358,29 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
     Args a{q, out, kplane, vplane, positions, row_req, req_start, requests, table, table_stride, page_tokens, n_heads, n_kv, hd, vd, window,
            scale, softcap, head_gate, gate_ld, sink, few_rows};
     if (tiles > 0) {
-        // Tiles of 32 rows when those of 64 would leave SMs without a second block: 256 rows at 950 keys, 16 heads 185 -> 138 us.
-        const int rows = (long long)tiles * n_heads >= 2 * 148 ? 64 : 32, wide = vd <= 64 ? 0 : 1;
-        auto smem = [rows](int h, int v) { return (int)sizeof(float) * ((rows + KEYS) * (h + 4) + KEYS * v + rows * (KEYS + 4)); };
+        // Tiles of 64 rows where an SM holds two of them and the step has two for every SM, else of 32.  What an SM holds is what hides the
+        // waits for keys: with heads of 128 a tile of 64 rows takes 115 KB and is alone (1,777 rows of 16 heads 728 us, with tiles of 32
+        // 713; 768 rows 187 and 172; 256 rows at 950 keys 185 and 137), with heads of 96 two fit (1,777 rows at 2,277 keys 925 and 987).
+        static int sms = 0, sm_bytes = 0;
+        if (!sms) {
+            int dev = 0;
+            cudaError_t e = cudaGetDevice(&dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return (int)e;
+        }
+        auto smem = [](int rows, int h, int v) { return (int)sizeof(float) * ((rows + KEYS) * (h + 4) + KEYS * v + rows * (KEYS + 4)); };
+        const bool two = 2 * (smem(64, hd, vd) + 1024) <= sm_bytes;
+        const int rows = two && (long long)tiles * n_heads >= 2 * sms ? 64 : 32, wide = vd <= 64 ? 0 : 1;
         auto kern = rows == 64 ? (wide ? attention_f32_tile_kernel<2, 64> : attention_f32_tile_kernel<1, 64>)
                                : (wide ? attention_f32_tile_kernel<2, 32> : attention_f32_tile_kernel<1, 32>);
         static bool sized[2][2] = {};
         if (!sized[rows == 64][wide]) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(MAX_DIM, MAX_DIM));
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(rows, MAX_DIM, MAX_DIM));
             if (e != cudaSuccess) return (int)e;
             sized[rows == 64][wide] = true;
         }
-        cj::launch(kern, dim3(rows == 64 ? tiles : tiles32, n_heads), dim3(4 * rows), smem(hd, vd), stream, a);
+        cj::launch(kern, dim3(rows == 64 ? tiles : tiles32, n_heads), dim3(4 * rows), smem(rows, hd, vd), stream, a);
         if (int st = launch_status()) return st;
     }
     if (tiles <= 0) a.req_start = nullptr;                     // no tile: every row by itself, whatever its request has

@@ -15,7 +15,8 @@ DEV = "cuda:0"
     ([130, 9, 70, 3], [50, 5, 33, 100], 6, 2, 128, 64, 40, 30.0, True, None, 16),
     ([65, 200], [7, 90], 4, 1, 24, 100, 33, 0.0, False, 0.0, 4),
     ([12], [600], 2, 1, 4, 128, 0, 0.0, False, None, 16),
-    ([640, 9, 65], [0, 700, 10], 32, 4, 128, 128, 0, 0.0, False, None, 16),      # tiles of 64 rows (the others: of 32)
+    ([640, 9, 65], [0, 700, 10], 32, 4, 128, 128, 0, 0.0, False, None, 16),
+    ([640, 9, 65], [0, 700, 10], 32, 4, 96, 96, 0, 0.0, False, None, 16),        # tiles of 64 rows (so the next; the others: of 32)
     ([600, 12], [3, 0], 32, 32, 60, 64, 50, 20.0, True, 0.5, 16)])
 def test_tiles_and_rows_agree(rows, prior, H, G, hd, vd, window, cap, gated, sink, page):
     from cajeta_llm_b200.csrc import kernels as K
