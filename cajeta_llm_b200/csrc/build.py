@@ -45,6 +45,7 @@ LIBRARIES: Dict[str, str] = {
     "attention_decode": "attention_decode.cu",
     "attention_prefill": "attention_prefill.cu",
     "attention_prefill_tc": "attention_prefill_tc.cu",
+    "attention_flash_tc": "attention_flash_tc.cu",
     "random_fill": "random_fill.cu",
     "recurrent": "recurrent.cu",
     "decay_attention": "decay_attention.cu",

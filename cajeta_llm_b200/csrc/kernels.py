@@ -478,6 +478,21 @@ def diff_tile_shape(head_dim: int, value_dim: int) -> bool:
     return head_dim in (32, 64, 128) and value_dim in (64, 128)
 
 
+def diff_attention_tc(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor, req_start: torch.Tensor,
+                      req_prior: torch.Tensor, n_requests: int, table: torch.Tensor, page_tokens: int, n_heads: int, n_kv: int, head_dim: int,
+                      value_dim: int, window: int, scale: float, lam: float, eps: float, out_scale: float) -> None:
+    """The tiled form of :func:`diff_attention` on the tcgen05 tensor cores: 128 rows of a request and a head a block.  Maps of 64 or 128,
+    values of 64 or 128, pages of a multiple of 16 tokens, a positive scale."""
+    for n, t in (("q", q), ("out", out), ("k_plane", k_plane), ("v_plane", v_plane)):
+        _need(t, n, torch.bfloat16)
+    _need(req_start, "req_start", torch.int32), _need(req_prior, "req_prior", torch.int32), _need(table, "table", torch.int32)
+    st = library("attention_flash_tc").cj_diff_attention_tc(
+        _ptr(q), _ptr(out), _ptr(k_plane), _ptr(v_plane), _i(k_plane.shape[0]), _ptr(req_start), _ptr(req_prior), _i(n_requests),
+        _i(q.shape[0]), _ptr(table), _i(table.stride(0)), _i(page_tokens), _i(n_heads), _i(n_kv), _i(head_dim), _i(value_dim), _i(window),
+        _f(scale), _f(lam), _f(eps), _f(out_scale), _stream())
+    _check(st, "diff_attention_tc")
+
+
 def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor, positions: torch.Tensor,
                    row_req: torch.Tensor, table: torch.Tensor, page_tokens: int, n_heads: int, n_kv: int, head_dim: int,
                    value_dim: int, window: int, scale: float, lam: float, eps: float, out_scale: float,
@@ -505,6 +520,14 @@ def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_
         _need(req_start, "req_start", torch.int32), _need(req_prior, "req_prior", torch.int32)
         if tile_rows not in (16, 64):
             raise KernelError(f"diff_attention: tile_rows must be 16 or 64, found {tile_rows}")
+        # On tcgen05 from 256 rows on (16 heads, us, tile by mma.sync -> tcgen05): 256 rows behind 3,000 120 -> 80, 8 times 40 rows 29 -> 25,
+        # 4 times 200 33 -> 21; below, where keys are dealt to several blocks or a tile of 128 rows is mostly empty, not: 64 rows behind
+        # 3,000 58 -> 72, 8 times 30 rows 13 -> 18
+        if (splits is None and tile_rows == 64 and T >= 256 and head_dim >= 64 and page_tokens % 16 == 0 and scale > 0.0 and window >= 0
+                and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
+            diff_attention_tc(q, out, k_plane, v_plane, req_start, req_prior, n_requests, table, page_tokens, n_heads, n_kv, head_dim, value_dim,
+                              window, scale, lam, eps, out_scale)
+            return
         blocks = (-(-T // tile_rows) + n_requests) * n_heads
         fill = _sm_count() * (3 if tile_rows == 16 else 1)            # blocks that fill the machine
         if splits is None:
@@ -1165,12 +1188,17 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, plane: torch.Tens
 
 # -- the plain form for long prompt portions: keys and values built per head, a flash kernel over them --
 def latent_gather(plane: torch.Tensor, rank: int, tok_req: torch.Tensor, tok_pos: torch.Tensor, table: torch.Tensor,
-                  page_tokens: int, c_all: torch.Tensor) -> None:
-    """c_all[n] = the latent of (request tok_req[n], position tok_pos[n]) from the paged cache; bfloat16."""
+                  page_tokens: int, c_all: torch.Tensor, kr: Optional[torch.Tensor] = None) -> None:
+    """c_all[n] = the latent of (request tok_req[n], position tok_pos[n]) from the paged cache, kr[n] (64 entries) its rotated key part and
+    zeros behind it; bfloat16."""
     _need(plane, "plane", torch.bfloat16), _need(c_all, "c_all", torch.bfloat16), _need(table, "table", torch.int32)
     _need(tok_req, "tok_req", torch.int32), _need(tok_pos, "tok_pos", torch.int32)
+    if kr is not None:
+        _need(kr, "kr", torch.bfloat16)
+        if tuple(kr.shape) != (tok_req.numel(), 64):
+            raise KernelError("latent_gather: kr must hold 64 entries a token")
     st = library("latent_prefill").cj_latent_gather(_ptr(plane), _i(plane.shape[-1]), _i(rank), _ptr(tok_req), _ptr(tok_pos), _ptr(table),
-                                                    _i(table.stride(0)), _i(page_tokens), _ptr(c_all), _i(tok_req.numel()), _stream())
+                                                    _i(table.stride(0)), _i(page_tokens), _ptr(c_all), _ptr(kr), _i(tok_req.numel()), _stream())
     _check(st, "latent_gather")
 
 
@@ -1219,6 +1247,36 @@ def latent_flash(qx: torch.Tensor, out: torch.Tensor, kx: torch.Tensor, vx: torc
                                                    _i(requests), _i(qx.shape[0]), _i(heads), _i(qx.shape[2]), _i(vx.shape[2]), _i(window),
                                                    _i(1 if exact_weights else 0), _f(scale), _ptr(sink), _stream())
     _check(st, "latent_flash")
+
+
+def latent_tc_shape(dim: int, rot: int, vdim: int, scale: float) -> bool:
+    """Whether :func:`latent_attention_tc` takes these sizes."""
+    return dim in (64, 128) and 0 < rot <= 64 and vdim in (64, 128) and scale > 0.0
+
+
+def latent_attention_tc(qx: torch.Tensor, out: torch.Tensor, kp: torch.Tensor, kr: torch.Tensor, vp: torch.Tensor, req_start: torch.Tensor,
+                        req_prior: torch.Tensor, req_base: torch.Tensor, requests: int, heads: int, dim: int, vdim: int, scale: float,
+                        sink: Optional[torch.Tensor] = None, window: int = 0, exact_weights: bool = False,
+                        gate: Optional[torch.Tensor] = None, gate_offset: int = 0, by_entry: bool = False) -> None:
+    """:func:`latent_flash` on the tcgen05 tensor cores, with the keys and values where the products left them and the gate of
+    :func:`latent_gate_rows` on the way out: qx [T, heads, dim + 64], kp [N, heads * dim], kr [N, 64], vp [N, heads * vdim],
+    out [T, heads * vdim], bfloat16."""
+    if sink is not None:
+        _need(sink, "sink", torch.float32)
+    for n, t in (("qx", qx), ("out", out), ("kp", kp), ("kr", kr), ("vp", vp)):
+        _need(t, n, torch.bfloat16)
+    for n, t in (("req_start", req_start), ("req_prior", req_prior), ("req_base", req_base)):
+        _need(t, n, torch.int32)
+    T, N = qx.shape[0], kp.shape[0]
+    if (qx.numel() != T * heads * (dim + 64) or kp.numel() != N * heads * dim or kr.numel() != N * 64 or vp.numel() != N * heads * vdim
+            or out.numel() != T * heads * vdim):
+        raise KernelError("latent_attention_tc: sizes do not agree")
+    gate_ptr, gate_ld = _gate(gate, gate_offset)
+    st = library("attention_flash_tc").cj_latent_attention_tc(
+        _ptr(qx), _ptr(out), _ptr(kp), _ptr(kr), _ptr(vp), _i(N), _ptr(req_start), _ptr(req_prior), _ptr(req_base), _i(requests), _i(T),
+        _i(heads), _i(dim), _i(vdim), _i(window), _i(1 if exact_weights else 0), _f(scale), _ptr(sink), gate_ptr, _i(gate_ld),
+        _i(1 if by_entry else 0), _stream())
+    _check(st, "latent_attention_tc")
 
 
 def latent_gate_rows(o: torch.Tensor, gate: Optional[torch.Tensor], gate_offset: int, heads: int, vdim: int, out: torch.Tensor,
@@ -1534,7 +1592,7 @@ def wait_errors() -> Dict[str, int]:
     when all is well.  Only libraries that are already loaded are asked."""
     found = {}
     for name, symbol in (("gemm_tc", "cj_gemm_tc_error"), ("gemm_tc2", "cj_gemm_tc2_error"), ("gemm_f32_tc", "cj_gemm_f32_tc_error"),
-                         ("attention_prefill_tc", "cj_prefill_attention_tc_error")):
+                         ("attention_prefill_tc", "cj_prefill_attention_tc_error"), ("attention_flash_tc", "cj_attention_flash_tc_error")):
         lib = _libs.get(name)
         if lib is not None:
             code = int(getattr(lib, symbol)())

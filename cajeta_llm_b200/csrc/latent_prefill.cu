@@ -10,7 +10,7 @@
 // than a few rows a request; decoding keeps the absorbed kernel, which reads a cache
 // entry once for all heads.
 //
-//   latent_gather   c of every token of the step's requests (cached and new) -> [N, kv_rank]
+//   latent_gather   c of every token of the step's requests (cached and new) -> [N, kv_rank], and r -> [N, 64]
 //   latent_kv_pack  [N, H, DK] = [k_plain(h) | r | 0], [N, H, DV] = [v(h) | 0]   (DK, DV: padded to 64)
 //   latent_q_pack   [T, H, DK] = [q_plain(h) | rotate(q_rot(h)) | 0]
 //   latent_flash    out [T, H, DV]
@@ -258,16 +258,25 @@ __global__ void __launch_bounds__(THREADS) latent_flash_kernel(
     }
 }
 
-__global__ void latent_gather_kernel(const __nv_bfloat16* __restrict__ plane, int width, int rank, const int* __restrict__ tok_req,
-                                     const int* __restrict__ tok_pos, const int* __restrict__ table, int table_stride,
-                                     int page_tokens, __nv_bfloat16* __restrict__ c_all) {
+// The latent of token n to c_all[n] and, where wanted, its rotated key part to kr[n] (64 entries, zeros past `rot`).  V entries (16 bytes,
+// or one where the sizes leave no such alignment) a thread.
+template <typename V>
+__global__ void __launch_bounds__(128) latent_gather_kernel(const __nv_bfloat16* __restrict__ plane, int width, int rank, const int* __restrict__ tok_req,
+                                                            const int* __restrict__ tok_pos, const int* __restrict__ table, int table_stride,
+                                                            int page_tokens, __nv_bfloat16* __restrict__ c_all, __nv_bfloat16* __restrict__ kr) {
     cj::after_predecessor();
     cj::release_successor();
+    constexpr int N = sizeof(V) / 2;
     const int n = blockIdx.x;
     const int pos = tok_pos[n];
     const int page = table[(size_t)tok_req[n] * table_stride + pos / page_tokens];
-    const __nv_bfloat16* src = plane + ((size_t)page * page_tokens + pos % page_tokens) * width;
-    for (int e = threadIdx.x; e < rank; e += blockDim.x) c_all[(size_t)n * rank + e] = src[e];
+    const V* src = (const V*)(plane + ((size_t)page * page_tokens + pos % page_tokens) * width);
+    V* c = (V*)(c_all + (size_t)n * rank);
+    const int mine = rank / N, all = mine + (kr ? 64 / N : 0);
+    for (int e = threadIdx.x; e < all; e += blockDim.x) {
+        if (e < mine) c[e] = src[e];
+        else ((V*)(kr + (size_t)n * 64))[e - mine] = e < width / N ? src[e] : V{};
+    }
 }
 
 __global__ void latent_kv_pack_kernel(const __nv_bfloat16* __restrict__ kp, const __nv_bfloat16* __restrict__ vp,
@@ -322,6 +331,61 @@ __global__ void latent_q_pack_kernel(const float* __restrict__ q, int ld, int he
     }
 }
 
+// The same for sizes in eights (the rotated part's halves too), 16-byte aligned rows: eight entries a thread, a row's angles worked out once
+// for its heads.  2,048 rows of 16 heads of 128 + 64 (25 MB read, 12.6 MB written, bound by memory), cold: 29 us
+// an entry a thread with its own angle, 14 us this way.
+__global__ void __launch_bounds__(256) latent_q_pack8_kernel(const float* __restrict__ q, int ld, int heads, int dim, int rot, int rotary, int halves,
+                                                             float mag, const float* __restrict__ inv_freq, const int* __restrict__ positions,
+                                                             int DK, __nv_bfloat16* __restrict__ qx) {
+    cj::after_predecessor();
+    cj::release_successor();
+    __shared__ float2 turn[128];
+    const int r = blockIdx.x;
+    const float* src = q + (size_t)r * ld;
+    const int per = dim + rot, hr = rotary / 2;
+    for (int i = threadIdx.x; i < hr; i += 256) {
+        const float a = (float)positions[r] * inv_freq[i];
+        turn[i] = make_float2(mag * cosf(a), mag * sinf(a));
+    }
+    __syncthreads();
+    __nv_bfloat16* dst = qx + (size_t)r * heads * DK;
+    const int groups = DK / 8;
+    for (int i = threadIdx.x; i < heads * groups; i += 256) {
+        const int h = i / groups, e = (i - h * groups) * 8;
+        float v[8];
+        if (e >= per) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = 0.0f;
+        } else {
+            const float* at = src + h * per + e;
+            *(float4*)v = *(const float4*)at;
+            *(float4*)(v + 4) = *(const float4*)(at + 4);
+            const int j = e - dim;
+            if (j >= 0 && j < rotary) {
+                if (halves) {
+                    const bool second = j >= hr;
+                    float o[8];
+                    const float* other = at + (second ? -hr : hr);
+                    *(float4*)o = *(const float4*)other;
+                    *(float4*)(o + 4) = *(const float4*)(other + 4);
+                    const float2* t = turn + (second ? j - hr : j);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] = second ? v[k] * t[k].x + o[k] * t[k].y : v[k] * t[k].x - o[k] * t[k].y;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 t = turn[j / 2 + k];
+                        const float u = v[2 * k], w = v[2 * k + 1];
+                        v[2 * k] = u * t.x - w * t.y;
+                        v[2 * k + 1] = w * t.x + u * t.y;
+                    }
+                }
+            }
+        }
+        *(uint4*)(dst + h * DK + e) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    }
+}
+
 __global__ void latent_gate_rows_kernel(const __nv_bfloat16* __restrict__ o, int DV, const float* __restrict__ gate, int ld_gate,
                                         int by_entry, int heads, int vdim, __nv_bfloat16* __restrict__ out) {
     cj::after_predecessor();
@@ -337,11 +401,14 @@ __global__ void latent_gate_rows_kernel(const __nv_bfloat16* __restrict__ o, int
 }  // namespace
 
 CJ_EXPORT int cj_latent_gather(const void* plane, int width, int rank, const int* tok_req, const int* tok_pos, const int* table,
-                               int table_stride, int page_tokens, void* c_all, int N, cudaStream_t stream) {
+                               int table_stride, int page_tokens, void* c_all, void* kr, int N, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (!plane || !tok_req || !tok_pos || !table || !c_all || rank <= 0 || width < rank || page_tokens <= 0) return CJ_ERR_ARG;
-    cj::launch(latent_gather_kernel, dim3(N), dim3(rank >= 512 ? 256 : 128), 0, stream, (const __nv_bfloat16*)plane, width, rank,
-               tok_req, tok_pos, table, table_stride, page_tokens, (__nv_bfloat16*)c_all);
+    if (kr && width - rank > 64) return CJ_ERR_SIZE;
+    const bool wide = rank % 8 == 0 && width % 8 == 0 && (((uintptr_t)plane | (uintptr_t)c_all | (uintptr_t)kr) & 15) == 0;
+    auto kern = wide ? latent_gather_kernel<uint4> : latent_gather_kernel<unsigned short>;
+    cj::launch(kern, dim3(N), dim3(128), 0, stream, (const __nv_bfloat16*)plane, width, rank, tok_req, tok_pos, table, table_stride, page_tokens,
+               (__nv_bfloat16*)c_all, (__nv_bfloat16*)kr);
     return launch_status();
 }
 
@@ -362,8 +429,10 @@ CJ_EXPORT int cj_latent_q_pack(const float* q, int ld, int heads, int dim, int r
     if (T <= 0) return 0;
     if (!q || !positions || !qx || heads <= 0 || dim <= 0 || rot < 0 || DK < dim + rot) return CJ_ERR_ARG;
     if ((rotary & 1) || rotary < 0 || rotary > rot || (rotary > 0 && !inv_freq)) return CJ_ERR_SIZE;
-    cj::launch(latent_q_pack_kernel, dim3(T), dim3(256), 0, stream, q, ld, heads, dim, rot, rotary, halves, mag, inv_freq, positions, DK,
-               (__nv_bfloat16*)qx);
+    const bool eights = dim % 8 == 0 && rot % 8 == 0 && DK % 8 == 0 && ld % 4 == 0 && rotary % (halves ? 16 : 8) == 0 && rotary <= 256
+                        && (((uintptr_t)q | (uintptr_t)qx) & 15) == 0;
+    auto kern = eights ? latent_q_pack8_kernel : latent_q_pack_kernel;
+    cj::launch(kern, dim3(T), dim3(256), 0, stream, q, ld, heads, dim, rot, rotary, halves, mag, inv_freq, positions, DK, (__nv_bfloat16*)qx);
     return launch_status();
 }
 

@@ -101,7 +101,7 @@ class DifferentialAttention(Part):
         return p
 
     def libraries(self) -> set:
-        libs = {"attention_diff", "attention_paged", "gemm_simt"}
+        libs = {"attention_diff", "attention_paged", "gemm_simt"} | ({"attention_flash_tc"} if self._tiled() else set())
         if self.has_conv:
             libs.add("recurrent")
         if self.runtime.fast_kernels and self.hidden >= 128:

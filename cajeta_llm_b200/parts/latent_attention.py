@@ -136,7 +136,7 @@ class LatentAttention(Part):
         return p
 
     def libraries(self) -> set:
-        libs = {"latent_attention", "gemm_simt"} | ({"latent_prefill"} if self.can_expand else set())
+        libs = {"latent_attention", "gemm_simt"} | ({"latent_prefill", "attention_flash_tc"} if self.can_expand else set())
         if self.runtime.fast_kernels and self.hidden >= 128:
             libs |= {"gemm_tc", "gemm_tc2"}
         return libs
@@ -265,13 +265,27 @@ class LatentAttention(Part):
         req_base, tok_req, tok_pos, N = layout
         plane = entry.k_plane
         c_all = torch.empty((N, self.rank), dtype=torch.bfloat16, device=dev)
+        # On tcgen05 the attention reads keys and values where the products below leave them, and the gate rides on its way out
+        fast = K.latent_tc_shape(self.dim, self.rot, self.vdim, self.scale)
+        kr = torch.empty((N, 64), dtype=torch.bfloat16, device=dev) if fast else None
         K.tag = "latent gather"
-        K.latent_gather(plane, self.rank, tok_req, tok_pos, entry.block_table, entry.page_tokens, c_all)
+        K.latent_gather(plane, self.rank, tok_req, tok_pos, entry.block_table, entry.page_tokens, c_all, kr)
         kp = torch.empty((N, H * self.dim), dtype=torch.bfloat16, device=dev)
         vp = torch.empty((N, H * self.vdim), dtype=torch.bfloat16, device=dev)
         K.tag = "key/value up"
         project(rt, c_all, self.w_uk, kp)
         project(rt, c_all, self.w_uv.view(H * self.vdim, self.rank), vp)
+        if fast:
+            qx = torch.empty((T, H, self.dim + 64), dtype=torch.bfloat16, device=dev)
+            K.tag = "q split + rope"
+            K.latent_q_pack(proj, H, self.dim, self.rot, self.rotary, self.position.inv_freq, ctx.positions, qx, halves=self.halves,
+                            magnitude=self.magnitude)
+            gated = torch.empty((T, H * self.vdim), dtype=torch.bfloat16, device=dev)
+            K.tag = "attention"
+            K.latent_attention_tc(qx, gated, kp, kr, vp, ctx.req_start, ctx.req_prior, req_base, ctx.n_requests, H, self.dim, self.vdim,
+                                  self.scale, sink=self.sink, window=self.window, exact_weights=self.exact_weights, gate=gate[0],
+                                  gate_offset=gate[1], by_entry=self.gate_by_entry)
+            return gated
         kx = torch.empty((N, H, self.dk_pad), dtype=torch.bfloat16, device=dev)
         vx = torch.empty((N, H, self.dv_pad), dtype=torch.bfloat16, device=dev)
         K.tag = "key/value pack"
