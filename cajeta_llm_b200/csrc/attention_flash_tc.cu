@@ -165,8 +165,10 @@ struct Args {
     // latent: request i's token p lies at row req_base[i] + p of the dense buffers
     const int* req_base;
     const float* sink;             // null, or [n_heads]: exp(sink) joins the divisor
-    const float* gate;             // null, or float32 [T, gate_ld]: the outputs are multiplied by sigmoid(gate)
-    int gate_ld, gate_by_entry;    // a gate for every entry, or one a head
+    // null, or float32 [T, gate_ld]: head h of row t is multiplied by sigmoid(gate[t, h]).  (A gate for every entry costs more here than in a
+    // kernel of its own: the rows' results leave a row a thread, and the block waits for its gates - 29 to 40 us of 2,250 rows' 70 to 80.)
+    const float* gate;
+    int gate_ld;
 };
 
 // What a softmax of the block covers: its rows, the position of the first, and the key tiles it needs, counted from the block's
@@ -590,9 +592,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const bool live = r < mine.n;
             if (p.sink) l += exp2f(p.sink[h] * 1.4426950408889634f - m_ref);           // the key without a value
             float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            const float* gate = p.gate && live ? p.gate + (size_t)row * p.gate_ld + (p.gate_by_entry ? h * DV : h) : nullptr;
-            if (gate && !p.gate_by_entry) inv *= 1.0f / (1.0f + expf(-gate[0]));
             __nv_bfloat16* dst = p.out + ((size_t)row * p.n_heads + h) * DV;
+            if (p.gate && live) inv *= 1.0f / (1.0f + expf(-p.gate[(size_t)row * p.gate_ld + h]));
 #pragma unroll 1
             for (int c0 = 0; c0 < DV; c0 += 16) {
                 uint32_t o[16];
@@ -602,10 +603,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     float x[16];
 #pragma unroll
                     for (int q = 0; q < 16; ++q) x[q] = __uint_as_float(o[q]) * inv;
-                    if (gate && p.gate_by_entry) {
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) x[q] *= 1.0f / (1.0f + expf(-gate[c0 + q]));
-                    }
                     *(uint4*)(dst + c0) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
                     *(uint4*)(dst + c0 + 8) = make_uint4(pack_bf16(x[8], x[9]), pack_bf16(x[10], x[11]), pack_bf16(x[12], x[13]), pack_bf16(x[14], x[15]));
                 }
@@ -677,12 +674,10 @@ CJ_EXPORT int cj_diff_attention_tc(const void* q, void* out, const void* kplane,
 
 // Latent attention's plain form.  q [T, heads, dim + 64]; kp [N, heads * dim], kr [N, 64] (the key part that the heads share), vp
 // [N, heads * vdim]; out [T, heads * vdim]; all bfloat16.  dim and vdim 64 or 128.  Request i's token p lies at row req_base[i] + p.
-// exact: weights as two bfloat16 terms.  sink: null or [heads]; gate: null or float32 with row stride gate_ld (by_entry: a column for
-// every entry, otherwise one a head).
+// exact: weights as two bfloat16 terms.  sink: null or [heads]; gate: null or float32 with row stride gate_ld, a column a head.
 CJ_EXPORT int cj_latent_attention_tc(const void* q, void* out, const void* kp, const void* kr, const void* vp, int N, const int* req_start,
                                      const int* req_prior, const int* req_base, int n_requests, int T, int heads, int dim, int vdim,
-                                     int window, int exact, float scale, const float* sink, const float* gate, int gate_ld, int by_entry,
-                                     cudaStream_t stream) {
+                                     int window, int exact, float scale, const float* sink, const float* gate, int gate_ld, cudaStream_t stream) {
     if (T <= 0 || n_requests <= 0) return 0;
     if (!q || !out || !kp || !kr || !vp || !req_start || !req_prior || !req_base || N <= 0) return CJ_ERR_ARG;
     if (heads <= 0 || window < 0 || !(scale > 0.0f) || (dim != 64 && dim != 128) || (vdim != 64 && vdim != 128)) return CJ_ERR_SIZE;
@@ -702,7 +697,7 @@ CJ_EXPORT int cj_latent_attention_tc(const void* q, void* out, const void* kp, c
     a.block_rows = 2 * blocks_256 <= sm_count() ? 128 : 256;
     const long long row_blocks = ((long long)T + a.block_rows - 1) / a.block_rows + n_requests;
     if (row_blocks > 65535) return CJ_ERR_SIZE;
-    a.req_base = req_base, a.sink = sink, a.gate = gate, a.gate_ld = gate_ld, a.gate_by_entry = by_entry;
+    a.req_base = req_base, a.sink = sink, a.gate = gate, a.gate_ld = gate_ld;
 #define START(D_, V_) (exact ? start<false, D_, V_, true>(mq, mk, mr, mv, a, row_blocks, stream) : start<false, D_, V_, false>(mq, mk, mr, mv, a, row_blocks, stream))
     if (dim == 64) return vdim == 64 ? START(128, 64) : START(128, 128);
     return vdim == 64 ? START(192, 64) : START(192, 128);

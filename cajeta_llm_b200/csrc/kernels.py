@@ -1257,9 +1257,9 @@ def latent_tc_shape(dim: int, rot: int, vdim: int, scale: float) -> bool:
 def latent_attention_tc(qx: torch.Tensor, out: torch.Tensor, kp: torch.Tensor, kr: torch.Tensor, vp: torch.Tensor, req_start: torch.Tensor,
                         req_prior: torch.Tensor, req_base: torch.Tensor, requests: int, heads: int, dim: int, vdim: int, scale: float,
                         sink: Optional[torch.Tensor] = None, window: int = 0, exact_weights: bool = False,
-                        gate: Optional[torch.Tensor] = None, gate_offset: int = 0, by_entry: bool = False) -> None:
-    """:func:`latent_flash` on the tcgen05 tensor cores, with the keys and values where the products left them and the gate of
-    :func:`latent_gate_rows` on the way out: qx [T, heads, dim + 64], kp [N, heads * dim], kr [N, 64], vp [N, heads * vdim],
+                        gate: Optional[torch.Tensor] = None, gate_offset: int = 0) -> None:
+    """:func:`latent_flash` on the tcgen05 tensor cores, with the keys and values where the products left them and a gate a head
+    (as :func:`latent_gate_rows` has it) on the way out: qx [T, heads, dim + 64], kp [N, heads * dim], kr [N, 64], vp [N, heads * vdim],
     out [T, heads * vdim], bfloat16."""
     if sink is not None:
         _need(sink, "sink", torch.float32)
@@ -1274,15 +1274,14 @@ def latent_attention_tc(qx: torch.Tensor, out: torch.Tensor, kp: torch.Tensor, k
     gate_ptr, gate_ld = _gate(gate, gate_offset)
     st = library("attention_flash_tc").cj_latent_attention_tc(
         _ptr(qx), _ptr(out), _ptr(kp), _ptr(kr), _ptr(vp), _i(N), _ptr(req_start), _ptr(req_prior), _ptr(req_base), _i(requests), _i(T),
-        _i(heads), _i(dim), _i(vdim), _i(window), _i(1 if exact_weights else 0), _f(scale), _ptr(sink), gate_ptr, _i(gate_ld),
-        _i(1 if by_entry else 0), _stream())
+        _i(heads), _i(dim), _i(vdim), _i(window), _i(1 if exact_weights else 0), _f(scale), _ptr(sink), gate_ptr, _i(gate_ld), _stream())
     _check(st, "latent_attention_tc")
 
 
 def latent_gate_rows(o: torch.Tensor, gate: Optional[torch.Tensor], gate_offset: int, heads: int, vdim: int, out: torch.Tensor,
                      by_entry: bool = False) -> None:
     """out[t, h * vdim + e] = o[t, h, e] * sigmoid(gate[t, gate_offset + h]); o bfloat16 [T, heads, DV], gate float32
-    (None: no gate, the heads' entries are only moved out of their padding).  ``by_entry``: the gate has a column for every entry,
+    (None: no gate, the heads' entries are only moved out of their padding); without padding out may be o.  ``by_entry``: the gate has a column for every entry,
     gate[t, gate_offset + h * vdim + e]."""
     _need(o, "o", torch.bfloat16), _need(out, "out", torch.bfloat16)
     gate_ptr, gate_ld = _gate(gate, gate_offset)

@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(256) latent_q_pack8_kernel(const float* __rest
     }
 }
 
-__global__ void latent_gate_rows_kernel(const __nv_bfloat16* __restrict__ o, int DV, const float* __restrict__ gate, int ld_gate,
-                                        int by_entry, int heads, int vdim, __nv_bfloat16* __restrict__ out) {
+__global__ void latent_gate_rows_kernel(const __nv_bfloat16* o, int DV, const float* __restrict__ gate, int ld_gate,
+                                        int by_entry, int heads, int vdim, __nv_bfloat16* out) {
     cj::after_predecessor();
     cj::release_successor();
     const int r = blockIdx.x;
@@ -395,6 +395,29 @@ __global__ void latent_gate_rows_kernel(const __nv_bfloat16* __restrict__ o, int
         const int h = i / vdim, e = i % vdim;
         const float g = gate ? 1.0f / (1.0f + expf(-gate[(size_t)r * ld_gate + (by_entry ? i : h)])) : 1.0f;
         out[(size_t)r * heads * vdim + i] = __float2bfloat16_rn(__bfloat162float(o[((size_t)r * heads + h) * DV + e]) * g);
+    }
+}
+
+// The same for a gate an entry, eight entries a thread: vdim in eights, everything on 16 bytes; out may be o (DV = vdim).  2,250 rows of 2,048
+// entries, 18 MB of gates and 18 MB of outputs, cold: 28.7 us an entry a
+// thread, 14.4 this way.
+__global__ void __launch_bounds__(256) latent_gate_rows8_kernel(const __nv_bfloat16* o, int DV, const float* __restrict__ gate, int ld_gate, int heads,
+                                                                int vdim, __nv_bfloat16* out) {
+    cj::after_predecessor();
+    cj::release_successor();
+    const int r = blockIdx.x;
+    for (int i = 8 * threadIdx.x; i < heads * vdim; i += 8 * 256) {
+        const int h = i / vdim, e = i - h * vdim;
+        const float4 a = *(const float4*)(gate + (size_t)r * ld_gate + i), b = *(const float4*)(gate + (size_t)r * ld_gate + i + 4);
+        const uint4 u = *(const uint4*)(o + ((size_t)r * heads + h) * DV + e);
+        const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const unsigned w[4] = {u.x, u.y, u.z, u.w};
+        unsigned v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            v[k] = pack_bf16(__uint_as_float(w[k] << 16) * (1.0f / (1.0f + expf(-g[2 * k]))),
+                             __uint_as_float(w[k] & 0xffff0000u) * (1.0f / (1.0f + expf(-g[2 * k + 1]))));
+        *(uint4*)(out + (size_t)r * heads * vdim + i) = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 
@@ -480,6 +503,10 @@ CJ_EXPORT int cj_latent_gate_rows(const void* o, int DV, const float* gate, int 
                                   cudaStream_t stream) {
     if (T <= 0) return 0;
     if (!o || !out || heads <= 0 || vdim <= 0 || DV < vdim) return CJ_ERR_ARG;
+    if (gate && by_entry && vdim % 8 == 0 && DV % 8 == 0 && ld_gate % 4 == 0 && (((uintptr_t)o | (uintptr_t)gate | (uintptr_t)out) & 15) == 0) {
+        cj::launch(latent_gate_rows8_kernel, dim3(T), dim3(256), 0, stream, (const __nv_bfloat16*)o, DV, gate, ld_gate, heads, vdim, (__nv_bfloat16*)out);
+        return launch_status();
+    }
     cj::launch(latent_gate_rows_kernel, dim3(T), dim3(heads * vdim >= 2048 ? 256 : 128), 0, stream, (const __nv_bfloat16*)o, DV, gate,
                ld_gate, by_entry, heads, vdim, (__nv_bfloat16*)out);
     return launch_status();

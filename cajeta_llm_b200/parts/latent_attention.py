@@ -265,7 +265,7 @@ class LatentAttention(Part):
         req_base, tok_req, tok_pos, N = layout
         plane = entry.k_plane
         c_all = torch.empty((N, self.rank), dtype=torch.bfloat16, device=dev)
-        # On tcgen05 the attention reads keys and values where the products below leave them, and the gate rides on its way out
+        # On tcgen05 the attention reads keys and values where the products below leave them, and a gate a head rides on its way out
         fast = K.latent_tc_shape(self.dim, self.rot, self.vdim, self.scale)
         kr = torch.empty((N, 64), dtype=torch.bfloat16, device=dev) if fast else None
         K.tag = "latent gather"
@@ -283,8 +283,11 @@ class LatentAttention(Part):
             gated = torch.empty((T, H * self.vdim), dtype=torch.bfloat16, device=dev)
             K.tag = "attention"
             K.latent_attention_tc(qx, gated, kp, kr, vp, ctx.req_start, ctx.req_prior, req_base, ctx.n_requests, H, self.dim, self.vdim,
-                                  self.scale, sink=self.sink, window=self.window, exact_weights=self.exact_weights, gate=gate[0],
-                                  gate_offset=gate[1], by_entry=self.gate_by_entry)
+                                  self.scale, sink=self.sink, window=self.window, exact_weights=self.exact_weights,
+                                  gate=None if self.gate_by_entry else gate[0], gate_offset=gate[1])
+            if self.gate_by_entry:
+                K.tag = "head gate"
+                K.latent_gate_rows(gated.view(T, H, self.vdim), gate[0], gate[1], H, self.vdim, gated, by_entry=True)
             return gated
         kx = torch.empty((N, H, self.dk_pad), dtype=torch.bfloat16, device=dev)
         vx = torch.empty((N, H, self.dv_pad), dtype=torch.bfloat16, device=dev)

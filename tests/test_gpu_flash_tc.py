@@ -104,7 +104,7 @@ def test_latent(H, dim, rot, vdim, window, sink, gate, requests):
         kr[lo:hi, :rot], kr[lo:hi, rot:] = torch.randn((hi - lo, rot), generator=g), 0.0
     kp, kr, vp = kp.bfloat16(), kr.bfloat16(), vp.bfloat16()
     sinks = torch.randn(H, generator=g) if sink else None
-    gates = torch.randn((T, 3 + (H * vdim if gate == "entry" else H)), generator=g)
+    gates = torch.randn((T, 4 + (H * vdim if gate == "entry" else H)), generator=g)
     scale, want = 1.5 * (dim + rot) ** -0.5, torch.zeros((T, H, vdim), dtype=torch.float64)
     for i, (p, r) in enumerate(requests):
         first = max(0, p + 1 - window) if window else 0
@@ -114,17 +114,20 @@ def test_latent(H, dim, rot, vdim, window, sink, gate, requests):
             k = torch.cat([kp[toks, h * dim:(h + 1) * dim], kr[toks]], 1).double()
             o = _attend(q[rows, h].double(), k, vp[toks, h * vdim:(h + 1) * vdim].double(), see, scale, sinks[h].double() if sink else None)
             if gate != "none":
-                z = gates[rows, 3:].double()
+                z = gates[rows, 3 if gate == "head" else 4:].double()
                 o = o * torch.sigmoid(z[:, h * vdim:(h + 1) * vdim] if gate == "entry" else z[:, h:h + 1])
             want[rows, h] = o
     errs = []
     for exact in (False, True):
         out = torch.full((T, H * vdim), NAN, dtype=torch.bfloat16, device=DEV)
+        # (a gate from the fourth column on lies on 16 bytes: eight entries a thread)
         K.latent_attention_tc(q.to(DEV), out, kp.to(DEV), kr.to(DEV), vp.to(DEV), torch.tensor(starts, dtype=torch.int32, device=DEV),
                               torch.tensor([p for p, _ in requests], dtype=torch.int32, device=DEV),
                               torch.tensor(base, dtype=torch.int32, device=DEV), len(requests), H, dim, vdim, scale,
                               sink=sinks.to(DEV) if sink else None, window=window, exact_weights=exact,
-                              gate=gates.to(DEV) if gate != "none" else None, gate_offset=3, by_entry=gate == "entry")
+                              gate=gates.to(DEV) if gate == "head" else None, gate_offset=3)
+        if gate == "entry":
+            K.latent_gate_rows(out.view(T, H, vdim), gates.to(DEV), 4, H, vdim, out, by_entry=True)
         err = (out.cpu().double().view(T, H, vdim) - want).abs()
         assert float(err.max()) < 2.0 ** -8 * 5.0, float(err.max())                # values of at most about five
         errs.append(float(err.pow(2).mean().sqrt()))
