@@ -24,16 +24,19 @@
 // product itself does not) or below 2^-100 (whose smaller parts' products are too small for float32).
 //
 // One block a tile of `feat_tile` (up to 128) features x N tokens; the weights are the rows of the product.  One thread sends for
-// the float32 tiles (TMA) into a ring as deep as shared memory allows; groups of eight warps split them into the six bfloat16
-// tiles of a stage, a group every G-th block of K; one warp issues the products; the last warps add the accumulators up
-// and store.  A block of K is a chain of short waits for a group (tile landed, stage free, stores visible to the products: some
-// 1,100 clocks, half of them waiting), so with few tokens several groups work side by side.  What bounds it: with few
-// tokens that chain, with many one group's going through read, split, write and wait (issue slots 61 % used, shared memory 44 %, integer and
-// conversion pipe 40 %, tensor pipe 33 %; shared memory has no room for a second group).
-// Rows x features x K, us, gemm_simt.cu before and now (cold weights): 1 x 2,048 x 2,048 190 and 32; 250 x 6,144 x 2,048 327 and 100;
-// 1,777 x 6,144 x 2,048 1,817 and 352; 64 groups of 1,408 gated features, 8 / 256 / 1,777 tokens of 4 picks among 60 of them
-// 796 / 1,449 / 3,162 and 147 / 392 / 866.  (With the float32 operands loaded into registers instead of by TMA 1,777 x 6,144 took 815: one
-// load's latency a block lay bare.  Three loading threads instead of one changed nothing.)
+// the float32 tiles (TMA) into a ring as deep as shared memory allows; groups of eight warps, a group every G-th block of K, split W into its
+// parts and put them in tensor memory, from where the products read them: a product of 128 rows and n tokens takes 12 + n / 2 clocks so,
+// 44 + n / 2 with W in shared memory (measured alone, back to back).  X goes to shared memory in its parts, split by the same warps or, for
+// tiles of 64 tokens and more, once for all tiles by split_rows_kernel.  Two warps issue the products, every other one each, since one's round
+// of waits, products and commits lasted longer than the products themselves; the last warps add the accumulators up, two sums an instruction,
+// and store.  What bounds it: issue slots with few tokens (of 0.37 us a block of 32 of K with 16 tokens splitting takes 0.13, the loads alone
+// 0.2), the products and the adding up with many (0.84 us with 128 tokens, 0.5 of them the products); and some 10 us of every tile
+// are its beginning and end.  Rows x features x K, us, cold weights; gemm_simt.cu, then W's parts in shared memory with one issuing warp,
+// then now: 8 x 2,048 x 2,048 190, 39 and 34; 264 x 6,144 x 2,048 327, 111 and 75; 1,777 x 6,144 x 2,048 1,817, 366 and 314; 60 groups of 1,408
+// gated features, 17 tokens each 380 and 340, 118 each 750 and 650.
+// Built and taken out: two blocks an SM with few tokens (60 groups of 17 tokens 333 us instead of 343, one of 24 groups the same).  (With the
+// float32 operands loaded into registers instead of by TMA 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading
+// threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
 #define CJ_LIB "gemm_f32_tc"
 #include "common.cuh"
@@ -44,18 +47,21 @@ using namespace tc;
 namespace {
 
 constexpr int BK = 32;                    // K of a stage: 128 bytes of float32 (TMA's swizzle row), 64 bytes of bfloat16
-// groups of eight splitting warps, each with stages of bfloat16 parts of its own, and warps that add up: as many as registers
-// and shared memory hold
+// groups of eight splitting warps, each with stages of bfloat16 parts of its own, and warps that add up: as many as registers and issue slots bear
 constexpr int GROUP_WARPS = 8;
-constexpr int split_groups(int n) { return n <= 32 ? 3 : n <= 64 ? 2 : 1; }
-constexpr int split_stages(int n) { return n <= 32 ? 3 : 2; }
-constexpr int epi_warps(int n) { return n >= 64 ? 8 : 4; }
-// warps: the splitting groups, product issue, loads (and, so that the warps that add up begin at a multiple of four, idle ones), adding up
-constexpr int first_epi(int n) { return (GROUP_WARPS * split_groups(n) + 2 + 3) / 4 * 4; }
+constexpr int split_groups(int n) { return n <= 16 ? 3 : n <= 32 ? 2 : 1; }
+constexpr int split_stages(int n) { return n <= 32 ? 6 : 4; }
+// tiles of many tokens take X in its parts, which split_rows_kernel made once for all of them; the others split their rows of X themselves
+constexpr bool ready_x(int n) { return n >= 64; }
+constexpr int epi_warps(int n) { return n >= 64 ? 16 : n >= 32 ? 8 : 4; }
+// warps: the splitting groups, two that issue products (every other unit each), two that load (one where the tile's X is not ready), adding up
+constexpr int first_epi(int n) { return GROUP_WARPS * split_groups(n) + 4; }
 constexpr int threads(int n) { return 32 * (first_epi(n) + epi_warps(n)); }
 
 struct Args {
     const float* X; long long ldx;
+    const int* x_index;                    // ready_x: the row of X that feeds a token (null: its own)
+    const int* x_odd;                      // ready_x: tokens whose row has an entry that is not the sum of three parts
     const float* W; const float* W2;       // W2: the gated form's second weight
     const float* bias; const float* bias2;
     float* C; long long ldc;
@@ -71,16 +77,44 @@ struct Args {
 };
 
 template <int N> struct Smem {
-    static constexpr int W_PART = 128 * 64, X_PART = N * 64;           // one bfloat16 tile
-    static constexpr int STAGE = 3 * (W_PART + X_PART);
-    static constexpr int W_RAW = 128 * 128, X_RAW = N * 128;           // one float32 tile
+    static constexpr int STAGE = 3 * N * 64;                           // the bfloat16 parts of X (those of W lie in tensor memory)
+    static constexpr int W_RAW = 128 * 128, X_RAW = ready_x(N) ? 0 : N * 128;       // one float32 tile
     static constexpr int RAW = W_RAW + X_RAW;
-    static constexpr int STAGES = split_stages(N);
+    static constexpr int STAGES = split_stages(N), GROUPS = split_groups(N);
     // a multiple of the groups, so that a slot is always read by the same group: a wait by phase parity must not be two phases off
-    static constexpr int RING = (225 * 1024 - STAGES * STAGE) / RAW / STAGES * STAGES;
+    static constexpr int RING = (225 * 1024 - STAGES * STAGE) / RAW / GROUPS * GROUPS;
     static constexpr int TOTAL = STAGES * STAGE + RING * RAW + 1024 /* alignment */;
-    static_assert(STAGES % split_groups(N) == 0, "a stage belongs to one group");
+    static_assert(STAGES % GROUPS == 0, "a stage belongs to one group");
+    // tensor memory: two accumulators of a unit of UNIT tokens (a tile of 128 tokens is two units), then the parts of W, three times 16
+    // columns a stage
+    static constexpr int UNIT = N < 64 ? N : 64, UNITS = N / UNIT;
+    static constexpr int A_AT = 4 * UNIT, COLS_USED = A_AT + 48 * STAGES;
+    static constexpr uint32_t TMEM_COLS = COLS_USED <= 256 ? 256 : 512;
+    static_assert(COLS_USED <= 512, "tensor memory of an SM");
 };
+
+// two float32 operations in one instruction
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 both_of(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 
 // eight float32 -> their three bfloat16 parts, packed; some bit of `odd` is set when one of the eight is not the sum of its parts: infinite,
 // no number, so large that its first part rounds to infinity, or so small that its last part falls below the smallest bfloat16
@@ -95,11 +129,12 @@ __device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& 
     for (int i = 0; i < 4; ++i) {
         const float a = f[2 * i], b = f[2 * i + 1];
         h[i] = pack(a, b);
-        const float ra = a - __uint_as_float(h[i] << 16), rb = b - __uint_as_float(h[i] & 0xffff0000u);
-        m[i] = pack(ra, rb);
-        const float la = ra - __uint_as_float(m[i] << 16), lb = rb - __uint_as_float(m[i] & 0xffff0000u);
-        l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);        // (a remainder has eight bits at most)
-        odd |= __float_as_uint(la) | __float_as_uint(lb);
+        const f32x2 r = sub2(pair(a, b), pair(__uint_as_float(h[i] << 16), __uint_as_float(h[i] & 0xffff0000u)));
+        const float2 rs = both_of(r);
+        m[i] = pack(rs.x, rs.y);
+        const float2 ls = both_of(sub2(r, pair(__uint_as_float(m[i] << 16), __uint_as_float(m[i] & 0xffff0000u))));
+        l[i] = __byte_perm(__float_as_uint(ls.x), __float_as_uint(ls.y), 0x7632);        // (a remainder has eight bits at most)
+        odd |= __float_as_uint(ls.x) | __float_as_uint(ls.y);
     }
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     mid = make_uint4(m[0], m[1], m[2], m[3]);
@@ -118,9 +153,42 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(const void* smem_tile) {
     return d;
 }
 
+// D[tmem] (+)= A[tmem] * B[smem] by the one thread of the warp with `on` set: A's rows are the lanes, two bfloat16 of neighbouring k a
+// column; B's descriptor in two words.  (The whole warp walks the loop, so that addresses stay in uniform registers.)
+__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t on, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                                 uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "mov.b64 b, {%2, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(on)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_by(uint32_t on, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(on) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 a, const uint4 b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// (x null: a row of zeros)
 __device__ __noinline__ float chain(const float* x, const float* w, int K) {
     float s = 0.0f;
-    for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
+    for (int k = 0; k < K; ++k) s = fmaf(x ? x[k] : 0.0f, w[k], s);
     return s;
 }
 
@@ -146,36 +214,21 @@ __global__ void __launch_bounds__(threads(N), 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_w2, const Args p) {
     using S = Smem<N>;
-    constexpr int G = split_groups(N), STAGES = S::STAGES, EPI_WARPS = epi_warps(N), RING = S::RING, ISSUE = GROUP_WARPS * G,
-                  LOAD = ISSUE + 1, FIRST_EPI = first_epi(N);
-    constexpr int XP = (N + 63) / 64;                         // rows of X a splitting thread takes (64 rows a pass)
-    constexpr int COLS = N * 4 / EPI_WARPS;                   // columns of an adding thread
-    constexpr uint32_t TMEM_COLS = 4 * N <= 64 ? 64 : 4 * N <= 128 ? 128 : 4 * N <= 256 ? 256 : 512;
+    constexpr int G = S::GROUPS, STAGES = S::STAGES, EPI_WARPS = epi_warps(N), RING = S::RING, ISSUE = GROUP_WARPS * G,
+                  LOAD = ISSUE + 2, LOAD_X = LOAD + 1, FIRST_EPI = first_epi(N);
+    constexpr bool READY = ready_x(N);
+    constexpr int XP = READY ? 0 : 1;                         // rows of X a splitting thread takes (64 rows a pass)
+    constexpr int UNIT = S::UNIT, UNITS = S::UNITS, UCOLS = UNIT * 4 / EPI_WARPS, COLS = UNITS * UCOLS;      // columns of an adding thread
+    constexpr uint32_t TMEM_COLS = S::TMEM_COLS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stages = raw + RING * S::RAW;
-    __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], x_full[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int odd_flag;                                  // some row of the tile has an entry that is not the sum of three parts
     __shared__ int place[3];                                  // group, first row, one past the last; group -1: no work
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        for (int s = 0; s < RING; ++s) {
-            mbar_init(&raw_full[s], 1);
-            mbar_init(&raw_empty[s], GROUP_WARPS);
-        }
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full_bar[s], GROUP_WARPS);
-            mbar_init(&empty_bar[s], 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], EPI_WARPS);
-        }
-        odd_flag = 0;
-        fence_barrier_init();
-    }
     if (warp == ISSUE) tmem_alloc(&tmem_slot, TMEM_COLS);
     const bool grouped = p.group_offsets != nullptr;
     if (grouped) cj::after_predecessor();
@@ -210,6 +263,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             place[1] = blockIdx.y * N;
             place[2] = min(p.tokens, place[1] + N);
         }
+        if (lane == 0) {
+            const int units = (place[2] - place[1] + UNIT - 1) / UNIT;
+            for (int s = 0; s < RING; ++s) {
+                mbar_init(&raw_full[s], 1);
+                mbar_init(&raw_empty[s], GROUP_WARPS);
+            }
+            for (int s = 0; s < STAGES; ++s) {
+                mbar_init(&full_bar[s], GROUP_WARPS);
+                mbar_init(&x_full[s], 1);
+                mbar_init(&empty_bar[s], max(units, 1));      // the products of every unit
+            }
+            for (int s = 0; s < 2; ++s) {
+                mbar_init(&acc_full[s], 1);
+                mbar_init(&acc_empty[s], EPI_WARPS);
+            }
+            odd_flag = 0;
+            fence_barrier_init();
+        }
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -220,7 +291,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     const int feat0 = blockIdx.x * p.feat_tile;
     const int n_kb = (p.K + BK - 1) / BK;
     const bool work = group >= 0 && n_tok > 0;
-    const int n16 = (n_tok + 15) & ~15;                       // the product's width; the parts of X lie n16 rows apart, side by side
+    const int units = (n_tok + UNIT - 1) / UNIT;
+    // the width of a unit's products; the parts of its X lie that many rows apart, side by side (those that came in parts UNIT rows)
+    auto width = [&](int u) { return (min(n_tok - u * UNIT, UNIT) + 15) & ~15; };
 
     if (work && warp == LOAD) {
         // ---- float32 tiles: the weights' first ones leave before the kernel before this one has ended (no kernel writes weights) ----
@@ -237,7 +310,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 mbar_expect_tx(&raw_full[kb], bytes);
                 weights(kb, kb);
             }
-            if (!grouped) cj::after_predecessor();
+            if (!READY && !grouped) cj::after_predecessor();
             bool ok = true;
             for (int kb = 0; kb < n_kb && ok; ++kb) {
                 const int s = kb % RING;
@@ -247,22 +320,33 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     mbar_expect_tx(&raw_full[s], bytes);
                     weights(kb, s);
                 }
-                tma_load_2d(raw + s * S::RAW + S::W_RAW, &map_x, &raw_full[s], kb * BK, tok0);
+                if (!READY) tma_load_2d(raw + s * S::RAW + S::W_RAW, &map_x, &raw_full[s], kb * BK, tok0);
+            }
+        }
+    } else if (READY && work && warp == LOAD_X) {
+        // ---- the parts of X, a stage's three side by side ----
+        if (elect_one()) {
+            if (!grouped) cj::after_predecessor();
+            for (int kb = 0; kb < n_kb; ++kb) {
+                const int s = kb % STAGES;
+                if (!mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 17)) break;
+                mbar_expect_tx(&x_full[s], units * 3 * UNIT * 64);
+                for (int u = 0; u < units; ++u) tma_load_3d(stages + s * S::STAGE + u * 3 * UNIT * 64, &map_x, &x_full[s], kb * BK, tok0 + u * UNIT, 0);
             }
         }
     } else if (work && warp < ISSUE) {
-        // ---- splitting: thread = (row of 64, eight of the row's 32 float32) ------------------------
+        // ---- splitting: of X a thread takes eight of a row's 32 float32 (a row of 64), of W half a row, its lane of tensor memory ----
         const int g = warp / GROUP_WARPS, piece = tid & 3, row0 = (tid & (32 * GROUP_WARPS - 1)) >> 2;
-        bool w_live[2], x_live[XP];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) w_live[i] = (DUAL ? row0 : row0 + 64 * i) < p.feat_tile;      // (rows past the last feature: read as they are, never stored)
+        const int w_row = (warp & 3) * 32 + lane, half = warp >> 2 & 1;
+        const bool w_live = (DUAL ? w_row & 63 : w_row) < p.feat_tile;      // (lanes past the tile's features: whatever they read, never stored)
+        const uint32_t w_to = tmem + S::A_AT + half * 8 + ((uint32_t)((warp & 3) * 32) << 16);
+        bool x_live[XP + 1];
 #pragma unroll
         for (int i = 0; i < XP; ++i) x_live[i] = row0 + 64 * i < n_tok;
         // 16-byte pieces 2 piece, 2 piece + 1 of a float32 row, piece `piece` of a bfloat16 row, each where its swizzle puts it
         // (64 rows apart the swizzles are the same)
         const int src0 = row0 * 128 + (((2 * piece) ^ (row0 & 7)) << 4), src1 = row0 * 128 + (((2 * piece + 1) ^ (row0 & 7)) << 4);
         const int dst = row0 * 64 + ((piece ^ ((row0 >> 1) & 3)) << 4);
-        const int x_part = n16 * 64;
         uint32_t odd = 0;
         bool ok = true;
         for (int kb = g; kb < n_kb && ok; kb += G) {
@@ -271,14 +355,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             if (!ok) break;
             const uint8_t* wr = raw + rs * S::RAW;
             const uint8_t* xr = wr + S::W_RAW;
-            float4 w[2][2], x[XP][2];
+            float4 w[4], x[XP + 1][2];
             auto read = [&]() {
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    if (w_live[i]) {
-                        w[i][0] = *(const float4*)(wr + i * 64 * 128 + src0);
-                        w[i][1] = *(const float4*)(wr + i * 64 * 128 + src1);
-                    }
+                for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(wr + w_row * 128 + (((4 * half + i) ^ (w_row & 7)) << 4));
 #pragma unroll
                 for (int i = 0; i < XP; ++i)
                     if (x_live[i]) {
@@ -290,117 +370,161 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             if (G == 1) read();
             ok = mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 11);
             if (!ok) break;
+            tcgen05_fence_after();
             if (G > 1) read();
-            uint8_t* wt = stages + s * S::STAGE;
-            uint8_t* xt = wt + 3 * S::W_PART;
-            uint4 hi, mid, lo;
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (w_live[i]) {
-                    split8(w[i][0], w[i][1], hi, mid, lo, odd);
-                    uint8_t* at = wt + i * 64 * 64 + dst;
-                    *(uint4*)at = hi;
-                    *(uint4*)(at + S::W_PART) = mid;
-                    *(uint4*)(at + 2 * S::W_PART) = lo;
-                }
+            {
+                uint4 hi[2], mid[2], lo[2];
+                uint32_t w_odd = 0;
+                split8(w[0], w[1], hi[0], mid[0], lo[0], w_odd);
+                split8(w[2], w[3], hi[1], mid[1], lo[1], w_odd);
+                if (w_live) odd |= w_odd;
+                const uint32_t to = w_to + s * 48;
+                tmem_st8(to, hi[0], hi[1]);
+                tmem_st8(to + 16, mid[0], mid[1]);
+                tmem_st8(to + 32, lo[0], lo[1]);
+            }
+            uint8_t* xt = stages + s * S::STAGE;
 #pragma unroll
             for (int i = 0; i < XP; ++i)
                 if (x_live[i]) {
+                    uint4 hi, mid, lo;
                     split8(x[i][0], x[i][1], hi, mid, lo, odd);
-                    uint8_t* at = xt + i * 64 * 64 + dst;
+                    uint8_t* at = xt + i * 3 * UNIT * 64 + dst;
+                    const int x_part = width(i) * 64;
                     *(uint4*)at = hi;
                     *(uint4*)(at + x_part) = mid;
                     *(uint4*)(at + 2 * x_part) = lo;
                 }
             if (kb + G >= n_kb && (odd & 0xffffu)) odd_flag = 1;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
+            if (!READY) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
+            tmem_st_wait();
+            tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&raw_empty[rs]);
                 mbar_arrive(&full_bar[s]);
             }
         }
-    } else if (work && warp == ISSUE) {
+    } else if (work && (warp == ISSUE || warp == ISSUE + 1)) {
         // ---- product issue --------------------------------------------------------------------------
-        if (elect_one()) {
-            // two accumulators a block of K, D0 | D1, n16 columns each: D0 takes the products of the leading parts alone, whose 16 bits an
-            // accumulator holds, D1 the others; the leading part of W meets the first two parts of X in one product twice as wide
-            const uint32_t one = umma_idesc_bf16(128, n16), both = umma_idesc_bf16(128, 2 * n16);
-            const uint64_t first = umma_desc_sw64(stages);
-            const uint64_t w_step = S::W_PART >> 4, x_hi = 3 * w_step, x_step = (uint64_t)(n16 * 64 >> 4);
-            bool ok = true;
-            for (int kb = 0; kb < n_kb && ok; ++kb) {
-                const int s = kb % STAGES, a = kb & 1;
-                ok = mbar_wait(&acc_empty[a], ((kb >> 1) & 1) ^ 1, 14) && mbar_wait(&full_bar[s], (kb / STAGES) & 1, 12);
-                if (!ok) break;
-                tcgen05_fence_after();
-                const uint64_t at = first + (uint64_t)((s * S::STAGE) >> 4);
-                const uint32_t d0 = tmem + a * 2 * N, d1 = d0 + n16;
-                auto add = [&](int pw, int px) {             // D1 += part pw of W . part px of X
+        // two accumulators a unit and block of K, D0 | D1, as wide as the unit each: D0 takes the products of the leading parts alone, whose
+        // 16 bits an accumulator holds, D1 the others; the leading part of W meets the first two parts of X in one product twice as wide
+        const uint32_t on = elect_one();
+        const uint64_t first = umma_desc_sw64(stages);
+        const uint32_t b_hi = (uint32_t)(first >> 32), b_first = (uint32_t)first;
+        // unit n of the tile (n counts units over all blocks of K) is warp n % 2's, and so is accumulator n % 2
+        const int mine = warp - ISSUE;
+        const uint32_t acc0 = tmem + mine * 2 * UNIT;
+        auto issue = [&](int u, int s, int times) {          // times: how often this warp has issued
+            const int wide = width(u);
+            const uint32_t one = umma_idesc_bf16(128, wide), both = umma_idesc_bf16(128, 2 * wide);
+            const uint32_t at = b_first + ((s * S::STAGE + u * 3 * UNIT * 64) >> 4), x_step = (READY ? UNIT : wide) * 64 >> 4;
+            const uint32_t w = tmem + S::A_AT + s * 48, d1 = acc0 + wide;
+            if (!mbar_wait(&acc_empty[mine], (times & 1) ^ 1, 14)) return false;
+            tcgen05_fence_after();
+            auto add = [&](int pw, int px) {                 // D1 += part pw of W . part px of X
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) umma_bf16(d1, at + pw * w_step + 2 * k, at + x_hi + px * x_step + 2 * k, one, 1);
-                };
+                for (int k = 0; k < BK / 16; ++k) umma_bf16_a_tmem(on, d1, w + pw * 16 + k * 8, at + px * x_step + 2 * k, b_hi, one, 1);
+            };
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_bf16(d0, at + 2 * k, at + x_hi + 2 * k, both, k > 0);                      // hi hi | hi mid
-                add(1, 0); add(0, 2); add(1, 1); add(2, 0);
-                umma_commit(&empty_bar[s]);
-                umma_commit(&acc_full[a]);
+            for (int k = 0; k < BK / 16; ++k) {               // hi hi | hi mid
+                const uint32_t wk = w + k * 8, xk = at + 2 * k;
+                if (!READY || wide == UNIT) {
+                    umma_bf16_a_tmem(on, acc0, wk, xk, b_hi, both, k > 0);
+                } else {
+                    umma_bf16_a_tmem(on, acc0, wk, xk, b_hi, one, k > 0);
+                    umma_bf16_a_tmem(on, d1, wk, xk + x_step, b_hi, one, k > 0);
+                }
             }
+            add(1, 0); add(0, 2); add(1, 1); add(2, 0);
+            umma_commit_by(on, &empty_bar[s]);
+            umma_commit_by(on, &acc_full[mine]);
+            return true;
+        };
+        const int step = units == 2 ? 1 : 2;                  // blocks of K between two units of this warp
+        int times = 0;
+        for (int kb = units == 2 ? 0 : mine; kb < n_kb; kb += step, ++times) {
+            const int s = kb % STAGES;
+            if (!mbar_wait(&full_bar[s], (kb / STAGES) & 1, 12) || (READY && !mbar_wait(&x_full[s], (kb / STAGES) & 1, 18)) || !issue(units == 2 ? mine : 0, s, times)) break;
         }
     } else if (work && warp >= FIRST_EPI) {
         // ---- adding up: a thread has one row of the product (a feature) and COLS of its tokens --------------
-        const int quarter = warp & 3, r = quarter * 32 + lane, c_first = ((warp - FIRST_EPI) >> 2) * COLS;
+        const int quarter = warp & 3, r = quarter * 32 + lane, c_first = ((warp - FIRST_EPI) >> 2) * UCOLS;
+        auto token = [&](int j) { return j / UCOLS * UNIT + c_first + j % UCOLS; };      // the token of the thread's column j
+        f32x2 acc2[COLS / 2];
+#pragma unroll
+        for (int j = 0; j < COLS / 2; ++j) acc2[j] = pair(0.0f, 0.0f);
+        bool ok = true;
+        int n = 0;
+        for (int kb = 0; kb < n_kb && ok; ++kb) {
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) {
+                if (u >= units || !ok) break;
+                const int a = n & 1, wide = width(u);
+                ok = mbar_wait(&acc_full[a], (n >> 1) & 1, 13);
+                if (!ok) break;
+                ++n;
+                tcgen05_fence_after();
+                const uint32_t at = tmem + a * 2 * UNIT + c_first + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+                for (int c = 0; c < UCOLS; c += 16) {
+                    uint32_t v[16], h[16];                    // (columns past the unit's width hold whatever they held: nothing asks for them)
+                    tmem_ld16(at + wide + c, v);
+                    tmem_ld16(at + c, h);
+                    tmem_ld_wait();
+                    if (c + 16 == UCOLS) {                    // the accumulator is free before its sums are added
+                        tcgen05_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty[a]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) {
+                        f32x2& s = acc2[(u * UCOLS + c + j) / 2];
+                        s = add2(add2(s, pair(__uint_as_float(v[j]), __uint_as_float(v[j + 1]))), pair(__uint_as_float(h[j]), __uint_as_float(h[j + 1])));
+                    }
+                }
+            }
+        }
         float acc[COLS];
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
-        bool ok = true;
-        for (int kb = 0; kb < n_kb && ok; ++kb) {
-            const int a = kb & 1;
-            ok = mbar_wait(&acc_full[a], (kb >> 1) & 1, 13);
-            if (!ok) break;
-            tcgen05_fence_after();
-            const uint32_t at = tmem + a * 2 * N + c_first + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll
-            for (int c = 0; c < COLS; c += 16) {
-                if (c_first + c >= n16) break;
-                uint32_t v[16];
-                tmem_ld16(at + n16 + c, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(v[j]);
-                tmem_ld16(at + c, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(v[j]);
-            }
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[a]);
+        for (int j = 0; j < COLS; j += 2) {
+            const float2 t = both_of(acc2[j / 2]);
+            acc[j] = t.x;
+            acc[j + 1] = t.y;
         }
         if (!grouped) cj::after_predecessor();
         const int fr = DUAL ? (r & 63) : r, feat = feat0 + fr;
         const bool live = ok && fr < p.feat_tile && feat < p.features;
         bool again = odd_flag != 0;
+        unsigned long long odd_x = 0;                         // the thread's tokens whose rows are not sums of three parts
+        if (READY) {
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) again = again || !chain_free(acc[j]);
+            for (int u = 0; u < UNITS; ++u) {
+                const int t = u * UNIT + c_first + lane;
+                odd_x |= (unsigned long long)__ballot_sync(0xffffffffu, lane < UCOLS && t < n_tok && p.x_odd[tok0 + t] != 0) << (u * UCOLS);
+            }
+            again = again || odd_x != 0;
+        }
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) again = again || (token(j) < n_tok && !chain_free(acc[j]));
         if (__any_sync(0xffffffffu, again)) {
             // (rarely: through an array in memory, so that the sums keep their registers)
             float sums[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
-            const int cols = min(COLS, n_tok - c_first);
-            const float* x = p.X + (size_t)(tok0 + c_first) * p.ldx;
             const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
-            unsigned long long odd_x = 0;
             bool odd_w = false;
             if (__any_sync(0xffffffffu, odd_flag != 0)) {
                 // some row of the tile: which of the warp's (its live features are its first lanes')
-                odd_x = odd_rows(x, p.ldx, cols, p.K);
+                if (!READY) odd_x = odd_rows(p.X + (size_t)(tok0 + c_first) * p.ldx, p.ldx, max(0, min(UCOLS, n_tok - c_first)), p.K);
                 odd_w = odd_rows(w - (long long)lane * p.K, p.K, __popc(__ballot_sync(0xffffffffu, live)), p.K) >> lane & 1;
             }
 #pragma unroll 1
-            for (int j = 0; j < cols && live; ++j)
-                if (odd_w || (odd_x >> j & 1) || !chain_free(sums[j])) sums[j] = chain(x + (size_t)j * p.ldx, w, p.K);
+            for (int j = 0; j < COLS; ++j) {
+                if (!live || token(j) >= n_tok || !(odd_w || (odd_x >> j & 1) || !chain_free(sums[j]))) continue;
+                const int row = READY && p.x_index ? p.x_index[tok0 + token(j)] : tok0 + token(j);
+                sums[j] = chain(row >= 0 && row < p.x_rows ? p.X + (size_t)row * p.ldx : nullptr, w, p.K);
+            }
 #pragma unroll
             for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
         }
@@ -409,26 +533,26 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             float* up = (float*)raw;
             if (r >= 64) {
 #pragma unroll
-                for (int j = 0; j < COLS; ++j) up[(c_first + j) * 64 + fr] = acc[j];
+                for (int j = 0; j < COLS; ++j) up[token(j) * 64 + fr] = acc[j];
             }
             asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
         }
         if (live && !(DUAL && r >= 64)) {
             const float b = p.bias ? p.bias[feat] : 0.0f;
             const float b2 = DUAL && p.bias2 ? p.bias2[feat] : 0.0f;
-            float* out = p.C + (size_t)(tok0 + c_first) * p.ldc + feat;
+            float* out = p.C + (size_t)tok0 * p.ldc + feat;
 #pragma unroll
             for (int j = 0; j < COLS; ++j) {
-                if (c_first + j >= n_tok) break;
+                if (token(j) >= n_tok) continue;
                 float v = p.bias ? acc[j] + b : acc[j];
                 if (DUAL) {
-                    const float u = ((const float*)raw)[(c_first + j) * 64 + fr];
+                    const float u = ((const float*)raw)[token(j) * 64 + fr];
                     v = cj::gated_act(v, p.bias2 ? u + b2 : u, p.act_limit, p.act_alpha, p.act_cubic);
                 } else if (p.act != cj::ACT_NONE && feat < p.act_feats) {
                     v = cj::plain_act(v, p.act);
                 }
                 v *= p.out_scale;
-                float* o = out + (size_t)j * p.ldc;
+                float* o = out + (size_t)token(j) * p.ldc;
                 *o = p.accumulate ? v + *o : v;
             }
         }
@@ -458,6 +582,48 @@ __global__ void __launch_bounds__(256) gather_group_rows_kernel(const float* __r
     for (int i = lane; i < K / 4; i += 32) dst[i] = there ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
+// The three parts of rows of x, [3][rows][Kp] bfloat16 (Kp: K rounded up to a block of K, the rest zeros), and whether a row has an entry that
+// is not their sum.  Rows and index as above.  A warp a row.  Bound by memory: 1,777 rows of 2,048 out of HBM 11 us; a tile of 128 tokens x
+// 128 features that splits its rows itself does so features / 128 times (1,777 x 6,144 x 2,048: see the head of the file).
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, int x_rows, const int* __restrict__ index,
+                                                         const int* __restrict__ group_offsets, int groups, int rows, int K, int Kp,
+                                                         __nv_bfloat16* __restrict__ out, int* __restrict__ odd_row) {
+    cj::after_predecessor();
+    cj::release_successor();
+    const int lane = threadIdx.x & 31, s = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lo = group_offsets ? group_offsets[0] : 0, hi = group_offsets ? min(rows, group_offsets[groups]) : rows;
+    if (s < lo || s >= hi) return;
+    const int from = index ? index[s] : s;
+    const bool there = from >= 0 && from < x_rows;
+    const float4* src = (const float4*)(x + (there ? from : 0) * ldx);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const size_t plane = (size_t)rows * Kp;
+    __nv_bfloat16* dst = out + (size_t)s * Kp;
+    uint32_t odd = 0;
+#pragma unroll 4
+    for (int i = lane; i < Kp / 8; i += 32) {
+        uint4 h, m, l;
+        split8(there && 8 * i < K ? src[2 * i] : zero, there && 8 * i + 4 < K ? src[2 * i + 1] : zero, h, m, l, odd);
+        *(uint4*)(dst + 8 * i) = h;
+        *(uint4*)(dst + plane + 8 * i) = m;
+        *(uint4*)(dst + 2 * plane + 8 * i) = l;
+    }
+    const bool any = __any_sync(0xffffffffu, (odd & 0xffffu) != 0);
+    if (lane == 0) odd_row[s] = any;
+}
+
+// the parts that split_rows_kernel left, in boxes of [3][box_rows][32] with the 64-byte swizzle; rows past the last read as zero
+bool make_map_parts(CUtensorMap* map, const void* base, long long rows, long long Kp, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, 3};
+    cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)rows * Kp * 2};
+    cuuint32_t box[3] = {BK, (cuuint32_t)box_rows, 3};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // a row-major float32 matrix in boxes of [box_rows, 32] with the 128-byte swizzle; out-of-range elements read as zero
 bool make_map_f32(CUtensorMap* map, const float* base, long long rows, long long cols, long long ld, int box_rows) {
     EncodeTiledFn fn = encode_fn();
@@ -471,21 +637,25 @@ bool make_map_f32(CUtensorMap* map, const float* base, long long rows, long long
 }
 
 template <int N, bool DUAL>
-int launch(const Args& a, int tok_tiles, cudaStream_t stream) {
+int launch(const Args& a, const void* parts, int tok_tiles, cudaStream_t stream) {
+    using S = Smem<N>;
     auto kern = gemm_f32_tc_kernel<N, DUAL>;
     static bool sized = false;
     if (!sized) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<N>::TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
         if (e != cudaSuccess) return (int)e;
         sized = true;
     }
     if (tok_tiles > 65535) return CJ_ERR_SIZE;
     const long long w_rows = (long long)(a.group_offsets ? a.groups : 1) * a.features;
     CUtensorMap mx, mw, mw2;
-    if (!make_map_f32(&mx, a.X, a.x_rows, a.K, a.ldx, N) || !make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
+    if (ready_x(N)) {
+        if (!parts || !a.x_odd || !make_map_parts(&mx, parts, a.tokens, (a.K + BK - 1) / BK * BK, S::UNIT)) return CJ_ERR_ARG;
+    } else if (!make_map_f32(&mx, a.X, a.x_rows, a.K, a.ldx, N)) return CJ_ERR_ARG;
+    if (!make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
     mw2 = mw;
     if (DUAL && !make_map_f32(&mw2, a.W2, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
-    cj::launch(kern, dim3((a.features + a.feat_tile - 1) / a.feat_tile, tok_tiles), dim3(threads(N)), Smem<N>::TOTAL, stream, mx, mw, mw2, a);
+    cj::launch(kern, dim3((a.features + a.feat_tile - 1) / a.feat_tile, tok_tiles), dim3(threads(N)), S::TOTAL, stream, mx, mw, mw2, a);
     return cj::launch_status();
 }
 
@@ -501,10 +671,23 @@ CJ_EXPORT int cj_gather_group_rows(const float* x, long long ldx, int x_rows, co
     return cj::launch_status();
 }
 
+// Rows of x in three bfloat16 parts, as cj_gemm_f32_tc takes them for tiles of 64 tokens and more: parts [3, rows, K rounded up to 32], odd_row
+// [rows].  index (may be null): the row of x for each; group_offsets (may be null): rows outside the groups are left alone.
+CJ_EXPORT int cj_split_rows(const float* x, long long ldx, int x_rows, const int* index, const int* group_offsets, int groups, int rows, int K,
+                            void* parts, int* odd_row, cudaStream_t stream) {
+    if (rows <= 0) return 0;
+    if (!x || !parts || !odd_row || K <= 0 || x_rows <= 0 || (group_offsets && groups <= 0)) return CJ_ERR_ARG;
+    if (K % 4 != 0 || ldx % 4 != 0 || ldx < K || (((uintptr_t)x | (uintptr_t)parts) & 15)) return CJ_ERR_ALIGN;
+    cj::launch(split_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, x, ldx, x_rows, index, group_offsets, groups, rows, K,
+               (K + BK - 1) / BK * BK, (__nv_bfloat16*)parts, odd_row);
+    return cj::launch_status();
+}
+
 // X [x_rows, K] float32 with row stride ldx (grouped: in the groups' order; no row from x_rows on is read), W (and W2) [groups, features, K]
 // contiguous float32; the
-// other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16, 32, 64 or 128); feat_tile: its features (32, 64 or 128; with W2 at most 64).
-CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
+// other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16 or 32; 64 or 128: the rows' parts and x_odd
+// from cj_split_rows, made for all `tokens` rows, and x_index, which may be null, that kernel's index: then X and x_rows are its x); feat_tile: its features (32, 64 or 128; with W2 at most 64).
+CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const void* parts, const int* x_index, const int* x_odd, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
                              long long ldc, int tokens, int features, int K, int accumulate, const int* group_offsets, int groups,
                              float act_limit, float act_alpha, float act_cubic, int act, int act_feats, float out_scale, int n_tok,
                              int feat_tile, cudaStream_t stream) {
@@ -515,10 +698,10 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const fl
     if (feat_tile != 32 && feat_tile != 64 && !(feat_tile == 128 && !W2)) return CJ_ERR_SIZE;
     if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2) & 15) return CJ_ERR_ALIGN;
-    Args a{X, ldx, W, W2, bias, bias2, C, ldc, tokens, features, K, x_rows, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
+    Args a{X, ldx, x_index, x_odd, W, W2, bias, bias2, C, ldc, tokens, features, K, x_rows, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
            act_feats > 0 ? act_feats : features, out_scale, feat_tile};
     const int tok_tiles = (tokens + n_tok - 1) / max(n_tok, 1) + (group_offsets ? groups : 0);
-#define CASE(N) case N: return W2 ? launch<N, true>(a, tok_tiles, stream) : launch<N, false>(a, tok_tiles, stream);
+#define CASE(N) case N: return W2 ? launch<N, true>(a, parts, tok_tiles, stream) : launch<N, false>(a, parts, tok_tiles, stream);
     switch (n_tok) {
         CASE(16) CASE(32) CASE(64) CASE(128)
     }
@@ -526,7 +709,7 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const fl
     return CJ_ERR_SIZE;
 }
 
-// 0, or the code of the first bounded wait that ran out (15 loads, 11 and 16 splitting, 12 and 14 product issue, 13 adding up);
+// 0, or the code of the first bounded wait that ran out (15 and 17 loads, 11 and 16 splitting, 12, 14 and 18 product issue, 13 adding up);
 // reading it synchronises the device.
 CJ_EXPORT int cj_gemm_f32_tc_error() {
     int v = 0;

@@ -287,13 +287,13 @@ def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
         n_tok = next((n for n in F32_TC_TOKENS if want <= n), F32_TC_TOKENS[-1])
         return n_tok, most if -(-features // most) * min(groups, rows) >= sms else most // 2
 
-    # rounds of the machine times what a block of K takes in a tile of these sizes (us, fitted to 2,048 x 2,048 for one row and
-    # 6,144 x 2,048 for 60, 250 and 1,777); 128 tokens only for many rows: with cold weights and one round 250 x 6,144 took 164 us
-    # with 128 and 114 with 64, 1,777 x 6,144 375 and 543
+    # rounds of the machine times what a block of K takes in a tile of that many tokens, a tile's beginning and end (10 us) included (us, fitted to
+    # 8, 60, 264 and 1,777 rows x 2,048 or 6,144 features x 2,048; the features of a tile change only the rounds): 264 x 6,144 75 us with 128
+    # tokens and 91 with 64, 264 x 2,048 41 with 32, 50 with 64 and 69 with 128
     def cost(n, f):
-        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.18 + 0.0056 * min(n, rows) + 0.0023 * f * (2 if gated else 1))
+        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.46 + 0.005 * min(n, -(-rows // 16) * 16))
 
-    return min(((n, f) for n in F32_TC_TOKENS if n <= 64 or rows >= 512 for f in (most, most // 2)), key=lambda t: cost(*t))
+    return min(((n, f) for n in F32_TC_TOKENS for f in (most, most // 2)), key=lambda t: cost(*t))
 
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -335,16 +335,26 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
     if a_row_index is not None:
         _need(a_row_index, "a_row_index", torch.int32)
     if f32_tc_takes(a, w, w_up, out):
-        if a_row_index is not None:
+        n_tok, feat_tile = f32_tc_tile(M, N, G, w_up is not None, _sm_count())
+        x_rows, parts, odd, index = (a.shape[0] if a_row_index is not None else min(M, a.shape[0])), None, None, None
+        if n_tok >= 64:
+            # X in its three parts, split once for all tiles (the rows in the groups' order)
+            index = a_row_index
+            parts = torch.empty((3, M, -(-K // 32) * 32), dtype=torch.bfloat16, device=a.device)
+            odd = torch.empty((M,), dtype=torch.int32, device=a.device)
+            st = library("gemm_f32_tc").cj_split_rows(_ptr(a), _ll(a.stride(0)), _i(x_rows), _ptr(index), _ptr(group_offsets), _i(G), _i(M), _i(K),
+                                                      _ptr(parts), _ptr(odd), _stream())
+            _check(st, "split_rows")
+        elif a_row_index is not None:
             # the groups' rows side by side (a row outside the groups has no index to follow, an index below 0 names a row of zeros)
             gathered = torch.empty((M, K), dtype=a.dtype, device=a.device)
             st = library("gemm_f32_tc").cj_gather_group_rows(_ptr(a), _ll(a.stride(0)), _i(a.shape[0]), _ptr(a_row_index), _ptr(group_offsets), _i(G),
                                                              _i(M), _i(K), _ptr(gathered), _stream())
             _check(st, "gather_rows")
-            a = gathered
-        n_tok, feat_tile = f32_tc_tile(M, N, G, w_up is not None, _sm_count())
+            a, x_rows = gathered, M
         st = library("gemm_f32_tc").cj_gemm_f32_tc(
-            _ptr(a), _ll(a.stride(0)), _i(min(M, a.shape[0])), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
+            _ptr(a), _ll(a.stride(0)), _i(x_rows), _ptr(parts), _ptr(index), _ptr(odd), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out),
+            _ll(out.stride(0)), _i(M), _i(N), _i(K),
             _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
             _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
         _check(st, "gemm")

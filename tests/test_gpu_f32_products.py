@@ -197,3 +197,26 @@ def test_rows_by_index_of_a_column_slice_and_slots_outside_the_groups(K):
     again = torch.full((slots, N), 7.0, device=DEV)
     K.gemm(rows[:30].contiguous(), w, again, group_offsets=offsets, rows=slots)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("n_tok", [64, 128])
+@pytest.mark.parametrize("Kd", [132, 192])
+def test_rows_split_ahead_follow_their_index(K, monkeypatch, n_tok, Kd):
+    """Tiles of many tokens take rows that were split once, through the index: the bits of tiles that split their own, rows of zeros and
+    rows that are not finite among them."""
+    x, w, up = rnd(90, Kd, seed=24), rnd(3, 70, Kd, seed=25), rnd(3, 70, Kd, seed=26)
+    x[5, 3], x[60, 131], w[1, 9, 0] = float("inf"), 1e-40, float("nan")
+    index = torch.randint(-1, 90, (300,), generator=torch.Generator().manual_seed(27)).int().to(DEV)
+    index[:2] = torch.tensor([5, 60])
+    offsets = torch.tensor([0, 130, 131, 290], dtype=torch.int32, device=DEV)
+    index[290:] = 1 << 20                                       # outside the groups: never followed
+    outs = []
+    for n in (16, n_tok):
+        monkeypatch.setattr(K, "f32_tc_tile", lambda *a, n=n: (n, 64))
+        out = torch.zeros(300, 70, device=DEV)
+        K.gemm(x, w, out, w_up=up, group_offsets=offsets, a_row_index=index)
+        outs.append(out)
+    assert torch.equal(outs[0].view(torch.int32), outs[1].view(torch.int32))
+    finite = torch.isfinite(outs[0][:130][index[:130] != 5])
+    assert bool(finite.all()) and bool(torch.isnan(outs[0][130, 9])) and not bool(outs[0][290:].any())
+    assert K.wait_errors() == {}
