@@ -987,11 +987,13 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
         _need(skip, "skip", torch.float32)
     if state[0].numel() < state_offset + state_scan_floats(heads, rows, cols, mode) or out.shape[1] != heads * cols:
         raise KernelError("state_scan: state or out too small")
+    # (the decays of a prompt's rows, worked out once for all of the scan's blocks)
+    decays = torch.empty((x.shape[0], heads * rows), dtype=torch.float32, device=x.device) if mode == SCAN_GLA and x.shape[0] >= 8 * requests else None
     st = library("recurrent").cj_state_scan(
         _i(mode), _ptr(x), _i(x.stride(0)), _i(off_a), _i(off_b), _i(off_v), _ptr(raw), _i(raw.stride(0)), _i(off_dt), _i(off_beta),
         _ptr(A_log), _ptr(dt_bias), _ptr(skip), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), _ll(state.stride(0)),
         _ll(state[0].numel() - state_offset), _ptr(req_start), _ptr(req_slot), _ptr(out), _i(requests),
-        _i(x.shape[0]), _i(heads), _i(groups), _i(rows), _i(cols), _f(q_scale), _f(c0), _f(c1), _stream())
+        _i(x.shape[0]), _i(heads), _i(groups), _i(rows), _i(cols), _f(q_scale), _f(c0), _f(c1), _ptr(decays), _stream())
     _check(st, "state_scan")
 
 

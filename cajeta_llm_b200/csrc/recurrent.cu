@@ -298,6 +298,7 @@ struct ScanArgs {
     float* out;          // [T, heads * cols]
     int heads, groups, rows, cols;           // rows: state rows (N or key dim); cols: value dim
     float q_scale;
+    int decays_ready;    // gla: raw holds the decays themselves
     float c0, c1;        // gla: c0 = 1 / tau ; mlstm: c0 = the gates' cap, c1 = the floor added to the read-out's divisor
 };
 
@@ -607,10 +608,13 @@ __global__ void __launch_bounds__(128) scan_kernel(ScanArgs p, int DP, int TOK) 
 // tree, the update - so a state or a row has the same bits whichever of the two walked it.  Half of a block's warps walk; the other half
 // fetch the next tokens and work out what needs no state (unit norms, gates, decays' exponentials), a batch ahead.  2,048 tokens of
 // one prompt, scan_kernel, this kernel with every warp doing both, and as it is: state-space, 64 heads of 128 x 64, 1,266, 356 and
-// 274 us; delta rule, 16 of 128 x 128, 1,412, 565 and 333 us; gated linear attention, 4 of 128 x 256, 1,214, 427 and 385 us;
+// 274 us; delta rule, 16 of 128 x 128, 1,412, 565 and 333 us; gated linear attention, 4 of 128 x 256, 1,214, 427 and 385 us (217 with its
+// decays worked out ahead, gla_decays_kernel);
 // matrix memory, 8 of 128 x 256, 1,488, 369 and 296 us.  Two columns a thread: with one 20 to 35 % slower (twice the loads), with
-// four up to 60 % (too few warps).  What bounds it: latencies with one walking warp a scheduler - in the delta rule the chain from one
-// token's state to the next (four dependent shuffles), in gated linear attention the 128 exponentials and logarithms a token.
+// four up to 60 % (too few warps).  What bounds it: latencies with one walking warp a scheduler (an instruction every 3.3 clocks, the FMA
+// pipe at most 47 % busy), in the delta rule the chain from one token's state to the next (four dependent shuffles).  Two rows packed
+// into one instruction (f32x2), operands read a token ahead and eight walking warps of a column each changed nothing or cost time
+// (state-space 282, 286 and 379 us).
 constexpr int WALK_COLS = 2, WALK_BUFS = 3;
 constexpr int walk_tok(int mode) { return mode == SCAN_GLA ? 16 : 32; }      // (with the decays staged too, 32 would leave an SM room for one block)
 
@@ -634,6 +638,16 @@ template <int DP, int N, int STEP, int V> __device__ __forceinline__ void halve_
             halve_sum<DP, 1, STEP + 1>(v, lane);
         }
     }
+}
+
+// The decays of gated linear attention for a step's rows, once: each of the walk's blocks of 8 or so columns (4 heads of 256 columns: 32 a
+// head) would work out all of its head's otherwise, and its walking warps wait for them: 2,048 tokens, 4 heads of 128 x 256, 388 us so,
+// 217 with this kernel before it (its own 4 included).
+__global__ void gla_decays_kernel(const float* __restrict__ raw, int ld, int off, int width, long long n, float c0, float* __restrict__ out) {
+    cj::after_predecessor();
+    cj::release_successor();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = expf(log_sigmoid_f(raw[i / width * ld + off + i % width]) * c0);
 }
 
 template <int DP, int NPER, int MODE, int C>
@@ -739,7 +753,7 @@ __global__ void __launch_bounds__(256, 1) walk_kernel(ScanArgs p) {
                 for (int e = tid; e < nt * ROWS; e += 128) {
                     float* tk = cur + (e / ROWS) * STRIDE + e % ROWS;
                     tk[0] *= p.q_scale;
-                    tk[2 * ROWS] = expf(log_sigmoid_f(tk[2 * ROWS]) * p.c0);
+                    if (!p.decays_ready) tk[2 * ROWS] = expf(log_sigmoid_f(tk[2 * ROWS]) * p.c0);
                 }
             } else if (MODE == SCAN_MLSTM) {
                 float li = 0.0f, lf = 0.0f;
@@ -1419,6 +1433,7 @@ static int launch_walk_as(const ScanArgs& p, int requests, cudaStream_t stream) 
     return launch_status();
 }
 
+static bool walk_built(int DP, int nper) { return DP * nper == 64 ? DP <= 16 : DP * nper == 128 && DP >= 8; }
 // CJ_ERR_SIZE: not built for this share of the rows
 static int launch_walk(int mode, int DP, int nper, const ScanArgs& p, int requests, cudaStream_t stream) {
 #define WALK(D, N)                                                                                                      \
@@ -1440,7 +1455,7 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
                             int off_dt, int off_beta, const float* A_log, const float* dt_bias, const float* skip, float* state,
                             long long slot_stride, long long state_floats, const int* req_start, const int* req_slot, float* out,
                             int requests, int total_rows, int heads, int groups, int rows, int cols, float q_scale, float c0, float c1,
-                            cudaStream_t stream) {
+                            float* decays, cudaStream_t stream) {
     if (requests <= 0) return 0;
     if (mode < 0 || mode > 3) return CJ_ERR_ARG;
     if (!x || !raw || !state || !req_start || !req_slot || !out) return CJ_ERR_ARG;
@@ -1454,13 +1469,23 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
     int nper = 1;
     while (nper < per) nper <<= 1;
     ScanArgs p{x, ld, off_a, off_b, off_v, raw, ld_raw, off_dt, off_beta, A_log, dt_bias, skip, state, slot_stride,
-               req_start, req_slot, out, heads, groups, rows, cols, q_scale, c0, c1};
+               req_start, req_slot, out, heads, groups, rows, cols, q_scale, 0, c0, c1};
     const int cols_per_block = 4 * (32 / DP);
     dim3 grid(requests, heads, (cols + cols_per_block - 1) / cols_per_block);
     if (total_rows >= WALK_MIN_ROWS * requests && rows == DP * nper && grid.y <= 65535
         && state_floats >= (long long)heads * grid.z * scan_tile_floats(mode, nper)) {
         // many tokens a request: the same results from the kernel that walks several columns and tokens at a time, where it is built
-        const int st = launch_walk(mode, DP, nper, p, requests, stream);
+        ScanArgs w = p;
+        if (mode == SCAN_GLA && decays && walk_built(DP, nper)) {
+            const long long n = (long long)total_rows * heads * rows;
+            cj::launch(gla_decays_kernel, dim3((unsigned)min((n + 255) / 256, (long long)148 * 16)), dim3(256), 0, stream, raw, ld_raw, off_dt,
+                       heads * rows, n, c0, decays);
+            w.raw = decays;
+            w.ld_raw = heads * rows;
+            w.off_dt = 0;
+            w.decays_ready = 1;
+        }
+        const int st = launch_walk(mode, DP, nper, w, requests, stream);
         if (st != CJ_ERR_SIZE) return st;
     }
     if (grid.y > 65535 || grid.z > 65535) return CJ_ERR_SIZE;
