@@ -465,22 +465,46 @@ __global__ void __launch_bounds__(32 * WARPS) chunk_kernel(ChunkArgs p) {
 template <typename TZ, typename TO>
 __global__ void gated_row_norm_kernel(const float* __restrict__ y, int n, const TZ* __restrict__ z, int ld_z, const float* __restrict__ w,
                                       float eps, TO* __restrict__ out) {
+    __shared__ float scratch[32];
+    // four entries a thread (all of them up to n = 2,048) are read once and side by side, the weights before the kernel before this one has
+    // ended (no kernel writes them): 4 rows of 2,048, cold, 6.7 -> 3.7 us; bound by two round trips
+    float v[4], g[4], f[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        g[k] = i < n ? w[i] : 0.0f;
+    }
     cj::after_predecessor();
     cj::release_successor();
-    __shared__ float scratch[32];
     const float* yr = y + (size_t)blockIdx.x * n;
     const TZ* zr = z + (size_t)blockIdx.x * ld_z;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        v[k] = i < n ? yr[i] : 0.0f;
+        f[k] = i < n ? to_f32(zr[i]) : 0.0f;
+    }
     float ss = 0.0f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ss = fmaf(yr[i], yr[i], ss);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ss = fmaf(v[k], v[k], ss);
+    const int more = threadIdx.x + 4 * blockDim.x;
+    for (int i = more; i < n; i += blockDim.x) ss = fmaf(yr[i], yr[i], ss);
     ss = warp_sum(ss);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (lane == 0) scratch[warp] = ss;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) f[k] = 1.0f + expf(-f[k]);
     __syncthreads();
     float total = 0.0f;
     for (int i = 0; i < nw; ++i) total += scratch[i];
     const float scale = 1.0f / sqrtf(total / (float)n + eps);
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        out[(size_t)blockIdx.x * n + i] = from_f32<TO>(yr[i] * scale * w[i] / (1.0f + expf(-to_f32(zr[i]))));
+    TO* dst = out + (size_t)blockIdx.x * n;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n) dst[i] = from_f32<TO>(v[k] * scale * g[k] / f[k]);
+    }
+    for (int i = more; i < n; i += blockDim.x) dst[i] = from_f32<TO>(yr[i] * scale * w[i] / (1.0f + expf(-to_f32(zr[i]))));
 }
 
 }  // namespace

@@ -144,3 +144,17 @@ def test_single_tokens_convolution_of_more_channels_than_a_grid_has_threads():
     want, out = w[:, 0] * state[0] + w[:, 1] * x[0], torch.empty(1, C, device=DEV)
     K.short_conv_moved(x, 0, C, taps, w, None, state, SimpleNamespace(row_req=at, req_slot=at, all_single=True), out, activate=False)
     assert torch.allclose(out[0], want, atol=1e-5, rtol=1e-5) and torch.equal(state, x)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (3, 100), (2, 1023), (4, 2048), (2, 2049), (3, 5000)])
+def test_row_norms_whose_first_entries_stay_in_registers(rows, n):
+    """Widths around what the threads hold (latent_q_norm 1,024 and 2,048, gated_row_norm 512 to 2,048), and past it."""
+    from cajeta_llm_b200.csrc import kernels as K
+    x, z, w = rnd(rows, n + 3, seed=31), rnd(rows, n + 5, seed=32), rnd(n, seed=33)
+    v = x[:, 2:2 + n].double()
+    want = v / torch.sqrt((v ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    out = torch.empty(rows, n, device=DEV)
+    K.latent_q_norm(x, 2, n, w, 1e-6, out)
+    assert torch.allclose(out.double(), want, atol=1e-5, rtol=1e-5)
+    K.gated_row_norm(x[:, 2:2 + n].contiguous(), z, 4, w, 1e-6, out)
+    assert torch.allclose(out.double(), want * torch.sigmoid(z[:, 4:4 + n].double()), atol=1e-5, rtol=1e-5)
