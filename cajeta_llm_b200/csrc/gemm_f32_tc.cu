@@ -646,11 +646,10 @@ int launch(const Args& a, const void* parts, int tok_tiles, cudaStream_t stream)
         if (e != cudaSuccess) return (int)e;
         sized = true;
     }
-    if (tok_tiles > 65535) return CJ_ERR_SIZE;
     const long long w_rows = (long long)(a.group_offsets ? a.groups : 1) * a.features;
     CUtensorMap mx, mw, mw2;
     if (ready_x(N)) {
-        if (!parts || !a.x_odd || !make_map_parts(&mx, parts, a.tokens, (a.K + BK - 1) / BK * BK, S::UNIT)) return CJ_ERR_ARG;
+        if (!make_map_parts(&mx, parts, a.tokens, (a.K + BK - 1) / BK * BK, S::UNIT)) return CJ_ERR_ARG;
     } else if (!make_map_f32(&mx, a.X, a.x_rows, a.K, a.ldx, N)) return CJ_ERR_ARG;
     if (!make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
     mw2 = mw;
@@ -661,47 +660,52 @@ int launch(const Args& a, const void* parts, int tok_tiles, cudaStream_t stream)
 
 }  // namespace
 
-// Rows of x (float32, row stride ldx, x_rows of them) in the groups' order, out [rows, K] contiguous: as cj_gemm_f32_tc takes them.
-CJ_EXPORT int cj_gather_group_rows(const float* x, long long ldx, int x_rows, const int* index, const int* group_offsets, int groups, int rows,
-                                   int K, float* out, cudaStream_t stream) {
-    if (rows <= 0) return 0;
-    if (!x || !index || !out || K <= 0 || x_rows <= 0 || (group_offsets && groups <= 0)) return CJ_ERR_ARG;
-    if (K % 4 != 0 || ldx % 4 != 0 || ldx < K || (((uintptr_t)x | (uintptr_t)out) & 15)) return CJ_ERR_ALIGN;
-    cj::launch(gather_group_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, x, ldx, x_rows, index, group_offsets, groups, rows, K, out);
-    return cj::launch_status();
+// Bytes of scratch that cj_gemm_f32_tc needs: the rows' parts and a flag a row for tiles of 64 tokens and more, the gathered rows for smaller ones
+// with an index, else none.
+CJ_EXPORT long long cj_gemm_f32_tc_scratch(int tokens, int K, int n_tok, int indexed) {
+    const long long Kp = (long long)(K + BK - 1) / BK * BK;
+    return n_tok >= 64 ? tokens * (6 * Kp + 4) : indexed ? (long long)tokens * K * 4 : 0;
 }
 
-// Rows of x in three bfloat16 parts, as cj_gemm_f32_tc takes them for tiles of 64 tokens and more: parts [3, rows, K rounded up to 32], odd_row
-// [rows].  index (may be null): the row of x for each; group_offsets (may be null): rows outside the groups are left alone.
-CJ_EXPORT int cj_split_rows(const float* x, long long ldx, int x_rows, const int* index, const int* group_offsets, int groups, int rows, int K,
-                            void* parts, int* odd_row, cudaStream_t stream) {
-    if (rows <= 0) return 0;
-    if (!x || !parts || !odd_row || K <= 0 || x_rows <= 0 || (group_offsets && groups <= 0)) return CJ_ERR_ARG;
-    if (K % 4 != 0 || ldx % 4 != 0 || ldx < K || (((uintptr_t)x | (uintptr_t)parts) & 15)) return CJ_ERR_ALIGN;
-    cj::launch(split_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, x, ldx, x_rows, index, group_offsets, groups, rows, K,
-               (K + BK - 1) / BK * BK, (__nv_bfloat16*)parts, odd_row);
-    return cj::launch_status();
-}
-
-// X [x_rows, K] float32 with row stride ldx (grouped: in the groups' order; no row from x_rows on is read), W (and W2) [groups, features, K]
+// X [x_rows, K] float32 with row stride ldx; x_index (may be null): the row of X for each of `tokens` rows, those outside the groups left alone, an
+// index that names no row of X for zeros; without it row s is row s, and those from x_rows on are zeros.  W (and W2) [groups, features, K]
 // contiguous float32; the
-// other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16 or 32; 64 or 128: the rows' parts and x_odd
-// from cj_split_rows, made for all `tokens` rows, and x_index, which may be null, that kernel's index: then X and x_rows are its x); feat_tile: its features (32, 64 or 128; with W2 at most 64).
-CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const void* parts, const int* x_index, const int* x_odd, const float* W, const float* W2, const float* bias, const float* bias2, float* C,
-                             long long ldc, int tokens, int features, int K, int accumulate, const int* group_offsets, int groups,
-                             float act_limit, float act_alpha, float act_cubic, int act, int act_feats, float out_scale, int n_tok,
-                             int feat_tile, cudaStream_t stream) {
+// other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16, 32, 64 or 128); feat_tile: its features (32, 64 or 128; with W2 at most 64).
+// scratch: cj_gemm_f32_tc_scratch bytes, 16-byte aligned.
+CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const int* x_index, void* scratch, const float* W, const float* W2,
+                             const float* bias, const float* bias2, float* C, long long ldc, int tokens, int features, int K, int accumulate,
+                             const int* group_offsets, int groups, float act_limit, float act_alpha, float act_cubic, int act, int act_feats,
+                             float out_scale, int n_tok, int feat_tile, cudaStream_t stream) {
     if (tokens <= 0 || features <= 0) return 0;
     if (!X || !W || !C || K <= 0 || x_rows <= 0) return CJ_ERR_ARG;
     if (group_offsets && groups <= 0) return CJ_ERR_ARG;
     if ((bias2 && !W2) || (act != cj::ACT_NONE && W2)) return CJ_ERR_ARG;
     if (feat_tile != 32 && feat_tile != 64 && !(feat_tile == 128 && !W2)) return CJ_ERR_SIZE;
+    if (n_tok != 16 && n_tok != 32 && n_tok != 64 && n_tok != 128) return CJ_ERR_SIZE;
     if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
-    if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2) & 15) return CJ_ERR_ALIGN;
+    if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2 | (uintptr_t)scratch) & 15) return CJ_ERR_ALIGN;
+    const int tok_tiles = (tokens + n_tok - 1) / n_tok + (group_offsets ? groups : 0);
+    if (tok_tiles > 65535) return CJ_ERR_SIZE;
+    if (cj_gemm_f32_tc_scratch(tokens, K, n_tok, x_index != nullptr) > 0 && !scratch) return CJ_ERR_ARG;
+    const int* x_odd = nullptr;
+    if (n_tok >= 64) {
+        const int Kp = (K + BK - 1) / BK * BK;
+        int* odd = (int*)((__nv_bfloat16*)scratch + 3 * (size_t)tokens * Kp);
+        cj::launch(split_rows_kernel, dim3((tokens + 7) / 8), dim3(256), 0, stream, X, ldx, x_rows, x_index, group_offsets, groups, tokens, K, Kp,
+                   (__nv_bfloat16*)scratch, odd);
+        x_odd = odd;
+    } else if (x_index) {
+        cj::launch(gather_group_rows_kernel, dim3((tokens + 7) / 8), dim3(256), 0, stream, X, ldx, x_rows, x_index, group_offsets, groups, tokens, K,
+                   (float*)scratch);
+        X = (const float*)scratch;
+        ldx = K;
+        x_rows = tokens;
+        x_index = nullptr;
+    }
+    if (int st = cj::launch_status()) return st;
     Args a{X, ldx, x_index, x_odd, W, W2, bias, bias2, C, ldc, tokens, features, K, x_rows, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
            act_feats > 0 ? act_feats : features, out_scale, feat_tile};
-    const int tok_tiles = (tokens + n_tok - 1) / max(n_tok, 1) + (group_offsets ? groups : 0);
-#define CASE(N) case N: return W2 ? launch<N, true>(a, parts, tok_tiles, stream) : launch<N, false>(a, parts, tok_tiles, stream);
+#define CASE(N) case N: return W2 ? launch<N, true>(a, scratch, tok_tiles, stream) : launch<N, false>(a, scratch, tok_tiles, stream);
     switch (n_tok) {
         CASE(16) CASE(32) CASE(64) CASE(128)
     }

@@ -7,6 +7,7 @@ no fallback: without a CUDA device and the built libraries these functions raise
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Dict, Optional, Sequence
@@ -277,6 +278,7 @@ def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor],
             and a.stride(0) % 4 == 0 and a.stride(0) >= K and (a.data_ptr() | w.data_ptr() | (w_up.data_ptr() if w_up is not None else 0)) % 16 == 0)
 
 
+@functools.lru_cache(maxsize=4096)
 def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
     """(tokens, features) of a tile of the float32 tensor-core product; a result's bits do not depend on them."""
     most = 64 if gated else 128
@@ -336,25 +338,14 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
         _need(a_row_index, "a_row_index", torch.int32)
     if f32_tc_takes(a, w, w_up, out):
         n_tok, feat_tile = f32_tc_tile(M, N, G, w_up is not None, _sm_count())
-        x_rows, parts, odd, index = (a.shape[0] if a_row_index is not None else min(M, a.shape[0])), None, None, None
-        if n_tok >= 64:
-            # X in its three parts, split once for all tiles (the rows in the groups' order)
-            index = a_row_index
-            parts = torch.empty((3, M, -(-K // 32) * 32), dtype=torch.bfloat16, device=a.device)
-            odd = torch.empty((M,), dtype=torch.int32, device=a.device)
-            st = library("gemm_f32_tc").cj_split_rows(_ptr(a), _ll(a.stride(0)), _i(x_rows), _ptr(index), _ptr(group_offsets), _i(G), _i(M), _i(K),
-                                                      _ptr(parts), _ptr(odd), _stream())
-            _check(st, "split_rows")
-        elif a_row_index is not None:
-            # the groups' rows side by side (a row outside the groups has no index to follow, an index below 0 names a row of zeros)
-            gathered = torch.empty((M, K), dtype=a.dtype, device=a.device)
-            st = library("gemm_f32_tc").cj_gather_group_rows(_ptr(a), _ll(a.stride(0)), _i(a.shape[0]), _ptr(a_row_index), _ptr(group_offsets), _i(G),
-                                                             _i(M), _i(K), _ptr(gathered), _stream())
-            _check(st, "gather_rows")
-            a, x_rows = gathered, M
-        st = library("gemm_f32_tc").cj_gemm_f32_tc(
-            _ptr(a), _ll(a.stride(0)), _i(x_rows), _ptr(parts), _ptr(index), _ptr(odd), _ptr(w), _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out),
-            _ll(out.stride(0)), _i(M), _i(N), _i(K),
+        # X in its three parts, split once for all tiles, or the groups' rows side by side (a row outside the groups has no index to
+        # follow, an index below 0 names a row of zeros)
+        lib, indexed = library("gemm_f32_tc"), a_row_index is not None
+        room = M * (6 * (-(-K // 32) * 32) + 4) if n_tok >= 64 else 4 * M * K if indexed else 0
+        scratch = torch.empty((room,), dtype=torch.uint8, device=a.device) if room else None
+        st = lib.cj_gemm_f32_tc(
+            _ptr(a), _ll(a.stride(0)), _i(a.shape[0] if indexed else min(M, a.shape[0])), _ptr(a_row_index), _ptr(scratch), _ptr(w), _ptr(w_up),
+            _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
             _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
             _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
         _check(st, "gemm")
@@ -461,7 +452,7 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v
     vd = value_dim or head_dim
     if (q.dtype == k_plane.dtype == torch.float32 and out.dtype == torch.float32 and head_dim % 4 == 0 and vd % 4 == 0
             and max(head_dim, vd) <= 128 and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
-        tiles, tiles32, singles, requests = 0, 0, True, 0
+        tiles, tiles32, singles, requests = 0, 0, T, 0
         if req_start is not None and h_req_start is not None and len(h_req_start) > 0:      # (an empty list: a step's lengths that nobody filled in)
             _need(req_start, "req_start", torch.int32)
             requests = len(h_req_start) - 1
@@ -469,11 +460,11 @@ def paged_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v
             if h_req_start[0] != 0 or h_req_start[-1] != T or min(rows, default=0) < 0 or req_start.numel() <= requests:
                 raise KernelError(f"paged_attention: h_req_start {list(h_req_start)} does not share out {T} rows")
             tiles, tiles32 = (sum(-(-n // t) for n in rows if n > F32_FEW_ROWS) for t in (64, 32))
-            singles = any(0 < n <= F32_FEW_ROWS for n in rows)
+            singles = sum(n for n in rows if n <= F32_FEW_ROWS)
         st = library("attention_f32").cj_attention_f32(
             _ptr(q), _ptr(out), _ptr(k_plane), _ptr(v_plane), _ptr(positions), _ptr(row_req), _ptr(req_start if requests else None), _i(requests),
             _ptr(table), _i(table.stride(0)), _i(page_tokens), _i(T), _i(n_heads), _i(n_kv), _i(head_dim), _i(vd), _i(window), _f(scale),
-            _f(softcap), gate_ptr, _i(gate_ld), _f(sink), _i(F32_FEW_ROWS), _i(tiles), _i(tiles32), _i(1 if singles else 0), _stream())
+            _f(softcap), gate_ptr, _i(gate_ld), _f(sink), _i(F32_FEW_ROWS), _i(tiles), _i(tiles32), _i(singles), _stream())
         _check(st, "paged_attention")
         return
     st = library("attention_paged").cj_paged_attention(
