@@ -11,9 +11,10 @@
 // Keys outside a row's [from, p] enter none of its sums (they are skipped, not multiplied by zero).
 //
 // The prompt form keeps a thread on 4 rows x 4 keys of the scores and 4 rows x 8 entries of the output, operands as float4 from
-// shared memory (12 shared-memory wavefronts a 16 FMA clocks): bound by the FMA pipe and by waiting for a chunk's keys, which nothing
-// fetches ahead but the SM's other block, where a second one fits.  1,777 rows of one prompt, 16 heads of 128: 713 us, where a row and head
-// a block with a key a lane took 12,700 us.  One row at 570 keys: 34 us, 120 us before.
+// shared memory, which gives an SM 128 bytes a clock: eight of them (32 clocks a warp) for 16 clocks of FMA, so shared memory bounds it, 315 us
+// for the 1,777 rows of one prompt with 16 heads of 128; it takes 685, 785 before a chunk's keys travelled while the chunk before was summed up
+// and its values while its scores were worked out (cold; a row and head a block with a key a lane took 12,700).  256 rows at 700 keys:
+// 199 -> 134 us.  One row at 570 keys: 73 -> 33 us, at 4,000 293 -> 156.
 #define CJ_LIB "attention_f32"
 #include "common.cuh"
 
@@ -23,7 +24,7 @@ using namespace cj;
 
 namespace {
 
-constexpr int KEYS = 64, MAX_DIM = 128, ROW_WARPS = 8;
+constexpr int KEYS = 64, MAX_DIM = 128;
 
 struct Args {
     const float* q; float* out; const float* kplane; const float* vplane;
@@ -54,6 +55,13 @@ __device__ __forceinline__ float chain4(float4 a, float4 b, float s) {
 __device__ __forceinline__ float gate_of(const Args& p, int row, int head) {
     return p.head_gate ? 1.0f / (1.0f + expf(-p.head_gate[(size_t)row * p.gate_ld + head])) : 1.0f;
 }
+
+// 16 bytes on their way to shared memory, zeros where `valid` is not set
+__device__ __forceinline__ void cp_async16(float* smem, const float* gmem, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // VC: float4 of the output a thread holds per row (values of up to 64 VC entries); ROWS: rows of a tile, 64 or 32
 template <int VC, int ROWS>
@@ -104,7 +112,7 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
     if (place[0] < 0) return;
     const int* tab = p.table + (size_t)place[0] * p.table_stride;
     const int pos0 = p.positions[row0];             // the tile's rows are neighbours
-    const int hd4 = p.hd / 4, vd4 = p.vd / 4;
+    const int hd4 = p.hd / 4;
     for (int i = tid; i < ROWS * hd4; i += TILE_THREADS) {
         const int r = i / hd4, d = i - r * hd4;
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -123,22 +131,27 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][c][e] = 0.0f;
     }
-    for (int k0 = first & ~(KEYS - 1); k0 <= last; k0 += KEYS) {
-        __syncthreads();                            // the chunk before has been read
+    // a chunk's keys travel while the chunk before is summed up, its values while its scores are worked out; four threads a key
+    auto fetch = [&](int k0, const float* plane, int size, float* to, int stride) {
+        const int size4 = size / 4;
         for (int i = tid; i < KEYS * 4; i += TILE_THREADS) {
-            const int j = i >> 2, key = k0 + j;     // four threads a key
+            const int j = i >> 2, key = k0 + j;
             const bool held = key >= first && key <= last;
             size_t base = 0;
             if (held) base = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
-            const float4* kr = (const float4*)(p.kplane + base * p.hd);
-            const float4* vr = (const float4*)(p.vplane + base * p.vd);
-            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
-            for (int d = i & 3; d < hd4; d += 4) *(float4*)(Ks + j * ks + 4 * d) = held ? kr[d] : zero;
-#pragma unroll 4
-            for (int d = i & 3; d < vd4; d += 4) *(float4*)(Vs + j * p.vd + 4 * d) = held ? vr[d] : zero;
+            const float* from = plane + base * size;
+#pragma unroll 8
+            for (int d = i & 3; d < size4; d += 4) cp_async16(to + j * stride + 4 * d, from + 4 * d, held);
         }
-        __syncthreads();
+        cp_async_commit();
+    };
+    const int k_first = first & ~(KEYS - 1);
+    fetch(k_first, p.kplane, p.hd, Ks, ks);
+    for (int k0 = k_first; k0 <= last; k0 += KEYS) {
+        if (k0 > k_first) __syncthreads();          // the values of the chunk before have been read
+        fetch(k0, p.vplane, p.vd, Vs, p.vd);
+        cp_async_wait<1>();
+        __syncthreads();                            // the chunk's keys (and, the first time, the queries)
         // scores: rows 4 ty + i, keys tx + 16 j
         float s[4][4];
 #pragma unroll
@@ -157,6 +170,9 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s[i][j] = chain4(a[i], b[j], s[i][j]);
         }
+        __syncthreads();                            // the keys have been read
+        if (k0 + KEYS <= last) fetch(k0 + KEYS, p.kplane, p.hd, Ks, ks);
+        else cp_async_commit();
         float keep[4], take[4];                     // factors of the sums so far and of this chunk's
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -189,7 +205,8 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
                 m[i] = mn;
             }
         }
-        __syncwarp();                               // a row's weights were written by this warp's own lanes
+        cp_async_wait<1>();
+        __syncthreads();                            // the chunk's values (a row's weights were written by its warp's own lanes)
         float o[4][VC][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -259,70 +276,131 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
     }
 }
 
+// floats of a warp's half chunk of keys or values in the kernel below
+__host__ __device__ constexpr int half_floats(int hd, int vd) { return 32 * (hd + 4 > vd ? hd + 4 : vd); }
+
 // A row and head a block: a warp a chunk of 64 keys, lane = keys lane and lane + 32 for the scores and four entries of the value for
-// the sums; after every round of chunks thread d joins them, in order, into entry d of the output.
+// the sums; after every round of chunks thread d joins them, in order, into entry d of the output.  A chunk's two halves of keys are
+// sent for together and its values as soon as the keys have been read, a warp a key (512 bytes side by side), so that a chunk is two
+// round trips to memory; with a lane reading its own key's row, eight pieces at a time, it was twelve, in lines of 128 bytes for 16.
+// HALVES 1: one half at a time, for room.  Bound by the round trips with few blocks, by what an SM draws from memory with many.
+template <int ROW_WARPS, int HALVES>
 __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const Args p) {
     cj::after_predecessor();
     cj::release_successor();
+    extern __shared__ __align__(16) float smem[];
     __shared__ __align__(16) float qs[MAX_DIM];
     __shared__ __align__(16) float oc[ROW_WARPS][MAX_DIM];
     __shared__ float mc_s[ROW_WARPS], lc_s[ROW_WARPS];
-    const int row = blockIdx.x, head = blockIdx.y, kvh = head / (p.n_heads / p.n_kv);
-    const int req = p.row_req[row];
-    if (p.req_start && p.req_start[req + 1] - p.req_start[req] > p.few_rows) return;      // the other kernel's
+    __shared__ int place[2];
+    const int head = blockIdx.y, kvh = head / (p.n_heads / p.n_kv);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (p.req_start) {
+        // the rows of requests with few rows, in order: which is this block's
+        if (warp == 0) {
+            int before = 0, row = -1, req = 0;
+            for (int r0 = 0; r0 < p.requests; r0 += 32) {
+                const int r = r0 + lane;
+                const int a = r < p.requests ? p.req_start[r] : 0, c = r < p.requests ? p.req_start[r + 1] - a : 0;
+                const int n = c <= p.few_rows ? max(c, 0) : 0;
+                int inc = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                const int t = (int)blockIdx.x - (before + inc - n);
+                const unsigned who = __ballot_sync(0xffffffffu, t >= 0 && t < n);
+                if (who) {
+                    const int l = __ffs(who) - 1;
+                    req = r0 + l;
+                    row = __shfl_sync(0xffffffffu, a + t, l);
+                    break;
+                }
+                before += __shfl_sync(0xffffffffu, inc, 31);
+            }
+            if (lane == 0) { place[0] = row; place[1] = req; }
+        }
+        __syncthreads();
+        if (place[0] < 0) return;
+    }
+    const int row = p.req_start ? place[0] : blockIdx.x, req = p.req_start ? place[1] : p.row_req[row];
     const int pos = p.positions[row], from = first_key(pos, p.window);
     const int* tab = p.table + (size_t)req * p.table_stride;
     if (tid < p.hd / 4) *(float4*)(qs + 4 * tid) = *(const float4*)(p.q + ((size_t)row * p.n_heads + head) * p.hd + 4 * tid);
     __syncthreads();
+    float* bufs[2];
+    bufs[0] = smem + warp * HALVES * half_floats(p.hd, p.vd);
+    bufs[1] = bufs[0] + (HALVES - 1) * half_floats(p.hd, p.vd);
+    const int ks = p.hd + 4;
     float m = p.sink, l = p.sink == -INFINITY ? 0.0f : 1.0f, acc = 0.0f;
     for (int k0 = from & ~(KEYS - 1); k0 <= pos; k0 += KEYS * ROW_WARPS) {
         const int c0 = k0 + warp * KEYS;
         if (c0 <= pos) {
             float s[2], e[2];
             size_t base[2];
+            bool seen[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int key = c0 + lane + 32 * j;
+                seen[j] = key >= from && key <= pos;
                 base[j] = 0;
-                s[j] = 0.0f;
-                if (key >= from && key <= pos)
-                    base[j] = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
+                if (seen[j]) base[j] = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
             }
-            const bool seen0 = c0 + lane >= from && c0 + lane <= pos, seen1 = c0 + lane + 32 >= from && c0 + lane + 32 <= pos;
-            const float4* k_a = (const float4*)(p.kplane + base[0] * p.hd);
-            const float4* k_b = (const float4*)(p.kplane + base[1] * p.hd);
-            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            auto fetch = [&](int h, const float* plane, int size, int stride) {
+                __syncwarp();                       // what the half held has been read
+                const unsigned there = __ballot_sync(0xffffffffu, seen[h]);
+#pragma unroll 4
+                for (int j = 0; j < 32; ++j) {
+                    const size_t b = __shfl_sync(0xffffffffu, (unsigned long long)base[h], j);
+                    if (4 * lane < size && (there >> j & 1)) cp_async16(bufs[h] + j * stride + 4 * lane, plane + b * size + 4 * lane, true);
+                }
+                cp_async_commit();
+            };
+            fetch(0, p.kplane, p.hd, ks);
+            if (HALVES == 2) fetch(1, p.kplane, p.hd, ks);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                cp_async_wait<HALVES - 1>();
+                __syncwarp();
+                float dot = 0.0f;
+                if (seen[h]) {
+                    const float* kr = bufs[h] + lane * ks;
 #pragma unroll 8
-            for (int d = 0; d < p.hd / 4; ++d) {
-                const float4 a = *(const float4*)(qs + 4 * d);
-                s[0] = chain4(a, seen0 ? k_a[d] : zero, s[0]);
-                s[1] = chain4(a, seen1 ? k_b[d] : zero, s[1]);
+                    for (int d = 0; d < p.hd; d += 4) dot = chain4(*(const float4*)(qs + d), *(const float4*)(kr + d), dot);
+                }
+                s[h] = seen[h] ? score(dot, p) : -INFINITY;
+                if (HALVES == 2) fetch(h, p.vplane, p.vd, p.vd);
+                else if (h == 0) fetch(1, p.kplane, p.hd, ks);
+                else fetch(0, p.vplane, p.vd, p.vd);
             }
-            s[0] = seen0 ? score(s[0], p) : -INFINITY;
-            s[1] = seen1 ? score(s[1], p) : -INFINITY;
             const float mc = warp_max(fmaxf(s[0], s[1]));
-            e[0] = seen0 ? weight(s[0], mc) : 0.0f;
-            e[1] = seen1 ? weight(s[1], mc) : 0.0f;
+            e[0] = seen[0] ? weight(s[0], mc) : 0.0f;
+            e[1] = seen[1] ? weight(s[1], mc) : 0.0f;
             // the tree of the other kernel: keys 32 apart, then 16 apart, then 1, 2, 4, 8
             float lc = __fadd_rn(e[0], e[1]);
             lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, 16));
 #pragma unroll
             for (int o = 1; o < 16; o <<= 1) lc = __fadd_rn(lc, __shfl_xor_sync(0xffffffffu, lc, o));
             if (lane == 0) { mc_s[warp] = mc; lc_s[warp] = lc; }
-            const int lo = max(from - c0, 0), hi = min(pos - c0, KEYS - 1);
-            float4 o = zero;
+            float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             const bool mine = 4 * lane < p.vd;
-#pragma unroll 8
-            for (int j = lo; j <= hi; ++j) {
-                const float w = __shfl_sync(0xffffffffu, j < 32 ? e[0] : e[1], j & 31);
-                const size_t b = __shfl_sync(0xffffffffu, (unsigned long long)(j < 32 ? base[0] : base[1]), j & 31);
-                if (mine) {
-                    const float4 v = *(const float4*)(p.vplane + b * p.vd + 4 * lane);
-                    o.x = fmaf(w, v.x, o.x);
-                    o.y = fmaf(w, v.y, o.y);
-                    o.z = fmaf(w, v.z, o.z);
-                    o.w = fmaf(w, v.w, o.w);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (HALVES == 1 && h == 1) fetch(1, p.vplane, p.vd, p.vd);
+                if (HALVES == 2 && h == 0) cp_async_wait<1>(); else cp_async_wait<0>();
+                __syncwarp();
+                const int lo = max(from - c0 - 32 * h, 0), hi = min(pos - c0 - 32 * h, 31);
+#pragma unroll 4
+                for (int j = lo; j <= hi; ++j) {
+                    const float w = __shfl_sync(0xffffffffu, e[h], j);
+                    if (mine) {
+                        const float4 v = *(const float4*)(bufs[h] + j * p.vd + 4 * lane);
+                        o.x = fmaf(w, v.x, o.x);
+                        o.y = fmaf(w, v.y, o.y);
+                        o.z = fmaf(w, v.z, o.z);
+                        o.w = fmaf(w, v.w, o.w);
+                    }
                 }
             }
             if (mine) *(float4*)(oc[warp] + 4 * lane) = o;
@@ -341,11 +419,23 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
         p.out[((size_t)row * p.n_heads + head) * p.vd + tid] = __fmul_rn(acc, __fmul_rn(1.0f / l, gate_of(p, row, head)));
 }
 
+int multiprocessors(int& n) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return (int)e;
+    }
+    n = sms;
+    return 0;
+}
+
 }  // namespace
 
 // Arguments as cj_paged_attention's, float32 throughout; req_start [requests + 1]: the step's rows by request (neighbouring rows of a
 // request at neighbouring positions), or null: every row goes by itself.  tiles: an upper bound of the 64-row tiles of the
-// requests with more than few_rows rows, 0 for none, tiles32 the same of 32 rows; singles: whether a request has at most few_rows rows.
+// requests with more than few_rows rows, 0 for none, tiles32 the same of 32 rows; singles: the rows of the others.
 CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, const float* vplane, const int* positions, const int* row_req,
                                const int* req_start, int requests, const int* table, int table_stride, int page_tokens, int T, int n_heads,
                                int n_kv, int hd, int vd, int window, float scale, float softcap, const float* head_gate, int gate_ld,
@@ -359,14 +449,15 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
            scale, softcap, head_gate, gate_ld, sink, few_rows};
     if (tiles > 0) {
         // Tiles of 64 rows where an SM holds two of them and the step has two for every SM, else of 32.  What an SM holds is what hides the
-        // waits for keys: with heads of 128 a tile of 64 rows takes 115 KB and is alone (1,777 rows of 16 heads 728 us, with tiles of 32
-        // 713; 768 rows 187 and 172; 256 rows at 950 keys 185 and 137), with heads of 96 two fit (1,777 rows at 2,277 keys 925 and 987).
-        static int sms = 0, sm_bytes = 0;
-        if (!sms) {
+        // waits for keys: with heads of 128 a tile of 64 rows takes 115 KB and is alone (before keys travelled ahead: 1,777 rows of 16 heads 728 us,
+        // with tiles of 32 713; 768 rows 187 and 172; 256 rows at 950 keys 185 and 137), with heads of 96 two fit (1,777 rows at 2,277 keys 925, 987).
+        int sms = 0;
+        if (int st = multiprocessors(sms)) return st;
+        static int sm_bytes = 0;
+        if (!sm_bytes) {
             int dev = 0;
             cudaError_t e = cudaGetDevice(&dev);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return (int)e;
         }
         auto smem = [](int rows, int h, int v) { return (int)sizeof(float) * ((rows + KEYS) * (h + 4) + KEYS * v + rows * (KEYS + 4)); };
@@ -384,6 +475,28 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
         if (int st = launch_status()) return st;
     }
     if (tiles <= 0) a.req_start = nullptr;                     // no tile: every row by itself, whatever its request has
-    if (singles || tiles <= 0) cj::launch(attention_f32_row_kernel, dim3(T, n_heads), dim3(ROW_WARPS * 32), 0, stream, a);
+    if (singles > 0 || tiles <= 0) {
+        const int rows = a.req_start ? singles : T;
+#define ROWS(W, HALVES)                                                                                                 \
+    do {                                                                                                                \
+        static bool row_sized = false;                                                                                  \
+        if (!row_sized) {                                                                                               \
+            cudaError_t e = cudaFuncSetAttribute(attention_f32_row_kernel<W, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                 HALVES * W * half_floats(MAX_DIM, MAX_DIM) * (int)sizeof(float));      \
+            if (e != cudaSuccess) return (int)e;                                                                        \
+            row_sized = true;                                                                                           \
+        }                                                                                                               \
+        cj::launch(attention_f32_row_kernel<W, HALVES>, dim3(rows, n_heads), dim3(W * 32),                              \
+                   HALVES * W * half_floats(hd, vd) * (int)sizeof(float), stream, a);                                   \
+    } while (0)
+        // With a block an SM at most, six warps whose chunks' halves travel together (8 rows at 520 keys, 16 heads: 36 us, 63 with the kernel
+        // before); with more, three smaller blocks an SM, one summing while another waits (64 rows at 1,000 keys: 303 us with the large blocks,
+        // 241 with these, 283 before; 64 rows at 512 keys 195, 133 and 154).
+        int sms = 0;
+        if (int st = multiprocessors(sms)) return st;
+        if ((long long)rows * n_heads <= sms) ROWS(6, 2);
+        else ROWS(4, 1);
+#undef ROWS
+    }
     return launch_status();
 }
