@@ -29,11 +29,11 @@
 // 44 + n / 2 with W in shared memory (measured alone, back to back).  X goes to shared memory in its parts, split by the same warps or, for
 // tiles of 64 tokens and more, once for all tiles by split_rows_kernel.  Two warps issue the products, every other one each, since one's round
 // of waits, products and commits lasted longer than the products themselves; the last warps add the accumulators up, two sums an instruction,
-// and store.  What bounds it: issue slots with few tokens (of 0.37 us a block of 32 of K with 16 tokens splitting takes 0.13, the loads alone
-// 0.2), the products and the adding up with many (0.84 us with 128 tokens, 0.5 of them the products); and some 10 us of every tile
-// are its beginning and end.  Rows x features x K, us, cold weights; gemm_simt.cu, then W's parts in shared memory with one issuing warp,
-// then now: 8 x 2,048 x 2,048 190, 39 and 34; 264 x 6,144 x 2,048 327, 111 and 75; 1,777 x 6,144 x 2,048 1,817, 366 and 314; 60 groups of 1,408
-// gated features, 17 tokens each 380 and 340, 118 each 750 and 650.
+// and store.  Blocks stay, one an SM, and every role runs across tile boundaries.  What bounds it: issue slots with few tokens (of 0.37 us a
+// block of 32 of K with 16 tokens splitting takes 0.13, the loads alone 0.2), the products and the adding up with many (0.84 us with 128
+// tokens, 0.5 of them the products).  Rows x features x K, us, cold weights; gemm_simt.cu, then W's parts in shared memory with one
+// issuing warp, then a tile a block, then now: 8 x 2,048 x 2,048 190, 39, 34 and 36; 264 x 6,144 x 2,048 327, 111, 75 and 69; 1,777 x 6,144 x 2,048
+// 1,817, 366, 314 and 280; 60 groups of 1,408 gated features, 17 tokens each 380, 340 and 316, 118 each 750, 650 and 625.
 // Built and taken out: two blocks an SM with few tokens (60 groups of 17 tokens 333 us instead of 343, one of 24 groups the same).  (With the
 // float32 operands loaded into registers instead of by TMA 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading
 // threads instead of one changed nothing.)
@@ -76,14 +76,17 @@ struct Args {
     int feat_tile;                         // features of a tile: at most 128, of the gated form at most 64
 };
 
-template <int N> struct Smem {
+constexpr int MAX_GROUPS = 1024;           // groups of a launch: the places of their tiles are a table in shared memory
+
+template <int N, bool DUAL> struct Smem {
     static constexpr int STAGE = 3 * N * 64;                           // the bfloat16 parts of X (those of W lie in tensor memory)
     static constexpr int W_RAW = 128 * 128, X_RAW = ready_x(N) ? 0 : N * 128;       // one float32 tile
     static constexpr int RAW = W_RAW + X_RAW;
     static constexpr int STAGES = split_stages(N), GROUPS = split_groups(N);
     // a multiple of the groups, so that a slot is always read by the same group: a wait by phase parity must not be two phases off
-    static constexpr int RING = (225 * 1024 - STAGES * STAGE) / RAW / GROUPS * GROUPS;
-    static constexpr int TOTAL = STAGES * STAGE + RING * RAW + 1024 /* alignment */;
+    static constexpr int CROSS = DUAL ? epi_warps(N) * 1024 : 0;       // where the second weight's sums cross to the first's threads
+    static constexpr int RING = (221 * 1024 - STAGES * STAGE - CROSS) / RAW / GROUPS * GROUPS;
+    static constexpr int TOTAL = STAGES * STAGE + RING * RAW + CROSS + 1024 /* alignment */;
     static_assert(STAGES % GROUPS == 0, "a stage belongs to one group");
     // tensor memory: two accumulators of a unit of UNIT tokens (a tile of 128 tokens is two units), then the parts of W, three times 16
     // columns a stage
@@ -209,214 +212,245 @@ __device__ __noinline__ unsigned long long odd_rows(const float* first, long lon
 // whether a sum of the parts' products stands as it is (see the head of the file)
 __device__ __forceinline__ bool chain_free(float v) { return (fabsf(v) >= 0x1p-100f && fabsf(v) <= 3.402823466e38f) || v == 0.0f; }
 
+// A tile of the launch: tile index t is (token tile t / feat_tiles, feature tile t % feat_tiles), the token tiles of the groups after one another
+struct Tile {
+    int group, tok0, n_tok, feat0;
+};
+template <int N>
+__device__ __forceinline__ Tile locate(const Args& p, int t, int feat_tiles, const int* before) {
+    const int tt = t / feat_tiles;
+    Tile c;
+    c.feat0 = (t - tt * feat_tiles) * p.feat_tile;
+    c.group = 0;
+    if (p.group_offsets) {
+        int lo = 0, hi = p.groups;                            // before[lo] <= tt < before[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (before[mid] <= tt) lo = mid; else hi = mid;
+        }
+        c.group = lo;
+        c.tok0 = p.group_offsets[lo] + (tt - before[lo]) * N;
+        c.n_tok = min(p.group_offsets[lo + 1] - c.tok0, N);
+    } else {
+        c.tok0 = tt * N;
+        c.n_tok = min(p.tokens - c.tok0, N);
+    }
+    return c;
+}
+
+// Blocks stay, a block an SM, and take every gridDim.x-th tile; all roles run across tile boundaries, so that a tile's first loads and its last
+// sums lie under its neighbours' products (they were 10 us of every tile bare).
 template <int N, bool DUAL>
 __global__ void __launch_bounds__(threads(N), 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                    const __grid_constant__ CUtensorMap map_w2, const Args p) {
-    using S = Smem<N>;
-    constexpr int G = S::GROUPS, STAGES = S::STAGES, EPI_WARPS = epi_warps(N), RING = S::RING, ISSUE = GROUP_WARPS * G,
+    using S = Smem<N, DUAL>;
+    // (blocks of K are counted without a sign: places in rings of odd sizes come cheaper so)
+    constexpr unsigned G = S::GROUPS, STAGES = S::STAGES, RING = S::RING;
+    constexpr int EPI_WARPS = epi_warps(N), ISSUE = GROUP_WARPS * G,
                   LOAD = ISSUE + 2, LOAD_X = LOAD + 1, FIRST_EPI = first_epi(N);
     constexpr bool READY = ready_x(N);
     constexpr int XP = READY ? 0 : 1;                         // rows of X a splitting thread takes (64 rows a pass)
     constexpr int UNIT = S::UNIT, UNITS = S::UNITS, UCOLS = UNIT * 4 / EPI_WARPS, COLS = UNITS * UCOLS;      // columns of an adding thread
-    constexpr uint32_t TMEM_COLS = S::TMEM_COLS;
+    static_assert(UCOLS == 16 && UNITS <= 2, "sixteen columns of a unit an adding thread, a unit an accumulator");
+    constexpr int FLAGS = 8;                                  // tiles that splitting may be ahead of adding up (a tile has four blocks of K at least)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stages = raw + RING * S::RAW;
     __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], x_full[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int odd_flag;                                  // some row of the tile has an entry that is not the sum of three parts
-    __shared__ int place[3];                                  // group, first row, one past the last; group -1: no work
+    __shared__ int odd_flag[FLAGS];                           // some row of the tile has an entry that is not the sum of three parts
+    __shared__ int gave_up;                                   // a wait of an adding warp ran out: all of them leave together
+    __shared__ int before[MAX_GROUPS + 1];                    // token tiles of the groups before one
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == ISSUE) tmem_alloc(&tmem_slot, TMEM_COLS);
+    if (tid == 0) {
+        for (int s = 0; s < RING; ++s) {
+            mbar_init(&raw_full[s], 1);
+            mbar_init(&raw_empty[s], GROUP_WARPS);
+        }
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], GROUP_WARPS);
+            mbar_init(&x_full[s], 1);
+            mbar_init(&empty_bar[s], UNITS);                  // the products of every unit
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], EPI_WARPS);
+        }
+        for (int i = 0; i < FLAGS; ++i) odd_flag[i] = 0;
+        gave_up = 0;
+        fence_barrier_init();
+    }
+    if (warp == ISSUE) tmem_alloc(&tmem_slot, S::TMEM_COLS);
     const bool grouped = p.group_offsets != nullptr;
     if (grouped) cj::after_predecessor();
-    if (warp == 0) {
-        // which rows: token tile blockIdx.y of the whole launch, or of the group that holds it
-        if (grouped) {
-            int before = 0, found = -1, lo = 0, hi = 0;
-            for (int g0 = 0; g0 < p.groups; g0 += 32) {
-                const int g = g0 + lane;
-                const int a = g < p.groups ? p.group_offsets[g] : 0, b = g < p.groups ? p.group_offsets[g + 1] : 0;
-                const int n = g < p.groups ? (b - a + N - 1) / N : 0;
-                int inc = n;
+    if (grouped && warp == 0) {
+        int carry = 0;
+        for (int g0 = 0; g0 < p.groups; g0 += 32) {
+            const int g = g0 + lane;
+            const int n = g < p.groups ? (p.group_offsets[g + 1] - p.group_offsets[g] + N - 1) / N : 0;
+            int inc = n;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
-                }
-                const int t = (int)blockIdx.y - (before + inc - n);
-                const unsigned who = __ballot_sync(0xffffffffu, t >= 0 && t < n);
-                if (who) {
-                    const int l = __ffs(who) - 1;
-                    found = g0 + l;
-                    lo = __shfl_sync(0xffffffffu, a, l) + __shfl_sync(0xffffffffu, t, l) * N;
-                    hi = min(__shfl_sync(0xffffffffu, b, l), lo + N);
-                    break;
-                }
-                before += __shfl_sync(0xffffffffu, inc, 31);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
             }
-            if (lane == 0) { place[0] = found; place[1] = lo; place[2] = hi; }
-        } else if (lane == 0) {
-            place[0] = 0;
-            place[1] = blockIdx.y * N;
-            place[2] = min(p.tokens, place[1] + N);
+            if (g < p.groups) before[g] = carry + inc - n;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
         }
-        if (lane == 0) {
-            const int units = (place[2] - place[1] + UNIT - 1) / UNIT;
-            for (int s = 0; s < RING; ++s) {
-                mbar_init(&raw_full[s], 1);
-                mbar_init(&raw_empty[s], GROUP_WARPS);
-            }
-            for (int s = 0; s < STAGES; ++s) {
-                mbar_init(&full_bar[s], GROUP_WARPS);
-                mbar_init(&x_full[s], 1);
-                mbar_init(&empty_bar[s], max(units, 1));      // the products of every unit
-            }
-            for (int s = 0; s < 2; ++s) {
-                mbar_init(&acc_full[s], 1);
-                mbar_init(&acc_empty[s], EPI_WARPS);
-            }
-            odd_flag = 0;
-            fence_barrier_init();
-        }
+        if (lane == 0) before[p.groups] = carry;
     }
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
     cj::release_successor();                                  // tensor memory is held
-    const int group = place[0], tok0 = place[1], n_tok = place[2] - place[1];
     const uint32_t tmem = tmem_slot;
-    const int feat0 = blockIdx.x * p.feat_tile;
-    const int n_kb = (p.K + BK - 1) / BK;
-    const bool work = group >= 0 && n_tok > 0;
-    const int units = (n_tok + UNIT - 1) / UNIT;
+    const int feat_tiles = (p.features + p.feat_tile - 1) / p.feat_tile;
+    const int n_tiles = (grouped ? before[p.groups] : (p.tokens + N - 1) / N) * feat_tiles;
+    const unsigned n_kb = (p.K + BK - 1) / BK;
     // the width of a unit's products; the parts of its X lie that many rows apart, side by side (those that came in parts UNIT rows)
-    auto width = [&](int u) { return (min(n_tok - u * UNIT, UNIT) + 15) & ~15; };
+    auto width = [](int n_tok, int u) { return (min(n_tok - u * UNIT, UNIT) + 15) & ~15; };
 
-    if (work && warp == LOAD) {
+    if (warp == LOAD) {
         // ---- float32 tiles: the weights' first ones leave before the kernel before this one has ended (no kernel writes weights) ----
         if (elect_one()) {
-            const int w_row = group * p.features + feat0;
             const uint32_t bytes = S::X_RAW + (DUAL ? 2u : 1u) * p.feat_tile * 128;
-            auto weights = [&](int kb, int s) {
+            auto weights = [&](unsigned kb, unsigned s, int w_row) {
                 uint8_t* at = raw + s * S::RAW;
                 tma_load_2d(at, &map_w, &raw_full[s], kb * BK, w_row);
                 if (DUAL) tma_load_2d(at + 64 * 128, &map_w2, &raw_full[s], kb * BK, w_row);
             };
-            const int early = grouped ? 0 : min(RING, n_kb);
-            for (int kb = 0; kb < early; ++kb) {
-                mbar_expect_tx(&raw_full[kb], bytes);
-                weights(kb, kb);
-            }
-            if (!READY && !grouped) cj::after_predecessor();
-            bool ok = true;
-            for (int kb = 0; kb < n_kb && ok; ++kb) {
-                const int s = kb % RING;
-                if (kb >= early) {
-                    ok = mbar_wait(&raw_empty[s], ((kb / RING) & 1) ^ 1, 15);
-                    if (!ok) break;
-                    mbar_expect_tx(&raw_full[s], bytes);
-                    weights(kb, s);
+            unsigned early = 0;
+            if (!grouped) {
+                if ((int)blockIdx.x < n_tiles) {
+                    const Tile c = locate<N>(p, blockIdx.x, feat_tiles, before);
+                    for (; early < min(RING, n_kb); ++early) {
+                        mbar_expect_tx(&raw_full[early], bytes);
+                        weights(early, early, c.feat0);
+                    }
                 }
-                if (!READY) tma_load_2d(raw + s * S::RAW + S::W_RAW, &map_x, &raw_full[s], kb * BK, tok0);
+                if (!READY) cj::after_predecessor();
+            }
+            bool ok = true;
+            unsigned it = 0;
+            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+                const Tile c = locate<N>(p, t, feat_tiles, before);
+                for (unsigned kb = 0; kb < n_kb; ++kb, ++it) {
+                    const unsigned s = it % RING;
+                    if (it >= early) {
+                        ok = mbar_wait(&raw_empty[s], ((it / RING) & 1) ^ 1, 15);
+                        if (!ok) break;
+                        mbar_expect_tx(&raw_full[s], bytes);
+                        weights(kb, s, c.group * p.features + c.feat0);
+                    }
+                    if (!READY) tma_load_2d(raw + s * S::RAW + S::W_RAW, &map_x, &raw_full[s], kb * BK, c.tok0);
+                }
             }
         }
-    } else if (READY && work && warp == LOAD_X) {
+    } else if (READY && warp == LOAD_X) {
         // ---- the parts of X, a stage's three side by side ----
         if (elect_one()) {
             if (!grouped) cj::after_predecessor();
-            for (int kb = 0; kb < n_kb; ++kb) {
-                const int s = kb % STAGES;
-                if (!mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 17)) break;
-                mbar_expect_tx(&x_full[s], units * 3 * UNIT * 64);
-                for (int u = 0; u < units; ++u) tma_load_3d(stages + s * S::STAGE + u * 3 * UNIT * 64, &map_x, &x_full[s], kb * BK, tok0 + u * UNIT, 0);
+            bool ok = true;
+            unsigned it = 0;
+            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+                const Tile c = locate<N>(p, t, feat_tiles, before);
+                const int units = (c.n_tok + UNIT - 1) / UNIT;
+                for (unsigned kb = 0; kb < n_kb; ++kb, ++it) {
+                    const unsigned s = it % STAGES;
+                    ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 17);
+                    if (!ok) break;
+                    mbar_expect_tx(&x_full[s], units * 3 * UNIT * 64);
+                    for (int u = 0; u < units; ++u)
+                        tma_load_3d(stages + s * S::STAGE + u * 3 * UNIT * 64, &map_x, &x_full[s], kb * BK, c.tok0 + u * UNIT, 0);
+                }
             }
         }
-    } else if (work && warp < ISSUE) {
+    } else if (warp < ISSUE) {
         // ---- splitting: of X a thread takes eight of a row's 32 float32 (a row of 64), of W half a row, its lane of tensor memory ----
-        const int g = warp / GROUP_WARPS, piece = tid & 3, row0 = (tid & (32 * GROUP_WARPS - 1)) >> 2;
+        const unsigned g = warp / GROUP_WARPS;
+        const int piece = tid & 3, row0 = (tid & (32 * GROUP_WARPS - 1)) >> 2;
         const int w_row = (warp & 3) * 32 + lane, half = warp >> 2 & 1;
         const bool w_live = (DUAL ? w_row & 63 : w_row) < p.feat_tile;      // (lanes past the tile's features: whatever they read, never stored)
         const uint32_t w_to = tmem + S::A_AT + half * 8 + ((uint32_t)((warp & 3) * 32) << 16);
-        bool x_live[XP + 1];
-#pragma unroll
-        for (int i = 0; i < XP; ++i) x_live[i] = row0 + 64 * i < n_tok;
         // 16-byte pieces 2 piece, 2 piece + 1 of a float32 row, piece `piece` of a bfloat16 row, each where its swizzle puts it
-        // (64 rows apart the swizzles are the same)
         const int src0 = row0 * 128 + (((2 * piece) ^ (row0 & 7)) << 4), src1 = row0 * 128 + (((2 * piece + 1) ^ (row0 & 7)) << 4);
         const int dst = row0 * 64 + ((piece ^ ((row0 >> 1) & 3)) << 4);
-        uint32_t odd = 0;
         bool ok = true;
-        for (int kb = g; kb < n_kb && ok; kb += G) {
-            const int rs = kb % RING, s = kb % STAGES;
-            ok = mbar_wait(&raw_full[rs], (kb / RING) & 1, 16);
-            if (!ok) break;
-            const uint8_t* wr = raw + rs * S::RAW;
-            const uint8_t* xr = wr + S::W_RAW;
-            float4 w[4], x[XP + 1][2];
-            auto read = [&]() {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(wr + w_row * 128 + (((4 * half + i) ^ (w_row & 7)) << 4));
-#pragma unroll
-                for (int i = 0; i < XP; ++i)
-                    if (x_live[i]) {
-                        x[i][0] = *(const float4*)(xr + i * 64 * 128 + src0);
-                        x[i][1] = *(const float4*)(xr + i * 64 * 128 + src1);
-                    }
-            };
-            // a lone group reads while the stage is still in use (1,777 x 6,144: 396 -> 375 us); several cover each other's
-            if (G == 1) read();
-            ok = mbar_wait(&empty_bar[s], ((kb / STAGES) & 1) ^ 1, 11);
-            if (!ok) break;
-            tcgen05_fence_after();
-            if (G > 1) read();
-            {
-                uint4 hi[2], mid[2], lo[2];
-                uint32_t w_odd = 0;
-                split8(w[0], w[1], hi[0], mid[0], lo[0], w_odd);
-                split8(w[2], w[3], hi[1], mid[1], lo[1], w_odd);
-                if (w_live) odd |= w_odd;
-                const uint32_t to = w_to + s * 48;
-                tmem_st8(to, hi[0], hi[1]);
-                tmem_st8(to + 16, mid[0], mid[1]);
-                tmem_st8(to + 32, lo[0], lo[1]);
+        unsigned it = g, end = 0, nth = 0;                    // this group's next block of K of all tiles', one past the tile's last, tiles before it
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++nth) {
+            end += n_kb;
+            bool x_live = false;
+            int x_part = 0;
+            if (!READY) {
+                const Tile c = locate<N>(p, t, feat_tiles, before);
+                x_live = row0 < c.n_tok;
+                x_part = width(c.n_tok, 0) * 64;
             }
-            uint8_t* xt = stages + s * S::STAGE;
+            uint32_t odd = 0;
+            for (; it < end; it += G) {
+                const unsigned rs = it % RING, s = it % STAGES;
+                ok = mbar_wait(&raw_full[rs], (it / RING) & 1, 16);
+                if (!ok) break;
+                const uint8_t* wr = raw + rs * S::RAW;
+                const uint8_t* xr = wr + S::W_RAW;
+                float4 w[4], x[2];
+                auto read = [&]() {
 #pragma unroll
-            for (int i = 0; i < XP; ++i)
-                if (x_live[i]) {
+                    for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(wr + w_row * 128 + (((4 * half + i) ^ (w_row & 7)) << 4));
+                    if (XP && x_live) {
+                        x[0] = *(const float4*)(xr + src0);
+                        x[1] = *(const float4*)(xr + src1);
+                    }
+                };
+                // a lone group reads while the stage is still in use (1,777 x 6,144: 396 -> 375 us); several cover each other's
+                if (G == 1) read();
+                ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 11);
+                if (!ok) break;
+                tcgen05_fence_after();
+                if (G > 1) read();
+                {
+                    uint4 hi[2], mid[2], lo[2];
+                    uint32_t w_odd = 0;
+                    split8(w[0], w[1], hi[0], mid[0], lo[0], w_odd);
+                    split8(w[2], w[3], hi[1], mid[1], lo[1], w_odd);
+                    if (w_live) odd |= w_odd;
+                    const uint32_t to = w_to + s * 48;
+                    tmem_st8(to, hi[0], hi[1]);
+                    tmem_st8(to + 16, mid[0], mid[1]);
+                    tmem_st8(to + 32, lo[0], lo[1]);
+                }
+                if (XP && x_live) {
                     uint4 hi, mid, lo;
-                    split8(x[i][0], x[i][1], hi, mid, lo, odd);
-                    uint8_t* at = xt + i * 3 * UNIT * 64 + dst;
-                    const int x_part = width(i) * 64;
+                    split8(x[0], x[1], hi, mid, lo, odd);
+                    uint8_t* at = stages + s * S::STAGE + dst;
                     *(uint4*)at = hi;
                     *(uint4*)(at + x_part) = mid;
                     *(uint4*)(at + 2 * x_part) = lo;
                 }
-            if (kb + G >= n_kb && (odd & 0xffffu)) odd_flag = 1;
-            if (!READY) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
-            tmem_st_wait();
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&raw_empty[rs]);
-                mbar_arrive(&full_bar[s]);
+                if (it + G >= end && (odd & 0xffffu)) odd_flag[nth % FLAGS] = 1;
+                if (!READY) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // generic writes before the products' reads
+                tmem_st_wait();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&raw_empty[rs]);
+                    mbar_arrive(&full_bar[s]);
+                }
             }
         }
-    } else if (work && (warp == ISSUE || warp == ISSUE + 1)) {
+    } else if (warp == ISSUE || warp == ISSUE + 1) {
         // ---- product issue --------------------------------------------------------------------------
         // two accumulators a unit and block of K, D0 | D1, as wide as the unit each: D0 takes the products of the leading parts alone, whose
         // 16 bits an accumulator holds, D1 the others; the leading part of W meets the first two parts of X in one product twice as wide
         const uint32_t on = elect_one();
         const uint64_t first = umma_desc_sw64(stages);
         const uint32_t b_hi = (uint32_t)(first >> 32), b_first = (uint32_t)first;
-        // unit n of the tile (n counts units over all blocks of K) is warp n % 2's, and so is accumulator n % 2
+        // tiles of one unit: every other block of K is a warp's (with the accumulator of its number), of two: every other unit
         const int mine = warp - ISSUE;
         const uint32_t acc0 = tmem + mine * 2 * UNIT;
-        auto issue = [&](int u, int s, int times) {          // times: how often this warp has issued
-            const int wide = width(u);
+        auto issue = [&](int wide, int u, unsigned s, unsigned times) {     // times: how often this warp has issued
             const uint32_t one = umma_idesc_bf16(128, wide), both = umma_idesc_bf16(128, 2 * wide);
             const uint32_t at = b_first + ((s * S::STAGE + u * 3 * UNIT * 64) >> 4), x_step = (READY ? UNIT : wide) * 64 >> 4;
             const uint32_t w = tmem + S::A_AT + s * 48, d1 = acc0 + wide;
@@ -441,127 +475,153 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             umma_commit_by(on, &acc_full[mine]);
             return true;
         };
-        const int step = units == 2 ? 1 : 2;                  // blocks of K between two units of this warp
-        int times = 0;
-        for (int kb = units == 2 ? 0 : mine; kb < n_kb; kb += step, ++times) {
-            const int s = kb % STAGES;
-            if (!mbar_wait(&full_bar[s], (kb / STAGES) & 1, 12) || (READY && !mbar_wait(&x_full[s], (kb / STAGES) & 1, 18)) || !issue(units == 2 ? mine : 0, s, times)) break;
-        }
-    } else if (work && warp >= FIRST_EPI) {
-        // ---- adding up: a thread has one row of the product (a feature) and COLS of its tokens --------------
-        const int quarter = warp & 3, r = quarter * 32 + lane, c_first = ((warp - FIRST_EPI) >> 2) * UCOLS;
-        auto token = [&](int j) { return j / UCOLS * UNIT + c_first + j % UCOLS; };      // the token of the thread's column j
-        f32x2 acc2[COLS / 2];
-#pragma unroll
-        for (int j = 0; j < COLS / 2; ++j) acc2[j] = pair(0.0f, 0.0f);
         bool ok = true;
-        int n = 0;
-        for (int kb = 0; kb < n_kb && ok; ++kb) {
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) {
-                if (u >= units || !ok) break;
-                const int a = n & 1, wide = width(u);
-                ok = mbar_wait(&acc_full[a], (n >> 1) & 1, 13);
+        unsigned it = UNITS == 2 ? 0 : mine, end = 0, times = 0;
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            end += n_kb;
+            const Tile c = locate<N>(p, t, feat_tiles, before);
+            const int u = UNITS == 2 ? mine : 0;
+            const bool live = u * UNIT < c.n_tok;
+            const int wide = live ? width(c.n_tok, u) : 16;
+            for (; it < end; it += UNITS == 2 ? 1 : 2) {
+                const unsigned s = it % STAGES;
+                ok = mbar_wait(&full_bar[s], (it / STAGES) & 1, 12) && (!READY || mbar_wait(&x_full[s], (it / STAGES) & 1, 18));
                 if (!ok) break;
-                ++n;
-                tcgen05_fence_after();
-                const uint32_t at = tmem + a * 2 * UNIT + c_first + ((uint32_t)(quarter * 32) << 16);
+                if (live) {
+                    ok = issue(wide, u, s, times);
+                    if (!ok) break;
+                    ++times;
+                } else if (lane == 0) {
+                    mbar_arrive(&empty_bar[s]);
+                }
+            }
+        }
+    } else if (warp >= FIRST_EPI) {
+        // ---- adding up: a thread has one row of the product (a feature) and COLS of its tokens --------------
+        const int quarter = warp & 3, r = quarter * 32 + lane, part = (warp - FIRST_EPI) >> 2, c_first = part * UCOLS;
+        auto token = [&](int j) { return j / UCOLS * UNIT + c_first + j % UCOLS; };      // the token of the thread's column j
+        if (!grouped) cj::after_predecessor();
+        bool ok = true;
+        unsigned it = 0, nth = 0, times[UNITS] = {};
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++nth) {
+            const Tile c = locate<N>(p, t, feat_tiles, before);
+            const int n_tok = c.n_tok, tok0 = c.tok0;
+            f32x2 acc2[COLS / 2];
 #pragma unroll
-                for (int c = 0; c < UCOLS; c += 16) {
+            for (int j = 0; j < COLS / 2; ++j) acc2[j] = pair(0.0f, 0.0f);
+            for (unsigned kb = 0; kb < n_kb && ok; ++kb, ++it) {
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u) {
+                    if (u * UNIT >= n_tok || !ok) break;
+                    const int a = UNITS == 2 ? u : it & 1, wide = width(n_tok, u);
+                    ok = mbar_wait(&acc_full[a], (UNITS == 2 ? times[u] : it >> 1) & 1, 13);
+                    if (!ok) break;
+                    ++times[u];
+                    tcgen05_fence_after();
+                    const uint32_t at = tmem + a * 2 * UNIT + c_first + ((uint32_t)(quarter * 32) << 16);
                     uint32_t v[16], h[16];                    // (columns past the unit's width hold whatever they held: nothing asks for them)
-                    tmem_ld16(at + wide + c, v);
-                    tmem_ld16(at + c, h);
+                    tmem_ld16(at + wide, v);
+                    tmem_ld16(at, h);
                     tmem_ld_wait();
-                    if (c + 16 == UCOLS) {                    // the accumulator is free before its sums are added
-                        tcgen05_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&acc_empty[a]);
-                    }
+                    tcgen05_fence_before();                   // the accumulator is free before its sums are added
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[a]);
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) {
-                        f32x2& s = acc2[(u * UCOLS + c + j) / 2];
+                        f32x2& s = acc2[(u * UCOLS + j) / 2];
                         s = add2(add2(s, pair(__uint_as_float(v[j]), __uint_as_float(v[j + 1]))), pair(__uint_as_float(h[j]), __uint_as_float(h[j + 1])));
                     }
                 }
             }
-        }
-        float acc[COLS];
+            if (!ok) gave_up = 1;
+            float acc[COLS];
 #pragma unroll
-        for (int j = 0; j < COLS; j += 2) {
-            const float2 t = both_of(acc2[j / 2]);
-            acc[j] = t.x;
-            acc[j + 1] = t.y;
-        }
-        if (!grouped) cj::after_predecessor();
-        const int fr = DUAL ? (r & 63) : r, feat = feat0 + fr;
-        const bool live = ok && fr < p.feat_tile && feat < p.features;
-        bool again = odd_flag != 0;
-        unsigned long long odd_x = 0;                         // the thread's tokens whose rows are not sums of three parts
-        if (READY) {
+            for (int j = 0; j < COLS; j += 2) {
+                const float2 d = both_of(acc2[j / 2]);
+                acc[j] = d.x;
+                acc[j + 1] = d.y;
+            }
+            const int fr = DUAL ? (r & 63) : r, feat = c.feat0 + fr;
+            const bool live = ok && fr < p.feat_tile && feat < p.features;
+            const bool odd_tile = odd_flag[nth % FLAGS] != 0;
+            bool again = odd_tile;
+            unsigned long long odd_x = 0;                     // the thread's tokens whose rows are not sums of three parts
+            if (READY) {
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u) {
+                    const int tok = u * UNIT + c_first + lane;
+                    odd_x |= (unsigned long long)__ballot_sync(0xffffffffu, lane < UCOLS && tok < n_tok && p.x_odd[tok0 + tok] != 0) << (u * UCOLS);
+                }
+                again = again || odd_x != 0;
+            }
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) again = again || (token(j) < n_tok && !chain_free(acc[j]));
+            if (__any_sync(0xffffffffu, again && ok)) {
+                // (rarely: through an array in memory, so that the sums keep their registers)
+                float sums[COLS];
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
+                const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)c.group * p.features + feat) * p.K;
+                bool odd_w = false;
+                if (__any_sync(0xffffffffu, odd_tile)) {
+                    // some row of the tile: which of the warp's (its live features are its first lanes')
+                    if (!READY) odd_x = odd_rows(p.X + (size_t)(tok0 + c_first) * p.ldx, p.ldx, max(0, min(UCOLS, n_tok - c_first)), p.K);
+                    odd_w = odd_rows(w - (long long)lane * p.K, p.K, __popc(__ballot_sync(0xffffffffu, live)), p.K) >> lane & 1;
+                }
+#pragma unroll 1
+                for (int j = 0; j < COLS; ++j) {
+                    if (!live || token(j) >= n_tok || !(odd_w || (odd_x >> j & 1) || !chain_free(sums[j]))) continue;
+                    const int row = READY && p.x_index ? p.x_index[tok0 + token(j)] : tok0 + token(j);
+                    sums[j] = chain(row >= 0 && row < p.x_rows ? p.X + (size_t)row * p.ldx : nullptr, w, p.K);
+                }
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
+            }
+            const float b = p.bias && live ? p.bias[feat] : 0.0f;
+            const float b2 = DUAL && p.bias2 && live ? p.bias2[feat] : 0.0f;
+            float* out = p.C + (size_t)tok0 * p.ldc + feat;
+            // the four warps of the same tokens
+            auto together = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory"); };
+            float* up = (float*)(stages + STAGES * S::STAGE) + part * 16 * 64;
 #pragma unroll
             for (int u = 0; u < UNITS; ++u) {
-                const int t = u * UNIT + c_first + lane;
-                odd_x |= (unsigned long long)__ballot_sync(0xffffffffu, lane < UCOLS && t < n_tok && p.x_odd[tok0 + t] != 0) << (u * UCOLS);
-            }
-            again = again || odd_x != 0;
-        }
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) again = again || (token(j) < n_tok && !chain_free(acc[j]));
-        if (__any_sync(0xffffffffu, again)) {
-            // (rarely: through an array in memory, so that the sums keep their registers)
-            float sums[COLS];
-#pragma unroll
-            for (int j = 0; j < COLS; ++j) sums[j] = acc[j];
-            const float* w = (DUAL && r >= 64 ? p.W2 : p.W) + ((size_t)group * p.features + feat) * p.K;
-            bool odd_w = false;
-            if (__any_sync(0xffffffffu, odd_flag != 0)) {
-                // some row of the tile: which of the warp's (its live features are its first lanes')
-                if (!READY) odd_x = odd_rows(p.X + (size_t)(tok0 + c_first) * p.ldx, p.ldx, max(0, min(UCOLS, n_tok - c_first)), p.K);
-                odd_w = odd_rows(w - (long long)lane * p.K, p.K, __popc(__ballot_sync(0xffffffffu, live)), p.K) >> lane & 1;
-            }
-#pragma unroll 1
-            for (int j = 0; j < COLS; ++j) {
-                if (!live || token(j) >= n_tok || !(odd_w || (odd_x >> j & 1) || !chain_free(sums[j]))) continue;
-                const int row = READY && p.x_index ? p.x_index[tok0 + token(j)] : tok0 + token(j);
-                sums[j] = chain(row >= 0 && row < p.x_rows ? p.X + (size_t)row * p.ldx : nullptr, w, p.K);
-            }
-#pragma unroll
-            for (int j = 0; j < COLS; ++j) acc[j] = sums[j];
-        }
-        if (DUAL) {
-            // the second weight's sums cross to the threads that hold the first's: through the ring, which nothing reads any more
-            float* up = (float*)raw;
-            if (r >= 64) {
-#pragma unroll
-                for (int j = 0; j < COLS; ++j) up[token(j) * 64 + fr] = acc[j];
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-        }
-        if (live && !(DUAL && r >= 64)) {
-            const float b = p.bias ? p.bias[feat] : 0.0f;
-            const float b2 = DUAL && p.bias2 ? p.bias2[feat] : 0.0f;
-            float* out = p.C + (size_t)tok0 * p.ldc + feat;
-#pragma unroll
-            for (int j = 0; j < COLS; ++j) {
-                if (token(j) >= n_tok) continue;
-                float v = p.bias ? acc[j] + b : acc[j];
                 if (DUAL) {
-                    const float u = ((const float*)raw)[token(j) * 64 + fr];
-                    v = cj::gated_act(v, p.bias2 ? u + b2 : u, p.act_limit, p.act_alpha, p.act_cubic);
-                } else if (p.act != cj::ACT_NONE && feat < p.act_feats) {
-                    v = cj::plain_act(v, p.act);
+                    // the second weight's sums cross to the threads that hold the first's, a unit at a time
+                    if (u > 0) together();
+                    if (r >= 64) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) up[j * 64 + fr] = acc[u * 16 + j];
+                    }
+                    together();
                 }
-                v *= p.out_scale;
-                float* o = out + (size_t)token(j) * p.ldc;
-                *o = p.accumulate ? v + *o : v;
+                if (live && !(DUAL && r >= 64)) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (token(u * 16 + j) >= n_tok) break;
+                        float v = p.bias ? acc[u * 16 + j] + b : acc[u * 16 + j];
+                        if (DUAL) {
+                            const float w2 = up[j * 64 + fr];
+                            v = cj::gated_act(v, p.bias2 ? w2 + b2 : w2, p.act_limit, p.act_alpha, p.act_cubic);
+                        } else if (p.act != cj::ACT_NONE && feat < p.act_feats) {
+                            v = cj::plain_act(v, p.act);
+                        }
+                        v *= p.out_scale;
+                        float* o = out + (size_t)token(u * 16 + j) * p.ldc;
+                        *o = p.accumulate ? v + *o : v;
+                    }
+                }
             }
+            // everyone has read the flag (and what crossed) before the next tile's
+            asm volatile("bar.sync 5, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+            if (warp == FIRST_EPI && lane == 0) odd_flag[nth % FLAGS] = 0;
+            ok = gave_up == 0;
         }
     }
     tcgen05_fence_before();
     __syncthreads();
     if (warp == ISSUE) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem, TMEM_COLS);
+        tmem_dealloc(tmem, S::TMEM_COLS);
     }
 }
 
@@ -638,7 +698,7 @@ bool make_map_f32(CUtensorMap* map, const float* base, long long rows, long long
 
 template <int N, bool DUAL>
 int launch(const Args& a, const void* parts, int tok_tiles, cudaStream_t stream) {
-    using S = Smem<N>;
+    using S = Smem<N, DUAL>;
     auto kern = gemm_f32_tc_kernel<N, DUAL>;
     static bool sized = false;
     if (!sized) {
@@ -654,7 +714,16 @@ int launch(const Args& a, const void* parts, int tok_tiles, cudaStream_t stream)
     if (!make_map_f32(&mw, a.W, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
     mw2 = mw;
     if (DUAL && !make_map_f32(&mw2, a.W2, w_rows, a.K, a.K, a.feat_tile)) return CJ_ERR_ARG;
-    cj::launch(kern, dim3((a.features + a.feat_tile - 1) / a.feat_tile, tok_tiles), dim3(threads(N)), S::TOTAL, stream, mx, mw, mw2, a);
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const long long tiles = (long long)((a.features + a.feat_tile - 1) / a.feat_tile) * tok_tiles;
+    if (tiles > 0x3fffffff) return CJ_ERR_SIZE;
+    cj::launch(kern, dim3((unsigned)min(tiles, (long long)sms)), dim3(threads(N)), S::TOTAL, stream, mx, mw, mw2, a);
     return cj::launch_status();
 }
 
@@ -685,7 +754,7 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const in
     if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2 | (uintptr_t)scratch) & 15) return CJ_ERR_ALIGN;
     const int tok_tiles = (tokens + n_tok - 1) / n_tok + (group_offsets ? groups : 0);
-    if (tok_tiles > 65535) return CJ_ERR_SIZE;
+    if (group_offsets && groups > MAX_GROUPS) return CJ_ERR_SIZE;
     if (cj_gemm_f32_tc_scratch(tokens, K, n_tok, x_index != nullptr) > 0 && !scratch) return CJ_ERR_ARG;
     const int* x_odd = nullptr;
     if (n_tok >= 64) {

@@ -267,6 +267,7 @@ def _gate_biases(w: torch.Tensor, w_up: Optional[torch.Tensor], bias: Optional[t
 
 
 F32_TC_TOKENS = (16, 32, 64, 128)      # token tiles of the float32 tensor-core product
+F32_TC_GROUPS = 1024                   # groups whose places a block of it holds
 
 
 def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor], out: torch.Tensor) -> bool:
@@ -275,6 +276,7 @@ def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor],
     number of rows is no part of it: a row's bits must not depend on the others."""
     N, K = w.shape[-2], w.shape[-1]
     return (a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K >= 128 and N >= 64 and K % 4 == 0
+            and (w.dim() < 3 or w.shape[0] <= F32_TC_GROUPS)
             and a.stride(0) % 4 == 0 and a.stride(0) >= K and (a.data_ptr() | w.data_ptr() | (w_up.data_ptr() if w_up is not None else 0)) % 16 == 0)
 
 
@@ -289,11 +291,11 @@ def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
         n_tok = next((n for n in F32_TC_TOKENS if want <= n), F32_TC_TOKENS[-1])
         return n_tok, most if -(-features // most) * min(groups, rows) >= sms else most // 2
 
-    # rounds of the machine times what a block of K takes in a tile of that many tokens, a tile's beginning and end (10 us) included (us, fitted to
-    # 8, 60, 264 and 1,777 rows x 2,048 or 6,144 features x 2,048; the features of a tile change only the rounds): 264 x 6,144 75 us with 128
-    # tokens and 91 with 64, 264 x 2,048 41 with 32, 50 with 64 and 69 with 128
+    # rounds of the machine times what a block of K takes in a tile of that many tokens (us, fitted to 8, 60, 264 and 1,777 rows x 2,048 or 6,144
+    # features x 2,048; the features of a tile change only the rounds): 264 x 6,144 69 us with 128 tokens and 90 with 64, 264 x 2,048 41 with
+    # 32, 52 with 64 and 65 with 128, 1,777 x 2,048 124 with 128 and 167 with 64
     def cost(n, f):
-        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.46 + 0.005 * min(n, -(-rows // 16) * 16))
+        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.31 + 0.0044 * min(n, -(-rows // 16) * 16))
 
     return min(((n, f) for n in F32_TC_TOKENS for f in (most, most // 2)), key=lambda t: cost(*t))
 

@@ -220,3 +220,30 @@ def test_rows_split_ahead_follow_their_index(K, monkeypatch, n_tok, Kd):
     finite = torch.isfinite(outs[0][:130][index[:130] != 5])
     assert bool(finite.all()) and bool(torch.isnan(outs[0][130, 9])) and not bool(outs[0][290:].any())
     assert K.wait_errors() == {}
+
+
+@pytest.mark.parametrize("Kd", [132, 260])                      # five and nine blocks of K: the rings' places and phases move from tile to tile
+def test_blocks_that_take_many_tiles(K, monkeypatch, Kd):
+    """More tiles than the machine has blocks, the last ones part-filled, a row and a feature that are not finite in the middle ones."""
+    a, w = rnd(2100, Kd, seed=28), rnd(1500, Kd, seed=29)
+    plain, want = torch.empty(2100, 1500, device=DEV), a.double() @ w.double().t()
+    K.gemm(a, w, plain)
+    held(plain, a, w, want)
+    a[1000, 5], w[700, 100] = float("inf"), 1e-40
+    rows, feats = torch.arange(2100, device=DEV) != 1000, torch.arange(1500, device=DEV) != 700
+    for n_tok in (16, 32, 64, 128):
+        monkeypatch.setattr(K, "f32_tc_tile", lambda *x: (n_tok, 64))
+        out = torch.empty(2100, 1500, device=DEV)
+        K.gemm(a, w, out)
+        assert torch.equal(out[rows][:, feats], plain[rows][:, feats]) and not bool(torch.isfinite(out[1000]).any())
+        # gated and in groups: the two weights' sums cross while the next tile is under way
+        offsets = torch.tensor([0, 1, 1, 700, 2100], dtype=torch.int32, device=DEV)
+        wg, wu = w[:1480].view(4, 370, Kd), w[20:].view(4, 370, Kd)
+        got = torch.empty(2100, 370, device=DEV)
+        K.gemm(a, wg, got, w_up=wu, group_offsets=offsets)
+        for g in range(4):
+            lo, hi = int(offsets[g]), int(offsets[g + 1])
+            x, y = (a[lo:hi].double() @ t[g].double().t() for t in (wg, wu))
+            fine = torch.arange(lo, hi, device=DEV) != 1000
+            assert torch.allclose(got[lo:hi].double()[fine], (x * torch.sigmoid(x) * y)[fine], atol=1e-3, rtol=1e-4)
+    assert K.wait_errors() == {}
