@@ -61,6 +61,20 @@ __global__ void cast_rows_kernel(const float* __restrict__ x, TO* __restrict__ o
         out[i] = from_f32<TO>(x[i]);
 }
 
+// The same, four at a time: 16-byte loads, 8- or 16-byte stores (n a multiple of four, both pointers on their boundaries).  2,048 rows of 2,048
+// to bfloat16, cold: 8.8 us with the kernel above, 6.1 so
+__device__ __forceinline__ void store_piece(float* dst, float4 v) { *(float4*)dst = v; }
+__device__ __forceinline__ void store_piece(__nv_bfloat16* dst, float4 v) {
+    __nv_bfloat162 two[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+    *(uint2*)dst = *(const uint2*)two;
+}
+template <typename TO>
+__global__ void __launch_bounds__(256) cast_rows4_kernel(const float4* __restrict__ x, TO* __restrict__ out, long long n4) {
+    cj::after_predecessor();
+    cj::release_successor();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) store_piece(out + 4 * i, x[i]);
+}
+
 __global__ void rmsnorm_add_kernel(float* __restrict__ hs, const float* __restrict__ y, const float* __restrict__ w, float eps, int H) {
     cj::after_predecessor();
     cj::release_successor();
@@ -1081,6 +1095,67 @@ __global__ void rmsnorm_mix2_kernel(const float* __restrict__ a, const float* __
     }
 }
 
+// The same for widths that are multiples of four, up to 4,096, everything on 16 bytes: a thread keeps its NV float4 of both rows, which are read
+// once.  The squares are added in the order of the kernel above with `order` threads, from shared memory, as in rmsnorm_add4_kernel: the
+// same bits.  Bound by memory: 1,511 rows of 2,048, cold, 20.2 us with the kernel above, 12.4 so
+template <int NV>
+__global__ void __launch_bounds__(256) rmsnorm_mix2_vec_kernel(const float* __restrict__ a, const float* __restrict__ wa, const float* __restrict__ b,
+                                                               const float* __restrict__ wb, float eps, float c, int accumulate, float* __restrict__ out,
+                                                               int H, int order) {
+    cj::after_predecessor();
+    cj::release_successor();
+    __shared__ __align__(16) float row[2][1024 * NV];
+    __shared__ float sums[2][16];
+    const float4* ra = (const float4*)(a + (size_t)blockIdx.x * H);
+    const float4* rb = (const float4*)(b + (size_t)blockIdx.x * H);
+    float4* dst = (float4*)(out + (size_t)blockIdx.x * H);
+    const int n4 = H / 4;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 va[NV], vb[NV], old[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        va[k] = vb[k] = old[k] = zero;
+        if (i < n4) {
+            va[k] = ra[i];
+            vb[k] = rb[i];
+            if (accumulate) old[k] = dst[i];
+            *(float4*)(row[0] + 4 * i) = va[k];
+            *(float4*)(row[1] + 4 * i) = vb[k];
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < order; t += 256) {
+        float sa = 0.0f, sb = 0.0f;
+        for (int i = t; i < H; i += order) {
+            sa = fmaf(row[0][i], row[0][i], sa);
+            sb = fmaf(row[1][i], row[1][i], sb);
+        }
+        sa = warp_sum(sa);
+        sb = warp_sum(sb);
+        if ((t & 31) == 0) { sums[0][t >> 5] = sa; sums[1][t >> 5] = sb; }
+    }
+    __syncthreads();
+    float sa = 0.0f, sb = 0.0f;
+    for (int i = 0; i < order / 32; ++i) {
+        sa += sums[0][i];
+        sb += sums[1][i];
+    }
+    const float fa = 1.0f / sqrtf(sa / (float)H + eps), fb = 1.0f / sqrtf(sb / (float)H + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i >= n4) continue;
+        const float4 ga = ((const float4*)wa)[i], gb = ((const float4*)wb)[i];
+        auto mixed = [&](float x, float g, float y, float h, float o) {
+            const float v = c * (x * fa * g + y * fb * h);
+            return accumulate ? o + v : v;
+        };
+        dst[i] = make_float4(mixed(va[k].x, ga.x, vb[k].x, gb.x, old[k].x), mixed(va[k].y, ga.y, vb[k].y, gb.y, old[k].y),
+                             mixed(va[k].z, ga.z, vb[k].z, gb.z, old[k].z), mixed(va[k].w, ga.w, vb[k].w, gb.w, old[k].w));
+    }
+}
+
 // x <- cap tanh(x / cap), in place, float32
 __global__ void softcap_rows_kernel(float* __restrict__ x, float cap, long long n) {
     cj::after_predecessor();
@@ -1292,11 +1367,17 @@ static int scan_lanes(int heads, int rows, int cols) {
 CJ_EXPORT int cj_cast_rows(const float* x, void* out, int out_dtype, long long n, cudaStream_t stream) {
     if (n <= 0) return 0;
     if (!x || !out) return CJ_ERR_ARG;
+    if (out_dtype != CJ_F32 && out_dtype != CJ_BF16) return CJ_ERR_DTYPE;
+    if (n % 4 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0) {
+        const dim3 grid((unsigned)min((n / 4 + 255) / 256, (long long)148 * 16));
+        if (out_dtype == CJ_F32) cj::launch(cast_rows4_kernel<float>, grid, dim3(256), 0, stream, (const float4*)x, (float*)out, n / 4);
+        else cj::launch(cast_rows4_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, (const float4*)x, (__nv_bfloat16*)out, n / 4);
+        return launch_status();
+    }
     long long blocks = (n + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (out_dtype == CJ_F32) cj::launch(cast_rows_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, x, (float*)out, n);
-    else if (out_dtype == CJ_BF16) cj::launch(cast_rows_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, stream, x, (__nv_bfloat16*)out, n);
-    else return CJ_ERR_DTYPE;
+    else cj::launch(cast_rows_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, stream, x, (__nv_bfloat16*)out, n);
     return launch_status();
 }
 
@@ -1617,6 +1698,14 @@ CJ_EXPORT int cj_rmsnorm_mix2(const float* a, const float* wa, const float* b, c
     if (rows <= 0) return 0;
     if (!a || !wa || !b || !wb || !out || H <= 0) return CJ_ERR_ARG;
     int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
+    if (H % 4 == 0 && H <= 4096 && (((uintptr_t)a | (uintptr_t)wa | (uintptr_t)b | (uintptr_t)wb | (uintptr_t)out) & 15) == 0) {
+#define MIX(NV) cj::launch(rmsnorm_mix2_vec_kernel<NV>, dim3(rows), dim3(256), 0, stream, a, wa, b, wb, eps, c, accumulate, out, H, threads)
+        if (H <= 1024) MIX(1);
+        else if (H <= 2048) MIX(2);
+        else MIX(4);
+#undef MIX
+        return launch_status();
+    }
     cj::launch(rmsnorm_mix2_kernel, dim3(rows), dim3(threads), 0, stream, a, wa, b, wb, eps, c, accumulate, out, H);
     return launch_status();
 }

@@ -25,6 +25,30 @@ __global__ void embed_gather_kernel(float* __restrict__ out, const TW* __restric
     for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] = ok ? to_f32(src[i]) * f : 0.0f;
 }
 
+// The same for tables of bfloat16 whose rows are whole pieces of 16 bytes: a thread takes eight entries at a time.  2,048 rows of 2,048,
+// cold: 13.8 us with the kernel above (two bytes a load), 8.8 so.
+__global__ void embed_gather8_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ table, const int* __restrict__ ids, int H, int V, float scale) {
+    cj::after_predecessor();
+    cj::release_successor();
+    const int t = blockIdx.x, id = ids[t];
+    const bool ok = id >= 0 && id < V;
+    const uint4* src = (const uint4*)(table + (size_t)(ok ? id : 0) * H);
+    float4* dst = (float4*)(out + (size_t)t * H);
+    const float f = scale != 0.0f ? scale : 1.0f;
+    for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+        const uint4 u = ok ? src[i] : make_uint4(0, 0, 0, 0);
+        const unsigned w[4] = {u.x, u.y, u.z, u.w};
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[2 * k] = ok ? __uint_as_float(w[k] << 16) * f : 0.0f;
+            v[2 * k + 1] = ok ? __uint_as_float(w[k] & 0xffff0000u) * f : 0.0f;
+        }
+        dst[2 * i] = make_float4(v[0], v[1], v[2], v[3]);
+        dst[2 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
 CJ_EXPORT int cj_embed_gather(float* out, const void* table, int table_dtype, const int* ids,
                               int T, int H, int V, float scale, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -32,6 +56,8 @@ CJ_EXPORT int cj_embed_gather(float* out, const void* table, int table_dtype, co
     int threads = H >= 1024 ? 256 : 128;
     if (table_dtype == CJ_F32)
         cj::launch(embed_gather_kernel<float>, dim3(T), dim3(threads), 0, stream, out, (const float*)table, ids, H, V, scale);
+    else if (table_dtype == CJ_BF16 && H % 8 == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
+        cj::launch(embed_gather8_kernel, dim3(T), dim3(min(256, max(32, (H / 8 + 31) / 32 * 32))), 0, stream, out, (const __nv_bfloat16*)table, ids, H, V, scale);
     else if (table_dtype == CJ_BF16)
         cj::launch(embed_gather_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, stream, out, (const __nv_bfloat16*)table, ids, H, V, scale);
     else

@@ -158,3 +158,34 @@ def test_row_norms_whose_first_entries_stay_in_registers(rows, n):
     assert torch.allclose(out.double(), want, atol=1e-5, rtol=1e-5)
     K.gated_row_norm(x[:, 2:2 + n].contiguous(), z, 4, w, 1e-6, out)
     assert torch.allclose(out.double(), want * torch.sigmoid(z[:, 4:4 + n].double()), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("H", [8, 20, 264, 2048, 2056])
+def test_embedding_rows_in_pieces_of_eight(H):
+    """Rows of whole 16-byte pieces and not, a scale, and an id out of range."""
+    from cajeta_llm_b200.csrc import kernels as K
+    table = rnd(7, H, seed=41).bfloat16()
+    ids = torch.tensor([6, 0, 3, 9, -1], dtype=torch.int32, device=DEV)
+    for scale in (0.0, 1.75):
+        out = torch.empty(5, H, device=DEV)
+        K.embed_gather(out, table, ids, scale)
+        want = torch.cat([table[[6, 0, 3]].float() * (scale or 1.0), torch.zeros(2, H, device=DEV)])
+        assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("rows,H", [(1, 4), (3, 7), (5, 1028), (2, 2048), (3, 4096), (2, 4100)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_two_normed_rows_mixed_and_cast(rows, H, accumulate):
+    from cajeta_llm_b200.csrc import kernels as K
+    a, b, wa, wb, out = rnd(rows, H, seed=42), rnd(rows, H, seed=43), rnd(H, seed=44), rnd(H, seed=45), rnd(rows, H, seed=46)
+
+    def normed(t, w):
+        return t.double() / torch.sqrt((t.double() ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+
+    want = 0.5 * (normed(a, wa) + normed(b, wb)) + (out.double() if accumulate else 0.0)
+    K.rmsnorm_mix2(a, wa, b, wb, 1e-6, 0.5, out, accumulate=accumulate)
+    assert torch.allclose(out.double(), want, atol=1e-5, rtol=1e-5)
+    for dtype in (torch.float32, torch.bfloat16):
+        cast = torch.empty(rows, H, device=DEV, dtype=dtype)
+        K.cast_rows(out, cast)
+        assert torch.equal(cast, out.to(dtype))
