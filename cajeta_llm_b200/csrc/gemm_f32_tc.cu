@@ -253,7 +253,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     constexpr int XP = READY ? 0 : 1;                         // rows of X a splitting thread takes (64 rows a pass)
     constexpr int UNIT = S::UNIT, UNITS = S::UNITS, UCOLS = UNIT * 4 / EPI_WARPS, COLS = UNITS * UCOLS;      // columns of an adding thread
     static_assert(UCOLS == 16 && UNITS <= 2, "sixteen columns of a unit an adding thread, a unit an accumulator");
-    constexpr int FLAGS = 8;                                  // tiles that splitting may be ahead of adding up (a tile has four blocks of K at least)
+    constexpr int FLAGS = 16;                                 // more tiles than splitting can be ahead of adding up: its stages and the accumulators
     extern __shared__ uint8_t smem_raw[];
     uint8_t* raw = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stages = raw + RING * S::RAW;
