@@ -430,7 +430,7 @@ NO_SINK = float("-inf")      # no key without a value joins the softmax
 
 
 # float32 attention: a request with at most this many rows in the step goes a row a block, one with more 64 or 32 rows a block.  Eight
-# rows at 520 keys in each of eight requests took 127 us a row a block; as a tile of 64 they would pay for 56 that are not there.
+# rows at 512 keys in each of eight requests take 133 us a row a block (cold); as a tile of 64 they would pay for 56 that are not there.
 F32_FEW_ROWS = 8
 
 
