@@ -565,7 +565,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 bool odd_w = false;
                 if (__any_sync(0xffffffffu, odd_tile)) {
                     // some row of the tile: which of the warp's (its live features are its first lanes')
-                    if (!READY) odd_x = odd_rows(p.X + (size_t)(tok0 + c_first) * p.ldx, p.ldx, max(0, min(UCOLS, n_tok - c_first)), p.K);
+                    // (rows from x_rows on are zeros, not memory of X)
+                    if (!READY)
+                        odd_x = odd_rows(p.X + (size_t)(tok0 + c_first) * p.ldx, p.ldx, max(0, min(UCOLS, min(n_tok, p.x_rows - tok0) - c_first)), p.K);
                     odd_w = odd_rows(w - (long long)lane * p.K, p.K, __popc(__ballot_sync(0xffffffffu, live)), p.K) >> lane & 1;
                 }
 #pragma unroll 1

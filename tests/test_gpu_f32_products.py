@@ -247,3 +247,23 @@ def test_blocks_that_take_many_tiles(K, monkeypatch, Kd):
             fine = torch.arange(lo, hi, device=DEV) != 1000
             assert torch.allclose(got[lo:hi].double()[fine], (x * torch.sigmoid(x) * y)[fine], atol=1e-3, rtol=1e-4)
     assert K.wait_errors() == {}
+
+
+@pytest.mark.parametrize("n_tok", [16, 32, 64, 128])
+@pytest.mark.parametrize("rows", [1, 17, 33])
+def test_tokens_past_the_rows_of_x_are_rows_of_zeros(K, monkeypatch, n_tok, rows):
+    """Fewer rows than tokens, and a row and a feature that send a tile to look for entries that are not the sum of three parts: the rows that
+    x does not have are not read (memory behind them holds what no number is)."""
+    monkeypatch.setattr(K, "f32_tc_tile", lambda *x: (n_tok, 64))
+    behind, w = torch.full((160, 192), float("nan"), device=DEV), rnd(70, 192, seed=34)
+    x = behind[:rows]
+    x.copy_(rnd(rows, 192, seed=35))
+    x[0, 5], w[66, 9] = 1e-40, 2.0 ** -126
+    out = torch.full((150, 70), 7.0, device=DEV)
+    K.gemm(x, w, out, rows=150)
+    want = x.double() @ w.double().t()
+    assert torch.allclose(out[:rows].double(), want, atol=1e-4, rtol=1e-5) and not bool(out[rows:].any())
+    offsets = torch.tensor([0, 40, 150], dtype=torch.int32, device=DEV)
+    K.gemm(x, torch.stack([w, w]), out, w_up=torch.stack([w, w]), group_offsets=offsets, rows=150)
+    assert torch.allclose(out[:rows].double(), want * torch.sigmoid(want) * want, atol=1e-3, rtol=1e-4) and not bool(out[rows:].any())
+    assert K.wait_errors() == {}
