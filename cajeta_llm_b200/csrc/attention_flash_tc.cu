@@ -303,7 +303,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int i = 0; i < n_tiles && ok; ++i) {
             const int key0 = (kt_begin + i) * BN;
             for (int c = 0; c < KC; ++c) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&k_empty[slot], phase, 11));
+                ok = mbar_wait_warp(&k_empty[slot], phase, 11);
                 if (!ok) break;
                 uint8_t* dst = smem + S::K_AT + slot * CHUNK;
                 if (leader) mbar_expect_tx(&k_full[slot], CHUNK);
@@ -330,7 +330,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         bool ok = true;
         int row = MAPS && lane < 4 ? plane_row(kt_begin * BN + 16 * lane) : 0;
         for (int i = 0; i < 2 * n_tiles && ok; ++i) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&v_empty[slot], phase, 19));
+            ok = mbar_wait_warp(&v_empty[slot], phase, 19);
             if (!ok) break;
             const int key0 = kt_begin * BN + i * 64;
             uint8_t* dst = smem + S::V_AT + slot * S::V_BYTES;
@@ -356,7 +356,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         // 64 keys.  S_g(i + 1) overwrites the columns PV_g(i) reads the weights from; one thread's products run in the order they
         // were issued.  The whole warp walks the loop (it clears what the values' tiles must not hold); one lane issues.
         const bool leader = elect_one();
-        bool ok = mbar_wait(q_full, 0, 12);
+        bool ok = mbar_wait_warp(q_full, 0, 12);
         int k_slot = 0;                           // where the next tile's chunks lie, and the phase of the first
         uint32_t k_phase = 0;
         int v_slot = 0;
@@ -371,7 +371,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 const int col = MAPS ? g * DK + 16 * k : 16 * k, c = col / 64, in = (col % 64) / 16;
                 const int slot = k_slot + c >= KS ? k_slot + c - KS : k_slot + c;
                 if ((k == 0 || in == 0) && there) {
-                    there = __all_sync(0xffffffffu, mbar_wait(&k_full[slot], k_phase ^ (k_slot + c >= KS ? 1u : 0u), 13));
+                    there = mbar_wait_warp(&k_full[slot], k_phase ^ (k_slot + c >= KS ? 1u : 0u), 13);
                     tcgen05_fence_after();
                 }
                 if (there && leader)
@@ -390,7 +390,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         };
         // 64 keys' values have landed, and what are no keys of the block reads as zero
         auto values_there = [&](int slot, uint32_t phase, int key0) {
-            if (!__all_sync(0xffffffffu, mbar_wait(&v_full[slot], phase, 14))) return false;
+            if (!mbar_wait_warp(&v_full[slot], phase, 14)) return false;
             if (key0 < key_from || key0 + 63 > p_last) {
                 uint8_t* v = smem + S::V_AT + slot * S::V_BYTES;
                 for (int i = lane; i < 64 * (DV / 64) * 8; i += 32) {       // 16 bytes each
@@ -402,7 +402,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
             return true;
         };
-        ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             tcgen05_fence_after();
 #pragma unroll
@@ -426,7 +425,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     there[half] = true;
                     if (!ok) break;
                     if (mine) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(&p_full[2 * g + half], p_phase[g], 15));
+                        ok = mbar_wait_warp(&p_full[2 * g + half], p_phase[g], 15);
                         if (!ok) break;
                         tcgen05_fence_after();
                         if (leader) {
@@ -470,7 +469,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         bool ok = true;
         const int n_mine = mine.end - mine.begin + 1;
         for (int j = 0; j < n_mine && ok; ++j) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&s_full[g], j & 1, 16));
+            ok = mbar_wait_warp(&s_full[g], j & 1, 16);
             if (!ok) break;
             tcgen05_fence_after();
             // columns [lo, lo + span] of this tile are keys this row may see (span < 0: none)
@@ -534,7 +533,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 // O may be rescaled once the product before is done: the one over the last tile's second half was done before this
                 // tile's scores were; the one over this tile's first half is waited for here
                 if (half == 1) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(&half_done[g], j & 1, 17));
+                    ok = mbar_wait_warp(&half_done[g], j & 1, 17);
                     if (!ok) break;
                     tcgen05_fence_after();
                 }
@@ -555,12 +554,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
         }
         // ---- the rows' results ---------------------------------------------------------------------------
-        if (ok && n_mine > 0) ok = __all_sync(0xffffffffu, mbar_wait(&o_done[g], 0, 18));
+        if (ok && n_mine > 0) ok = mbar_wait_warp(&o_done[g], 0, 18);
         if (MAPS) {
             // the second map's warps hand over what divides their rows; the first map's read both outputs from tensor memory
             if (g == 1) inv2[r] = ok && l > 0.0f ? 1.0f / l : 0.0f;
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (g == 0 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_done[1], 0, 18));
+            if (g == 0 && ok) ok = mbar_wait_warp(&o_done[1], 0, 18);
             if (g == 0 && ok) {
                 tcgen05_fence_after();
                 const float ia = l > 0.0f ? 1.0f / l : 0.0f, ib = inv2[r];

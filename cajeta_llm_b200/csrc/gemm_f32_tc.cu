@@ -188,6 +188,21 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// whether `ok` holds in all of the block's THREADS threads that come here, after all of them have
+template <int THREADS>
+__device__ __forceinline__ bool all_of(bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 5, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)ok), "n"(THREADS)
+        : "memory");
+    return r != 0;
+}
+
 // (x null: a row of zeros)
 __device__ __noinline__ float chain(const float* x, const float* w, int K) {
     float s = 0.0f;
@@ -260,7 +275,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], x_full[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int odd_flag[FLAGS];                           // some row of the tile has an entry that is not the sum of three parts
-    __shared__ int gave_up;                                   // a wait of an adding warp ran out: all of them leave together
     __shared__ int before[MAX_GROUPS + 1];                    // token tiles of the groups before one
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -279,7 +293,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             mbar_init(&acc_empty[s], EPI_WARPS);
         }
         for (int i = 0; i < FLAGS; ++i) odd_flag[i] = 0;
-        gave_up = 0;
         fence_barrier_init();
     }
     if (warp == ISSUE) tmem_alloc(&tmem_slot, S::TMEM_COLS);
@@ -391,7 +404,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             uint32_t odd = 0;
             for (; it < end; it += G) {
                 const unsigned rs = it % RING, s = it % STAGES;
-                ok = mbar_wait(&raw_full[rs], (it / RING) & 1, 16);
+                ok = mbar_wait_warp(&raw_full[rs], (it / RING) & 1, 16);
                 if (!ok) break;
                 const uint8_t* wr = raw + rs * S::RAW;
                 const uint8_t* xr = wr + S::W_RAW;
@@ -406,7 +419,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 };
                 // a lone group reads while the stage is still in use (1,777 x 6,144: 396 -> 375 us); several cover each other's
                 if (G == 1) read();
-                ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 11);
+                ok = mbar_wait_warp(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 11);
                 if (!ok) break;
                 tcgen05_fence_after();
                 if (G > 1) read();
@@ -454,7 +467,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const uint32_t one = umma_idesc_bf16(128, wide), both = umma_idesc_bf16(128, 2 * wide);
             const uint32_t at = b_first + ((s * S::STAGE + u * 3 * UNIT * 64) >> 4), x_step = (READY ? UNIT : wide) * 64 >> 4;
             const uint32_t w = tmem + S::A_AT + s * 48, d1 = acc0 + wide;
-            if (!mbar_wait(&acc_empty[mine], (times & 1) ^ 1, 14)) return false;
+            if (!mbar_wait_warp(&acc_empty[mine], (times & 1) ^ 1, 14)) return false;
             tcgen05_fence_after();
             auto add = [&](int pw, int px) {                 // D1 += part pw of W . part px of X
 #pragma unroll
@@ -485,7 +498,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const int wide = live ? width(c.n_tok, u) : 16;
             for (; it < end; it += UNITS == 2 ? 1 : 2) {
                 const unsigned s = it % STAGES;
-                ok = mbar_wait(&full_bar[s], (it / STAGES) & 1, 12) && (!READY || mbar_wait(&x_full[s], (it / STAGES) & 1, 18));
+                ok = mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, 12) && (!READY || mbar_wait_warp(&x_full[s], (it / STAGES) & 1, 18));
                 if (!ok) break;
                 if (live) {
                     ok = issue(wide, u, s, times);
@@ -514,7 +527,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 for (int u = 0; u < UNITS; ++u) {
                     if (u * UNIT >= n_tok || !ok) break;
                     const int a = UNITS == 2 ? u : it & 1, wide = width(n_tok, u);
-                    ok = mbar_wait(&acc_full[a], (UNITS == 2 ? times[u] : it >> 1) & 1, 13);
+                    ok = mbar_wait_warp(&acc_full[a], (UNITS == 2 ? times[u] : it >> 1) & 1, 13);
                     if (!ok) break;
                     ++times[u];
                     tcgen05_fence_after();
@@ -533,7 +546,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     }
                 }
             }
-            if (!ok) gave_up = 1;
             float acc[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; j += 2) {
@@ -613,10 +625,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     }
                 }
             }
-            // everyone has read the flag (and what crossed) before the next tile's
-            asm volatile("bar.sync 5, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+            // everyone has read the flag (and what crossed) before the next tile's; where a wait ran out, all of these warps leave together
+            ok = all_of<EPI_WARPS * 32>(ok);
             if (warp == FIRST_EPI && lane == 0) odd_flag[nth % FLAGS] = 0;
-            ok = gave_up == 0;
         }
     }
     tcgen05_fence_before();

@@ -351,7 +351,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             TileCoord c = decode_tile<TOK_TILE>(p, tile, feat_tiles, tok_tiles, tiles_before, feat_tile);
             if (!c.valid) continue;
             const int as = acc_it % ACC_STAGES;
-            ok = mbar_wait(&acc_full[as], (acc_it / ACC_STAGES) & 1, 3);
+            ok = mbar_wait_warp(&acc_full[as], (acc_it / ACC_STAGES) & 1, 3);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t lane_base = tmem_base + as * STAGE_COLS + ((uint32_t)(quarter * 32) << 16);

@@ -73,6 +73,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
     return mbar_wait_slow(bar, parity, code);
 }
 
+// The same by a whole warp that goes on to instructions all of its lanes must take (tcgen05.ld and .st, __syncwarp): one answer
+// for all lanes.  Lane by lane, a limit that runs out while the phase completes would send some of them on and some to the exit, and
+// both would wait there for each other without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, code));
+}
+
 // TMA: one 2-D tile [box rows x box cols] into shared memory, completion counted in bytes
 // on an mbarrier.  c0 is the innermost (contiguous) coordinate; c0 * element size must be
 // a multiple of 16 bytes.  No cluster multicast is used anywhere.
