@@ -980,8 +980,10 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
         _need(skip, "skip", torch.float32)
     if state[0].numel() < state_offset + state_scan_floats(heads, rows, cols, mode) or out.shape[1] != heads * cols:
         raise KernelError("state_scan: state or out too small")
-    # (the decays of a prompt's rows, worked out once for all of the scan's blocks)
-    decays = torch.empty((x.shape[0], heads * rows), dtype=torch.float32, device=x.device) if mode == SCAN_GLA and x.shape[0] >= 8 * requests else None
+    # the decays of a prompt's rows, worked out once for all of the scan's blocks; of all rows of x, so not where raw ends with the requests'
+    decays = None
+    if mode == SCAN_GLA and x.shape[0] >= 8 * requests and raw.shape[0] >= x.shape[0]:
+        decays = torch.empty((x.shape[0], heads * rows), dtype=torch.float32, device=x.device)
     st = library("recurrent").cj_state_scan(
         _i(mode), _ptr(x), _i(x.stride(0)), _i(off_a), _i(off_b), _i(off_v), _ptr(raw), _i(raw.stride(0)), _i(off_dt), _i(off_beta),
         _ptr(A_log), _ptr(dt_bias), _ptr(skip), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), _ll(state.stride(0)),

@@ -43,3 +43,19 @@ def test_walked_and_single_tokens_agree(mode, heads, groups, rows, cols, lengths
             outs.append(out)
         assert bool(outs[0].abs().sum() > 0) and bool(states[0][slots.long()].abs().sum(1).min() > 0)
         assert torch.equal(outs[0], outs[1]) and torch.equal(states[0], states[1])
+
+
+def test_raw_rows_that_end_with_the_requests():
+    """x may have rows behind the requests' (of another step's length, say) that raw has not: the same bits."""
+    from cajeta_llm_b200.csrc import kernels as K
+    heads, rows, cols, T, more = 4, 128, 64, 40, 24
+    g = torch.Generator().manual_seed(12)
+    x, raw = torch.randn(T + more, heads * (2 * rows + cols), generator=g).to(DEV), torch.randn(T, heads * rows, generator=g).to(DEV)
+    start, slot = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for n in (T, T + more):
+        state, out = torch.zeros(1, K.state_scan_floats(heads, rows, cols, K.SCAN_GLA), device=DEV), torch.zeros(n, heads * cols, device=DEV)
+        K.state_scan(K.SCAN_GLA, x[:n], 0, heads * rows, 2 * heads * rows, raw, 0, 0, None, None, None, state, 0, start, slot, out, 1, heads, heads,
+                     rows, cols, q_scale=0.125, c0=0.25)
+        outs.append((out[:T], state))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])

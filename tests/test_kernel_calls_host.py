@@ -1,0 +1,47 @@
+"""What the kernels' Python face hands to the libraries, on the CPU: the libraries are stood in for, nothing is launched."""
+import ctypes
+
+import pytest
+import torch
+
+from cajeta_llm_b200.csrc import kernels as K
+
+
+class Calls:
+    """A library whose every function takes its arguments down and succeeds; ``answers``: what a function returns instead of 0."""
+
+    def __init__(self, **answers):
+        self.answers, self.made = answers, []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.made.append((name, [a.value if isinstance(a, ctypes._SimpleCData) else a for a in args]))
+            return self.answers.get(name, 0)
+        return call
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    lib = Calls()
+    monkeypatch.setattr(K, "library", lambda name: lib)
+    monkeypatch.setattr(K, "_need", lambda *a: None)
+    monkeypatch.setattr(K, "_stream", lambda: ctypes.c_void_p(0))
+    monkeypatch.setattr(K, "_sm_count", lambda: 148)
+    return lib
+
+
+def scan(mode, tokens, raw_rows, requests, **kw):
+    heads, rows, cols = 4, 128, 256
+    x, raw = torch.zeros(tokens, heads * (2 * rows + cols)), torch.zeros(raw_rows, heads * rows)
+    K.state_scan(mode, x, 0, heads * rows, 2 * heads * rows, raw, 0, heads, *[torch.zeros(heads)] * 3, torch.zeros(2, K.state_scan_floats(heads, rows, cols, mode)),
+                 0, torch.zeros(requests + 1, dtype=torch.int32), torch.zeros(requests, dtype=torch.int32), torch.zeros(tokens, heads * cols), requests, heads,
+                 heads, rows, cols, c0=0.25, **kw)
+
+
+def test_decays_of_all_rows_only_where_all_rows_have_them(calls):
+    """Gated linear attention works the decays of all of x's rows out ahead; the scan alone needs those of the requests' rows."""
+    scan(K.SCAN_GLA, 64, 64, 1)
+    scan(K.SCAN_GLA, 64, 40, 1)
+    scan(K.SCAN_DELTA, 64, 64, 1)
+    pointers = [args[-2] for name, args in calls.made if name == "cj_state_scan"]
+    assert pointers[0] and not pointers[1] and not pointers[2]
