@@ -753,11 +753,11 @@ CJ_EXPORT long long cj_gemm_f32_tc_scratch(int tokens, int K, int n_tok, int ind
 // index that names no row of X for zeros; without it row s is row s, and those from x_rows on are zeros.  W (and W2) [groups, features, K]
 // contiguous float32; the
 // other arguments as cj_gemm_simt's.  n_tok: tokens of a tile (16, 32, 64 or 128); feat_tile: its features (32, 64 or 128; with W2 at most 64).
-// scratch: cj_gemm_f32_tc_scratch bytes, 16-byte aligned.
-CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const int* x_index, void* scratch, const float* W, const float* W2,
-                             const float* bias, const float* bias2, float* C, long long ldc, int tokens, int features, int K, int accumulate,
-                             const int* group_offsets, int groups, float act_limit, float act_alpha, float act_cubic, int act, int act_feats,
-                             float out_scale, int n_tok, int feat_tile, cudaStream_t stream) {
+// scratch: scratch_bytes of memory, 16-byte aligned, at least what cj_gemm_f32_tc_scratch says.
+CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const int* x_index, void* scratch, long long scratch_bytes, const float* W,
+                             const float* W2, const float* bias, const float* bias2, float* C, long long ldc, int tokens, int features, int K,
+                             int accumulate, const int* group_offsets, int groups, float act_limit, float act_alpha, float act_cubic, int act,
+                             int act_feats, float out_scale, int n_tok, int feat_tile, cudaStream_t stream) {
     if (tokens <= 0 || features <= 0) return 0;
     if (!X || !W || !C || K <= 0 || x_rows <= 0) return CJ_ERR_ARG;
     if (group_offsets && groups <= 0) return CJ_ERR_ARG;
@@ -768,7 +768,8 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const in
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2 | (uintptr_t)scratch) & 15) return CJ_ERR_ALIGN;
     const int tok_tiles = (tokens + n_tok - 1) / n_tok + (group_offsets ? groups : 0);
     if (group_offsets && groups > MAX_GROUPS) return CJ_ERR_SIZE;
-    if (cj_gemm_f32_tc_scratch(tokens, K, n_tok, x_index != nullptr) > 0 && !scratch) return CJ_ERR_ARG;
+    const long long room = cj_gemm_f32_tc_scratch(tokens, K, n_tok, x_index != nullptr);
+    if (room > 0 && (!scratch || scratch_bytes < room)) return CJ_ERR_ARG;
     const int* x_odd = nullptr;
     if (n_tok >= 64) {
         const int Kp = (K + BK - 1) / BK * BK;

@@ -300,6 +300,14 @@ def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
     return min(((n, f) for n in F32_TC_TOKENS for f in (most, most // 2)), key=lambda t: cost(*t))
 
 
+@functools.lru_cache(maxsize=4096)
+def _f32_tc_scratch(rows: int, K: int, n_tok: int, indexed: bool) -> int:
+    """Bytes of scratch that the float32 tensor-core product wants, as its library says."""
+    size = library("gemm_f32_tc").cj_gemm_f32_tc_scratch
+    size.restype = ctypes.c_longlong
+    return int(size(_i(rows), _i(K), _i(n_tok), _i(1 if indexed else 0)))
+
+
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
          accumulate: bool = False, w_up: Optional[torch.Tensor] = None, group_offsets: Optional[torch.Tensor] = None,
          a_row_index: Optional[torch.Tensor] = None, rows: Optional[int] = None, act_limit: float = 0.0,
@@ -343,11 +351,11 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
         # X in its three parts, split once for all tiles, or the groups' rows side by side (a row outside the groups has no index to
         # follow, an index below 0 names a row of zeros)
         lib, indexed = library("gemm_f32_tc"), a_row_index is not None
-        room = M * (6 * (-(-K // 32) * 32) + 4) if n_tok >= 64 else 4 * M * K if indexed else 0
+        room = _f32_tc_scratch(M, K, n_tok, indexed)
         scratch = torch.empty((room,), dtype=torch.uint8, device=a.device) if room else None
         st = lib.cj_gemm_f32_tc(
-            _ptr(a), _ll(a.stride(0)), _i(a.shape[0] if indexed else min(M, a.shape[0])), _ptr(a_row_index), _ptr(scratch), _ptr(w), _ptr(w_up),
-            _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
+            _ptr(a), _ll(a.stride(0)), _i(a.shape[0] if indexed else min(M, a.shape[0])), _ptr(a_row_index), _ptr(scratch), _ll(room), _ptr(w),
+            _ptr(w_up), _ptr(bias), _ptr(bias_up), _ptr(out), _ll(out.stride(0)), _i(M), _i(N), _i(K),
             _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
             _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
         _check(st, "gemm")

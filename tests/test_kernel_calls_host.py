@@ -45,3 +45,20 @@ def test_decays_of_all_rows_only_where_all_rows_have_them(calls):
     scan(K.SCAN_DELTA, 64, 64, 1)
     pointers = [args[-2] for name, args in calls.made if name == "cj_state_scan"]
     assert pointers[0] and not pointers[1] and not pointers[2]
+
+
+@pytest.mark.parametrize("n_tok,indexed", [(16, False), (32, True), (64, False), (128, True)])
+def test_a_float32_product_refuses_scratch_that_is_too_small(n_tok, indexed):
+    """The library's own entry (its host side launches nothing before the check): a byte short, and no scratch at all."""
+    lib, one = K.library("gemm_f32_tc"), ctypes.c_void_p(1 << 20)
+    need = K._f32_tc_scratch(100, 260, n_tok, indexed)
+    assert need == (100 * (6 * 288 + 4) if n_tok >= 64 else 100 * 260 * 4 if indexed else 0)
+
+    def call(scratch, size):
+        null = ctypes.c_void_p(0)
+        return lib.cj_gemm_f32_tc(one, K._ll(260), K._i(100), one if indexed else null, scratch, K._ll(size), one, null, null, null, one, K._ll(64), K._i(100),
+                                  K._i(64), K._i(260), K._i(0), null, K._i(0), K._f(0), K._f(1), K._f(0), K._i(0), K._i(0), K._f(1), K._i(n_tok), K._i(64),
+                                  null)
+
+    if need:
+        assert call(one, need - 1) == -5 and call(ctypes.c_void_p(0), need) == -5
