@@ -74,9 +74,11 @@ struct Args {
     int act, act_feats;
     float out_scale;
     int feat_tile;                         // features of a tile: at most 128, of the gated form at most 64
+    int span, spans;                       // groups a place of the table, and its places
 };
 
-constexpr int MAX_GROUPS = 1024;           // groups of a launch: the places of their tiles are a table in shared memory
+constexpr int SPANS = 1024;                // places of the table in shared memory that says where groups' tiles begin: of every group up to 1,024,
+                                           // of every n-th beyond
 
 template <int N, bool DUAL> struct Smem {
     static constexpr int STAGE = 3 * N * 64;                           // the bfloat16 parts of X (those of W lie in tensor memory)
@@ -232,20 +234,25 @@ struct Tile {
     int group, tok0, n_tok, feat0;
 };
 template <int N>
+__device__ __forceinline__ int group_tiles(const Args& p, int g) { return (p.group_offsets[g + 1] - p.group_offsets[g] + N - 1) / N; }
+template <int N>
 __device__ __forceinline__ Tile locate(const Args& p, int t, int feat_tiles, const int* before) {
     const int tt = t / feat_tiles;
     Tile c;
     c.feat0 = (t - tt * feat_tiles) * p.feat_tile;
     c.group = 0;
     if (p.group_offsets) {
-        int lo = 0, hi = p.groups;                            // before[lo] <= tt < before[hi]
+        int lo = 0, hi = p.spans;                             // before[lo] <= tt < before[hi]
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (before[mid] <= tt) lo = mid; else hi = mid;
         }
-        c.group = lo;
-        c.tok0 = p.group_offsets[lo] + (tt - before[lo]) * N;
-        c.n_tok = min(p.group_offsets[lo + 1] - c.tok0, N);
+        int first = before[lo];
+        c.group = lo * p.span;
+        if (p.span > 1)                                       // (tt lies before the span's end, so some group of it holds it)
+            for (int n; tt >= first + (n = group_tiles<N>(p, c.group)); ++c.group) first += n;
+        c.tok0 = p.group_offsets[c.group] + (tt - first) * N;
+        c.n_tok = min(p.group_offsets[c.group + 1] - c.tok0, N);
     } else {
         c.tok0 = tt * N;
         c.n_tok = min(p.tokens - c.tok0, N);
@@ -275,7 +282,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], x_full[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int odd_flag[FLAGS];                           // some row of the tile has an entry that is not the sum of three parts
-    __shared__ int before[MAX_GROUPS + 1];                    // token tiles of the groups before one
+    __shared__ int before[SPANS + 1];                         // token tiles of the groups before a span's first
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
@@ -302,17 +309,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         int carry = 0;
         for (int g0 = 0; g0 < p.groups; g0 += 32) {
             const int g = g0 + lane;
-            const int n = g < p.groups ? (p.group_offsets[g + 1] - p.group_offsets[g] + N - 1) / N : 0;
+            const int n = g < p.groups ? group_tiles<N>(p, g) : 0;
             int inc = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int v = __shfl_up_sync(0xffffffffu, inc, o);
                 if (lane >= o) inc += v;
             }
-            if (g < p.groups) before[g] = carry + inc - n;
+            if (g < p.groups && g % p.span == 0) before[g / p.span] = carry + inc - n;
             carry += __shfl_sync(0xffffffffu, inc, 31);
         }
-        if (lane == 0) before[p.groups] = carry;
+        if (lane == 0) before[p.spans] = carry;
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -320,7 +327,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     cj::release_successor();                                  // tensor memory is held
     const uint32_t tmem = tmem_slot;
     const int feat_tiles = (p.features + p.feat_tile - 1) / p.feat_tile;
-    const int n_tiles = (grouped ? before[p.groups] : (p.tokens + N - 1) / N) * feat_tiles;
+    const int n_tiles = (grouped ? before[p.spans] : (p.tokens + N - 1) / N) * feat_tiles;
     const unsigned n_kb = (p.K + BK - 1) / BK;
     // the width of a unit's products; the parts of its X lie that many rows apart, side by side (those that came in parts UNIT rows)
     auto width = [](int n_tok, int u) { return (min(n_tok - u * UNIT, UNIT) + 15) & ~15; };
@@ -767,7 +774,6 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const in
     if (K % 4 != 0 || ldx % 4 != 0 || ldx < K) return CJ_ERR_ALIGN;               // TMA: strides of 16 bytes
     if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)W2 | (uintptr_t)scratch) & 15) return CJ_ERR_ALIGN;
     const int tok_tiles = (tokens + n_tok - 1) / n_tok + (group_offsets ? groups : 0);
-    if (group_offsets && groups > MAX_GROUPS) return CJ_ERR_SIZE;
     const long long room = cj_gemm_f32_tc_scratch(tokens, K, n_tok, x_index != nullptr);
     if (room > 0 && (!scratch || scratch_bytes < room)) return CJ_ERR_ARG;
     const int* x_odd = nullptr;
@@ -787,7 +793,11 @@ CJ_EXPORT int cj_gemm_f32_tc(const float* X, long long ldx, int x_rows, const in
     }
     if (int st = cj::launch_status()) return st;
     Args a{X, ldx, x_index, x_odd, W, W2, bias, bias2, C, ldc, tokens, features, K, x_rows, accumulate, group_offsets, groups, act_limit, act_alpha, act_cubic, act,
-           act_feats > 0 ? act_feats : features, out_scale, feat_tile};
+           act_feats > 0 ? act_feats : features, out_scale, feat_tile, 1, 0};
+    if (group_offsets) {
+        a.span = (groups + SPANS - 1) / SPANS;
+        a.spans = (groups + a.span - 1) / a.span;
+    }
 #define CASE(N) case N: return W2 ? launch<N, true>(a, scratch, tok_tiles, stream) : launch<N, false>(a, scratch, tok_tiles, stream);
     switch (n_tok) {
         CASE(16) CASE(32) CASE(64) CASE(128)

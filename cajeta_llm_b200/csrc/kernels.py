@@ -267,7 +267,6 @@ def _gate_biases(w: torch.Tensor, w_up: Optional[torch.Tensor], bias: Optional[t
 
 
 F32_TC_TOKENS = (16, 32, 64, 128)      # token tiles of the float32 tensor-core product
-F32_TC_GROUPS = 1024                   # groups whose places a block of it holds
 
 
 def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor], out: torch.Tensor) -> bool:
@@ -276,7 +275,6 @@ def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor],
     number of rows is no part of it: a row's bits must not depend on the others."""
     N, K = w.shape[-2], w.shape[-1]
     return (a.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and K >= 128 and N >= 64 and K % 4 == 0
-            and (w.dim() < 3 or w.shape[0] <= F32_TC_GROUPS)
             and a.stride(0) % 4 == 0 and a.stride(0) >= K and (a.data_ptr() | w.data_ptr() | (w_up.data_ptr() if w_up is not None else 0)) % 16 == 0)
 
 

@@ -267,3 +267,27 @@ def test_tokens_past_the_rows_of_x_are_rows_of_zeros(K, monkeypatch, n_tok, rows
     K.gemm(x, torch.stack([w, w]), out, w_up=torch.stack([w, w]), group_offsets=offsets, rows=150)
     assert torch.allclose(out[:rows].double(), want * torch.sigmoid(want) * want, atol=1e-3, rtol=1e-4) and not bool(out[rows:].any())
     assert K.wait_errors() == {}
+
+
+@pytest.mark.parametrize("groups", [1023, 1024, 1025, 2500])
+def test_any_number_of_groups(K, monkeypatch, groups):
+    """More groups than a block holds places for, empty ones at both ends and in runs, one with several tiles: the bits of the groups alone."""
+    H, N = 128, 64
+    g = torch.Generator().manual_seed(36)
+    sizes = torch.randint(0, 3, (groups,), generator=g)
+    sizes[:5], sizes[-40:], sizes[groups // 2:groups // 2 + 70] = 0, 0, 0
+    sizes[7], sizes[groups - 41] = 150, 33
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), sizes.cumsum(0)])
+    T = int(offsets[-1])
+    x, w = rnd(T, H, seed=37), rnd(groups, N, H, seed=38)
+    want = torch.empty(T, N, device=DEV)
+    for e in range(groups):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        if hi > lo:
+            K.gemm(x[lo:hi], w[e], want[lo:hi])
+    for n_tok in (16, 64):
+        monkeypatch.setattr(K, "f32_tc_tile", lambda *a: (n_tok, 64))
+        out = torch.empty(T, N, device=DEV)
+        K.gemm(x, w, out, group_offsets=offsets.int().to(DEV))
+        assert torch.equal(out, want)
+    assert K.wait_errors() == {}
