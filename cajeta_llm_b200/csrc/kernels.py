@@ -85,7 +85,7 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-launches = 0      # kernels launched through this module since import (each wrapper launches one)
+launches = 0      # kernels launched through this module since import (each wrapper launches one, unless it adds the others)
 # Measurement: parts name the class of work their next launches belong to (``tag``: "qkv", "expert
 # gate/up", ...; costs an assignment); while a trace is open every launch is followed by an event
 # on the stream, so that the time between two events is one launch's device time with the launches
@@ -357,6 +357,9 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[tor
             _i(1 if accumulate else 0), _ptr(group_offsets), _i(G), _f(act_limit), _f(act_alpha), _f(act_cubic),
             _i(ACTS[act]), _i(act_features), _f(out_scale), _i(n_tok), _i(feat_tile), _stream())
         _check(st, "gemm")
+        if room:
+            global launches
+            launches += 1              # rows are split, or gathered, by a kernel of their own
         return
     st = library("gemm_simt").cj_gemm_simt(
         _ptr(a), _ll(a.stride(0)), _i(_code(a)), _ptr(w), _ptr(w_up), _ll(K), _i(_code(w)), _ptr(bias), _ptr(bias_up),
@@ -958,6 +961,12 @@ def state_scan_floats(heads: int, rows: int, cols: int, mode: int = SCAN_SSD) ->
     return heads * -(-cols // cols_per_block) * tile
 
 
+@functools.lru_cache(maxsize=4096)
+def _scan_walks(mode: int, heads: int, rows: int, cols: int, requests: int, total_rows: int, state_floats: int) -> bool:
+    """Whether a step's scan walks several tokens at a time, as its library says."""
+    return bool(library("recurrent").cj_state_scan_walks(_i(mode), _i(heads), _i(rows), _i(cols), _i(requests), _i(total_rows), _ll(state_floats)))
+
+
 def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, raw: torch.Tensor, off_dt: int, off_beta: int,
                A_log: Optional[torch.Tensor], dt_bias: Optional[torch.Tensor], skip: Optional[torch.Tensor], state: torch.Tensor,
                state_offset: int, req_start: torch.Tensor, req_slot: torch.Tensor, out: torch.Tensor, requests: int, heads: int,
@@ -988,7 +997,8 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
         raise KernelError("state_scan: state or out too small")
     # the decays of a prompt's rows, worked out once for all of the scan's blocks; of all rows of x, so not where raw ends with the requests'
     decays = None
-    if mode == SCAN_GLA and x.shape[0] >= 8 * requests and raw.shape[0] >= x.shape[0]:
+    if (mode == SCAN_GLA and raw.shape[0] >= x.shape[0]
+            and _scan_walks(mode, heads, rows, cols, requests, x.shape[0], state[0].numel() - state_offset)):
         decays = torch.empty((x.shape[0], heads * rows), dtype=torch.float32, device=x.device)
     st = library("recurrent").cj_state_scan(
         _i(mode), _ptr(x), _i(x.stride(0)), _i(off_a), _i(off_b), _i(off_v), _ptr(raw), _i(raw.stride(0)), _i(off_dt), _i(off_beta),
@@ -996,6 +1006,9 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
         _ll(state[0].numel() - state_offset), _ptr(req_start), _ptr(req_slot), _ptr(out), _i(requests),
         _i(x.shape[0]), _i(heads), _i(groups), _i(rows), _i(cols), _f(q_scale), _f(c0), _f(c1), _ptr(decays), _stream())
     _check(st, "state_scan")
+    if decays is not None:
+        global launches
+        launches += 1                  # the decays are a kernel of their own
 
 
 def gated_scan(x: torch.Tensor, off_z: int, off_x: int, off_g: int, width: int, state: torch.Tensor, state_offset: int,

@@ -1532,6 +1532,17 @@ static int launch_walk(int mode, int DP, int nper, const ScanArgs& p, int reques
     return CJ_ERR_SIZE;
 }
 
+// Whether cj_state_scan takes the kernel that walks several columns and tokens at a time (in mode 2 with a kernel ahead of it that works out the
+// decays, where it is given room for them).
+CJ_EXPORT int cj_state_scan_walks(int mode, int heads, int rows, int cols, int requests, int total_rows, long long state_floats) {
+    if (heads <= 0 || rows <= 0 || cols <= 0 || requests <= 0 || heads > 65535 || total_rows < (long long)WALK_MIN_ROWS * requests) return 0;
+    const int DP = scan_lanes(heads, rows, cols), per = (rows + DP - 1) / DP, cols_per_block = 4 * (32 / DP);
+    int nper = 1;
+    while (nper < per) nper <<= 1;
+    const int tiles = (cols + cols_per_block - 1) / cols_per_block;
+    return rows == DP * nper && walk_built(DP, nper) && state_floats >= (long long)heads * tiles * scan_tile_floats(mode, nper);
+}
+
 CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off_b, int off_v, const float* raw, int ld_raw,
                             int off_dt, int off_beta, const float* A_log, const float* dt_bias, const float* skip, float* state,
                             long long slot_stride, long long state_floats, const int* req_start, const int* req_slot, float* out,
@@ -1553,11 +1564,10 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
                req_start, req_slot, out, heads, groups, rows, cols, q_scale, 0, c0, c1};
     const int cols_per_block = 4 * (32 / DP);
     dim3 grid(requests, heads, (cols + cols_per_block - 1) / cols_per_block);
-    if (total_rows >= WALK_MIN_ROWS * requests && rows == DP * nper && grid.y <= 65535
-        && state_floats >= (long long)heads * grid.z * scan_tile_floats(mode, nper)) {
+    if (cj_state_scan_walks(mode, heads, rows, cols, requests, total_rows, state_floats)) {
         // many tokens a request: the same results from the kernel that walks several columns and tokens at a time, where it is built
         ScanArgs w = p;
-        if (mode == SCAN_GLA && decays && walk_built(DP, nper)) {
+        if (mode == SCAN_GLA && decays) {
             const long long n = (long long)total_rows * heads * rows;
             cj::launch(gla_decays_kernel, dim3((unsigned)min((n + 255) / 256, (long long)148 * 16)), dim3(256), 0, stream, raw, ld_raw, off_dt,
                        heads * rows, n, c0, decays);

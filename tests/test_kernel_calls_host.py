@@ -16,7 +16,8 @@ class Calls:
     def __getattr__(self, name):
         def call(*args):
             self.made.append((name, [a.value if isinstance(a, ctypes._SimpleCData) else a for a in args]))
-            return self.answers.get(name, 0)
+            answer = self.answers.get(name, 0)
+            return answer(args) if callable(answer) else answer
         return call
 
 
@@ -27,6 +28,11 @@ def calls(monkeypatch):
     monkeypatch.setattr(K, "_need", lambda *a: None)
     monkeypatch.setattr(K, "_stream", lambda: ctypes.c_void_p(0))
     monkeypatch.setattr(K, "_sm_count", lambda: 148)
+    real = K._libs.get("recurrent") or ctypes.CDLL(K._build.build("recurrent"))
+    lib.answers["cj_state_scan_walks"] = lambda args: real.cj_state_scan_walks(*args)
+    scratch = ctypes.CDLL(K._build.build("gemm_f32_tc")).cj_gemm_f32_tc_scratch
+    scratch.restype = ctypes.c_longlong
+    lib.answers["cj_gemm_f32_tc_scratch"] = lambda args: scratch(*args)
     return lib
 
 
@@ -43,8 +49,26 @@ def test_decays_of_all_rows_only_where_all_rows_have_them(calls):
     scan(K.SCAN_GLA, 64, 64, 1)
     scan(K.SCAN_GLA, 64, 40, 1)
     scan(K.SCAN_DELTA, 64, 64, 1)
+    scan(K.SCAN_GLA, 64, 64, 9)                                               # (seven rows a request: too few to walk)
     pointers = [args[-2] for name, args in calls.made if name == "cj_state_scan"]
-    assert pointers[0] and not pointers[1] and not pointers[2]
+    assert pointers[0] and not any(pointers[1:])
+
+
+def counted(call, *args, **kw):
+    before = K.launches
+    call(*args, **kw)
+    return K.launches - before
+
+
+def test_every_kernel_of_a_call_is_counted(calls, monkeypatch):
+    """A product that splits or gathers its rows first, and a scan whose decays are worked out first, are two kernels."""
+    x, w, out = torch.zeros(300, 256), torch.zeros(3, 128, 256), torch.zeros(300, 128)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+    offsets, index = torch.tensor([0, 100, 200, 300], dtype=torch.int32), torch.arange(300, dtype=torch.int32)
+    for n_tok, many, index_given, kernels in ((16, False, None, 1), (16, True, None, 1), (32, True, index, 2), (64, False, None, 2), (128, True, index, 2)):
+        monkeypatch.setattr(K, "f32_tc_tile", lambda *a: (n_tok, 64))
+        assert counted(K.gemm, x, w if many else w[0], out, group_offsets=offsets if many else None, a_row_index=index_given) == kernels
+    assert counted(scan, K.SCAN_GLA, 64, 64, 1) == 2 and counted(scan, K.SCAN_GLA, 64, 40, 1) == 1 and counted(scan, K.SCAN_SSD, 64, 64, 1) == 1
 
 
 @pytest.mark.parametrize("n_tok,indexed", [(16, False), (32, True), (64, False), (128, True)])
