@@ -970,7 +970,8 @@ def _scan_walks(mode: int, heads: int, rows: int, cols: int, requests: int, tota
 def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, raw: torch.Tensor, off_dt: int, off_beta: int,
                A_log: Optional[torch.Tensor], dt_bias: Optional[torch.Tensor], skip: Optional[torch.Tensor], state: torch.Tensor,
                state_offset: int, req_start: torch.Tensor, req_slot: torch.Tensor, out: torch.Tensor, requests: int, heads: int,
-               groups: int, rows: int, cols: int, q_scale: float = 1.0, c0: float = 0.0, c1: float = 0.0) -> None:
+               groups: int, rows: int, cols: int, q_scale: float = 1.0, c0: float = 0.0, c1: float = 0.0,
+               single: Optional[bool] = None) -> None:
     """Walks every request's rows of the step in order through its recurrent state
     (``state[slot, state_offset:]``, ``state_scan_floats(heads, rows, cols)`` float32 entries in the
     scan's own layout; zero = the empty state) and writes a row's
@@ -986,7 +987,9 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
     ``SCAN_MLSTM``: off_a = q (times ``q_scale``), off_b = k, off_v = v; raw columns off_dt + h and off_beta + h = the
     input and forget gates before their bias (``dt_bias`` = the input gate's, ``A_log`` = the forget gate's);
     i = c0 tanh((. + b) / c0), f = log sigmoid(c0 tanh((. + b) / c0)); m_t = max(f + m, i), m_0 = 0;
-    S = e^(f + m - m_t) S + e^(i - m_t) k v^T, n likewise with k alone; o = S^T q / (max(|n . q|, e^(-m_t)) + c1)."""
+    S = e^(f + m - m_t) S + e^(i - m_t) k v^T, n likewise with k alone; o = S^T q / (max(|n . q|, e^(-m_t)) + c1).
+
+    ``single``: every request of the step brings one token (None: when there are no more rows than requests)."""
     _need(x, "x", torch.float32), _need(raw, "raw", torch.float32), _need(state, "state", torch.float32), _need(out, "out", torch.float32)
     if mode != SCAN_GLA:
         _need(A_log, "A_log", torch.float32), _need(dt_bias, "dt_bias", torch.float32)
@@ -1004,7 +1007,8 @@ def state_scan(mode: int, x: torch.Tensor, off_a: int, off_b: int, off_v: int, r
         _i(mode), _ptr(x), _i(x.stride(0)), _i(off_a), _i(off_b), _i(off_v), _ptr(raw), _i(raw.stride(0)), _i(off_dt), _i(off_beta),
         _ptr(A_log), _ptr(dt_bias), _ptr(skip), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), _ll(state.stride(0)),
         _ll(state[0].numel() - state_offset), _ptr(req_start), _ptr(req_slot), _ptr(out), _i(requests),
-        _i(x.shape[0]), _i(heads), _i(groups), _i(rows), _i(cols), _f(q_scale), _f(c0), _f(c1), _ptr(decays), _stream())
+        _i(x.shape[0]), _i(heads), _i(groups), _i(rows), _i(cols), _f(q_scale), _f(c0), _f(c1), _ptr(decays),
+        _i(1 if (x.shape[0] <= requests if single is None else single) else 0), _stream())
     _check(st, "state_scan")
     if decays is not None:
         global launches

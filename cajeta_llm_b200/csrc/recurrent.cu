@@ -1547,7 +1547,7 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
                             int off_dt, int off_beta, const float* A_log, const float* dt_bias, const float* skip, float* state,
                             long long slot_stride, long long state_floats, const int* req_start, const int* req_slot, float* out,
                             int requests, int total_rows, int heads, int groups, int rows, int cols, float q_scale, float c0, float c1,
-                            float* decays, cudaStream_t stream) {
+                            float* decays, int single, cudaStream_t stream) {
     if (requests <= 0) return 0;
     if (mode < 0 || mode > 3) return CJ_ERR_ARG;
     if (!x || !raw || !state || !req_start || !req_slot || !out) return CJ_ERR_ARG;
@@ -1585,8 +1585,9 @@ CJ_EXPORT int cj_state_scan(int mode, const float* x, int ld, int off_a, int off
     const size_t token_bytes = (size_t)((mode == 2 ? 3 : 2) * DP * nper + cols_per_block + 4) * sizeof(float);
     int TOK = (int)((96 * 1024) / (2 * token_bytes));
     if (TOK > 16) TOK = 16;
-    // single tokens: seven blocks an SM instead of six (8 requests, state-space and delta rule, cold: 13.0 and 13.6 us -> 11.2 and 11.4)
-    if (TOK > 1 && total_rows <= requests) TOK = 1;
+    // single tokens: seven blocks an SM instead of six (8 requests, state-space and delta rule, cold: 13.0 and 13.6 us -> 11.2 and 11.4).  Said by
+    // the caller: fewer rows than requests may also be a few of them with many, in a layout filled up with requests that bring none
+    if (TOK > 1 && single) TOK = 1;
     if (TOK < 1) return CJ_ERR_SIZE;
     const size_t smem = 2 * (size_t)TOK * token_bytes;
 #define LAUNCH_MODE(N, M)                                                                                               \

@@ -170,7 +170,7 @@ class StateSpaceMixer(_StateMixer):
         K.tag = "scan"
         K.state_scan(K.SCAN_SSD, conv, self.inner, self.inner + gn, 0, proj, 2 * self.inner + 2 * gn, 0, self.A_log, self.dt_bias,
                      self.D, entry.state, getattr(entry, "state_offset", 0) + self.conv_state, ctx.req_start, ctx.req_slot, y, ctx.n_requests, self.heads,
-                     self.groups, self.n_state, self.vdim)
+                     self.groups, self.n_state, self.vdim, single=getattr(ctx, "all_single", False))
         gated = torch.empty((T, self.inner), dtype=rt.act_dtype, device=x.device)
         K.tag = "gate + norm"
         K.gated_group_norm(y, self.inner // self.norm_groups, proj, 0, self.w_norm, self.eps, True, gated)
@@ -239,7 +239,7 @@ class GatedDeltaMixer(_StateMixer):
         K.tag = "scan"
         K.state_scan(K.SCAN_DELTA, conv, 0, self.qk, 2 * self.qk, proj, C, C + self.heads, self.A_log, self.dt_bias, None,
                      entry.state, getattr(entry, "state_offset", 0) + self.conv_state, ctx.req_start, ctx.req_slot, o, ctx.n_requests, self.heads, self.kv_heads,
-                     self.dim, self.vdim, q_scale=float(self.dim) ** -0.5)
+                     self.dim, self.vdim, q_scale=float(self.dim) ** -0.5, single=getattr(ctx, "all_single", False))
         gated = torch.empty((T, self.v), dtype=rt.act_dtype, device=x.device)
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, C + 2 * self.heads, self.w_norm, self.eps, False, gated)
@@ -304,7 +304,7 @@ class GatedLinearAttention(_StateMixer):
         K.tag = "scan"
         K.state_scan(K.SCAN_GLA, proj, 0, self.qk, 2 * self.qk, z, 0, 0, None, None, None, entry.state,
                      getattr(entry, "state_offset", 0), ctx.req_start, ctx.req_slot, o, ctx.n_requests, self.heads, self.heads,
-                     self.dim, self.vdim, q_scale=float(self.dim) ** -0.5, c0=1.0 / self.tau)
+                     self.dim, self.vdim, q_scale=float(self.dim) ** -0.5, c0=1.0 / self.tau, single=getattr(ctx, "all_single", False))
         gated = torch.empty((T, self.v), dtype=rt.act_dtype, device=x.device)
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, off_g, self.w_norm, self.eps, False, gated)
@@ -366,7 +366,7 @@ class MatrixMemoryMixer(_StateMixer):
         K.tag = "scan"
         K.state_scan(K.SCAN_MLSTM, proj, 0, self.qk, 2 * self.qk, proj, off_i, off_i + self.heads, self.b_f, self.b_i, None,
                      entry.state, getattr(entry, "state_offset", 0), ctx.req_start, ctx.req_slot, o, ctx.n_requests, self.heads,
-                     self.heads, self.dim, self.vdim, q_scale=float(self.dim) ** -0.5, c0=self.cap, c1=self.floor)
+                     self.heads, self.dim, self.vdim, q_scale=float(self.dim) ** -0.5, c0=self.cap, c1=self.floor, single=getattr(ctx, "all_single", False))
         gated = torch.empty((T, self.v), dtype=rt.act_dtype, device=x.device)
         K.tag = "gate + norm"
         K.gated_group_norm(o, self.vdim, proj, off_g, self.w_norm, self.eps, False, gated, sigmoid_gate=True)

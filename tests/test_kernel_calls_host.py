@@ -50,8 +50,18 @@ def test_decays_of_all_rows_only_where_all_rows_have_them(calls):
     scan(K.SCAN_GLA, 64, 40, 1)
     scan(K.SCAN_DELTA, 64, 64, 1)
     scan(K.SCAN_GLA, 64, 64, 9)                                               # (seven rows a request: too few to walk)
-    pointers = [args[-2] for name, args in calls.made if name == "cj_state_scan"]
+    pointers = [args[-3] for name, args in calls.made if name == "cj_state_scan"]
     assert pointers[0] and not any(pointers[1:])
+
+
+def test_a_few_requests_with_many_tokens_are_not_single_ones(calls):
+    """62 rows in a layout of 64 requests: 32 single tokens and one request of 30, say.  The caller knows; without it no more rows than requests
+    count as single tokens."""
+    scan(K.SCAN_SSD, 62, 62, 64, single=False)
+    scan(K.SCAN_SSD, 62, 62, 64, single=True)
+    scan(K.SCAN_SSD, 62, 62, 64)
+    scan(K.SCAN_SSD, 65, 65, 64)
+    assert [args[-2] for name, args in calls.made if name == "cj_state_scan"] == [0, 1, 1, 0]
 
 
 def counted(call, *args, **kw):
