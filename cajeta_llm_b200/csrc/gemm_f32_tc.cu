@@ -282,9 +282,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     __shared__ uint64_t raw_full[RING], raw_empty[RING], full_bar[STAGES], empty_bar[STAGES], x_full[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int odd_flag[FLAGS];                           // some row of the tile has an entry that is not the sum of three parts
+    __shared__ unsigned expired[threads(N) / 32];             // a warp's lanes whose waits ran out
     __shared__ int before[SPANS + 1];                         // token tiles of the groups before a span's first
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (lane == 0) expired[warp] = 0;
     if (tid == 0) {
         for (int s = 0; s < RING; ++s) {
             mbar_init(&raw_full[s], 1);
@@ -411,7 +413,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             uint32_t odd = 0;
             for (; it < end; it += G) {
                 const unsigned rs = it % RING, s = it % STAGES;
-                ok = mbar_wait_warp(&raw_full[rs], (it / RING) & 1, 16);
+                ok = mbar_wait_warp(&raw_full[rs], (it / RING) & 1, 16, expired);
                 if (!ok) break;
                 const uint8_t* wr = raw + rs * S::RAW;
                 const uint8_t* xr = wr + S::W_RAW;
@@ -426,7 +428,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 };
                 // a lone group reads while the stage is still in use (1,777 x 6,144: 396 -> 375 us); several cover each other's
                 if (G == 1) read();
-                ok = mbar_wait_warp(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 11);
+                ok = mbar_wait_warp(&empty_bar[s], ((it / STAGES) & 1) ^ 1, 11, expired);
                 if (!ok) break;
                 tcgen05_fence_after();
                 if (G > 1) read();
@@ -474,7 +476,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const uint32_t one = umma_idesc_bf16(128, wide), both = umma_idesc_bf16(128, 2 * wide);
             const uint32_t at = b_first + ((s * S::STAGE + u * 3 * UNIT * 64) >> 4), x_step = (READY ? UNIT : wide) * 64 >> 4;
             const uint32_t w = tmem + S::A_AT + s * 48, d1 = acc0 + wide;
-            if (!mbar_wait_warp(&acc_empty[mine], (times & 1) ^ 1, 14)) return false;
+            if (!mbar_wait_warp(&acc_empty[mine], (times & 1) ^ 1, 14, expired)) return false;
             tcgen05_fence_after();
             auto add = [&](int pw, int px) {                 // D1 += part pw of W . part px of X
 #pragma unroll
@@ -505,7 +507,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const int wide = live ? width(c.n_tok, u) : 16;
             for (; it < end; it += UNITS == 2 ? 1 : 2) {
                 const unsigned s = it % STAGES;
-                ok = mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, 12) && (!READY || mbar_wait_warp(&x_full[s], (it / STAGES) & 1, 18));
+                ok = mbar_wait_warp(&full_bar[s], (it / STAGES) & 1, 12, expired) && (!READY || mbar_wait_warp(&x_full[s], (it / STAGES) & 1, 18, expired));
                 if (!ok) break;
                 if (live) {
                     ok = issue(wide, u, s, times);
@@ -534,7 +536,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 for (int u = 0; u < UNITS; ++u) {
                     if (u * UNIT >= n_tok || !ok) break;
                     const int a = UNITS == 2 ? u : it & 1, wide = width(n_tok, u);
-                    ok = mbar_wait_warp(&acc_full[a], (UNITS == 2 ? times[u] : it >> 1) & 1, 13);
+                    ok = mbar_wait_warp(&acc_full[a], (UNITS == 2 ? times[u] : it >> 1) & 1, 13, expired);
                     if (!ok) break;
                     ++times[u];
                     tcgen05_fence_after();

@@ -41,17 +41,19 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {      // bar: an address in shared memory
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
+
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
 
 // Bounded wait: true when the phase completed, false (and the flag set) after the limit.
 __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int code) {
@@ -79,6 +81,46 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int code) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, code));
+}
+
+// The same where a vote in every wait costs too much (the float32 product's warps wait twice a block of K: 3 to 4 % of tiles of 64
+// and 128 tokens).  A lane whose limit has run out says so in `expired`, of which every warp has a word in shared memory, zero at first,
+// and goes on looking: it leaves when all 32 have said so, and takes its word back when the phase completes after all.  All bits set is
+// the end: nobody takes a word back then.  So either every lane leaves or none, and a lane waits no longer than the slowest of them.
+// (parity and code in one word: with an argument more the products of 64 and 128 tokens lost 2 %.)
+__device__ __noinline__ bool mbar_wait_slow_warp(uint32_t bar, uint32_t parity_code, unsigned* expired) {
+    const unsigned long long start = globaltimer_ns();
+    const uint32_t parity = parity_code & 1;
+    const unsigned mine = 1u << (threadIdx.x & 31);
+    expired += threadIdx.x >> 5;
+    bool late = false;
+#pragma unroll 1
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 256; ++i) {
+            if (!mbar_try_wait_at(bar, parity)) continue;
+            if (!late) return true;
+            unsigned said = *(volatile unsigned*)expired;
+            while (said != 0xffffffffu) {
+                const unsigned was = atomicCAS(expired, said, said & ~mine);
+                if (was == said) return true;
+                said = was;
+            }
+            return false;
+        }
+        if (late) {
+            if (*(volatile unsigned*)expired == 0xffffffffu) return false;
+        } else if (globaltimer_ns() - start > WAIT_LIMIT_NS) {
+            atomicCAS(&g_error_flag, 0, (int)(parity_code >> 1));
+            atomicOr(expired, mine);
+            late = true;
+        }
+    }
+}
+
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int code, unsigned* expired) {
+    if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_slow_warp(smem_u32(bar), parity | (uint32_t)code << 1, expired);
 }
 
 // TMA: one 2-D tile [box rows x box cols] into shared memory, completion counted in bytes
