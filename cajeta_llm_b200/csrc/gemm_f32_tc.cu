@@ -577,6 +577,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             }
 #pragma unroll
             for (int j = 0; j < COLS; ++j) again = again || (token(j) < n_tok && !chain_free(acc[j]));
+            again = again && fr < p.feat_tile;                // the other rows' sums are of whatever lay behind the tile's weights
             if (__any_sync(0xffffffffu, again && ok)) {
                 // (rarely: through an array in memory, so that the sums keep their registers)
                 float sums[COLS];

@@ -281,21 +281,23 @@ def f32_tc_takes(a: torch.Tensor, w: torch.Tensor, w_up: Optional[torch.Tensor],
 @functools.lru_cache(maxsize=4096)
 def f32_tc_tile(rows: int, features: int, groups: int, gated: bool, sms: int):
     """(tokens, features) of a tile of the float32 tensor-core product; a result's bits do not depend on them."""
+    # As many features as a tile takes.  Half as many make the blocks twice as many and none of them shorter (a block of K lasts what its chain of
+    # waits, splitting and products lasts; with the dead rows' splitting left out, too): us with 128 and 64, 8 rows x 2,048 x 2,048 38.7 and 38.7, 8 x
+    # 6,144 36.9 and 38.1, 60 x 6,144 41.0 and 71.3; gated, 64 and 32, 64 rows in 16 groups of 512 x 1,024 27.4 and 41.0, 500 rows 39.8 and 60.4
     most = 64 if gated else 128
     if groups:
         # tiles that most groups of an even split fill once (mean and two standard deviations), as their weights are read once a tile
         mean = rows / groups
         want = min(rows, mean + 2.0 * mean ** 0.5)
-        n_tok = next((n for n in F32_TC_TOKENS if want <= n), F32_TC_TOKENS[-1])
-        return n_tok, most if -(-features // most) * min(groups, rows) >= sms else most // 2
+        return next((n for n in F32_TC_TOKENS if want <= n), F32_TC_TOKENS[-1]), most
 
     # rounds of the machine times what a block of K takes in a tile of that many tokens (us, fitted to 8, 60, 264 and 1,777 rows x 2,048 or 6,144
-    # features x 2,048; the features of a tile change only the rounds): 264 x 6,144 69 us with 128 tokens and 90 with 64, 264 x 2,048 41 with
-    # 32, 52 with 64 and 65 with 128, 1,777 x 2,048 124 with 128 and 167 with 64
-    def cost(n, f):
-        return -(-(-(-rows // n) * -(-features // f)) // sms) * (0.31 + 0.0044 * min(n, -(-rows // 16) * 16))
+    # features x 2,048): 264 x 6,144 69 us with 128 tokens and 90 with 64, 264 x 2,048 41 with 32, 52 with 64 and 65 with 128, 1,777 x 2,048 124
+    # with 128 and 167 with 64
+    def cost(n):
+        return -(-(-(-rows // n) * -(-features // most)) // sms) * (0.31 + 0.0044 * min(n, -(-rows // 16) * 16))
 
-    return min(((n, f) for n in F32_TC_TOKENS for f in (most, most // 2)), key=lambda t: cost(*t))
+    return min(F32_TC_TOKENS, key=cost), most
 
 
 @functools.lru_cache(maxsize=4096)

@@ -96,3 +96,14 @@ def test_a_float32_product_refuses_scratch_that_is_too_small(n_tok, indexed):
 
     if need:
         assert call(one, need - 1) == -5 and call(ctypes.c_void_p(0), need) == -5
+
+
+@pytest.mark.parametrize("rows,features,groups,gated,tile", [
+    (1, 2048, 0, False, (16, 128)), (8, 6144, 0, False, (16, 128)), (60, 2048, 0, False, (16, 128)), (60, 6144, 0, False, (32, 128)),
+    (264, 2048, 0, False, (32, 128)), (264, 6144, 0, False, (128, 128)), (512, 2048, 0, False, (64, 128)), (1777, 2048, 0, False, (128, 128)),
+    (8, 5632, 0, True, (16, 64)), (60, 5632, 0, True, (64, 64)), (264, 5632, 0, True, (128, 64)),
+    (64, 512, 16, True, (16, 64)), (500, 512, 16, True, (64, 64)), (8, 1408, 8, True, (16, 64)), (16, 1024, 16, False, (16, 128)),
+    (1056, 1408, 60, True, (32, 64)), (7108, 1408, 60, True, (128, 64))])
+def test_tiles_of_float32_products(rows, features, groups, gated, tile):
+    """Tiles as measured; no tile is cut in half along its features: that makes rounds, not shorter blocks."""
+    assert K.f32_tc_tile(rows, features, groups, gated, 148) == tile
