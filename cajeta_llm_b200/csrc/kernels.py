@@ -507,11 +507,39 @@ def diff_attention_tc(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor,
     _check(st, "diff_attention_tc")
 
 
+def diff_tc_pays(rows: Sequence[int], priors: Sequence[int], heads: int, window: int, split_keys: int, sms: int) -> bool:
+    """Whether a step's differential attention is faster on tcgen05 (128 rows of a request and a head a block, one block an SM) than in tiles of
+    64 rows by mma.sync, whose keys go to several blocks in stretches of ``split_keys`` where the row blocks leave SMs idle (0: they do not).
+
+    What a form takes is the work of its blocks over the SMs, or its longest block, and a few us around them.  A block of 64 rows takes 5.2 us
+    and 3.6 a 64 keys, one of 128 rows 12.6 and 2.75 a 128 keys (fitted to 847 points: 2 to 32 heads of maps of 64 with values of 128, portions of
+    256 to 2,000 rows beside 0 to 60 single rows, 1 to 64 requests of 4 to 1,024 rows, 0 to 3,000 keys before them; where it takes the slower form
+    that is behind by 8 % at most but at three points, 16 to 19 %).  us, mma.sync and tcgen05, 16 heads: 256 rows behind
+    3,000 121 and 79, a portion of 256 beside 60 rows at 500 keys 210 and 163, at 2,000 730 and 382, at 50 72 and 114, 32 prompts of 8 tokens 34 and 58,
+    8 of 100 25 and 19; 256 rows behind 3,000 with 8 heads 70 and 78, with 2 37 and 76."""
+    def work(tile: int, start: float, step: float):
+        total = longest = 0.0
+        most = -(-window // tile) + 1 if window else 1 << 30          # a tile's steps of as many keys
+        for n, p in zip(rows, priors):
+            tiles = -(-n // tile)
+            if tiles:
+                last = min(-(-(p + n) // tile), most)
+                total += tiles * start + step * min((tiles - 1) * -(-p // tile) + tiles * (tiles - 1) // 2 + last, tiles * most)
+                longest = max(longest, start + step * last)
+        return total * heads / sms, longest
+
+    (mma, mma_block), (tc, tc_block) = work(64, 5.2, 3.6), work(128, 12.6, 2.75)
+    if split_keys:
+        return max(tc, tc_block) + 4.0 <= max(mma, min(mma_block, 5.2 + 3.6 * split_keys / 64)) + 18.0
+    return max(tc, tc_block) + 4.0 <= max(mma, mma_block) + 6.0
+
+
 def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor, positions: torch.Tensor,
                    row_req: torch.Tensor, table: torch.Tensor, page_tokens: int, n_heads: int, n_kv: int, head_dim: int,
                    value_dim: int, window: int, scale: float, lam: float, eps: float, out_scale: float,
                    req_start: Optional[torch.Tensor] = None, req_prior: Optional[torch.Tensor] = None, n_requests: int = 0,
-                   reach: int = 0, splits: Optional[int] = None, tile_rows: int = 64) -> None:
+                   reach: int = 0, splits: Optional[int] = None, tile_rows: int = 64, h_rows: Optional[Sequence[int]] = None,
+                   h_prior: Optional[Sequence[int]] = None) -> None:
     """Differential attention of every row over its request's cached keys [from, position]: a query head is
     [q1 | q2] (``head_dim`` entries each), a cached key [k1 | k2]; each map is a softmax attention of its own over the
     same values, ``o = a1 - lam a2``, then ``o / sqrt(mean(o^2) + eps) * out_scale`` over the head's ``value_dim`` entries.
@@ -521,7 +549,8 @@ def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_
     rows of a request and a head a block, the products on tensor cores.  ``reach``: a bound on the longest row's keys that
     the step's shape fixes; with few row blocks their keys are dealt to several blocks in stretches cut from it
     (``splits``: how many, instead of as many as fill the machine).  ``tile_rows``: 64, or 16 when no request of the step brings
-    more than 16 rows (single decoded tokens): blocks of two warps, three of them a SM."""
+    more than 16 rows (single decoded tokens): blocks of two warps, three of them a SM.  ``h_rows`` and ``h_prior``: the requests' rows
+    and the tokens before them, on the host; they only decide which of two forms is the faster one."""
     _need(q, "q"), _need(out, "out", q.dtype), _need(k_plane, "k_plane"), _need(v_plane, "v_plane", k_plane.dtype)
     _need(positions, "positions", torch.int32), _need(row_req, "row_req", torch.int32), _need(table, "table", torch.int32)
     T = q.shape[0]
@@ -534,22 +563,21 @@ def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_
         _need(req_start, "req_start", torch.int32), _need(req_prior, "req_prior", torch.int32)
         if tile_rows not in (16, 64):
             raise KernelError(f"diff_attention: tile_rows must be 16 or 64, found {tile_rows}")
-        # On tcgen05 from 256 rows on (16 heads, us, tile by mma.sync -> tcgen05): 256 rows behind 3,000 120 -> 80, 8 times 40 rows 29 -> 25,
-        # 4 times 200 33 -> 21; below, where keys are dealt to several blocks or a tile of 128 rows is mostly empty, not: 64 rows behind
-        # 3,000 58 -> 72, 8 times 30 rows 13 -> 18
-        if (splits is None and tile_rows == 64 and T >= 256 and head_dim >= 64 and page_tokens % 16 == 0 and scale > 0.0 and window >= 0
-                and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0):
-            diff_attention_tc(q, out, k_plane, v_plane, req_start, req_prior, n_requests, table, page_tokens, n_heads, n_kv, head_dim, value_dim,
-                              window, scale, lam, eps, out_scale)
-            return
         blocks = (-(-T // tile_rows) + n_requests) * n_heads
         fill = _sm_count() * (3 if tile_rows == 16 else 1)            # blocks that fill the machine
+        chosen = splits is None
         if splits is None:
             splits = min(32, -(-fill // blocks)) if blocks < fill else 1
         split_keys, partial = 0, None
         if splits > 1 and reach > 128:
             split_keys = max(128, -(-(-(-reach // splits)) // 64) * 64)
             splits = -(-reach // split_keys)
+        if (chosen and tile_rows == 64 and T >= 256 and head_dim >= 64 and page_tokens % 16 == 0 and scale > 0.0 and window >= 0
+                and (q.data_ptr() | out.data_ptr() | k_plane.data_ptr() | v_plane.data_ptr()) % 16 == 0
+                and (not h_rows or h_prior is None or diff_tc_pays(h_rows, h_prior, n_heads, window, split_keys, _sm_count()))):
+            diff_attention_tc(q, out, k_plane, v_plane, req_start, req_prior, n_requests, table, page_tokens, n_heads, n_kv, head_dim, value_dim,
+                              window, scale, lam, eps, out_scale)
+            return
         if splits > 1 and split_keys > 0:
             partial = torch.empty((splits, T, n_heads, 2, value_dim + 2), dtype=torch.float32, device=q.device)
         else:

@@ -163,11 +163,14 @@ class DifferentialAttention(Part):
         reach = 0
         if tiled:
             reach = ctx.max_context if getattr(ctx, "all_single", False) else entry.block_table.shape[1] * entry.page_tokens
+        # the rows and lengths the step has (a captured step keeps the form that was the faster one when it was captured)
+        start, h_prior = getattr(ctx, "h_req_start", ()), getattr(ctx, "h_req_prior", None)
+        h_rows = [b - a for a, b in zip(start, start[1:])] if T >= 256 else None
         K.diff_attention(q, out, entry.k_plane, entry.v_plane, ctx.positions, ctx.row_req, entry.block_table, entry.page_tokens,
                          self.heads, self.kv_heads, self.dim, self.vdim, self.window, self.scale, self.lam, self.eps,
                          1.0 - self.lambda_init, req_start=ctx.req_start if tiled else None,
                          req_prior=ctx.req_prior if tiled else None, n_requests=ctx.n_requests if tiled else 0, reach=reach,
-                         tile_rows=16 if getattr(ctx, "all_single", False) else 64)
+                         tile_rows=16 if getattr(ctx, "all_single", False) else 64, h_rows=h_rows, h_prior=h_prior)
         K.tag = "o"
         project(rt, out.view(T, self.o_dim), self.w_o, residual, accumulate=True)
         K.tag = None

@@ -76,6 +76,34 @@ def test_differential(H, G, hd, vd, page, window, requests):
     assert not K.wait_errors()
 
 
+@pytest.mark.parametrize("requests,tcgen05", [([(0, 128), (40, 127)], False), ([(0, 128), (40, 128)], True), ([(0, 8)] * 33, False), ([(300, 8)] * 33, True)])
+def test_the_forms_of_differential_attention_agree(monkeypatch, requests, tcgen05):
+    """What the entry takes on both sides of its lines, against the tiles of 64 rows."""
+    from cajeta_llm_b200.csrc import kernels as K
+    g, H, G, hd, vd, page = torch.Generator().manual_seed(5), 8, 4, 64, 128, 16
+    T, totals, taken = sum(r for _, r in requests), [p + r for p, r in requests], []
+    real = K.diff_attention_tc
+    monkeypatch.setattr(K, "diff_attention_tc", lambda *a: (taken.append(1), real(*a)))
+    need = [-(-t // page) for t in totals]
+    kp, vp = (torch.randn((sum(need), G, page, w), generator=g).bfloat16().to(DEV) for w in (2 * hd, vd))
+    table, at = torch.full((len(requests), max(need)), -1, dtype=torch.int32), 0
+    for i, n in enumerate(need):
+        table[i, :n] = torch.arange(at, at + n)
+        at += n
+    q, starts = torch.randn((T, H, 2 * hd), generator=g).bfloat16().to(DEV), [sum(r for _, r in requests[:i]) for i in range(len(requests) + 1)]
+    i32 = [torch.tensor(x, dtype=torch.int32, device=DEV) for x in (
+        [p + j for p, r in requests for j in range(r)], [i for i, (_, r) in enumerate(requests) for _ in range(r)], starts, [p for p, _ in requests])]
+    outs = []
+    for kw in (dict(h_rows=[r for _, r in requests], h_prior=[p for p, _ in requests]), dict(splits=1)):
+        out = torch.full((T, H, vd), NAN, dtype=torch.bfloat16, device=DEV)
+        K.diff_attention(q, out, kp, vp, i32[0], i32[1], table.to(DEV), page, H, G, hd, vd, 0, hd ** -0.5, 0.55, 1e-5, 0.4, i32[2], i32[3], len(requests),
+                         table.shape[1] * page, **kw)
+        outs.append(out.double())
+    assert bool(taken) == tcgen05
+    assert float((outs[0] - outs[1]).abs().max()) < 2 * 0.02 * max(1.0, float(outs[1].abs().max()))        # (each within 0.02 of the formula)
+    assert not K.wait_errors()
+
+
 @pytest.mark.parametrize("H,dim,rot,vdim,window,sink,gate,requests", [
     (2, 128, 64, 128, 0, True, "none", [(0, 256), (0, 257), (0, 1), (65, 127)]),
     (2, 128, 64, 128, 0, False, "head", [(100, 300), (0, 640)]),

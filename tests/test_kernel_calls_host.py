@@ -107,3 +107,35 @@ def test_a_float32_product_refuses_scratch_that_is_too_small(n_tok, indexed):
 def test_tiles_of_float32_products(rows, features, groups, gated, tile):
     """Tiles as measured; no tile is cut in half along its features: that makes rounds, not shorter blocks."""
     assert K.f32_tc_tile(rows, features, groups, gated, 148) == tile
+
+
+@pytest.mark.parametrize("heads,requests,split_keys,tcgen05", [
+    # (tokens before, rows) of the requests; what the tiles of 64 rows cut the keys into; which form was the faster one
+    (16, [(3000, 256)], 2048, True), (8, [(3000, 256)], 1024, False), (2, [(3000, 256)], 320, False), (8, [(1000, 256)], 1024, True),
+    (4, [(2000, 512)], 832, False), (4, [(3000, 512)], 832, False), (8, [(3000, 1024)], 0, True), (16, [(0, 256)], 2048, True),
+    (16, [(0, 8)] * 32, 0, False), (16, [(0, 32)] * 8, 0, False), (16, [(0, 100)] * 8, 0, True), (16, [(500, 8)] * 32, 0, True),
+    (16, [(0, 256)] + [(500, 1)] * 60, 0, True), (16, [(0, 256)] + [(2000, 1)] * 16, 0, True), (16, [(0, 256)] + [(50, 1)] * 60, 0, False),
+    (16, [(0, 1000)] + [(50, 1)] * 30, 0, True), (32, [(100, 16)] * 16, 0, False), (16, [(0, 256), (7, 0), (0, 0)], 2048, True)])
+def test_which_form_differential_attention_takes(heads, requests, split_keys, tcgen05):
+    assert K.diff_tc_pays([r for _, r in requests], [p for p, _ in requests], heads, 0, split_keys, 148) == tcgen05
+
+
+def test_a_window_bounds_what_a_tile_reads():
+    """Far behind its window a portion costs what its window costs."""
+    near, far = ([K.diff_tc_pays([256] * n, [p] * n, h, 512, 0, 148) for n in (1, 4, 16) for h in (2, 8, 32)] for p in (512, 100000))
+    assert near == far
+
+
+def test_differential_attention_asks_from_256_rows_on(calls, monkeypatch):
+    asked = []
+    monkeypatch.setattr(K, "diff_tc_pays", lambda *a: asked.append(a) or False)
+    for rows, given in (([255], True), ([256], True), ([200, 56], True), ([256], False)):
+        T, H = sum(rows), 16
+        start = torch.tensor([0] + list(torch.tensor(rows).cumsum(0)), dtype=torch.int32)
+        q, out = torch.zeros(T, H, 128, dtype=torch.bfloat16), torch.zeros(T, H, 128, dtype=torch.bfloat16)
+        k, v = torch.zeros(40, 8, 16, 128, dtype=torch.bfloat16), torch.zeros(40, 8, 16, 128, dtype=torch.bfloat16)
+        z = torch.zeros(T, dtype=torch.int32)
+        K.diff_attention(q, out, k, v, z, z, torch.zeros(len(rows), 4, dtype=torch.int32), 16, H, 8, 64, 128, 0, 0.125, 0.5, 1e-6, 0.5, start,
+                         torch.zeros(len(rows), dtype=torch.int32), len(rows), 64, h_rows=rows if given else None, h_prior=[0] * len(rows) if given else None)
+    assert [a[0] for a in asked] == [[256], [200, 56]]
+    assert [name for name, _ in calls.made] == ["cj_diff_attention_tile"] * 3 + ["cj_diff_attention_tc"]
