@@ -276,16 +276,18 @@ __global__ void __launch_bounds__(4 * ROWS, 2) attention_f32_tile_kernel(const A
     }
 }
 
-// floats of a warp's half chunk of keys or values in the kernel below
-__host__ __device__ constexpr int half_floats(int hd, int vd) { return 32 * (hd + 4 > vd ? hd + 4 : vd); }
+// floats of a piece of a warp's chunk of keys or values in the kernel below
+__host__ __device__ constexpr int piece_floats(int piece, int hd, int vd) { return piece * (hd + 4 > vd ? hd + 4 : vd); }
 
 // A row and head a block: a warp a chunk of 64 keys, lane = keys lane and lane + 32 for the scores and four entries of the value for
-// the sums; after every round of chunks thread d joins them, in order, into entry d of the output.  A chunk's two halves of keys are
-// sent for together and its values as soon as the keys have been read, a warp a key (512 bytes side by side), so that a chunk is two
-// round trips to memory; with a lane reading its own key's row, eight pieces at a time, it was twelve, in lines of 128 bytes for 16.
-// HALVES 1: one half at a time, for room.  Bound by the round trips with few blocks, by what an SM draws from memory with many.
-template <int ROW_WARPS, int HALVES>
+// the sums; after every round of chunks thread d joins them, in order, into entry d of the output.  A chunk comes in pieces of PIECE keys, a warp
+// a key (512 bytes side by side).  BUFS 2: its two halves of keys are sent for together and its values as soon as the keys have been read, so
+// that a chunk is two round trips to memory; with a lane reading its own key's row, eight pieces at a time, it was twelve, in lines of 128 bytes
+// for 16.  BUFS 1: one piece at a time, for room (a lane holds keys lane and lane + 32 whatever the piece).  Bound by the round trips with few blocks, by what an SM draws from memory with many.
+template <int ROW_WARPS, int PIECE, int BUFS>
 __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const Args p) {
+    constexpr int PIECES = (KEYS + PIECE - 1) / PIECE;
+    static_assert(PIECE <= 32 && (BUFS == 1 || PIECES == BUFS), "a lane has a key of a piece; all pieces of a chunk in buffers of their own, or one at a time");
     cj::after_predecessor();
     cj::release_successor();
     extern __shared__ __align__(16) float smem[];
@@ -330,8 +332,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
     if (tid < p.hd / 4) *(float4*)(qs + 4 * tid) = *(const float4*)(p.q + ((size_t)row * p.n_heads + head) * p.hd + 4 * tid);
     __syncthreads();
     float* bufs[2];
-    bufs[0] = smem + warp * HALVES * half_floats(p.hd, p.vd);
-    bufs[1] = bufs[0] + (HALVES - 1) * half_floats(p.hd, p.vd);
+    bufs[0] = smem + warp * BUFS * piece_floats(PIECE, p.hd, p.vd);
+    bufs[1] = bufs[0] + (BUFS - 1) * piece_floats(PIECE, p.hd, p.vd);
     const int ks = p.hd + 4;
     float m = p.sink, l = p.sink == -INFINITY ? 0.0f : 1.0f, acc = 0.0f;
     for (int k0 = from & ~(KEYS - 1); k0 <= pos; k0 += KEYS * ROW_WARPS) {
@@ -347,32 +349,45 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
                 base[j] = 0;
                 if (seen[j]) base[j] = ((size_t)tab[key / p.page_tokens] * p.n_kv + kvh) * p.page_tokens + key % p.page_tokens;
             }
-            auto fetch = [&](int h, const float* plane, int size, int stride) {
-                __syncwarp();                       // what the half held has been read
-                const unsigned there = __ballot_sync(0xffffffffu, seen[h]);
+            // whether key k of the chunk, in the piece that begins at `first`, is one of its second half
+            auto half = [](int first, int k) { return (PIECE == 32 ? first : k) >= 32; };
+            unsigned there[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) there[j] = __ballot_sync(0xffffffffu, seen[j]);
+            // the chunk's keys or values [first, first + PIECE) into buffer h
+            auto fetch = [&](int h, int first, const float* plane, int size, int stride) {
+                __syncwarp();                       // what the buffer held has been read
 #pragma unroll 4
-                for (int j = 0; j < 32; ++j) {
-                    const size_t b = __shfl_sync(0xffffffffu, (unsigned long long)base[h], j);
-                    if (4 * lane < size && (there >> j & 1)) cp_async16(bufs[h] + j * stride + 4 * lane, plane + b * size + 4 * lane, true);
+                for (int j = 0; j < PIECE; ++j) {
+                    const int k = first + j;
+                    if (PIECE * PIECES > KEYS && k >= KEYS) break;
+                    const size_t b = __shfl_sync(0xffffffffu, (unsigned long long)(half(first, k) ? base[1] : base[0]), k & 31);
+                    if (4 * lane < size && ((half(first, k) ? there[1] : there[0]) >> (k & 31) & 1))
+                        cp_async16(bufs[h] + j * stride + 4 * lane, plane + b * size + 4 * lane, true);
                 }
                 cp_async_commit();
             };
-            fetch(0, p.kplane, p.hd, ks);
-            if (HALVES == 2) fetch(1, p.kplane, p.hd, ks);
+            fetch(0, 0, p.kplane, p.hd, ks);
+            if (BUFS == 2) fetch(1, PIECE, p.kplane, p.hd, ks);
+            s[0] = s[1] = -INFINITY;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                cp_async_wait<HALVES - 1>();
+            for (int i = 0; i < PIECES; ++i) {
+                const int h = BUFS == 2 ? i : 0;
+                cp_async_wait<BUFS - 1>();
                 __syncwarp();
-                float dot = 0.0f;
-                if (seen[h]) {
-                    const float* kr = bufs[h] + lane * ks;
+                const int row = (lane - i * PIECE) & 31, k = i * PIECE + row;          // this lane's key of the piece
+                const bool second = half(i * PIECE, k);
+                if (row < PIECE && k < KEYS && (second ? seen[1] : seen[0])) {
+                    float dot = 0.0f;
+                    const float* kr = bufs[h] + row * ks;
 #pragma unroll 8
                     for (int d = 0; d < p.hd; d += 4) dot = chain4(*(const float4*)(qs + d), *(const float4*)(kr + d), dot);
+                    dot = score(dot, p);
+                    if (second) s[1] = dot; else s[0] = dot;
                 }
-                s[h] = seen[h] ? score(dot, p) : -INFINITY;
-                if (HALVES == 2) fetch(h, p.vplane, p.vd, p.vd);
-                else if (h == 0) fetch(1, p.kplane, p.hd, ks);
-                else fetch(0, p.vplane, p.vd, p.vd);
+                if (BUFS == 2) fetch(h, i * PIECE, p.vplane, p.vd, p.vd);
+                else if (i + 1 < PIECES) fetch(0, (i + 1) * PIECE, p.kplane, p.hd, ks);
+                else fetch(0, 0, p.vplane, p.vd, p.vd);
             }
             const float mc = warp_max(fmaxf(s[0], s[1]));
             e[0] = seen[0] ? weight(s[0], mc) : 0.0f;
@@ -386,16 +401,17 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
             float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             const bool mine = 4 * lane < p.vd;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (HALVES == 1 && h == 1) fetch(1, p.vplane, p.vd, p.vd);
-                if (HALVES == 2 && h == 0) cp_async_wait<1>(); else cp_async_wait<0>();
+            for (int i = 0; i < PIECES; ++i) {
+                const int h = BUFS == 2 ? i : 0;
+                if (BUFS == 1 && i > 0) fetch(0, i * PIECE, p.vplane, p.vd, p.vd);
+                if (BUFS == 2 && i == 0) cp_async_wait<1>(); else cp_async_wait<0>();
                 __syncwarp();
-                const int lo = max(from - c0 - 32 * h, 0), hi = min(pos - c0 - 32 * h, 31);
+                const int lo = max(from - c0, i * PIECE), hi = min(pos - c0, min(KEYS, (i + 1) * PIECE) - 1);
 #pragma unroll 4
-                for (int j = lo; j <= hi; ++j) {
-                    const float w = __shfl_sync(0xffffffffu, e[h], j);
+                for (int k = lo; k <= hi; ++k) {
+                    const float w = __shfl_sync(0xffffffffu, half(i * PIECE, k) ? e[1] : e[0], k & 31);
                     if (mine) {
-                        const float4 v = *(const float4*)(bufs[h] + j * p.vd + 4 * lane);
+                        const float4 v = *(const float4*)(bufs[h] + (k - i * PIECE) * p.vd + 4 * lane);
                         o.x = fmaf(w, v.x, o.x);
                         o.y = fmaf(w, v.y, o.y);
                         o.z = fmaf(w, v.z, o.z);
@@ -419,15 +435,19 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) attention_f32_row_kernel(const
         p.out[((size_t)row * p.n_heads + head) * p.vd + tid] = __fmul_rn(acc, __fmul_rn(1.0f / l, gate_of(p, row, head)));
 }
 
-int multiprocessors(int& n) {
-    static int sms = 0;
+// multiprocessors, and the shared memory of one
+int machine(int& n, int& bytes) {
+    static int sms = 0, sm_bytes = 0;
     if (!sms) {
-        int dev = 0;
+        int dev = 0, count = 0;
         cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return (int)e;
+        sms = count;
     }
     n = sms;
+    bytes = sm_bytes;
     return 0;
 }
 
@@ -451,15 +471,8 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
         // Tiles of 64 rows where an SM holds two of them and the step has two for every SM, else of 32.  What an SM holds is what hides the
         // waits for keys: with heads of 128 a tile of 64 rows takes 115 KB and is alone (before keys travelled ahead: 1,777 rows of 16 heads 728 us,
         // with tiles of 32 713; 768 rows 187 and 172; 256 rows at 950 keys 185 and 137), with heads of 96 two fit (1,777 rows at 2,277 keys 925, 987).
-        int sms = 0;
-        if (int st = multiprocessors(sms)) return st;
-        static int sm_bytes = 0;
-        if (!sm_bytes) {
-            int dev = 0;
-            cudaError_t e = cudaGetDevice(&dev);
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-            if (e != cudaSuccess) return (int)e;
-        }
+        int sms, sm_bytes;
+        if (int st = machine(sms, sm_bytes)) return st;
         auto smem = [](int rows, int h, int v) { return (int)sizeof(float) * ((rows + KEYS) * (h + 4) + KEYS * v + rows * (KEYS + 4)); };
         const bool two = 2 * (smem(64, hd, vd) + 1024) <= sm_bytes;
         const int rows = two && (long long)tiles * n_heads >= 2 * sms ? 64 : 32, wide = vd <= 64 ? 0 : 1;
@@ -477,25 +490,33 @@ CJ_EXPORT int cj_attention_f32(const float* q, float* out, const float* kplane, 
     if (tiles <= 0) a.req_start = nullptr;                     // no tile: every row by itself, whatever its request has
     if (singles > 0 || tiles <= 0) {
         const int rows = a.req_start ? singles : T;
-#define ROWS(W, HALVES)                                                                                                 \
+#define ROWS(W, PIECE, BUFS)                                                                                            \
     do {                                                                                                                \
         static bool row_sized = false;                                                                                  \
         if (!row_sized) {                                                                                               \
-            cudaError_t e = cudaFuncSetAttribute(attention_f32_row_kernel<W, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                 HALVES * W * half_floats(MAX_DIM, MAX_DIM) * (int)sizeof(float));      \
+            cudaError_t e = cudaFuncSetAttribute(attention_f32_row_kernel<W, PIECE, BUFS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                 BUFS * W * piece_floats(PIECE, MAX_DIM, MAX_DIM) * (int)sizeof(float)); \
             if (e != cudaSuccess) return (int)e;                                                                        \
             row_sized = true;                                                                                           \
         }                                                                                                               \
-        cj::launch(attention_f32_row_kernel<W, HALVES>, dim3(rows, n_heads), dim3(W * 32),                              \
-                   HALVES * W * half_floats(hd, vd) * (int)sizeof(float), stream, a);                                   \
+        cj::launch(attention_f32_row_kernel<W, PIECE, BUFS>, dim3(rows, n_heads), dim3(W * 32),                         \
+                   BUFS * W * piece_floats(PIECE, hd, vd) * (int)sizeof(float), stream, a);                             \
     } while (0)
-        // With a block an SM at most, six warps whose chunks' halves travel together (8 rows at 520 keys, 16 heads: 36 us, 63 with the kernel
-        // before); with more, three smaller blocks an SM, one summing while another waits (64 rows at 1,000 keys: 303 us with the large blocks,
-        // 241 with these, 283 before; 64 rows at 512 keys 195, 133 and 154).
-        int sms = 0;
-        if (int st = multiprocessors(sms)) return st;
-        if ((long long)rows * n_heads <= sms) ROWS(6, 2);
-        else ROWS(4, 1);
+        // With a block an SM at most, six warps whose chunks travel whole (8 rows at 520 keys, 16 heads: 36 us, 63 with the kernel
+        // before); with more, smaller blocks, one summing while another waits.  Those take a piece of 32, 24 or 16 keys at a time, so that an SM
+        // holds three, four or six of them (heads of 128): the size with the fewest rounds, of those with as few the largest.  us with pieces of 32, 24
+        // and 16, 16 heads, rows at 500 keys: 384 blocks 47, 51 and 53, 512 (32 decoding requests) 90, 73 and 72, 640 84, 86 and 63, 1,024 129,
+        // 117 and 136, 2,048 186, 180 and 161 (with the kernel before 60, 77, 78, 145 and 199).
+        int sms, sm_bytes;
+        if (int st = machine(sms, sm_bytes)) return st;
+        auto rounds = [&](int piece) {                         // (3.6 KB: what a block holds besides, and what an SM keeps for itself a block)
+            const int held = min(16, sm_bytes / ((int)sizeof(float) * 4 * piece_floats(piece, hd, vd) + 3686));
+            return ((long long)rows * n_heads + (long long)sms * held - 1) / ((long long)sms * held);
+        };
+        if ((long long)rows * n_heads <= sms) ROWS(6, 32, 2);
+        else if (rounds(32) <= min(rounds(24), rounds(16))) ROWS(4, 32, 1);
+        else if (rounds(24) <= rounds(16)) ROWS(4, 24, 1);
+        else ROWS(4, 16, 1);
 #undef ROWS
     }
     return launch_status();

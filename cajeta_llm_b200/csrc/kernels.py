@@ -440,8 +440,10 @@ def _gate(head_gate: Optional[torch.Tensor], gate_offset: int):
 NO_SINK = float("-inf")      # no key without a value joins the softmax
 
 
-# float32 attention: a request with at most this many rows in the step goes a row a block, one with more 64 or 32 rows a block.  Eight
-# rows at 512 keys in each of eight requests take 133 us a row a block (cold); as a tile of 64 they would pay for 56 that are not there.
+# float32 attention: a request with at most this many rows in the step goes a row a block, one with more 64 or 32 rows a block.  Rows at 500 keys,
+# cold, us a row a block and in tiles of 32: 8 rows of one request 31 and 73, of eight requests 53 and 74 with 8 heads, 99 and 76 with 16; 4 rows of
+# eight 41 and 74, 55 and 75; 16 of one 46 and 81, of eight (16 heads) 212 and 83.  What decides is how many blocks the step's few rows make; a line on
+# a request's rows alone is drawn where most steps are on the right side of it.
 F32_FEW_ROWS = 8
 
 

@@ -124,3 +124,27 @@ def test_keys_whose_scores_are_minus_infinity_have_no_weight(tiled):
         s = s.masked_fill(torch.arange(336, device=DEV)[None] > pos[:4, None], -math.inf)
         assert bool(torch.isinf(s[:, :64]).all())
         assert torch.allclose(out[:4, h].double(), torch.softmax(s, 1) @ values[h], atol=2e-5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("rows,heads,hd,vd", [(37, 4, 128, 128), (70, 4, 128, 96), (130, 4, 100, 128), (180, 4, 128, 128), (300, 4, 64, 64), (260, 8, 64, 128)])
+@pytest.mark.parametrize("window", [0, 41])
+def test_rows_in_pieces_of_any_size(monkeypatch, rows, heads, hd, vd, window):
+    """One row a request, as many blocks as go with chunks whole and in pieces of 32, 24 and 16 keys; keys that end at pieces' and chunks' edges."""
+    from cajeta_llm_b200.csrc import kernels as K
+    g, page = torch.Generator().manual_seed(13), 16
+    ends = [(0, 1, 15, 16, 17, 23, 24, 25, 31, 32, 47, 48, 49, 63, 64, 65, 87, 88, 111, 112, 130, 191, 192, 300, 450)[i % 25] for i in range(rows)]
+    pages = [e // page + 1 for e in ends]
+    kp, vp = (torch.randn(sum(pages), heads, page, d, generator=g).to(DEV) for d in (hd, vd))
+    table, at = torch.full((rows, max(pages)), -1, dtype=torch.int32), 0
+    for r, n in enumerate(pages):
+        table[r, :n] = torch.arange(at, at + n)
+        at += n
+    q, pos, req = torch.randn(rows, heads, hd, generator=g).to(DEV), torch.tensor(ends).int().to(DEV), torch.arange(rows).int().to(DEV)
+    starts, outs = list(range(rows + 1)), []
+    for few in (K.F32_FEW_ROWS, 0):
+        monkeypatch.setattr(K, "F32_FEW_ROWS", few)
+        out = torch.full((rows, heads, vd), math.nan, device=DEV)
+        K.paged_attention(q, out, kp, vp, pos, req, table.to(DEV), page, heads, heads, hd, window, hd ** -0.5, value_dim=vd,
+                          req_start=torch.tensor(starts, dtype=torch.int32, device=DEV), h_req_start=starts)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
