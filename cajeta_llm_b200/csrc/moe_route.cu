@@ -443,6 +443,17 @@ __global__ void __launch_bounds__(GROUP_WARPS * 32) moe_group_kernel(
 
 }  // namespace
 
+// Experts of a block of the logits' kernel: they are spread over blocks (8 to 32 a block) as far as `room` goes, two blocks for every SM or
+// the one that an SM holds, and all in one where the row blocks by themselves are many; every block reads its rows again.  us with 8, 16, 32 a block
+// and all: 60 experts of 2,048, 99 rows 30, 38, 52 and 79; 264 rows 36, 42, 55 and 83; 512 rows 54, 42, 56 and 82; 1,777 rows 130, 95, 83 and 83;
+// 256 experts of 2,048, with 32 and all, 512 rows 105 and 257, 1,000 rows 156 and 265; 16 of 4,096 (a block an SM), with 8 and 16, 1,000 rows 83 and 71.
+CJ_EXPORT int cj_router_experts_a_block(int row_blocks, int n_cols, int room) {
+    auto fits = [&](int n) { return (long long)row_blocks * ((n_cols + n - 1) / n) <= room; };
+    int n = 8;
+    while (n < 32 && n < n_cols && !fits(n)) n *= 2;
+    return n == 32 && row_blocks >= 128 && !fits(n) ? n_cols : n;
+}
+
 // logits: scratch [T, E + 1] float32 (column E holds the shared gate's dot when a gate is given).
 // tickets: int32 [4], zero before the first use (the kernel leaves them zero); may be null, the two-launch form is then used.
 // pin: int32 [T, k] experts given instead of chosen, or null.  gap: float32 [T] routing margins out, or null.
@@ -468,18 +479,18 @@ CJ_EXPORT int cj_router_topk(const float* x, const float* Wr, const float* share
     if ((size_t)tokb * H * sizeof(float) > 200 * 1024) return CJ_ERR_SIZE;
     size_t smem = (size_t)tokb * H * sizeof(float);
     int row_blocks = (T + tokb - 1) / tokb;
-    // the experts spread over blocks (8 to 32 a block) as far as the machine holds them in two rounds; every block reads its rows again
-    // (60 experts of 2,048, us with 8, 16, 32 a block and all: 99 rows 30, 38, 52 and 79; 264 rows 36, 42, 55 and 83; 512 rows 54, 42, 56 and
-    // 82; 1,777 rows 130, 95, 83 and 83)
-    static int sms = 0;
+    static int sms = 0, sm_bytes = 0;
     if (!sms) {
-        int dev = 0;
+        int dev = 0, n = 0;
         cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return (int)e;
+        sms = n;
     }
-    int per_block = 8;
-    while (per_block < n_cols && (long long)row_blocks * ((n_cols + per_block - 1) / per_block) > 2 * sms) per_block = per_block < 32 ? 2 * per_block : n_cols;
+    // (few rows and hundreds of experts: as many as an SM holds; 33 rows of 1,024, 512 experts, 38 us with 8 a block and 42 with 16)
+    const int held = max(1, (int)((size_t)sm_bytes / (smem + 1024)));
+    const int per_block = cj_router_experts_a_block(row_blocks, n_cols, sms * (row_blocks <= 8 ? held : min(held, 2)));
     dim3 grid(row_blocks, (n_cols + per_block - 1) / per_block);
 #define LAUNCH(TB)                                                                                                   \
     {                                                                                                                \

@@ -139,3 +139,17 @@ def test_differential_attention_asks_from_256_rows_on(calls, monkeypatch):
                          torch.zeros(len(rows), dtype=torch.int32), len(rows), 64, h_rows=rows if given else None, h_prior=[0] * len(rows) if given else None)
     assert [a[0] for a in asked] == [[256], [200, 56]]
     assert [name for name, _ in calls.made] == ["cj_diff_attention_tile"] * 3 + ["cj_diff_attention_tc"]
+
+
+@pytest.mark.parametrize("rows,columns,a_block", [(40, 61, 8), (99, 61, 8), (264, 61, 8), (512, 61, 16), (1000, 61, 32), (1777, 61, 61), (33, 257, 8), (264, 257, 32),
+                                                  (512, 257, 32), (1000, 257, 32), (1000, 129, 32), (1777, 257, 257), (4000, 17, 17), (600, 3, 8), (5000, 3, 8)])
+def test_experts_of_a_router_block(rows, columns, a_block):
+    """Many experts are spread over blocks until the row blocks by themselves fill the machine."""
+    lib = ctypes.CDLL(K._build.build("moe_route"))
+    assert lib.cj_router_experts_a_block(-(-rows // 8), columns, 2 * 148) == a_block
+
+
+@pytest.mark.parametrize("rows,columns,a_block", [(700, 16, 16), (1000, 16, 16), (512, 61, 32), (264, 129, 32), (99, 61, 8), (2000, 61, 61)])
+def test_experts_of_a_router_block_that_has_an_sm_to_itself(rows, columns, a_block):
+    lib = ctypes.CDLL(K._build.build("moe_route"))
+    assert lib.cj_router_experts_a_block(-(-rows // 8), columns, 148) == a_block
