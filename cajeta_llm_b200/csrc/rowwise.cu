@@ -25,8 +25,8 @@ __global__ void embed_gather_kernel(float* __restrict__ out, const TW* __restric
     for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] = ok ? to_f32(src[i]) * f : 0.0f;
 }
 
-// The same for tables of bfloat16 whose rows are whole pieces of 16 bytes: a thread takes eight entries at a time.  2,048 rows of 2,048,
-// cold: 13.8 us with the kernel above (two bytes a load), 8.8 so.
+// The same for tables of bfloat16 whose rows are whole pieces of 16 bytes, 32 of them or more: a thread takes eight entries at a time.  2,048 rows of
+// 2,048, cold: 13.8 us with the kernel above (two bytes a load), 8.8 so; 1,500 rows of 128 6.6 and 7.3.
 __global__ void embed_gather8_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ table, const int* __restrict__ ids, int H, int V, float scale) {
     cj::after_predecessor();
     cj::release_successor();
@@ -56,7 +56,7 @@ CJ_EXPORT int cj_embed_gather(float* out, const void* table, int table_dtype, co
     int threads = H >= 1024 ? 256 : 128;
     if (table_dtype == CJ_F32)
         cj::launch(embed_gather_kernel<float>, dim3(T), dim3(threads), 0, stream, out, (const float*)table, ids, H, V, scale);
-    else if (table_dtype == CJ_BF16 && H % 8 == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
+    else if (table_dtype == CJ_BF16 && H % 8 == 0 && H >= 256 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
         cj::launch(embed_gather8_kernel, dim3(T), dim3(min(256, max(32, (H / 8 + 31) / 32 * 32))), 0, stream, out, (const __nv_bfloat16*)table, ids, H, V, scale);
     else if (table_dtype == CJ_BF16)
         cj::launch(embed_gather_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, stream, out, (const __nv_bfloat16*)table, ids, H, V, scale);

@@ -189,3 +189,15 @@ def test_two_normed_rows_mixed_and_cast(rows, H, accumulate):
         cast = torch.empty(rows, H, device=DEV, dtype=dtype)
         K.cast_rows(out, cast)
         assert torch.equal(cast, out.to(dtype))
+
+
+@pytest.mark.parametrize("H", [248, 256, 508, 512, 516])
+def test_rows_on_both_sides_of_the_widths_that_go_in_pieces(H):
+    from cajeta_llm_b200.csrc import kernels as K
+    a, b, wa, wb, out = rnd(3, H, seed=51), rnd(3, H, seed=52), rnd(H, seed=53), rnd(H, seed=54), torch.empty(3, H, device=DEV)
+    K.rmsnorm_mix2(a, wa, b, wb, 1e-6, 0.5, out)
+    x, y = (t.double() / torch.sqrt((t.double() ** 2).mean(-1, keepdim=True) + 1e-6) * w.double() for t, w in ((a, wa), (b, wb)))
+    assert torch.allclose(out.double(), 0.5 * (x + y), atol=1e-5, rtol=1e-5)
+    table, ids = rnd(7, H, seed=55).bfloat16(), torch.tensor([6, 0, -1], dtype=torch.int32, device=DEV)
+    K.embed_gather(out, table, ids, 0.0)
+    assert torch.equal(out, torch.cat([table[[6, 0]].float(), torch.zeros(1, H, device=DEV)]))
