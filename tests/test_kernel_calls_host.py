@@ -153,3 +153,35 @@ def test_experts_of_a_router_block(rows, columns, a_block):
 def test_experts_of_a_router_block_that_has_an_sm_to_itself(rows, columns, a_block):
     lib = ctypes.CDLL(K._build.build("moe_route"))
     assert lib.cj_router_experts_a_block(-(-rows // 8), columns, 148) == a_block
+
+
+def test_products_and_scans_run_without_room_for_scratch(calls, monkeypatch):
+    """Where the memory for split rows or for decays is not there, the forms that need none (or the gathered rows alone) run."""
+    real, limit = torch.empty, [0]
+
+    def empty(*size, **kw):
+        n = 1
+        for d in size[0]:
+            n *= d
+        if n * (4 if kw.get("dtype") == torch.float32 else 1) > limit[0]:
+            raise torch.OutOfMemoryError("no room")
+        return real(*size, **kw)
+
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+    monkeypatch.setattr(torch, "empty", empty)
+    x, w, out = torch.zeros(300, 256), torch.zeros(3, 128, 256), torch.zeros(300, 128)
+    offsets, index = torch.tensor([0, 100, 200, 300], dtype=torch.int32), torch.arange(300, dtype=torch.int32)
+    monkeypatch.setattr(K, "f32_tc_tile", lambda *a: (128, 64))
+    K.gemm(x, w[0], out)
+    K.gemm(x, w, out, group_offsets=offsets)
+    with pytest.raises(torch.OutOfMemoryError):
+        K.gemm(x, w, out, group_offsets=offsets, a_row_index=index)
+    limit[0] = 300 * 256 * 4
+    K.gemm(x, w, out, group_offsets=offsets, a_row_index=index)
+    limit[0] = 300 * (256 * 6 + 4)
+    K.gemm(x, w, out, group_offsets=offsets, a_row_index=index)
+    products = [args for name, args in calls.made if name == "cj_gemm_f32_tc"]
+    assert [args[-3] for args in products] == [32, 32, 32, 128] and [bool(args[4]) for args in products] == [False, False, True, True]
+    limit[0] = 0
+    scan(K.SCAN_GLA, 64, 64, 1)
+    assert not calls.made[-1][1][-3]
