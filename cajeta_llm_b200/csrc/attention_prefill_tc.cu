@@ -62,80 +62,6 @@ constexpr uint32_t TM_S = 0, TM_O = 256, TM_COLS = 512;
 constexpr uint32_t IDESC_QK = umma_idesc_bf16(128, 128);
 constexpr uint32_t IDESC_PV = umma_idesc_bf16(128, 128) | (1u << 16);
 
-// MN-major operand, 128-byte swizzle: 64 contiguous dims (128 bytes) per key row, 8 key rows
-// per 1024-byte group (stride byte offset), the next 64 dims one half tile further (leading
-// byte offset).
-__device__ __forceinline__ uint64_t umma_desc_mn_sw128(const void* smem_tile) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(smem_tile) & 0x3FFFF) >> 4);
-    d |= (uint64_t)(HALF_BYTES >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
-}
-// 32 consecutive 32-bit columns of this thread's lane from v[OFF .. OFF + 31]
-template <int OFF, int N>
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[N]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(v[OFF + 0]), "r"(v[OFF + 1]), "r"(v[OFF + 2]), "r"(v[OFF + 3]), "r"(v[OFF + 4]), "r"(v[OFF + 5]),
-          "r"(v[OFF + 6]), "r"(v[OFF + 7]), "r"(v[OFF + 8]), "r"(v[OFF + 9]), "r"(v[OFF + 10]), "r"(v[OFF + 11]),
-          "r"(v[OFF + 12]), "r"(v[OFF + 13]), "r"(v[OFF + 14]), "r"(v[OFF + 15]), "r"(v[OFF + 16]), "r"(v[OFF + 17]),
-          "r"(v[OFF + 18]), "r"(v[OFF + 19]), "r"(v[OFF + 20]), "r"(v[OFF + 21]), "r"(v[OFF + 22]), "r"(v[OFF + 23]),
-          "r"(v[OFF + 24]), "r"(v[OFF + 25]), "r"(v[OFF + 26]), "r"(v[OFF + 27]), "r"(v[OFF + 28]), "r"(v[OFF + 29]),
-          "r"(v[OFF + 30]), "r"(v[OFF + 31])
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]: A's rows are the lanes, two bf16 of consecutive k per column
-__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// two float32 operations in one instruction (sm_100 f32x2), and the maximum of three
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
 // cap log2(e) tanh(x) - sub for a raw score s with x = s scale / cap; a masked score (-inf) stays -inf.
 // The softmax pass is bound by the special-function unit and by instruction issue, so the hyperbolic
 // tangent is the unit's own (tanh.approx.f32, relative error 2^-11: a capped score is off by at most that
@@ -159,18 +85,6 @@ inline float cap_reach(int terms) { return terms == 3 ? 0.21f : terms == 4 ? 0.4
 constexpr double CAP_P[3][CAP_TERMS] = {{0.9999998594, -0.3332758288, 0.1298347298, 0, 0},
                                         {0.9999999019, -0.3333136246, 0.1327097676, -0.04755360348, 0},
                                         {0.9999998931, -0.3333195425, 0.1330452599, -0.05182186644, 0.01505094485}};
-
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-__device__ __forceinline__ float ex2(float x) {       // 2^x, 0 for -inf
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 __device__ __forceinline__ float capped_score_exp(float s, float in_cap, float cap_log2) {
     const float e = ex2(s * in_cap * 2.8853900817779268f);                   // e^2x
@@ -399,7 +313,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const bool next = i + 1 < n_tiles;
                 ok = mbar_wait(&v_full[s], (i / KV_STAGES) & 1, 19);
                 if (!ok) break;
-                const uint64_t dv = umma_desc_mn_sw128(smem + SMEM_V + s * TILE_BYTES);
+                const uint64_t dv = umma_desc_mn_sw128(smem + SMEM_V + s * TILE_BYTES, HALF_BYTES);
                 bool k_there = false;
 #pragma unroll
                 for (int g = 0; g < QT; ++g) {

@@ -98,29 +98,6 @@ template <int N, bool DUAL> struct Smem {
     static_assert(COLS_USED <= 512, "tensor memory of an SM");
 };
 
-// two float32 operations in one instruction
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 both_of(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // eight float32 -> their three bfloat16 parts, packed; some bit of `odd` is set when one of the eight is not the sum of its parts: infinite,
 // no number, so large that its first part rounds to infinity, or so small that its last part falls below the smallest bfloat16
 __device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& hi, uint4& mid, uint4& lo, uint32_t& odd) {
@@ -134,10 +111,10 @@ __device__ __forceinline__ void split8(const float4 f0, const float4 f1, uint4& 
     for (int i = 0; i < 4; ++i) {
         const float a = f[2 * i], b = f[2 * i + 1];
         h[i] = pack(a, b);
-        const f32x2 r = sub2(pair(a, b), pair(__uint_as_float(h[i] << 16), __uint_as_float(h[i] & 0xffff0000u)));
-        const float2 rs = both_of(r);
+        const f32x2 r = sub2(pack2(a, b), pack2(__uint_as_float(h[i] << 16), __uint_as_float(h[i] & 0xffff0000u)));
+        const float2 rs = unpack2(r);
         m[i] = pack(rs.x, rs.y);
-        const float2 ls = both_of(sub2(r, pair(__uint_as_float(m[i] << 16), __uint_as_float(m[i] & 0xffff0000u))));
+        const float2 ls = unpack2(sub2(r, pack2(__uint_as_float(m[i] << 16), __uint_as_float(m[i] & 0xffff0000u))));
         l[i] = __byte_perm(__float_as_uint(ls.x), __float_as_uint(ls.y), 0x7632);        // (a remainder has eight bits at most)
         odd |= __float_as_uint(ls.x) | __float_as_uint(ls.y);
     }
@@ -188,8 +165,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // whether `ok` holds in all of the block's THREADS threads that come here, after all of them have
 template <int THREADS>
 __device__ __forceinline__ bool all_of(bool ok) {
@@ -530,7 +505,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const int n_tok = c.n_tok, tok0 = c.tok0;
             f32x2 acc2[COLS / 2];
 #pragma unroll
-            for (int j = 0; j < COLS / 2; ++j) acc2[j] = pair(0.0f, 0.0f);
+            for (int j = 0; j < COLS / 2; ++j) acc2[j] = pack2(0.0f, 0.0f);
             for (unsigned kb = 0; kb < n_kb && ok; ++kb, ++it) {
 #pragma unroll
                 for (int u = 0; u < UNITS; ++u) {
@@ -551,14 +526,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) {
                         f32x2& s = acc2[(u * UCOLS + j) / 2];
-                        s = add2(add2(s, pair(__uint_as_float(v[j]), __uint_as_float(v[j + 1]))), pair(__uint_as_float(h[j]), __uint_as_float(h[j + 1])));
+                        s = add2(add2(s, pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]))), pack2(__uint_as_float(h[j]), __uint_as_float(h[j + 1])));
                     }
                 }
             }
             float acc[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; j += 2) {
-                const float2 d = both_of(acc2[j / 2]);
+                const float2 d = unpack2(acc2[j / 2]);
                 acc[j] = d.x;
                 acc[j + 1] = d.y;
             }
