@@ -29,12 +29,14 @@
 // 44 + n / 2 with W in shared memory (measured alone, back to back).  X goes to shared memory in its parts, split by the same warps or, for
 // tiles of 64 tokens and more, once for all tiles by split_rows_kernel.  Two warps issue the products, every other one each, since one's round
 // of waits, products and commits lasted longer than the products themselves; the last warps add the accumulators up, two sums an instruction,
-// and store.  Blocks stay, one an SM, and every role runs across tile boundaries.  What bounds it: issue slots with few tokens (of 0.37 us a
-// block of 32 of K with 16 tokens splitting takes 0.13, the loads alone 0.2), the products and the adding up with many (0.84 us with 128
-// tokens, 0.5 of them the products).  Rows x features x K, us, cold weights; gemm_simt.cu, then W's parts in shared memory with one
-// issuing warp, then a tile a block, then now: 8 x 2,048 x 2,048 190, 39, 34 and 36; 264 x 6,144 x 2,048 327, 111, 75 and 69; 1,777 x 6,144 x 2,048
-// 1,817, 366, 314 and 280; 60 groups of 1,408 gated features, 17 tokens each 380, 340 and 316, 118 each 750, 650 and 625.
-// Built and taken out: two blocks an SM with few tokens (60 groups of 17 tokens 333 us instead of 343, one of 24 groups the same).  (With the
+// and store.  Blocks stay, one an SM, and every role runs across tile boundaries.  What bounds it: with few tokens the chain that a
+// block of 32 of K goes through, 0.37 us with 16 tokens (splitting 0.13, the loads alone 0.2) whether 16 or 32 blocks share the features, the products
+// and the adding up with many (0.84 us with 128 tokens, 0.5 of them the products).  Rows x features x K, us, cold weights; gemm_simt.cu, then W's parts
+// in shared memory with one issuing warp, then a tile a block, then now: 8 x 2,048 x 2,048 190, 39, 34 and 37; 264 x 6,144 x 2,048 327, 111, 75 and 70;
+// 1,777 x 6,144 x 2,048 1,817, 366, 314 and 284; the last three of 60 groups of 1,408 gated features, 17 tokens each 380, 340 and 304, 118 each
+// 750, 650 and 610.
+// Built and taken out: two blocks an SM with few tokens (60 groups of 17 tokens 333 us instead of 343, one of 24 groups the same); splitting warps
+// that leave rows past a tile's features out (tiles of 64 features took what tiles of 128 take, 264 x 2,048 x 2,048 45 us instead of 41).  (With the
 // float32 operands loaded into registers instead of by TMA 1,777 x 6,144 took 815: one load's latency a block lay bare.  Three loading
 // threads instead of one changed nothing.)
 // Grouped form as in gemm_simt.cu, with the rows of X already in the groups' order.
