@@ -515,6 +515,21 @@ def diff_attention_tc(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor,
     _check(st, "diff_attention_tc")
 
 
+def _attention_work(rows: Sequence[int], priors: Sequence[int], tile: int, keys: int, window: int, start: float, step: float):
+    """What the row blocks of a step's requests take for one head, all of them and the longest: a block has ``tile`` rows of a request and takes
+    ``start`` and a ``step`` for every ``keys`` keys that its rows see."""
+    total = longest = 0.0
+    more = tile // keys                                               # steps from one block of a request to the next
+    most = -(-window // keys) + more if window else 1 << 30
+    for n, p in zip(rows, priors):
+        blocks = -(-n // tile)
+        if blocks:
+            last = min(-(-(p + n) // keys), most)
+            total += blocks * start + step * min((blocks - 1) * -(-p // keys) + more * (blocks * (blocks - 1) // 2) + last, blocks * most)
+            longest = max(longest, start + step * last)
+    return total, longest
+
+
 def diff_tc_pays(rows: Sequence[int], priors: Sequence[int], heads: int, window: int, split_keys: int, sms: int) -> bool:
     """Whether a step's differential attention is faster on tcgen05 (128 rows of a request and a head a block, one block an SM) than in tiles of
     64 rows by mma.sync, whose keys go to several blocks in stretches of ``split_keys`` where the row blocks leave SMs idle (0: they do not).
@@ -522,24 +537,15 @@ def diff_tc_pays(rows: Sequence[int], priors: Sequence[int], heads: int, window:
     What a form takes is the work of its blocks over the SMs, or its longest block, and a few us around them.  A block of 64 rows takes 5.2 us
     and 3.6 a 64 keys, one of 128 rows 12.6 and 2.75 a 128 keys (fitted to 847 points: 2 to 32 heads of maps of 64 with values of 128, portions of
     256 to 2,000 rows beside 0 to 60 single rows, 1 to 64 requests of 4 to 1,024 rows, 0 to 3,000 keys before them; where it takes the slower form
-    that is behind by 8 % at most but at three points, 16 to 19 %).  us, mma.sync and tcgen05, 16 heads: 256 rows behind
+    that is behind by 8 % at most but at three points, 16 to 19 %; of 300 more with maps and values of 64 and 128 and windows of 512, one was the
+    slower form's, by 6 %).  us, mma.sync and tcgen05, 16 heads: 256 rows behind
     3,000 121 and 79, a portion of 256 beside 60 rows at 500 keys 210 and 163, at 2,000 730 and 382, at 50 72 and 114, 32 prompts of 8 tokens 34 and 58,
     8 of 100 25 and 19; 256 rows behind 3,000 with 8 heads 70 and 78, with 2 37 and 76."""
-    def work(tile: int, start: float, step: float):
-        total = longest = 0.0
-        most = -(-window // tile) + 1 if window else 1 << 30          # a tile's steps of as many keys
-        for n, p in zip(rows, priors):
-            tiles = -(-n // tile)
-            if tiles:
-                last = min(-(-(p + n) // tile), most)
-                total += tiles * start + step * min((tiles - 1) * -(-p // tile) + tiles * (tiles - 1) // 2 + last, tiles * most)
-                longest = max(longest, start + step * last)
-        return total * heads / sms, longest
-
-    (mma, mma_block), (tc, tc_block) = work(64, 5.2, 3.6), work(128, 12.6, 2.75)
+    mma, mma_block = _attention_work(rows, priors, 64, 64, window, 5.2, 3.6)
+    tc, tc_block = _attention_work(rows, priors, 128, 128, window, 12.6, 2.75)
     if split_keys:
-        return max(tc, tc_block) + 4.0 <= max(mma, min(mma_block, 5.2 + 3.6 * split_keys / 64)) + 18.0
-    return max(tc, tc_block) + 4.0 <= max(mma, mma_block) + 6.0
+        return max(tc * heads / sms, tc_block) + 4.0 <= max(mma * heads / sms, min(mma_block, 5.2 + 3.6 * split_keys / 64)) + 18.0
+    return max(tc * heads / sms, tc_block) + 4.0 <= max(mma * heads / sms, mma_block) + 6.0
 
 
 def diff_attention(q: torch.Tensor, out: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor, positions: torch.Tensor,
