@@ -1331,6 +1331,23 @@ def latent_tc_shape(dim: int, rot: int, vdim: int, scale: float) -> bool:
     return dim in (64, 128) and 0 < rot <= 64 and vdim in (64, 128) and scale > 0.0
 
 
+def latent_tc_pays(rows: Sequence[int], priors: Sequence[int], heads: int, dim: int, vdim: int, window: int, sms: int) -> bool:
+    """Whether a step's latent attention in its plain form is faster on tcgen05 (256 or 128 rows of a request and a head a block, one block an SM)
+    than with every head's keys and values copied side by side and tiles of 64 rows by mma.sync (:func:`latent_kv_pack`, :func:`latent_flash`).
+
+    As in :func:`diff_tc_pays`; the copies cost with the tokens, which a step of many short requests has few of.  Fitted to 1,836 points (4 to 32
+    heads of 64 and 128, windows and none, 1 to 64 requests of 4 to 2,000 rows, 0 to 3,000 tokens before them): tcgen05 is the slower form at 72 of them, up
+    to 2.3 times; 20 choices of this rule are the slower form's, by 3 to 21 %.  us, with copies and tcgen05, heads of 128, gather and packing of queries
+    included: 16 heads, 64 requests of 4 rows 63 and 112, 32 prompts of 8 tokens 47 and 54, a portion of 256 beside 60 rows at 500 keys 524 and 169, 256 rows
+    alone 49 and 22."""
+    total = sum(rows)
+    most = (-(-total // 256) + len(rows) - 1) * heads
+    tokens = sum(n + (min(p, window - 1) if window else p) for n, p in zip(rows, priors))
+    copied, copied_block = _attention_work(rows, priors, 64, 64, window, 3.3, 2.0)
+    tc, tc_block = _attention_work(rows, priors, 128 if 2 * most <= sms else 256, 128, window, 18.2, 3.0)
+    return max(tc * heads / sms, tc_block) + 14.0 <= max(copied * heads / sms, copied_block) + 36.0 + 6.8e-6 * tokens * heads * (dim + 64 + vdim)
+
+
 def latent_attention_tc(qx: torch.Tensor, out: torch.Tensor, kp: torch.Tensor, kr: torch.Tensor, vp: torch.Tensor, req_start: torch.Tensor,
                         req_prior: torch.Tensor, req_base: torch.Tensor, requests: int, heads: int, dim: int, vdim: int, scale: float,
                         sink: Optional[torch.Tensor] = None, window: int = 0, exact_weights: bool = False,

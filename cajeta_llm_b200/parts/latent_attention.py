@@ -265,8 +265,15 @@ class LatentAttention(Part):
         req_base, tok_req, tok_pos, N = layout
         plane = entry.k_plane
         c_all = torch.empty((N, self.rank), dtype=torch.bfloat16, device=dev)
-        # On tcgen05 the attention reads keys and values where the products below leave them, and a gate a head rides on its way out
+        # On tcgen05 the attention reads keys and values where the products below leave them, and a gate a head rides on its way out.  (The rows
+        # and lengths are the step's; a captured step keeps the form that was the faster one when it was captured.)
         fast = K.latent_tc_shape(self.dim, self.rot, self.vdim, self.scale)
+        if fast:
+            known, key = ctx.__dict__.setdefault("_latent_tc", {}), (H, self.dim, self.vdim, self.window)
+            if key not in known:
+                rows = [b - a for a, b in zip(ctx.h_req_start, ctx.h_req_start[1:])]
+                known[key] = K.latent_tc_pays(rows, ctx.h_req_prior, H, self.dim, self.vdim, self.window, K._sm_count())
+            fast = known[key]
         kr = torch.empty((N, 64), dtype=torch.bfloat16, device=dev) if fast else None
         K.tag = "latent gather"
         K.latent_gather(plane, self.rank, tok_req, tok_pos, entry.block_table, entry.page_tokens, c_all, kr)

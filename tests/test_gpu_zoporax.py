@@ -343,6 +343,35 @@ def test_window_edges_page_borders_and_far_keys(folders, name):
             r.release(s)
 
 
+@pytest.mark.parametrize("window", [None, 100])
+def test_both_plain_forms_of_latent_attention(folders, monkeypatch, window):
+    """Heads that tcgen05 takes, in the form that copies keys and values and in the one that does not, whichever the step's sizes would choose:
+    a whole prompt, portions beside cached tokens, and many short prompts in one step."""
+    from cajeta_llm_b200.csrc import kernels as K
+    from cajeta_llm_b200.engine.step import StepEntry
+    from cajeta_llm_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(LatentAttention, "EXPAND_MIN_ROWS", 8)
+    d, (cfg, W) = folders(f"heads64_{window}", config_of([latent(heads=2, dim=64, rot_dim=24, vdim=64, kv_rank=64, q_rank=32, scale=0.1, window=window)], width=64), seed=11)
+    toks = helpers.random_tokens(90, 300, seed=6)
+    want = torch.from_numpy(P.forward(cfg, W, toks))
+    short = [helpers.random_tokens(90, n, seed=60 + n) for n in (9, 30, 14, 21)]
+    wants = [torch.from_numpy(P.forward(cfg, W, t)) for t in short]
+    real, taken = K.latent_attention_tc, []
+    monkeypatch.setattr(K, "latent_attention_tc", lambda *a, **kw: (taken.append(1), real(*a, **kw)))
+    for pays in (False, True):
+        taken.clear()
+        monkeypatch.setattr(K, "latent_tc_pays", lambda *a: pays)
+        r = runner_for(d, "bfloat16", max_tokens=320)
+        for cuts in ([300], [40, 130, 9, 121]):
+            s = r.admit()
+            check(feed(r, s, toks, cuts), want, "bfloat16", f"window {window} tcgen05 {pays} cuts {cuts}")
+            r.release(s)
+        slots = [r.admit() for _ in short]
+        out = r.step([StepEntry(s, t, list(range(len(t)))) for s, t in zip(slots, short)]).cpu()
+        check(out, torch.cat(wants), "bfloat16", f"window {window} tcgen05 {pays} short prompts")
+        assert bool(taken) == pays
+
+
 def test_a_windowed_request_gives_pages_back(folders):
     """A pool that holds a window and little more: a request much longer than the pool runs through it."""
     d, (cfg, W) = folders("far_window", config_of(FAR["window"], width=32, vocab=2000), seed=9, touch=sharp)

@@ -185,3 +185,13 @@ def test_products_and_scans_run_without_room_for_scratch(calls, monkeypatch):
     limit[0] = 0
     scan(K.SCAN_GLA, 64, 64, 1)
     assert not calls.made[-1][1][-3]
+
+
+@pytest.mark.parametrize("heads,dim,vdim,window,requests,tcgen05", [
+    # (tokens before, rows) of the requests; which form was the faster one
+    (16, 128, 128, 0, [(0, 4)] * 64, False), (32, 64, 64, 0, [(0, 4)] * 64, False), (16, 128, 128, 0, [(0, 8)] * 32, False), (32, 128, 128, 512, [(0, 8)] * 32, False),
+    (16, 128, 128, 0, [(0, 16)] * 16, True), (16, 128, 128, 0, [(0, 256)], True), (16, 128, 128, 0, [(0, 2000)], True), (8, 128, 128, 0, [(3000, 256)], True),
+    (16, 128, 128, 0, [(0, 256)] + [(500, 1)] * 60, True), (16, 128, 128, 0, [(0, 256)] + [(20, 1)] * 60, False), (16, 128, 128, 0, [(500, 8)] * 32, True),
+    (16, 64, 64, 0, [(200, 4)] * 64, True), (4, 128, 128, 0, [(0, 100)] * 8, True), (16, 128, 128, 0, [(0, 300), (9, 0)], True)])
+def test_which_form_latent_attention_takes(heads, dim, vdim, window, requests, tcgen05):
+    assert K.latent_tc_pays([r for _, r in requests], [p for p, _ in requests], heads, dim, vdim, window, 148) == tcgen05
